@@ -157,6 +157,7 @@ namespace
 		// Default: 2 points per thread for the culled export, 4 for the dense one (measured).
 		o.Lanes = (lanes == 1 || lanes == 2 || lanes == 4) ? lanes : (o.Dense ? 4 : 2);
 		o.Staged = (flags & TG_MESH_STAGED) != 0;
+		o.Tapes = (flags & TG_MESH_TAPES) != 0;
 		return o;
 	}
 

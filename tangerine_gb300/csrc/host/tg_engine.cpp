@@ -145,6 +145,7 @@ namespace tg
 			p.View.MaxStack = p.Host.Header.MaxStack;
 			p.View.FullSurfaceCode = p.Host.Header.FullSurfaceCode;
 			p.View.Lipschitz = p.Host.Header.Lipschitz;
+			p.View.Form = p.Host.Header.Form;
 		}
 	}
 
@@ -327,6 +328,36 @@ namespace tg
 		return cudaSuccess;
 	}
 
+	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
+	// A tape saves about what its cell's program has beyond a dozen quads (two brushes), on
+	// every pass over the brick, and costs one pass of the whole program and two launches: it
+	// pays from a number of bricks that falls as the programs get longer.  Measured on a
+	// GB300, export to the device, tapes against whole programs, in us: 64 primitives (23
+	// quads a cell) 384^3 356 / 333, 512^3 414 / 417, 700^3 596 / 660; 16 primitives (16
+	// quads) 512^3 256 / 241, 700^3 346 / 356; 256 primitives (54 quads) 256^3 695 / 735,
+	// 512^3 861 / 1062, and 128^3 721 / 653.
+	static bool TapesPay(const Program& p, int64_t bricks)
+	{
+		const double quads = (double)p.Host.DistanceQuadsTotal / std::max(1, p.Host.Header.NodeCount);
+		return (double)bricks * (quads - 12.0) >= 3.5e6;
+	}
+
+	cudaError_t Engine::ReserveTapes(int64_t bricks, BrickTapes& out)
+	{
+		out.PartCapacity = (uint32_t)std::min<size_t>(BrickPartCapacity(bricks), 0x7FFFFFFFu);
+		out.EventCapacity = (uint32_t)std::min<size_t>(BrickEventCapacity(bricks), 0x7FFFFFFFu);
+		TG_TRY(TapeBricks.Reserve((size_t)bricks * sizeof(uint2)));
+		TG_TRY(TapeParts.Reserve((size_t)out.PartCapacity * sizeof(BrickPart)));
+		TG_TRY(TapeEvents.Reserve((size_t)out.EventCapacity * sizeof(uint2)));
+		TG_TRY(TapeCounters.Reserve((kBrickTapeCounters + kLongParts) * sizeof(uint32_t)));
+		out.Bricks = TapeBricks.As<uint2>();
+		out.Parts = TapeParts.As<BrickPart>();
+		out.Events = TapeEvents.As<uint2>();
+		out.Counters = TapeCounters.As<uint32_t>();
+		out.Long = out.Counters + kBrickTapeCounters;
+		return cudaSuccess;
+	}
+
 	cudaError_t Engine::Export(const Program& p, const GridSpec& g, const ExportOptions& opt, DeviceMesh& out, cudaStream_t s)
 	{
 		// Bits PreClassify left for this export (any other export voids them).
@@ -363,6 +394,7 @@ namespace tg
 		TG_TRY(Counts.Reserve(8 * sizeof(uint32_t)));
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4));
 
+		BrickTapes tapes{};
 		if (opt.Dense)
 		{
 			Bricks = ActiveBricks = 0;
@@ -427,13 +459,26 @@ namespace tg
 			TG_TRY(ActiveCells.Reserve((size_t)(nb * (int64_t)B * B * B < cells ? nb * (int64_t)B * B * B : cells) * 4));
 			int* evalStatus = reinterpret_cast<int*>(Counts.As<uint32_t>() + 4);      // status and work counter
 			TG_TRY(cudaMemsetAsync(evalStatus, 0, 2 * sizeof(int), s));
-			if (B == 7 && !opt.Staged)
+			if (B == 7 && !opt.Staged && !(opt.Tapes || TapesPay(p, nb)))
 			{
 				// The cell pass runs inside the brick evaluation, on each brick's values in
 				// shared memory.
 				Begin("eval_bricks", s);
 				TG_TRY(LaunchEvalBricksCells(p.View, g, BrickList.As<uint32_t>(), brickCount, tops, LatticeBuf.As<float>(),
 					Words.As<uint32_t>(), ActiveCells.As<uint32_t>(), Counts.As<uint32_t>() + 3, SmCount, s, opt.Lanes, evalStatus));
+				End(s);
+			}
+			else if (B == 7 && !opt.Staged)
+			{
+				// Each brick's shortened programs, then the evaluation by them with the cell pass
+				// folded in, on each brick's values in shared memory.
+				TG_TRY(ReserveTapes(nb, tapes));
+				Begin("brick_tapes", s);
+				TG_TRY(LaunchBrickTapes(p.View, g, B, BrickList.As<uint32_t>(), brickCount, tops, tapes, SmCount, s));
+				End(s);
+				Begin("eval_bricks", s);
+				TG_TRY(LaunchEvalBrickTapes(p.View, g, B, BrickList.As<uint32_t>(), brickCount, tapes, LatticeBuf.As<float>(),
+					Words.As<uint32_t>(), ActiveCells.As<uint32_t>(), Counts.As<uint32_t>() + 3, SmCount, s));
 				End(s);
 			}
 			else
@@ -569,7 +614,12 @@ namespace tg
 			if (!opt.Dense) order = { ActiveCells.As<uint32_t>(), Words.As<uint32_t>(), WordBase.As<uint32_t>() };
 			if (restaged.Event) TG_TRY(cudaStreamWaitEvent(s, restaged.Event, 0));
 			Begin("attributes", s);
-			TG_TRY(LaunchVertexAttributes(p.View, Vertices.As<float>(), vcount, Normals.As<float>(), colors, s, order));
+			// The tapes' lists name surface records by the order of the distance program's.
+			if (tapes.Bricks && (p.View.Form & kFormPlain))
+				TG_TRY(LaunchBrickAttributes(p.View, g, opt.BrickSize, tapes, order.Cells, order.Words, order.Base, Vertices.As<float>(),
+					vcount, Normals.As<float>(), colors, s));
+			else
+				TG_TRY(LaunchVertexAttributes(p.View, Vertices.As<float>(), vcount, Normals.As<float>(), colors, s, order));
 			End(s);
 			out.Normals = Normals.As<float>();
 			out.Colors = colors;

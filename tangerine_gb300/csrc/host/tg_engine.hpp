@@ -72,6 +72,7 @@ namespace tg
 		int BrickSize = 7;          // cells per brick edge when culling (1..32)
 		int Lanes = 2;              // lattice points per thread sharing one pass over records
 		bool Staged = false;        // brick evaluation reads single-cell bricks' programs from shared memory
+		bool Tapes = false;         // 7^3-cell bricks by tapes (LaunchBrickTapes) on any grid
 		const FieldNet* Field = nullptr;    // learned bound for the brick test (else exact)
 		bool Refine = true;                 // with Field: network-kept bricks also take the exact test
 		// The exact brick test already ran on the root cell's program (Engine::PreClassify,
@@ -198,10 +199,13 @@ namespace tg
 
 		cudaStream_t Stream = nullptr;
 		cudaStream_t CopyStream = nullptr;          // early device-to-host copies of an export
+		// The buffers of a grid's brick tapes (LaunchBrickTapes), kept between exports.
+		cudaError_t ReserveTapes(int64_t bricks, BrickTapes& out);
 		cudaEvent_t MeshReady = nullptr;
 		cudaEvent_t CodeReady = nullptr;            // RestageCode's copy of an export is done
 		DeviceBuffer LatticeBuf, Words, WordBase, Scratch, Counts, Vertices, Cubes, FaceCounts, FaceBase, Faces, Normals, Colors;
 		DeviceBuffer Points, PointOut, BrickBits, BrickList, BrickTops, ClassCounts, ProgramScratch, ActiveCells;
+		DeviceBuffer TapeBricks, TapeParts, TapeEvents, TapeCounters;    // ReserveTapes
 		DeviceBuffer RayIn, RayOut, Cameras, Image, RenderCounters;
 		DeviceBuffer SodaBoxes, SodaCache, SodaColors;
 		void* Staging = nullptr;

@@ -76,6 +76,11 @@ namespace tg
 		int32_t MaxStack;
 		int32_t FullSurfaceCode;    // quad offset of the whole tree's surface program
 		int32_t Lipschitz;          // 1 when every brush is 1-Lipschitz (no ellipsoid)
-		int32_t Reserved;
+		int32_t Form;               // kForm* below
 	};
+
+	// What the shortened programs (kernels/tg_tape.cuh) may assume of the whole tree.
+	constexpr int32_t kFormPrunable = 1;     // every rotation within 1e-3 of a unit quaternion, finite scales
+	constexpr int32_t kFormPlain = 2;        // no stencils: a surface program's records follow the distance program's
+	constexpr int32_t kFormPainted = 4;      // plain, and every brush has a material
 }

@@ -839,6 +839,26 @@ namespace tg
 		return true;
 	}
 
+	// kForm* bits of the tree (tg_layout.hpp).
+	static int32_t FormOf(const Node& n)
+	{
+		switch (n.Kind)
+		{
+		case NodeKind::Brush:
+		{
+			const Quat& q = n.Xf.Rotation;
+			const double norm = (double)q.w * q.w + (double)q.x * q.x + (double)q.y * q.y + (double)q.z * q.z;
+			const bool unit = norm > 1.0 - 2e-3 && norm < 1.0 + 2e-3;
+			const bool scaled = std::isfinite(n.Xf.Scalation) && n.Xf.Scalation != 0.0f;
+			return (unit && scaled ? kFormPrunable : 0) | kFormPlain | (n.Mat ? kFormPainted : 0);
+		}
+		case NodeKind::Set: return FormOf(*n.Lhs) & FormOf(*n.Rhs);
+		case NodeKind::Flate: return FormOf(*n.Lhs);
+		case NodeKind::Stencil: return FormOf(*n.Lhs) & kFormPrunable;
+		}
+		return 0;
+	}
+
 	std::vector<uint32_t> CompileReferenceWords(const Node& tree)
 	{
 		std::vector<uint32_t> w;
@@ -1127,6 +1147,7 @@ namespace tg
 		if (programs[evaluators].Stack > maxStack) maxStack = programs[evaluators].Stack;
 		out.Header.FullSurfaceCode = full;
 		out.Header.Lipschitz = HasNonLipschitzBrush(*root) ? 0 : 1;
+		out.Header.Form = FormOf(*root);
 		if (maxStack > kMaxStack)
 		{
 			error = "tree needs a deeper evaluation stack than the kernels hold";

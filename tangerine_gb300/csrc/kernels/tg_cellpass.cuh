@@ -1,0 +1,141 @@
+// The cell pass of one brick (surface nets' active cells) and the brick geometry it shares
+// with the brick evaluation.
+#pragma once
+
+#include "tg_device.cuh"
+#include "tg_kernels.hpp"
+#include "tg_surface.cuh"
+
+namespace tg
+{
+	struct BrickGrid
+	{
+		int B;                  // cells per brick edge
+		int NBX, NBY, NBZ;      // bricks per axis
+	};
+
+	// The cells of listed bricks, a CTA per brick with a grid stride over the list.
+	// Cells of unlisted bricks hold no surface and are never visited: the active-cell
+	// bitmask starts zeroed and only listed cells can set their bit.
+	struct BrickCells
+	{
+		int64_t i0, j0, k0;
+		int nx, ny, nz;
+	};
+
+	__device__ __forceinline__ BrickCells CellsOf(uint32_t b, const BrickGrid& bg, const CellGeom& cg)
+	{
+		const int bx = (int)(b % (uint32_t)bg.NBX), by = (int)((b / (uint32_t)bg.NBX) % (uint32_t)bg.NBY);
+		const int bz = (int)(b / ((uint32_t)bg.NBX * (uint32_t)bg.NBY));
+		BrickCells bc;
+		bc.i0 = (int64_t)bx * bg.B; bc.j0 = (int64_t)by * bg.B; bc.k0 = (int64_t)bz * bg.B;
+		bc.nx = (int)min((int64_t)bg.B, cg.sx - bc.i0);
+		bc.ny = (int)min((int64_t)bg.B, cg.sy - bc.j0);
+		bc.nz = (int)min((int64_t)bg.B, cg.sz - bc.k0);
+		return bc;
+	}
+
+	constexpr int kTiledBox = 8;
+	constexpr int kTiledThreads = 128;
+	constexpr int kTiledRounds = 3;   // 7^3 = 343 cells <= 3 x 128
+
+	// BT: the brick edge in cells when known at compile time (the cell coordinates then
+	// come from constant divisions, edge bricks masking their missing cells), or 0.
+	// The cell pass of one kept brick from its corner box in shared memory (kTiledBox^3,
+	// x fastest): every cell with corners of both signs sets its bit in `words` and is
+	// appended to `cells` (one atomic per brick).  Called by the whole CTA (it
+	// synchronises); `warpBase` is shared scratch, one word per warp.
+	template<int BT>
+	__device__ __forceinline__ void BrickCellFlags(const float* box, const BrickCells& bc, const CellGeom& cg, uint32_t* __restrict__ words,
+		uint32_t* __restrict__ cells, uint32_t* __restrict__ cell_count, uint32_t* warpBase)
+	{
+		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+		const int ex = BT ? BT : bc.nx, ey = BT ? BT : bc.ny;
+		const int total = BT ? BT * BT * BT : bc.nx * bc.ny * bc.nz;
+		const int64_t sxy = cg.sx * cg.sy;
+		const int64_t c0 = bc.i0 + bc.j0 * cg.sx + bc.k0 * sxy;
+		unsigned ballots[kTiledRounds];
+		uint32_t cellOf[kTiledRounds];
+		uint32_t mine = 0;
+#pragma unroll
+		for (int r = 0; r < kTiledRounds; ++r)
+		{
+			const int t = r * kTiledThreads + (int)threadIdx.x;
+			bool active = false;
+			cellOf[r] = 0;
+			const int x = t % ex, y = (t / ex) % ey, z = t / (ex * ey);
+			if (t < total && x < bc.nx && y < bc.ny && z < bc.nz)
+			{
+				const float* b = box + (z * kTiledBox + y) * kTiledBox + x;
+				constexpr int dy = kTiledBox, dz = kTiledBox * kTiledBox;
+				const float v[8] = { b[0], b[1], b[dy + 1], b[dy], b[dz], b[dz + 1], b[dz + dy + 1], b[dz + dy] };
+				unsigned pos = 0;
+#pragma unroll
+				for (int q = 0; q < 8; ++q) pos |= (v[q] >= 0.0f ? 1u : 0u) << q;
+				active = pos != 0u && pos != 0xFFu;
+				const int64_t c = c0 + x + y * cg.sx + z * sxy;
+				cellOf[r] = (uint32_t)c;
+				if (active) atomicOr(words + (c >> 5), 1u << (c & 31));
+			}
+			ballots[r] = __ballot_sync(0xFFFFFFFFu, active);
+			mine += (uint32_t)__popc(ballots[r]);
+		}
+		if (lane == 0) warpBase[warp] = mine;
+		__syncthreads();
+		if (threadIdx.x == 0)
+		{
+			uint32_t sum = 0;
+			uint32_t counts[kTiledThreads / 32];
+#pragma unroll
+			for (int w = 0; w < kTiledThreads / 32; ++w) { counts[w] = warpBase[w]; sum += counts[w]; }
+			uint32_t at = sum ? atomicAdd(cell_count, sum) : 0u;
+#pragma unroll
+			for (int w = 0; w < kTiledThreads / 32; ++w) { warpBase[w] = at; at += counts[w]; }
+		}
+		__syncthreads();
+		uint32_t at = warpBase[warp];
+		const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+		for (int r = 0; r < kTiledRounds; ++r)
+		{
+			if ((ballots[r] >> lane) & 1u) cells[at + __popc(ballots[r] & below)] = cellOf[r];
+			at += (uint32_t)__popc(ballots[r]);
+		}
+	}
+
+	// The box of a part's corner points (LaunchBrickTapes), `grow` lattice steps wider towards
+	// the rest of its brick.
+	__device__ __forceinline__ void PartBox(const GridSpec& g, const BrickGrid& bg, uint32_t b, uint32_t box, int grow, float (&lo)[3],
+		float (&hi)[3])
+	{
+		const uint32_t row = b / (uint32_t)bg.NBX, bz = row / (uint32_t)bg.NBY;
+		const int first[3] = { (int)(b - row * (uint32_t)bg.NBX) * bg.B, (int)(row - bz * (uint32_t)bg.NBY) * bg.B, (int)bz * bg.B };
+		const int last[3] = { min(first[0] + bg.B, g.NX - 1), min(first[1] + bg.B, g.NY - 1), min(first[2] + bg.B, g.NZ - 1) };
+		const float origin[3] = { g.X0, g.Y0, g.Z0 }, step[3] = { g.DX, g.DY, g.DZ };
+#pragma unroll
+		for (int a = 0; a < 3; ++a)
+		{
+			const int x0 = first[a] + (int)((box >> (8 * a)) & 15u), x1 = first[a] + (int)((box >> (8 * a + 4)) & 15u);
+			lo[a] = LatticeCoord(origin[a], max(x0 - grow, first[a]), step[a]);
+			hi[a] = LatticeCoord(origin[a], min(x1 + grow, last[a]), step[a]);
+		}
+	}
+
+	__device__ __forceinline__ void PartCorners(const GridSpec& g, const BrickGrid& bg, uint32_t b, uint32_t box, float (&lo)[3], float (&hi)[3])
+	{
+		PartBox(g, bg, b, box, 0, lo, hi);
+	}
+
+	// The space a part's tape is built for: one step more than its points towards the rest of
+	// the brick (the next part's points begin there, and a vertex between the two may descend
+	// to either part's cell).
+	__device__ __forceinline__ void PartRegion(const GridSpec& g, const BrickGrid& bg, uint32_t b, uint32_t box, float (&lo)[3], float (&hi)[3])
+	{
+		PartBox(g, bg, b, box, 1, lo, hi);
+	}
+
+	inline BrickGrid MakeBrickGrid(const GridSpec& g, int B)
+	{
+		return { B, (g.NX - 1 + B - 1) / B, (g.NY - 1 + B - 1) / B, (g.NZ - 1 + B - 1) / B };
+	}
+}

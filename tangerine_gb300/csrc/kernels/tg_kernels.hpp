@@ -18,6 +18,7 @@ namespace tg
 		int MaxStack;
 		int FullSurfaceCode;    // the whole tree's surface program
 		int Lipschitz;          // every brush 1-Lipschitz
+		int Form;               // kForm* (tg_layout.hpp): what may be left out of its programs
 	};
 
 	// Pinhole camera: pixel (x, y) looks along forward + right*u + up*v with
@@ -97,6 +98,44 @@ namespace tg
 	cudaError_t LaunchEvalBricksCells(const DeviceProgram& prog, const GridSpec& g, const uint32_t* list, const uint32_t* count,
 		const uint32_t* tops, float* lattice, uint32_t* words, uint32_t* cells, uint32_t* cell_count, int sms, cudaStream_t stream,
 		int lanes, int* status);
+	// The evaluation of 7^3-cell bricks through shortened programs (tg_bricktape.cu).  A kept
+	// brick's points lie in one octree cell or, where it straddles pivots, in a few; each such
+	// part of a brick gets a tape of its cell's program, which its points and its vertices run.
+	struct alignas(16) BrickPart
+	{
+		int Cell;               // octree cell; -1: a dead slot
+		uint32_t Box;           // corner points relative to the brick: x0 x1 y0 y1 z0 z1, 4 bits each
+		uint32_t Value;         // first event of the distance and gradient list
+		uint32_t Counts;        // events of the two lists, 16 bits each (0xFFFF: none, run the whole program)
+		int Distance, Surface;  // first quads of the cell's two programs
+		uint32_t Material;      // first event of the material list
+		uint32_t Brick;
+	};
+	constexpr int kBrickTapeCounters = 5;   // parts, parts taken for building, events, bricks evaluated, long parts
+	struct BrickTapes
+	{
+		uint2* Bricks;          // per brick of the grid (written for listed ones): first part, parts (0: none)
+		BrickPart* Parts;
+		uint2* Events;
+		uint32_t* Counters;
+		uint32_t* Long;         // parts with long programs (kLongParts of them at most), built first
+		uint32_t PartCapacity, EventCapacity;
+	};
+	constexpr uint32_t kLongParts = 16384;
+	size_t BrickPartCapacity(int64_t bricks);
+	size_t BrickEventCapacity(int64_t bricks);
+	// Parts and tapes of the listed bricks.  tops: as LaunchEvalBricks.
+	cudaError_t LaunchBrickTapes(const DeviceProgram& prog, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,
+		const uint32_t* tops, const BrickTapes& tapes, int sms, cudaStream_t stream);
+	// LaunchEvalBricks and LaunchCellFlagsListed in one launch through those tapes: the same
+	// lattice, cell bits and active-cell list (list order differs).
+	cudaError_t LaunchEvalBrickTapes(const DeviceProgram& prog, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,
+		const BrickTapes& tapes, float* lattice, uint32_t* words, uint32_t* cells, uint32_t* cell_count, int sms, cudaStream_t stream);
+	// LaunchVertexAttributes of the same export: normals and colours (null: none) of its
+	// `vertex_count` vertices by their parts' tapes, visited in the active-cell list's order.
+	cudaError_t LaunchBrickAttributes(const DeviceProgram& prog, const GridSpec& g, int B, const BrickTapes& tapes, const uint32_t* cells,
+		const uint32_t* words, const uint32_t* word_base, const float* vertices, uint32_t vertex_count, float* normals, uint8_t* colors,
+		cudaStream_t stream);
 	cudaError_t LaunchCellFlagsBricks(const float* lattice, const GridSpec& g, int B, const uint32_t* brick_bits, uint32_t* words,
 		cudaStream_t stream);
 	// Cell pass over the cells of listed bricks only: clears and fills the bitmask and

@@ -1,0 +1,594 @@
+// Shortened programs ("tapes") for a small box of space.
+//
+// An octree cell's program covers a cube of up to 0.25 units; a brick of a fine export is a
+// few hundredths.  Inside such a box most set operators always take the same operand: every
+// brush here (the ellipsoid, and trees with rotations that are not unit quaternions, excepted)
+// is 1-Lipschitz and union, intersection, difference, the polynomial blends, flate and uniform
+// scale keep that, so when two operands differ at the centre of a ball of radius r by more than
+// 2r (and the rounding of both sides), the same one wins at every point of the ball.  The other
+// operand's records can then be left out: min, max and the blends (where the operands are at
+// least the blend radius apart) return the winning operand's value itself, so the shortened
+// program's value at a point is the whole program's, bit for bit.
+//
+// BuildTape runs one program once per box, a warp at 64 points (two per lane, the centres of
+// the box's 4 x 4 x 4 sub-boxes), and votes on every set operator: a side is left out when it
+// loses in every sub-box.  A tape is a list of events, one per record that is left, in the
+// program's own order; the records themselves stay where they are, shared by all tapes of the
+// program.  Each event also names the record's place in the cell's surface program, so the
+// same list serves the gradient (SDFNode::Eval's form); a second list keeps what GetMaterial
+// needs (the left operand of a difference has the material even where the right one decides
+// the distance).
+#pragma once
+
+#include "tg_device.cuh"
+#include "tg_kernels.hpp"
+#include "tg_pair.cuh"
+
+namespace tg
+{
+	// Event: x = distance record (quad offset in the cell's distance program) << 16 | opcode |
+	// record flags; y = quad offset of the record in the cell's surface program.
+	constexpr uint32_t kTapeHead = 0xFFu | RecMatrix | RecOffset | RecScale | RecThenSet;
+	// Opcodes of events without a record: the operand a difference left alone is negated, and a
+	// blend's sum with its zero term turns -0 into +0.
+	enum : uint32_t { OpTapeNegate = 40, OpTapeAddZero = 41 };
+
+	constexpr int kTapeCap = 128;               // events of a list while it is built
+	constexpr uint32_t kNoTape = 0xFFFFu;       // an event count: run the cell's whole program
+
+	__device__ __forceinline__ uint32_t ProgramHead(float word) { return __float_as_uint(word) & kTapeHead; }
+
+	__device__ __forceinline__ int DistanceRecordQuads(uint32_t head)
+	{
+		const uint32_t op = head & 0xFFu;
+		if (op < OpSphere || op > OpPlane) return 1;
+		return 1 + ((head & RecMatrix) ? 3 : (head & RecOffset) ? 1 : 0) + ((head & RecScale) ? 1 : 0);
+	}
+
+	// The brushes a modeller uses least, out of line: one copy of their code for all callers.
+	static __device__ __noinline__ float RareBrushDistance(uint32_t op, float a, float b, float c, float x, float y, float z)
+	{
+		const float prm[3] = { a, b, c };
+		return BrushDistance(op, prm, Vec3(x, y, z));
+	}
+
+	__device__ __forceinline__ float CommonBrushDistance(uint32_t op, const float (&prm)[3], Vec3 p)
+	{
+		switch (op)
+		{
+		case OpSphere: return SdSphere(p, prm[0]);
+		case OpBox: return SdBox(p, Vec3(prm[0], prm[1], prm[2]));
+		case OpTorus: return SdTorus(p, prm[0], prm[1]);
+		default: return SdCylinder(p, prm[0], prm[1]);
+		}
+	}
+
+	// BrushDistance2 and SetDistance2 (tg_pair.cuh), the same values from less code: the
+	// evaluations by tapes are short, and a kernel that holds several interpreters waited for
+	// instructions more than for anything else (10 of 18 stall cycles an issue in the vertex
+	// attributes with the three blends and three rare brushes expanded for every lane).
+	__device__ __forceinline__ float2 TapeBrush2(uint32_t op, const float4& h, float2 x, float2 y, float2 z, const PairUnits& u)
+	{
+		switch (op)
+		{
+		case OpSphere: return SdSphere2(x, y, z, h.y, u);
+		case OpBox: return SdBox2(x, y, z, h.y, h.z, h.w, u);
+		case OpTorus: return SdTorus2(x, y, z, h.y, h.z, u);
+		case OpCylinder: return SdCylinder2(x, y, z, h.y, h.z, u);
+		case OpPlane: return SdPlane2(x, y, z, h.y, h.z, h.w, u);
+		default:
+			return make_float2(RareBrushDistance(op, h.y, h.z, h.w, x.x, y.x, z.x), RareBrushDistance(op, h.y, h.z, h.w, x.y, y.y, z.y));
+		}
+	}
+
+	// The blends share one term: the difference blends as the intersection with its right
+	// operand negated (|l + r| is |l - -r|).
+	__device__ __forceinline__ float TapeBlend(bool unions, float l, float r, float k)
+	{
+		const float m = unions ? fminf(l, r) : fmaxf(l, r);
+		return BlendTerm(m, fmaxf(k - fabsf(l - r), 0.0f), k, unions);
+	}
+
+	__device__ __forceinline__ float2 TapeSet2(uint32_t op, float2 l, float2 r, float k)
+	{
+		if (op == OpDiff || op == OpBlendDiff) r = make_float2(-r.x, -r.y);
+		if (op >= OpBlendUnion)
+		{
+			const bool unions = op == OpBlendUnion;
+			return make_float2(TapeBlend(unions, l.x, r.x, k), TapeBlend(unions, l.y, r.y, k));
+		}
+		if (op == OpUnion) return make_float2(fminf(l.x, r.x), fminf(l.y, r.y));
+		return make_float2(fmaxf(l.x, r.x), fmaxf(l.y, r.y));
+	}
+
+	// A brush's distance (RunDistancePairs' step) from its record at `pc`, whose head is known;
+	// q is left at the points in the brush's own frame, h at the record's first quad.
+	template<int NP, typename Load>
+	__device__ __forceinline__ void BrushStep(Load load, int pc, uint32_t head, const float2 (&px)[NP], const float2 (&py)[NP],
+		const float2 (&pz)[NP], const PairUnits& u, float2 (&qx)[NP], float2 (&qy)[NP], float2 (&qz)[NP], float4& h, float2 (&d)[NP])
+	{
+		h = load(pc);
+#pragma unroll
+		for (int j = 0; j < NP; ++j) { qx[j] = px[j]; qy[j] = py[j]; qz[j] = pz[j]; }
+		int at = pc + 1;
+		if (head & RecMatrix)
+		{
+			const float4 X = load(at), Y = load(at + 1), Z = load(at + 2);
+			at += 3;
+#pragma unroll
+			for (int j = 0; j < NP; ++j)
+			{
+				qx[j] = AffineRow2(X, px[j], py[j], pz[j], u);
+				qy[j] = AffineRow2(Y, px[j], py[j], pz[j], u);
+				qz[j] = AffineRow2(Z, px[j], py[j], pz[j], u);
+			}
+		}
+		else if (head & RecOffset)
+		{
+			const float4 O = load(at++);
+#pragma unroll
+			for (int j = 0; j < NP; ++j)
+			{
+				qx[j] = Add2(px[j], Pair(O.x), u);
+				qy[j] = Add2(py[j], Pair(O.y), u);
+				qz[j] = Add2(pz[j], Pair(O.z), u);
+			}
+		}
+#pragma unroll
+		for (int j = 0; j < NP; ++j) d[j] = TapeBrush2(head & 0xFFu, h, qx[j], qy[j], qz[j], u);
+		if (head & RecScale)
+		{
+			const float4 S = load(at);
+#pragma unroll
+			for (int j = 0; j < NP; ++j) d[j] = Mul2(d[j], Pair(S.x), u);
+		}
+	}
+
+	// The distance at NP pairs of points by a tape of `count` (at least one) events over the
+	// program at `base`; `event(i)` returns event i (from global or shared memory).  Operands
+	// below the top of the stack are at spill[(depth * NP + pair) * stride].  The set
+	// operator's code appears once: a brush that is its right operand falls through to it.
+	template<int NP, typename Load, typename Event>
+	__device__ __forceinline__ void RunTapePairs(Load load, int base, Event event, uint32_t count, const float2 (&px)[NP],
+		const float2 (&py)[NP], const float2 (&pz)[NP], const PairUnits& u, float2 (&acc)[NP], float2* spill, int stride)
+	{
+		float2 left[NP];
+#pragma unroll
+		for (int j = 0; j < NP; ++j) acc[j] = left[j] = make_float2(0.0f, 0.0f);
+		int depth = 0;
+		uint32_t e = 0, x = event(0u).x;
+		for (;;)
+		{
+			uint32_t op = x & 0xFFu;
+			int at = base + (int)(x >> 16);
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const uint32_t head = x;
+				if (++e < count) x = event(e).x;
+				if (!(head & RecThenSet))
+				{
+					if (depth > 0)
+					{
+#pragma unroll
+						for (int j = 0; j < NP; ++j) spill[((depth - 1) * NP + j) * stride] = acc[j];
+					}
+					++depth;
+				}
+#pragma unroll
+				for (int j = 0; j < NP; ++j) left[j] = acc[j];
+				float2 qx[NP], qy[NP], qz[NP];
+				float4 h;
+				BrushStep<NP>(load, at, head, px, py, pz, u, qx, qy, qz, h, acc);
+				if (e >= count) break;
+				if (!(head & RecThenSet)) continue;
+				op = x & 0xFFu;
+				at = base + (int)(x >> 16);
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+#pragma unroll
+				for (int j = 0; j < NP; ++j) left[j] = spill[((depth - 1) * NP + j) * stride];
+			}
+			if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				const float k = op >= OpBlendUnion ? load(at).y : 0.0f;
+#pragma unroll
+				for (int j = 0; j < NP; ++j) acc[j] = TapeSet2(op, left[j], acc[j], k);
+			}
+			else if (op == OpFlate)
+			{
+				const float k = load(at).y;
+#pragma unroll
+				for (int j = 0; j < NP; ++j) acc[j] = Sub2(acc[j], Pair(k), u);
+			}
+			else
+			{
+#pragma unroll
+				for (int j = 0; j < NP; ++j)
+					acc[j] = op == OpTapeNegate ? make_float2(-acc[j].x, -acc[j].y) : make_float2(acc[j].x + 0.0f, acc[j].y + 0.0f);
+			}
+			if (++e >= count) break;
+			x = event(e).x;
+		}
+	}
+
+	// The whole distance program at one pair of points, where there is no tape.  Out of line:
+	// rare beside the tapes, and the callers' code stays small.
+	static __device__ __noinline__ float2 RunWholePair(const float4* __restrict__ code, int pc, float2 px, float2 py, float2 pz, float2* spill,
+		int stride)
+	{
+		const float2 x[1] = { px }, y[1] = { py }, z[1] = { pz };
+		float2 d[1];
+		RunDistancePairs<1>([&](int q) { return __ldg(code + q); }, pc, x, y, z, d, spill, stride);
+		return d[0];
+	}
+
+	// SDFNode::Eval at NP pairs of points (RunSurfacePair's steps) by the surface records a
+	// tape names, those of the surface program at `base`.
+	template<int NP, typename Load, typename Event>
+	__device__ __forceinline__ void RunSurfaceTapePairs(Load load, int base, Event event, uint32_t count, const float2 (&px)[NP],
+		const float2 (&py)[NP], const float2 (&pz)[NP], const PairUnits& u, float2 (&acc)[NP], float2* spill, int stride)
+	{
+		float2 left[NP];
+#pragma unroll
+		for (int j = 0; j < NP; ++j) acc[j] = left[j] = make_float2(0.0f, 0.0f);
+		int depth = 0;
+		uint32_t e = 0;
+		uint2 ev = event(0u);
+		for (;;)
+		{
+			uint32_t op = ev.x & 0xFFu;
+			int at = base + (int)ev.y;
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const uint32_t head = ev.x;
+				if (++e < count) ev = event(e);
+				if (!(head & RecThenSet))
+				{
+					if (depth > 0)
+					{
+#pragma unroll
+						for (int j = 0; j < NP; ++j) spill[((depth - 1) * NP + j) * stride] = acc[j];
+					}
+					++depth;
+				}
+				const float4 h = load(at), Q = load(at + 1), T = load(at + 2);
+				const bool scaled = T.w != 1.0f;    // x / 1 and x * 1 are x exactly
+#pragma unroll
+				for (int j = 0; j < NP; ++j)
+				{
+					left[j] = acc[j];
+					const float2 vx = Sub2(px[j], Pair(T.x), u), vy = Sub2(py[j], Pair(T.y), u), vz = Sub2(pz[j], Pair(T.z), u);
+					// The quad holds the inverse quaternion as (w, x, y, z).
+					float2 ux, uy, uz, wx, wy, wz;
+					CrossPair(Q.y, Q.z, Q.w, vx, vy, vz, ux, uy, uz, u);
+					CrossPair(Q.y, Q.z, Q.w, ux, uy, uz, wx, wy, wz, u);
+					float2 lx = Add2(vx, Mul2(Add2(Mul2(ux, Pair(Q.x), u), wx, u), Pair(2.0f), u), u);
+					float2 ly = Add2(vy, Mul2(Add2(Mul2(uy, Pair(Q.x), u), wy, u), Pair(2.0f), u), u);
+					float2 lz = Add2(vz, Mul2(Add2(Mul2(uz, Pair(Q.x), u), wz, u), Pair(2.0f), u), u);
+					if (scaled)
+					{
+						lx = make_float2(lx.x / T.w, lx.y / T.w);
+						ly = make_float2(ly.x / T.w, ly.y / T.w);
+						lz = make_float2(lz.x / T.w, lz.y / T.w);
+					}
+					acc[j] = TapeBrush2(op, h, lx, ly, lz, u);
+					if (scaled) acc[j] = Mul2(acc[j], Pair(T.w), u);
+				}
+				if (e >= count) break;
+				if (!(head & RecThenSet)) continue;
+				op = ev.x & 0xFFu;
+				at = base + (int)ev.y;
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+#pragma unroll
+				for (int j = 0; j < NP; ++j) left[j] = spill[((depth - 1) * NP + j) * stride];
+			}
+			if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				const float k = op >= OpBlendUnion ? load(at).y : 0.0f;
+#pragma unroll
+				for (int j = 0; j < NP; ++j) acc[j] = TapeSet2(op, left[j], acc[j], k);
+			}
+			else if (op == OpFlate)
+			{
+				const float k = load(at).y;
+#pragma unroll
+				for (int j = 0; j < NP; ++j) acc[j] = Sub2(acc[j], Pair(k), u);
+			}
+			else
+			{
+#pragma unroll
+				for (int j = 0; j < NP; ++j)
+					acc[j] = op == OpTapeNegate ? make_float2(-acc[j].x, -acc[j].y) : make_float2(acc[j].x + 0.0f, acc[j].y + 0.0f);
+			}
+			if (++e >= count) break;
+			ev = event(e);
+		}
+	}
+
+	// The whole surface program at one pair of points, and GetMaterial's walk of it at one
+	// point: where there is no tape.
+	static __device__ __noinline__ float2 RunWholeSurfacePair(const float4* __restrict__ code, int pc, float2 px, float2 py, float2 pz,
+		float2* spill, int stride)
+	{
+		return RunSurfacePair([&](int q) { return __ldg(code + q); }, pc, px, py, pz, spill, stride);
+	}
+
+	static __device__ __noinline__ int RunWholeMaterial(const float4* __restrict__ code, int pc, Vec3 p, float* spill, int stride)
+	{
+		const float px[1] = { p.x }, py[1] = { p.y }, pz[1] = { p.z };
+		float d[1];
+		int m = -1;
+		RunSurfaceBatch<1>(code, pc, px, py, pz, d, 0, &m, spill, stride);
+		return m;
+	}
+
+	// GetMaterial at one point over a painted tree without stencils (every brush has a
+	// material, so intersections and blends choose by distance): the material list of a tape.
+	// `spill` as RunSurfaceBatch<1>'s, which other threads of the block may run meanwhile.
+	template<typename Load, typename Event>
+	__device__ __forceinline__ int RunMaterialTape(Load load, int base, Event event, uint32_t count, Vec3 p, float* spill, int stride)
+	{
+		// One brush left: its material, whatever its distance.
+		if (count == 1) return __float_as_int(load(base + (int)event(0u).y + 3).x);
+		float acc = 0.0f, left = 0.0f;
+		int macc = -1, mleft = -1;
+		int depth = 0;
+		for (uint32_t e = 0; e < count; )
+		{
+			uint2 ev = event(e++);
+			uint32_t op = ev.x & 0xFFu;
+			int at = base + (int)ev.y;
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const bool thenSet = (ev.x & RecThenSet) != 0;
+				left = acc;
+				mleft = macc;
+				if (!thenSet)
+				{
+					if (depth > 0)
+					{
+						spill[(depth - 1) * 2 * stride] = acc;
+						spill[((depth - 1) * 2 + 1) * stride] = __int_as_float(macc);
+					}
+					++depth;
+				}
+				const float4 h = load(at), Q = load(at + 1), T = load(at + 2), M = load(at + 3);
+				const Quat qi{ Q.x, Q.y, Q.z, Q.w };
+				Vec3 local = Rotate(qi, p - Vec3(T.x, T.y, T.z));
+				const bool scaled = T.w != 1.0f;
+				if (scaled) local = local / T.w;
+				const float prm[3] = { h.y, h.z, h.w };
+				acc = op == OpSphere || op == OpBox || op == OpTorus || op == OpCylinder ? CommonBrushDistance(op, prm, local)
+					: RareBrushDistance(op, h.y, h.z, h.w, local.x, local.y, local.z);
+				if (scaled) acc = acc * T.w;
+				macc = __float_as_int(M.x);
+				if (!thenSet) continue;
+				if (e >= count) break;
+				ev = event(e++);
+				op = ev.x & 0xFFu;
+				at = base + (int)ev.y;
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+				left = spill[(depth - 1) * 2 * stride];
+				mleft = __float_as_int(spill[((depth - 1) * 2 + 1) * stride]);
+			}
+			else
+			{
+				if (op == OpFlate) acc = acc - load(at).y;
+				else acc = acc + 0.0f;      // OpTapeAddZero; this list negates nothing
+				continue;
+			}
+			const float k = op >= OpBlendUnion ? load(at).y : 0.0f;
+			const float2 both = TapeSet2(op, make_float2(left, left), make_float2(acc, acc), k);
+			const float d = both.x;
+			// SetNode::GetMaterial (sdf_evaluator.cpp:957-1012).
+			const bool blend = op == OpBlendUnion || op == OpBlendInter;
+			const bool takeLeft = (op == OpDiff || op == OpBlendDiff) || (blend ? (fabsf(left - d) <= fabsf(acc - d)) : (d == left));
+			if (takeLeft) macc = mleft;
+			acc = d;
+		}
+		return macc;
+	}
+
+	// The warp's scratch while it builds a tape.
+	struct TapeScratch
+	{
+		uint2 Value[kTapeCap];              // events of the distance
+		uint2 Material[kTapeCap];           // events of the material walk
+		uint2 Start[kMaxStack + 1];         // each operand on the stack: its first events
+		uint2 Unused;
+		float4 Window[64];                  // the records around the one being run
+	};
+
+	struct TapeCounts
+	{
+		int Value, Material;
+		bool Same;              // no difference was decided by its right operand: one list serves both
+		int Sign;               // 1 or -1: the program keeps that sign in the box; 0: it may not
+	};
+
+	// Builds the tape of the distance program of `quads` records at `code`, stop included, for
+	// a box, by all lanes of a warp: lane l's pair of points are centres of two balls, and the
+	// balls of all lanes cover the box.  `reach` is how far the difference of two operands can
+	// move inside a ball, with the fixed part of the rounding (TapeReach); the part that grows
+	// with the operands' own coordinates (brushes far from the box) is added here: each brush's
+	// float error is at most a few roundings of its local coordinates and sizes.  Returns false
+	// when a list outgrows its scratch.
+	//
+	// The records come through a window in shared memory, 32 quads at a time, the next 32 in
+	// flight: read one by one from memory, every record's first use waited for L2, and a
+	// program of some hundred records held its warp longer than all others took together.
+	__device__ __forceinline__ bool BuildTape(const float4* __restrict__ code, int quads, float2 px, float2 py, float2 pz, float reach,
+		const PairUnits& u, float2* spill, int stride, TapeScratch& ts, TapeCounts& out)
+	{
+		const float2 x1[1] = { px }, y1[1] = { py }, z1[1] = { pz };
+		const int lane = (int)(threadIdx.x & 31);
+		float2 acc = make_float2(0.0f, 0.0f), left = acc;
+		float2 size = make_float2(0.0f, 0.0f);
+		int depth = 0, pc = 0, surface = 0;
+		int nv = 0, nm = 0;
+		bool same = true;
+		if (quads > 0xFFF0) return false;
+		// The window holds quads [32 * chunk, 32 * chunk + 64); `ahead` the 32 after those.
+		int chunk = 0;
+		auto fetch = [&](int q) { return __ldg(code + min(q, quads - 1)); };
+		ts.Window[lane] = fetch(lane);
+		ts.Window[lane + 32] = fetch(lane + 32);
+		float4 ahead = fetch(lane + 64);
+		__syncwarp();
+		auto load = [&](int q) { return ts.Window[q & 63]; };
+		// [from, to) of a list moves down to `down`.
+		auto move = [&](uint2* list, int down, int from, int to)
+		{
+			for (int i = 0; from + i < to; i += 32)
+			{
+				uint2 ev = make_uint2(0u, 0u);
+				if (from + i + lane < to) ev = list[from + i + lane];
+				__syncwarp();
+				if (from + i + lane < to) list[down + i + lane] = ev;
+				__syncwarp();
+			}
+		};
+		for (int guard = 0; guard < (1 << 24); ++guard)
+		{
+			if (nv + 4 > kTapeCap || nm + 4 > kTapeCap) return false;
+			if ((pc >> 5) != chunk)
+			{
+				__syncwarp();
+				ts.Window[(chunk & 1) * 32 + lane] = ahead;
+				++chunk;
+				ahead = fetch(32 * chunk + 64 + lane);
+				__syncwarp();
+			}
+			uint32_t head = ProgramHead(load(pc).x);
+			uint32_t op = head & 0xFFu;
+			uint32_t event = ((uint32_t)pc << 16) | (head & ~RecThenSet);
+			int rv = nv, rm = nm;       // first events of the right operand
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const bool thenSet = (head & RecThenSet) != 0;
+				left = acc;
+				if (!thenSet)
+				{
+					if (depth > 0) spill[(depth - 1) * stride] = acc;
+					ts.Start[depth] = make_uint2((uint32_t)nv, (uint32_t)nm);
+					++depth;
+				}
+				ts.Value[nv++] = make_uint2(event, (uint32_t)surface);
+				ts.Material[nm++] = make_uint2(event, (uint32_t)surface);
+				float2 qx[1], qy[1], qz[1], d[1];
+				float4 h;
+				BrushStep<1>(load, pc, head, x1, y1, z1, u, qx, qy, qz, h, d);
+				acc = d[0];
+				const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
+				size.x = fmaxf(size.x, fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(acc.x));
+				size.y = fmaxf(size.y, fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(acc.y));
+				pc += DistanceRecordQuads(head);
+				surface += 4;
+				if (!thenSet) continue;
+				head = ProgramHead(load(pc).x);
+				op = head & 0xFFu;
+				event = ((uint32_t)pc << 16) | head;
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+				const uint2 r = ts.Start[depth];
+				rv = (int)r.x; rm = (int)r.y;
+				left = spill[(depth - 1) * stride];
+			}
+			else if (op == OpFlate)
+			{
+				ts.Value[nv++] = make_uint2(event, (uint32_t)surface);
+				ts.Material[nm++] = make_uint2(event, (uint32_t)surface);
+				acc = Sub2(acc, Pair(load(pc).y), u);
+				++pc;
+				++surface;
+				continue;
+			}
+			else
+			{
+				break;   // OpStop
+			}
+			const float k = load(pc).y;
+			const bool blend = op >= OpBlendUnion;
+			const bool diff = op == OpDiff || op == OpBlendDiff;
+			const bool unions = op == OpUnion || op == OpBlendUnion;
+			// s > 0 where the left operand wins: by more than the reach everywhere, it always does.
+			const float2 s = unions ? make_float2(acc.x - left.x, acc.y - left.y)
+				: diff ? make_float2(left.x + acc.x, left.y + acc.y) : make_float2(left.x - acc.x, left.y - acc.y);
+			const float2 t = make_float2(reach + 2e-5f * size.x + (blend ? k : 0.0f), reach + 2e-5f * size.y + (blend ? k : 0.0f));
+			const bool decides = !blend || k > 0.0f;
+			__syncwarp();       // every lane's list writes so far come before any slot is reused
+			const bool leftWins = __all_sync(0xFFFFFFFFu, decides && s.x > t.x && s.y > t.y);
+			const bool rightWins = __all_sync(0xFFFFFFFFu, decides && s.x < -t.x && s.y < -t.y);
+			const uint2 l = ts.Start[depth - 1];
+			const uint2 set = make_uint2(event, (uint32_t)surface);
+			const uint2 addZero = make_uint2(OpTapeAddZero, 0u);
+			if (leftWins)
+			{
+				nv = rv;
+				nm = rm;
+				if (blend && !unions) { ts.Value[nv++] = addZero; ts.Material[nm++] = addZero; }
+			}
+			else
+			{
+				if (rightWins)
+				{
+					move(ts.Value, (int)l.x, rv, nv);
+					nv -= rv - (int)l.x;
+					if (diff) ts.Value[nv++] = make_uint2(OpTapeNegate, 0u);
+					if (blend && !unions) ts.Value[nv++] = addZero;
+				}
+				else
+				{
+					// A right operand that is now a single brush is combined in its own step.
+					if (nv - rv == 1 && (ts.Value[rv].x & 0xFFu) <= OpPlane) ts.Value[rv].x |= RecThenSet;
+					ts.Value[nv++] = set;
+				}
+				if (rightWins && !diff)
+				{
+					move(ts.Material, (int)l.y, rm, nm);
+					nm -= rm - (int)l.y;
+					if (blend && !unions) ts.Material[nm++] = addZero;
+				}
+				else
+				{
+					if (rightWins) same = false;
+					if (nm - rm == 1 && (ts.Material[rm].x & 0xFFu) <= OpPlane) ts.Material[rm].x |= RecThenSet;
+					ts.Material[nm++] = set;
+				}
+			}
+			acc = TapeSet2(op, left, acc, k);
+			++pc;
+			++surface;
+		}
+		__syncwarp();
+		out.Value = nv;
+		out.Material = nm;
+		out.Same = same;
+		// |f| beyond a ball's radius (half the reach covers it) at every centre: no sign change.
+		const float2 far = make_float2(0.5f * reach + 2e-5f * size.x, 0.5f * reach + 2e-5f * size.y);
+		out.Sign = __all_sync(0xFFFFFFFFu, acc.x > far.x && acc.y > far.y) ? 1
+			: __all_sync(0xFFFFFFFFu, acc.x < -far.x && acc.y < -far.y) ? -1 : 0;
+		return true;
+	}
+
+	// How far the difference of two operands can move inside a ball of radius r about a point
+	// near c, for trees whose rotations are within 1e-3 of unit quaternions, and the rounding
+	// of two operands at two points near c (as the brick test's margin, four times).
+	__device__ __forceinline__ float TapeReach(float r, float cx, float cy, float cz, float rootClip)
+	{
+		return 2.0f * 1.01f * r + 2e-4f * (1.0f + fabsf(cx) + fabsf(cy) + fabsf(cz) + fabsf(rootClip));
+	}
+
+	// The gradient's evaluation points lie up to this far from the point itself.
+	constexpr float kTetraReach = 1.8e-4f;
+}

@@ -1,0 +1,75 @@
+"""Shortened programs (tg_tape.cuh) against whole ones: a tape leaves out only operands that
+lose everywhere in its box, so every value it gives is the whole program's, bit for bit (the
+tolerance is 0)."""
+
+import numpy as np
+import pytest
+
+from conftest import golden_names
+from tangerine_gb300 import _lib, sdf
+from tangerine_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+ALL_OPS = ((W.UNION, 0.2), (W.DIFF, 0.2), (W.INTER, 0.1), (W.BLEND_UNION, 0.2), (W.BLEND_DIFF, 0.15), (W.BLEND_INTER, 0.15))
+# Coarse (bricks larger than octree cells, many parts a brick), fine, cut bricks on every
+# axis, a step per axis, one brick, one cell.
+GRIDS = {
+    "coarse": (-2.0, -2.0, -2.0, 0.11, 38, 38, 38),
+    "fine": (-0.75, -0.6, -0.4, 0.004, 150, 142, 129),
+    "ragged": (-1.9, -1.7, -2.0, 0.021, 173, 120, 191, 0.027, 0.019),
+    "brick": (-0.3, -0.2, -0.3, 0.03, 8, 8, 8),
+    "cell": (0.1, 0.1, 0.1, 0.5, 2, 2, 2),
+}
+
+
+def _same(a, b):
+    for x, y in ((a.vertices, b.vertices), (a.cubes, b.cubes), (a.faces, b.faces), (a.normals, b.normals)):
+        np.testing.assert_array_equal(x, y)
+    assert (a.colors is None) == (b.colors is None)
+    if a.colors is not None:
+        np.testing.assert_array_equal(a.colors, b.colors)
+
+
+@pytest.mark.parametrize("grid", sorted(GRIDS))
+@pytest.mark.parametrize("prims,ops,paint", [(1, ALL_OPS, True), (2, ALL_OPS, True), (40, ALL_OPS, True), (150, W.OPS_60_20_10_10, True),
+                                             (60, ALL_OPS, False)])
+def test_brick_tapes_equal_dense_export(lib, grid, prims, ops, paint):
+    seed = 3
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops, paint=paint))):
+        seed += 1
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        g = _lib.Grid(*GRIDS[grid])
+        _same(prog.export_mesh(g, dense=True), prog.export_mesh(g, tapes=True))
+
+
+@pytest.mark.parametrize("name", golden_names())
+def test_brick_tapes_equal_dense_export_fixture_trees(lib, golden, name):
+    """Every brush and operator (ellipsoids, cones, stencils, scales, flates, unpainted brushes)."""
+    g = golden[name]
+    if "octree_nodes" not in g:
+        pytest.skip("no octree")
+    with sdf.compile(sdf.from_spec(g["spec"])) as prog:
+        info = prog.info()
+        lo, hi = np.asarray(info.bounds_min[:]), np.asarray(info.bounds_max[:])
+        for cells in (20, 130):
+            step = float(np.max(hi - lo)) * 1.1 / cells
+            n = [int(np.ceil((h - l) * 1.1 / step)) + 3 for l, h in zip(lo, hi)]
+            start = [float(l - 0.05 * (h - l) - step) for l, h in zip(lo, hi)]
+            grid = _lib.Grid(*start, step, *n)
+            _same(prog.export_mesh(grid, dense=True), prog.export_mesh(grid, tapes=True))
+
+
+def test_brick_tapes_far_large_and_stretched_operands(lib):
+    """Operands whose own float error is large (a sphere of radius 3000 seen near its surface),
+    a thin blend, and rotations that are not unit quaternions (never shortened)."""
+    cut = sdf.sphere(3000.0).move(0.0, 0.0, -2999.9)
+    body = sdf.blend_union(0.003, sdf.box(0.5, 0.4, 0.6), sdf.torus(0.5, 0.1).move(0.2, 0.1, 0.3))
+    tree = sdf.inter(sdf.blend_diff(0.05, body, sdf.sphere(0.3).move(0.4, 0.3, 0.2)), cut)
+    stretched = sdf.union(sdf.box(0.4, 0.2, 0.3).rotate(0.1, 0.3, 0.2, 1.4), sdf.cylinder(0.2, 0.5).move(0.3, 0.0, 0.0))
+    grid = _lib.Grid(-0.9, -0.8, -0.8, 0.013, 140, 120, 131)
+    for t in (tree, stretched):
+        with sdf.compile(t) as prog:
+            whole = prog.export_mesh(grid, brick=6)
+            assert whole.vertices.shape[0] > 1000
+            _same(whole, prog.export_mesh(grid, tapes=True))
