@@ -817,23 +817,14 @@ extern "C"
 		if (!VoxPlan(p->Host.Bounds, grid_size, vs, err)) { SetError(err); return TG_ERR_UNSUPPORTED; }
 		Engine& eng = Engine::Get();
 		std::lock_guard<std::mutex> lock(eng.Mutex);
-		std::vector<uint32_t> cells;
-		cudaError_t e = eng.Voxels(*p, vs, cells, StreamOf(stream));
-		if (e != cudaSuccess) return CudaFail(e, "voxelising the tree");
-		out->voxels = (int32_t*)std::malloc(sizeof(int32_t) * 4 * (cells.empty() ? 1 : cells.size()));
-		if (!out->voxels) { SetError("out of host memory for the voxels"); return TG_ERR_MEMORY; }
-		// int z = i / Slice, y = (i % Slice) / Size.x, x = i % Size.x; abs(ColorIndex) % 255 + 1
-		const int32_t slice = vs.SX * vs.SY;
+		// abs(ColorIndex) % 255 + 1
 		const int32_t color = std::abs(color_index) % 255 + 1;
-		for (size_t v = 0; v < cells.size(); ++v)
-		{
-			const int32_t i = (int32_t)cells[v];
-			out->voxels[v * 4 + 0] = i % vs.SX;
-			out->voxels[v * 4 + 1] = (i % slice) / vs.SX;
-			out->voxels[v * 4 + 2] = i / slice;
-			out->voxels[v * 4 + 3] = color;
-		}
-		out->count = cells.size();
+		size_t count = 0;
+		bool hostFull = false;
+		cudaError_t e = eng.Voxels(*p, vs, color, out->voxels, count, hostFull, StreamOf(stream));
+		if (hostFull) { SetError("out of host memory for the voxels"); return TG_ERR_MEMORY; }
+		if (e != cudaSuccess) return CudaFail(e, "voxelising the tree");
+		out->count = count;
 		out->size[0] = vs.SX; out->size[1] = vs.SY; out->size[2] = vs.SZ;
 		out->radius = vs.Radius;
 		return TG_OK;
@@ -842,7 +833,7 @@ extern "C"
 	TANGERINE_API void tg_voxels_free(tg_voxels* v)
 	{
 		if (!v) return;
-		std::free(v->voxels);
+		if (v->voxels && !HostPool::Get().Give(v->voxels)) std::free(v->voxels);
 		std::memset(v, 0, sizeof *v);
 	}
 

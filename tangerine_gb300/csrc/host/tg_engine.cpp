@@ -146,6 +146,7 @@ namespace tg
 			p.View.FullSurfaceCode = p.Host.Header.FullSurfaceCode;
 			p.View.Lipschitz = p.Host.Header.Lipschitz;
 			p.View.Form = p.Host.Header.Form;
+			p.View.CodeQuads = p.Host.Header.CodeQuads;
 		}
 	}
 
@@ -342,6 +343,14 @@ namespace tg
 		return (double)bricks * (quads - 12.0) >= 3.5e6;
 	}
 
+	cudaError_t Engine::ReadSmCount()
+	{
+		if (SmCount) return cudaSuccess;
+		int dev = 0;
+		TG_TRY(cudaGetDevice(&dev));
+		return cudaDeviceGetAttribute(&SmCount, cudaDevAttrMultiProcessorCount, dev);
+	}
+
 	cudaError_t Engine::ReserveTapes(int64_t bricks, BrickTapes& out)
 	{
 		out.PartCapacity = (uint32_t)std::min<size_t>(BrickPartCapacity(bricks), 0x7FFFFFFFu);
@@ -416,12 +425,7 @@ namespace tg
 			// The exact classifier stores each kept brick's descent for the evaluation; the
 			// network alone leaves the evaluation to descend.
 			uint32_t* tops = (!opt.Field || opt.Refine) ? BrickTops.As<uint32_t>() : nullptr;
-			if (!SmCount)
-			{
-				int dev = 0;
-				TG_TRY(cudaGetDevice(&dev));
-				TG_TRY(cudaDeviceGetAttribute(&SmCount, cudaDevAttrMultiProcessorCount, dev));
-			}
+			TG_TRY(ReadSmCount());
 			uint32_t* brickCount = Counts.As<uint32_t>() + 2;
 			uint32_t* bits = BrickBits.As<uint32_t>();
 			if (opt.Field)

@@ -174,8 +174,10 @@ namespace tg
 		// voxel number, Faces nothing.
 		cudaError_t PointCloud(const Program& p, const CloudSpec& s, int refine, bool attributes, DeviceMesh& out, cudaStream_t st,
 			const ExportOptions* control = nullptr);
-		// VoxExport's voxel test on the GPU: the kept voxel numbers in order, to the host.
-		cudaError_t Voxels(const Program& p, const VoxSpec& s, std::vector<uint32_t>& cells, cudaStream_t st);
+		// VoxExport's voxels on the GPU in cell order, four words each (x, y, z, color), in a
+		// host block the caller owns (HostPool's, or malloc's where the pool has none).
+		cudaError_t Voxels(const Program& p, const VoxSpec& s, int color, int32_t*& voxels, size_t& count, bool& host_full,
+			cudaStream_t st);
 		// Network iterations and exact steps of the last network-stepped render.
 		uint64_t LastNetworkSteps = 0, LastExactSteps = 0;
 		DeviceBuffer& Lattice() { return LatticeBuf; }
@@ -201,6 +203,7 @@ namespace tg
 		cudaStream_t CopyStream = nullptr;          // early device-to-host copies of an export
 		// The buffers of a grid's brick tapes (LaunchBrickTapes), kept between exports.
 		cudaError_t ReserveTapes(int64_t bricks, BrickTapes& out);
+		cudaError_t ReadSmCount();
 		cudaEvent_t MeshReady = nullptr;
 		cudaEvent_t CodeReady = nullptr;            // RestageCode's copy of an export is done
 		DeviceBuffer LatticeBuf, Words, WordBase, Scratch, Counts, Vertices, Cubes, FaceCounts, FaceBase, Faces, Normals, Colors;
@@ -208,6 +211,7 @@ namespace tg
 		DeviceBuffer TapeBricks, TapeParts, TapeEvents, TapeCounters;    // ReserveTapes
 		DeviceBuffer RayIn, RayOut, Cameras, Image, RenderCounters;
 		DeviceBuffer SodaBoxes, SodaCache, SodaColors;
+		DeviceBuffer VoxScratch, VoxelsOut;
 		void* Staging = nullptr;
 		size_t StagingBytes = 0;
 		// PreClassify's one-cell program: pinned staging, its device copy, the event after

@@ -5,6 +5,7 @@
 
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <functional>
 #include <string>
 #include <unordered_map>
@@ -153,32 +154,50 @@ namespace tg
 		return cudaSuccess;
 	}
 
-	cudaError_t Engine::Voxels(const Program& p, const VoxSpec& s, std::vector<uint32_t>& cells, cudaStream_t st)
+	cudaError_t Engine::Voxels(const Program& p, const VoxSpec& s, int color, int32_t*& voxels, size_t& count, bool& host_full,
+		cudaStream_t st)
 	{
-		cells.clear();
+		voxels = nullptr;
+		count = 0;
 		const int64_t words = (s.Total + 31) / 32;
 		if (!HostCounts) TG_TRY(cudaMallocHost(&HostCounts, 8 * sizeof(uint32_t)));
 		TG_TRY(Words.Reserve((size_t)(words ? words : 1) * 4));
 		TG_TRY(WordBase.Reserve((size_t)(words ? words : 1) * 4));
 		TG_TRY(Counts.Reserve(4 * sizeof(uint32_t)));
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4 + 4));
-		TG_TRY(Cubes.Reserve((size_t)(words ? words : 1) * 32 * 4));
-		PreValid = false;   // these bits replace a pending PreClassify's
-		TG_TRY(BrickBits.Reserve(VoxelBrickWords(s.SX, s.SY, s.SZ) * 4));
+		TG_TRY(VoxScratch.Reserve(VoxScratchBytes(p.View, s)));
+		TG_TRY(ReadSmCount());
 		Begin("vox_flags", st);
-		TG_TRY(LaunchVoxFlags(p.View, s, BrickBits.As<uint32_t>(), Words.As<uint32_t>(), st));
+		TG_TRY(LaunchVoxFlags(p.View, s, VoxScratch.Ptr, Words.As<uint32_t>(), SmCount, st));
 		End(st);
 		Begin("list_cells", st);
-		TG_TRY(LaunchListBricks(Words.As<uint32_t>(), s.Total, WordBase.As<uint32_t>(), Scratch.As<uint32_t>(), Cubes.As<uint32_t>(),
-			Counts.As<uint32_t>(), st));
+		TG_TRY(LaunchExclusiveScan(Words.As<uint32_t>(), words, true, WordBase.As<uint32_t>(), Counts.As<uint32_t>(), Scratch.As<uint32_t>(), st));
 		End(st);
 		TG_TRY(cudaMemcpyAsync(HostCounts, Counts.Ptr, 4, cudaMemcpyDeviceToHost, st));
 		TG_TRY(cudaStreamSynchronize(st));
 		const uint32_t n = HostCounts[0];
-		cells.resize(n);
-		if (n) TG_TRY(cudaMemcpyAsync(cells.data(), Cubes.Ptr, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
-		TG_TRY(cudaStreamSynchronize(st));
+		// The voxels are written out on the GPU, straight in the caller's layout, and come back
+		// in one copy to a page-locked block.
+		const size_t bytes = (size_t)(n ? n : 1) * sizeof(int4);
+		void* block = HostPool::Get().Take(bytes);
+		if (!block) block = std::malloc(bytes);
+		host_full = !block;
+		if (!block) return cudaErrorMemoryAllocation;
+		cudaError_t e = VoxelsOut.Reserve(bytes);
+		if (e == cudaSuccess && n)
+		{
+			e = LaunchVoxList(s, Words.As<uint32_t>(), WordBase.As<uint32_t>(), color, VoxelsOut.As<int4>(), st);
+			if (e == cudaSuccess) e = cudaMemcpyAsync(block, VoxelsOut.Ptr, (size_t)n * sizeof(int4), cudaMemcpyDeviceToHost, st);
+		}
+		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
 		Collect();
+		if (e != cudaSuccess)
+		{
+			if (!HostPool::Get().Give(block)) std::free(block);
+			return e;
+		}
+		voxels = static_cast<int32_t*>(block);
+		count = n;
 		return cudaSuccess;
 	}
 

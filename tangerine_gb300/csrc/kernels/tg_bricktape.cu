@@ -207,6 +207,14 @@ namespace tg
 			}
 		}
 
+		// A warp's scratch while it builds a part's tape.
+		struct TapeScratch
+		{
+			uint2 Value[kTapeCap], Material[kTapeCap];
+			uint2 Start[kMaxStack + 2];
+			float4 Window[64];
+		};
+
 		// One warp per part, drawn from a counter, those with long programs first (a single one
 		// of several hundred records keeps a warp busy longer than the whole launch otherwise
 		// takes).  Bound by issue and by the latency of the one pass over the cell's program.
@@ -216,6 +224,7 @@ namespace tg
 			extern __shared__ __align__(16) uint8_t shared[];
 			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
 			TapeScratch& ts = reinterpret_cast<TapeScratch*>(shared)[warp];
+			const TapeLists lists{ ts.Value, ts.Material, ts.Start, kTapeCap };
 			float2* spill = reinterpret_cast<float2*>(shared + kWarps * sizeof(TapeScratch)) + warp * spill_pairs * 32 + lane;
 			const uint32_t n = min(tapes.Counters[0], tapes.PartCapacity), longs = min(tapes.Counters[4], kLongParts);
 			const float rootClip = __ldg(&prog.Nodes[0].ClipRadius);
@@ -248,8 +257,11 @@ namespace tg
 					const float r = 0.5f * sqrtf(wx * wx + wy * wy + wz * wz) + kTetraReach;
 					const float reach = TapeReach(r, fmaxf(fabsf(lo[0]), fabsf(hi[0])), fmaxf(fabsf(lo[1]), fabsf(hi[1])),
 						fmaxf(fabsf(lo[2]), fabsf(hi[2])), rootClip);
-					ok = BuildTape(code + base, part.Surface - base, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach, units, spill, 32,
-						ts, counts);
+					DistanceSource src;
+					const int quads = part.Surface - base;
+					src.In.Open(code + base, quads, ts.Window);
+					ok = quads <= 0xFFF0 && BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach,
+						units, spill, 32, lists, counts);
 				}
 				if (!ok) continue;
 				if (lane == 0 && counts.Sign) part.Box = box | (counts.Sign > 0 ? kBoxPositive : kBoxNegative);

@@ -10,6 +10,7 @@
 #include "tg_device.cuh"
 #include "tg_kernels.hpp"
 #include "tg_surface.cuh"
+#include "tg_tape.cuh"
 
 namespace tg
 {
@@ -220,7 +221,226 @@ namespace tg
 			return Mix(lo, hi, (float)((double)x + 0.5) / (float)size);
 		}
 
-		// One thread per brick of VoxExport's voxels: the whole tree's program at the centre
+		// The ball through the voxel centres [lo, hi], and the margin for rounding.  mix()
+		// rounds each centre separately, so the box is widened by a relative 1e-6 of its
+		// coordinates.
+		__device__ __forceinline__ void VoxBall(const VoxSpec& s, const int (&lo)[3], const int (&hi)[3], float scale, float (&c)[3], float& r,
+			float& margin)
+		{
+			const int size[3] = { s.SX, s.SY, s.SZ };
+			float clo[3], chi[3];
+#pragma unroll
+			for (int a = 0; a < 3; ++a)
+			{
+				const float u = VoxCentre(s.Min[a], s.Max[a], lo[a], size[a]);
+				const float v = VoxCentre(s.Min[a], s.Max[a], hi[a], size[a]);
+				const float slack = 1e-6f * (fabsf(u) + fabsf(v) + fabsf(s.Min[a]) + fabsf(s.Max[a]));
+				clo[a] = fminf(u, v) - slack;
+				chi[a] = fmaxf(u, v) + slack;
+			}
+			BallOf(clo, chi, c, r, margin, scale);
+		}
+
+		// VoxExport's test (magica.cpp:52-64) is on the whole tree (SDFNode::Eval), some
+		// hundreds of records.  Blocks of 64^3 voxels, then the 16^3 blocks in them that may
+		// hold a kept voxel, then the 4^3 boxes in those, are decided by a ball each, and every
+		// level shortens the tree's surface program for the next (tg_tape.cuh): a warp per
+		// block runs the program it was given at its 64 parts' centres.
+		constexpr int kVoxCoarse = 64, kVoxBlock = 16, kVoxFine = 4;
+		constexpr int kVoxCoarseCap = 2048, kVoxBlockCap = 192;
+		constexpr int kVoxWarps = 4, kVoxCtasPerSm = 6;
+
+		struct VoxGrid
+		{
+			int NX, NY, NZ;         // 64^3 blocks per axis
+		};
+
+		struct VoxState
+		{
+			uint2* Events;          // kVoxCoarseCap per 64^3 block: its tape
+			uint32_t* Counts;       // its length (kNoTape: none)
+			uint32_t* List;         // 16^3 blocks to look at: 64^3 block * 64 + part
+			uint32_t* Counters;     // their number, and how many are taken
+		};
+
+		// Part `part` (0..63, x fastest) of a block that starts at voxel `from` and has 4 x 4 x 4
+		// parts of `edge` voxels an axis; false when it lies outside the lattice (the box is then
+		// the nearest voxel).
+		__device__ __forceinline__ bool VoxPart(const VoxSpec& s, const int (&from)[3], int part, int edge, int (&lo)[3], int (&hi)[3])
+		{
+			const int size[3] = { s.SX, s.SY, s.SZ };
+			const int at[3] = { part & 3, (part >> 2) & 3, part >> 4 };
+			bool in = true;
+#pragma unroll
+			for (int a = 0; a < 3; ++a)
+			{
+				lo[a] = from[a] + at[a] * edge;
+				in = in && lo[a] < size[a];
+				lo[a] = min(lo[a], size[a] - 1);
+				hi[a] = min(lo[a] + edge - 1, size[a] - 1);
+			}
+			return in;
+		}
+
+		// The two balls of this lane in a block: parts lane and lane + 32.
+		struct VoxLane
+		{
+			float2 X, Y, Z, R, Margin;
+			bool In[2];
+		};
+
+		__device__ __forceinline__ VoxLane VoxLaneOf(const VoxSpec& s, const int (&from)[3], int edge, float scale)
+		{
+			VoxLane l;
+			float c[2][3], r[2], m[2];
+#pragma unroll
+			for (int j = 0; j < 2; ++j)
+			{
+				int lo[3], hi[3];
+				l.In[j] = VoxPart(s, from, (int)(threadIdx.x & 31) + 32 * j, edge, lo, hi);
+				VoxBall(s, lo, hi, scale, c[j], r[j], m[j]);
+			}
+			l.X = make_float2(c[0][0], c[1][0]);
+			l.Y = make_float2(c[0][1], c[1][1]);
+			l.Z = make_float2(c[0][2], c[1][2]);
+			l.R = make_float2(r[0], r[1]);
+			l.Margin = make_float2(m[0], m[1]);
+			return l;
+		}
+
+		__device__ __forceinline__ float VoxReach(const VoxLane& l, float rootClip)
+		{
+			return fmaxf(TapeReach(l.R.x, l.X.x, l.Y.x, l.Z.x, rootClip), TapeReach(l.R.y, l.X.y, l.Y.y, l.Z.y, rootClip));
+		}
+
+		// One warp per 64^3 block: bound by the latency of one pass over the whole tree.
+		__global__ void __launch_bounds__(32) VoxCoarseKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st, int spill_pairs)
+		{
+			extern __shared__ __align__(16) uint8_t shared[];
+			float4* window = reinterpret_cast<float4*>(shared);
+			uint2* value = reinterpret_cast<uint2*>(window + 64);
+			uint2* start = value + kVoxCoarseCap;
+			float2* spill = reinterpret_cast<float2*>(start + kMaxStack + 2) + threadIdx.x;
+			const int lane = (int)threadIdx.x, b = (int)blockIdx.x;
+			const int from[3] = { (b % vg.NX) * kVoxCoarse, ((b / vg.NX) % vg.NY) * kVoxCoarse, (b / (vg.NX * vg.NY)) * kVoxCoarse };
+			const float rootClip = fabsf(__ldg(&prog.Nodes[0].ClipRadius));
+			const VoxLane l = VoxLaneOf(s, from, kVoxBlock, rootClip);
+			SurfaceSource src;
+			src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, window);
+			TapeCounts counts;
+			const bool ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), LoadPairUnits(), spill, 32,
+				TapeLists{ value, nullptr, start, kVoxCoarseCap }, counts);
+			if (ok)
+				for (int i = lane; i < counts.Value; i += 32) st.Events[(int64_t)b * kVoxCoarseCap + i] = value[i];
+			if (lane == 0) st.Counts[b] = ok ? (uint32_t)counts.Value : kNoTape;
+#pragma unroll
+			for (int j = 0; j < 2; ++j)
+			{
+				const float d = j ? counts.Distance.y : counts.Distance.x, r = j ? l.R.y : l.R.x;
+				const float margin = (j ? l.Margin.y : l.Margin.x) + (j ? counts.Error.y : counts.Error.x);
+				const bool keep = l.In[j] && !(ok && fabsf(d) > r + s.Radius + margin);
+				const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+				uint32_t at = 0;
+				if (lane == 0 && kept) at = atomicAdd(st.Counters, (uint32_t)__popc(kept));
+				at = __shfl_sync(0xFFFFFFFFu, at, 0);
+				if (keep) st.List[at + (uint32_t)__popc(kept & ((1u << lane) - 1u))] = (uint32_t)b * 64u + (uint32_t)(lane + 32 * j);
+			}
+		}
+
+		// One warp per listed 16^3 block, drawn from a counter: its tape from its 64^3 block's,
+		// then the voxels of the 4^3 boxes that may hold a kept one, two a lane.
+		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxCtasPerSm) VoxFineKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
+			uint32_t* __restrict__ words, int spill_pairs)
+		{
+			extern __shared__ __align__(16) uint8_t shared[];
+			struct Scratch
+			{
+				float4 Window[64];
+				uint2 Heads[16], Value[kVoxBlockCap], Start[kMaxStack + 2];
+				float Axis[3][kVoxBlock];
+			};
+			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+			Scratch& sc = reinterpret_cast<Scratch*>(shared)[warp];
+			float2* spill = reinterpret_cast<float2*>(shared + kVoxWarps * sizeof(Scratch)) + warp * spill_pairs * 32 + lane;
+			const float4* code = prog.Code + prog.FullSurfaceCode;
+			auto load = [&](int q) { return __ldg(code + q); };
+			const float rootClip = fabsf(__ldg(&prog.Nodes[0].ClipRadius));
+			const PairUnits units = LoadPairUnits();
+			const int size[3] = { s.SX, s.SY, s.SZ };
+			const uint32_t n = st.Counters[0];
+			for (;;)
+			{
+				uint32_t item = 0;
+				if (lane == 0) item = atomicAdd(st.Counters + 1, 1u);
+				item = __shfl_sync(0xFFFFFFFFu, item, 0);
+				if (item >= n) break;
+				const uint32_t entry = __ldg(st.List + item);
+				const int b = (int)(entry >> 6), part = (int)(entry & 63u);
+				const int from[3] = { (b % vg.NX) * kVoxCoarse + (part & 3) * kVoxBlock, ((b / vg.NX) % vg.NY) * kVoxCoarse + ((part >> 2) & 3) * kVoxBlock,
+					(b / (vg.NX * vg.NY)) * kVoxCoarse + (part >> 4) * kVoxBlock };
+				const uint32_t given = __ldg(st.Counts + b);
+				const uint2* events = st.Events + (int64_t)b * kVoxCoarseCap;
+				__syncwarp();       // the previous block is done with the scratch
+				for (int i = lane; i < 3 * kVoxBlock; i += 32)
+				{
+					const int a = i / kVoxBlock, q = i % kVoxBlock;
+					sc.Axis[a][q] = VoxCentre(s.Min[a], s.Max[a], min(from[a] + q, size[a] - 1), size[a]);
+				}
+				const VoxLane l = VoxLaneOf(s, from, kVoxFine, rootClip);
+				bool ok = false;
+				TapeCounts counts;
+				if (given != kNoTape)
+				{
+					SurfaceEventSource src;
+					src.Open(code, events, (int)given, sc.Window, sc.Heads);
+					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32,
+						TapeLists{ sc.Value, nullptr, sc.Start, kVoxBlockCap }, counts);
+				}
+				__syncwarp();
+				unsigned kept[2];
+#pragma unroll
+				for (int j = 0; j < 2; ++j)
+				{
+					const float d = j ? counts.Distance.y : counts.Distance.x, r = j ? l.R.y : l.R.x;
+					const float margin = (j ? l.Margin.y : l.Margin.x) + (j ? counts.Error.y : counts.Error.x);
+					kept[j] = __ballot_sync(0xFFFFFFFFu, l.In[j] && !(ok && fabsf(d) > r + s.Radius + margin));
+				}
+				const int vx = lane & 3, vy = (lane >> 2) & 3, vz = lane >> 4;
+				while (kept[0] | kept[1])
+				{
+					const int half = kept[0] ? 0 : 1;
+					const int box = __ffs((int)kept[half]) - 1 + 32 * half;
+					kept[half] &= kept[half] - 1u;
+					const int ox = (box & 3) * kVoxFine + vx, oy = ((box >> 2) & 3) * kVoxFine + vy, oz = (box >> 4) * kVoxFine + vz;
+					const float2 px[1] = { make_float2(sc.Axis[0][ox], sc.Axis[0][ox]) }, py[1] = { make_float2(sc.Axis[1][oy], sc.Axis[1][oy]) };
+					const float2 pz[1] = { make_float2(sc.Axis[2][oz], sc.Axis[2][oz + 2]) };
+					float2 d[1];
+					if (given == kNoTape) d[0] = RunWholeSurfacePair(prog.Code, prog.FullSurfaceCode, px[0], py[0], pz[0], spill, 32);
+					else
+						RunSurfaceTapePairs<1>(load, 0, [&](uint32_t e) { return ok ? sc.Value[e] : __ldg(events + e); },
+							ok ? (uint32_t)counts.Value : given, px, py, pz, units, d, spill, 32);
+#pragma unroll
+					for (int j = 0; j < 2; ++j)
+					{
+						const int x = from[0] + ox, y = from[1] + oy, z = from[2] + oz + 2 * j;
+						const bool keep = x < s.SX && y < s.SY && z < s.SZ && fabsf(j ? d[0].y : d[0].x) <= s.Radius;
+						const unsigned bits = __ballot_sync(0xFFFFFFFFu, keep);
+						// A row of four voxels of the box is four neighbouring lanes.
+						const uint32_t row = (bits >> (lane & 28)) & 15u;
+						if (vx == 0 && row)
+						{
+							const int64_t t = x + (int64_t)s.SX * (y + (int64_t)s.SY * z);
+							const int shift = (int)(t & 31);
+							atomicOr(words + (t >> 5), row << shift);
+							if (shift > 28 && (row >> (32 - shift))) atomicOr(words + (t >> 5) + 1, row >> (32 - shift));
+						}
+					}
+				}
+			}
+		}
+
+		// Trees whose programs cannot be shortened (a brush that is not 1-Lipschitz, rotations that
+		// are not unit quaternions): one thread per brick of VoxExport's voxels: the whole tree's program at the centre
 		// of the ball through the brick's voxel centres decides (a tree with a brush that is
 		// not 1-Lipschitz keeps every brick).  mix() rounds each centre separately, so the
 		// box is widened by a relative 1e-6 of its coordinates.
@@ -256,7 +476,7 @@ namespace tg
 			if (keep) atomicOr(brick_bits + (b >> 5), 1u << (b & 31));
 		}
 
-		// VoxExport's test (magica.cpp:52-64): the voxel centre mix(Min, Max, (x + .5) / Size)
+		// VoxExport's test at every voxel of the bricks kept: the voxel centre mix(Min, Max, (x + .5) / Size)
 		// on the whole tree (SDFNode::Eval), kept when |d| <= Radius.
 		__global__ void __launch_bounds__(128) VoxFlagsKernel(DeviceProgram prog, VoxSpec s, VoxelBricks vb,
 			const uint32_t* __restrict__ brick_bits, uint32_t* __restrict__ words)
@@ -285,6 +505,23 @@ namespace tg
 			}
 			const unsigned ballot = __ballot_sync(0xFFFFFFFFu, keep);
 			if ((threadIdx.x & 31) == 0 && t < s.Total) words[t >> 5] = ballot;
+		}
+
+		__global__ void __launch_bounds__(128) VoxListKernel(VoxSpec s, const uint32_t* __restrict__ words, const uint32_t* __restrict__ base,
+			int64_t n, int color, int4* __restrict__ out)
+		{
+			const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+			if (w >= n) return;
+			uint32_t m = __ldg(words + w);
+			if (!m) return;
+			uint32_t at = __ldg(base + w);
+			const int slice = s.SX * s.SY;
+			while (m)
+			{
+				const int i = (int)(w * 32) + __ffs((int)m) - 1;
+				m &= m - 1u;
+				out[at++] = make_int4(i % s.SX, (i % slice) / s.SX, i / slice, color);
+			}
 		}
 	}
 
@@ -346,24 +583,75 @@ namespace tg
 		return cudaGetLastError();
 	}
 
-	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, uint32_t* brick_bits, uint32_t* words, cudaStream_t stream)
+	static VoxGrid VoxGridOf(const VoxSpec& s)
+	{
+		return { (s.SX + kVoxCoarse - 1) / kVoxCoarse, (s.SY + kVoxCoarse - 1) / kVoxCoarse, (s.SZ + kVoxCoarse - 1) / kVoxCoarse };
+	}
+
+	static bool VoxByBlocks(const DeviceProgram& prog) { return prog.Lipschitz && (prog.Form & kFormPrunable); }
+
+	size_t VoxScratchBytes(const DeviceProgram& prog, const VoxSpec& s)
+	{
+		if (s.Total <= 0) return 16;
+		if (!VoxByBlocks(prog)) return VoxelBrickWords(s.SX, s.SY, s.SZ) * sizeof(uint32_t);
+		const VoxGrid vg = VoxGridOf(s);
+		const size_t blocks = (size_t)vg.NX * vg.NY * vg.NZ;
+		return blocks * (kVoxCoarseCap * sizeof(uint2) + sizeof(uint32_t) + 64 * sizeof(uint32_t)) + 4 * sizeof(uint32_t);
+	}
+
+	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream)
 	{
 		if (s.Total <= 0) return cudaSuccess;
-		const VoxelBricks vb = BricksOf(s.SX, s.SY, s.SZ);
-		const int nb = vb.NX * vb.NY * vb.NZ;
-		cudaError_t e = cudaMemsetAsync(brick_bits, 0, VoxelBrickWords(s.SX, s.SY, s.SZ) * 4, stream);
-		if (e != cudaSuccess) return e;
-		const size_t smem = DistanceSpillBytes(prog, 128);
-		if (smem > 48 * 1024)
+		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
+		if (!VoxByBlocks(prog))
 		{
-			e = cudaFuncSetAttribute(VoxFlagsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-			if (e == cudaSuccess) e = cudaFuncSetAttribute(VoxBricksKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			uint32_t* brick_bits = static_cast<uint32_t*>(scratch);
+			const VoxelBricks vb = BricksOf(s.SX, s.SY, s.SZ);
+			const int nb = vb.NX * vb.NY * vb.NZ;
+			cudaError_t e = cudaMemsetAsync(brick_bits, 0, VoxelBrickWords(s.SX, s.SY, s.SZ) * 4, stream);
 			if (e != cudaSuccess) return e;
+			const size_t smem = DistanceSpillBytes(prog, 128);
+			if (smem > 48 * 1024)
+			{
+				e = cudaFuncSetAttribute(VoxFlagsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+				if (e == cudaSuccess) e = cudaFuncSetAttribute(VoxBricksKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+				if (e != cudaSuccess) return e;
+			}
+			VoxBricksKernel<<<Blocks(nb, 128), 128, smem, stream>>>(prog, s, vb, brick_bits);
+			e = cudaGetLastError();
+			if (e != cudaSuccess) return e;
+			VoxFlagsKernel<<<Blocks(s.Total, 128), 128, smem, stream>>>(prog, s, vb, brick_bits, words);
+			return cudaGetLastError();
 		}
-		VoxBricksKernel<<<Blocks(nb, 128), 128, smem, stream>>>(prog, s, vb, brick_bits);
+		const VoxGrid vg = VoxGridOf(s);
+		const int64_t blocks = (int64_t)vg.NX * vg.NY * vg.NZ;
+		VoxState st;
+		st.Events = static_cast<uint2*>(scratch);
+		st.Counts = reinterpret_cast<uint32_t*>(st.Events + blocks * kVoxCoarseCap);
+		st.List = st.Counts + blocks;
+		st.Counters = st.List + blocks * 64;
+		cudaError_t e = cudaMemsetAsync(words, 0, (size_t)((s.Total + 31) / 32) * 4, stream);
+		if (e == cudaSuccess) e = cudaMemsetAsync(st.Counters, 0, 2 * sizeof(uint32_t), stream);
+		if (e != cudaSuccess) return e;
+		const size_t coarse = 64 * sizeof(float4) + (kVoxCoarseCap + kMaxStack + 2) * sizeof(uint2) + (size_t)depth * 32 * sizeof(float2);
+		// The kernel's own scratch struct: window, events' heads, tape, stack starts, axes.
+		const size_t warp = 64 * sizeof(float4) + (16 + kVoxBlockCap + kMaxStack + 2) * sizeof(uint2) + 3 * kVoxBlock * sizeof(float);
+		const size_t fine = kVoxWarps * (warp + (size_t)depth * 32 * sizeof(float2));
+		if (coarse > 48 * 1024) e = cudaFuncSetAttribute(VoxCoarseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coarse);
+		if (e == cudaSuccess && fine > 48 * 1024) e = cudaFuncSetAttribute(VoxFineKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fine);
+		if (e != cudaSuccess) return e;
+		VoxCoarseKernel<<<(unsigned)blocks, 32, coarse, stream>>>(prog, s, vg, st, depth);
 		e = cudaGetLastError();
 		if (e != cudaSuccess) return e;
-		VoxFlagsKernel<<<Blocks(s.Total, 128), 128, smem, stream>>>(prog, s, vb, brick_bits, words);
+		VoxFineKernel<<<sms * kVoxCtasPerSm, kVoxWarps * 32, fine, stream>>>(prog, s, vg, st, words, depth);
+		return cudaGetLastError();
+	}
+
+	cudaError_t LaunchVoxList(const VoxSpec& s, const uint32_t* words, const uint32_t* word_base, int color, int4* out, cudaStream_t stream)
+	{
+		const int64_t n = (s.Total + 31) / 32;
+		if (n <= 0) return cudaSuccess;
+		VoxListKernel<<<Blocks(n, 128), 128, 0, stream>>>(s, words, word_base, n, color, out);
 		return cudaGetLastError();
 	}
 }

@@ -19,6 +19,7 @@ namespace tg
 		int FullSurfaceCode;    // the whole tree's surface program
 		int Lipschitz;          // every brush 1-Lipschitz
 		int Form;               // kForm* (tg_layout.hpp): what may be left out of its programs
+		int CodeQuads;          // quads of Code; the whole tree's surface program is the last in it
 	};
 
 	// Pinhole camera: pixel (x, y) looks along forward + right*u + up*v with
@@ -266,8 +267,11 @@ namespace tg
 	// Refined point of each listed cell (*count of them, at most `capacity`).
 	cudaError_t LaunchCloudRefine(const DeviceProgram& prog, const CloudSpec& s, const uint32_t* cells, const uint32_t* count,
 		uint32_t capacity, int iterations, float* points, cudaStream_t stream);
-	// One bit per voxel: |full-tree distance at the centre| <= Radius.
-	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, uint32_t* brick_bits, uint32_t* words, cudaStream_t stream);
+	// One bit per voxel: |full-tree distance at the centre| <= Radius.  scratch: VoxScratchBytes.
+	size_t VoxScratchBytes(const DeviceProgram& prog, const VoxSpec& s);
+	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream);
+	// The flagged voxels in order, each x, y, z, color; word_base: LaunchExclusiveScan of the words.
+	cudaError_t LaunchVoxList(const VoxSpec& s, const uint32_t* words, const uint32_t* word_base, int color, int4* out, cudaStream_t stream);
 }
 
 namespace tg

@@ -33,7 +33,7 @@ namespace tg
 	// blend's sum with its zero term turns -0 into +0.
 	enum : uint32_t { OpTapeNegate = 40, OpTapeAddZero = 41 };
 
-	constexpr int kTapeCap = 128;               // events of a list while it is built
+	constexpr int kTapeCap = 128;               // events of a brick's list while it is built
 	constexpr uint32_t kNoTape = 0xFFFFu;       // an event count: run the cell's whole program
 
 	__device__ __forceinline__ uint32_t ProgramHead(float word) { return __float_as_uint(word) & kTapeHead; }
@@ -224,6 +224,29 @@ namespace tg
 		return d[0];
 	}
 
+	// A brush's distance in a surface program (RunSurfacePair's step): T the translation and
+	// scale, Q the inverse quaternion as (w, x, y, z).
+	__device__ __forceinline__ float2 SurfaceBrushStep(uint32_t op, const float4& h, const float4& Q, const float4& T, float2 px, float2 py,
+		float2 pz, const PairUnits& u)
+	{
+		const float2 vx = Sub2(px, Pair(T.x), u), vy = Sub2(py, Pair(T.y), u), vz = Sub2(pz, Pair(T.z), u);
+		float2 ux, uy, uz, wx, wy, wz;
+		CrossPair(Q.y, Q.z, Q.w, vx, vy, vz, ux, uy, uz, u);
+		CrossPair(Q.y, Q.z, Q.w, ux, uy, uz, wx, wy, wz, u);
+		float2 lx = Add2(vx, Mul2(Add2(Mul2(ux, Pair(Q.x), u), wx, u), Pair(2.0f), u), u);
+		float2 ly = Add2(vy, Mul2(Add2(Mul2(uy, Pair(Q.x), u), wy, u), Pair(2.0f), u), u);
+		float2 lz = Add2(vz, Mul2(Add2(Mul2(uz, Pair(Q.x), u), wz, u), Pair(2.0f), u), u);
+		const bool scaled = T.w != 1.0f;    // x / 1 and x * 1 are x exactly
+		if (scaled)
+		{
+			lx = make_float2(lx.x / T.w, lx.y / T.w);
+			ly = make_float2(ly.x / T.w, ly.y / T.w);
+			lz = make_float2(lz.x / T.w, lz.y / T.w);
+		}
+		const float2 d = TapeBrush2(op, h, lx, ly, lz, u);
+		return scaled ? Mul2(d, Pair(T.w), u) : d;
+	}
+
 	// SDFNode::Eval at NP pairs of points (RunSurfacePair's steps) by the surface records a
 	// tape names, those of the surface program at `base`.
 	template<int NP, typename Load, typename Event>
@@ -254,27 +277,11 @@ namespace tg
 					++depth;
 				}
 				const float4 h = load(at), Q = load(at + 1), T = load(at + 2);
-				const bool scaled = T.w != 1.0f;    // x / 1 and x * 1 are x exactly
 #pragma unroll
 				for (int j = 0; j < NP; ++j)
 				{
 					left[j] = acc[j];
-					const float2 vx = Sub2(px[j], Pair(T.x), u), vy = Sub2(py[j], Pair(T.y), u), vz = Sub2(pz[j], Pair(T.z), u);
-					// The quad holds the inverse quaternion as (w, x, y, z).
-					float2 ux, uy, uz, wx, wy, wz;
-					CrossPair(Q.y, Q.z, Q.w, vx, vy, vz, ux, uy, uz, u);
-					CrossPair(Q.y, Q.z, Q.w, ux, uy, uz, wx, wy, wz, u);
-					float2 lx = Add2(vx, Mul2(Add2(Mul2(ux, Pair(Q.x), u), wx, u), Pair(2.0f), u), u);
-					float2 ly = Add2(vy, Mul2(Add2(Mul2(uy, Pair(Q.x), u), wy, u), Pair(2.0f), u), u);
-					float2 lz = Add2(vz, Mul2(Add2(Mul2(uz, Pair(Q.x), u), wz, u), Pair(2.0f), u), u);
-					if (scaled)
-					{
-						lx = make_float2(lx.x / T.w, lx.y / T.w);
-						ly = make_float2(ly.x / T.w, ly.y / T.w);
-						lz = make_float2(lz.x / T.w, lz.y / T.w);
-					}
-					acc[j] = TapeBrush2(op, h, lx, ly, lz, u);
-					if (scaled) acc[j] = Mul2(acc[j], Pair(T.w), u);
+					acc[j] = SurfaceBrushStep(op, h, Q, T, px[j], py[j], pz[j], u);
 				}
 				if (e >= count) break;
 				if (!(head & RecThenSet)) continue;
@@ -397,14 +404,198 @@ namespace tg
 		return macc;
 	}
 
-	// The warp's scratch while it builds a tape.
-	struct TapeScratch
+	// A program read by a whole warp through a window in shared memory, 32 quads at a time,
+	// the next 32 in flight: read one by one from memory, every record's first use waited for
+	// L2, and a program of some hundred records held its warp longer than all others took
+	// together.
+	struct WindowReader
 	{
-		uint2 Value[kTapeCap];              // events of the distance
-		uint2 Material[kTapeCap];           // events of the material walk
-		uint2 Start[kMaxStack + 1];         // each operand on the stack: its first events
-		uint2 Unused;
-		float4 Window[64];                  // the records around the one being run
+		const float4* Code;
+		int Quads;
+		float4* Window;         // 64 quads: [32 * Chunk, 32 * Chunk + 64)
+		int Chunk;
+		float4 Ahead;           // this lane's quad of the 32 after those
+
+		__device__ __forceinline__ float4 Fetch(int q) const { return __ldg(Code + min(q, Quads - 1)); }
+		__device__ __forceinline__ void Open(const float4* code, int quads, float4* window)
+		{
+			const int lane = (int)(threadIdx.x & 31);
+			Code = code;
+			Quads = quads;
+			Window = window;
+			Chunk = 0;
+			Window[lane] = Fetch(lane);
+			Window[lane + 32] = Fetch(lane + 32);
+			Ahead = Fetch(lane + 64);
+			__syncwarp();
+		}
+		// Makes the record at pc readable: at most 33 quads from pc's chunk on.
+		__device__ __forceinline__ void Seek(int pc)
+		{
+			const int lane = (int)(threadIdx.x & 31);
+			while (Chunk < (pc >> 5))
+			{
+				__syncwarp();
+				Window[(Chunk & 1) * 32 + lane] = Ahead;
+				++Chunk;
+				Ahead = Fetch(32 * Chunk + 64 + lane);
+				__syncwarp();
+			}
+		}
+		__device__ __forceinline__ float4 Load(int q) const { return Window[q & 63]; }
+	};
+
+	// What BuildTape reads: the records of a program in order, each with its event.
+	//
+	// A cell's distance program; events name the surface records too (the same brushes and
+	// operators in the same order, a brush 4 quads and an operator 1).
+	struct DistanceSource
+	{
+		WindowReader In;
+		int Pc = 0, Surface = 0;
+
+		__device__ __forceinline__ uint32_t Head()
+		{
+			In.Seek(Pc);
+			return ProgramHead(In.Load(Pc).x);
+		}
+		__device__ __forceinline__ uint2 Event(uint32_t head) const { return make_uint2(((uint32_t)Pc << 16) | (head & ~RecThenSet), (uint32_t)Surface); }
+		__device__ __forceinline__ float Operand() const { return In.Load(Pc).y; }
+		__device__ __forceinline__ void Advance(uint32_t head)
+		{
+			Pc += DistanceRecordQuads(head);
+			Surface += (head & 0xFFu) <= OpPlane ? 4 : 1;
+		}
+		// The brush's distance at the two points, and the size its float error goes with.
+		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
+		{
+			const float2 x[1] = { px }, y[1] = { py }, z[1] = { pz };
+			float2 qx[1], qy[1], qz[1], d[1];
+			float4 h;
+			BrushStep<1>([&](int q) { return In.Load(q); }, Pc, head, x, y, z, u, qx, qy, qz, h, d);
+			const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
+			size = make_float2(fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(d[0].x),
+				fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(d[0].y));
+			return d[0];
+		}
+	};
+
+	__device__ __forceinline__ float2 SurfaceBrushSize(float4 h, float4 T, float2 px, float2 py, float2 pz, float2 d)
+	{
+		const float sizes = (fabsf(h.y) + fabsf(h.z) + fabsf(h.w)) * fabsf(T.w) + fabsf(T.x) + fabsf(T.y) + fabsf(T.z);
+		return make_float2(fabsf(px.x) + fabsf(py.x) + fabsf(pz.x) + sizes + fabsf(d.x),
+			fabsf(px.y) + fabsf(py.y) + fabsf(pz.y) + sizes + fabsf(d.y));
+	}
+
+	// A surface program (stencils' masks are passed over: they change no distance).
+	struct SurfaceSource
+	{
+		WindowReader In;
+		int Pc = 0;
+
+		__device__ __forceinline__ uint32_t Head()
+		{
+			for (;;)
+			{
+				In.Seek(Pc);
+				const float4 h = In.Load(Pc);
+				const uint32_t head = __float_as_uint(h.x) & (0xFFu | RecThenSet);
+				if ((head & 0xFFu) != OpMaskBegin) return head;
+				Pc += 1 + (int)__float_as_uint(h.y);
+			}
+		}
+		__device__ __forceinline__ uint2 Event(uint32_t head) const { return make_uint2(head & ~RecThenSet, (uint32_t)Pc); }
+		__device__ __forceinline__ float Operand() const { return In.Load(Pc).y; }
+		__device__ __forceinline__ void Advance(uint32_t head) { Pc += (head & 0xFFu) <= OpPlane ? 4 : 1; }
+		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
+		{
+			const float4 h = In.Load(Pc), T = In.Load(Pc + 2);
+			const float2 d = SurfaceBrushStep(head & 0xFFu, h, In.Load(Pc + 1), T, px, py, pz, u);
+			size = SurfaceBrushSize(h, T, px, py, pz, d);
+			return d;
+		}
+	};
+
+	// The surface records that a tape of a larger box has left: eight events at a time, four
+	// quads each, with the next eight in flight.
+	struct SurfaceEventSource
+	{
+		const float4* Code;     // the surface program
+		const uint2* Events;
+		int Count;
+		float4* Window;         // 16 events x 4 quads
+		uint2* Heads;           // 16 events
+		int At = 0, Chunk = 0;
+		float4 Ahead;           // of this lane's event of the chunk after the two in the window,
+		uint2 AheadEvent, NextEvent;    // its event, and that of the chunk after it
+
+		__device__ __forceinline__ uint2 FetchEvent(int chunk) const
+		{
+			const int e = chunk * 8 + (int)((threadIdx.x & 31) >> 2);
+			return e < Count ? __ldg(Events + e) : make_uint2(0u, 0u);
+		}
+		__device__ __forceinline__ float4 FetchQuad(uint2 ev) const
+		{
+			const int q = (int)(threadIdx.x & 3);
+			const uint32_t op = ev.x & 0xFFu;
+			const bool brush = op >= OpSphere && op <= OpPlane;
+			return brush || (q == 0 && op != 0u && op < OpTapeNegate) ? __ldg(Code + ev.y + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+		}
+		__device__ __forceinline__ void Put(int half, uint2 ev, float4 quad)
+		{
+			const int lane = (int)(threadIdx.x & 31);
+			Window[half * 32 + lane] = quad;
+			if ((lane & 3) == 0) Heads[half * 8 + (lane >> 2)] = ev;
+		}
+		__device__ __forceinline__ void Open(const float4* code, const uint2* events, int count, float4* window, uint2* heads)
+		{
+			Code = code;
+			Events = events;
+			Count = count;
+			Window = window;
+			Heads = heads;
+			const uint2 e0 = FetchEvent(0), e1 = FetchEvent(1);
+			AheadEvent = FetchEvent(2);
+			NextEvent = FetchEvent(3);
+			Put(0, e0, FetchQuad(e0));
+			Put(1, e1, FetchQuad(e1));
+			Ahead = FetchQuad(AheadEvent);
+			__syncwarp();
+		}
+		__device__ __forceinline__ uint32_t Head()
+		{
+			while (Chunk < (At >> 3))
+			{
+				__syncwarp();
+				Put(Chunk & 1, AheadEvent, Ahead);
+				++Chunk;
+				AheadEvent = NextEvent;
+				Ahead = FetchQuad(AheadEvent);
+				NextEvent = FetchEvent(Chunk + 3);
+				__syncwarp();
+			}
+			return At < Count ? Heads[At & 15].x & 0xFFFFu : OpStop;
+		}
+		__device__ __forceinline__ float4 Quad(int q) const { return Window[(At & 15) * 4 + q]; }
+		__device__ __forceinline__ uint2 Event(uint32_t head) const { return make_uint2(head & ~RecThenSet, Heads[At & 15].y); }
+		__device__ __forceinline__ float Operand() const { return Quad(0).y; }
+		__device__ __forceinline__ void Advance(uint32_t) { ++At; }
+		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
+		{
+			const float4 h = Quad(0), T = Quad(2);
+			const float2 d = SurfaceBrushStep(head & 0xFFu, h, Quad(1), T, px, py, pz, u);
+			size = SurfaceBrushSize(h, T, px, py, pz, d);
+			return d;
+		}
+	};
+
+	// The lists a warp writes its tape to, in shared memory.
+	struct TapeLists
+	{
+		uint2* Value;           // events of the distance
+		uint2* Material;        // events of the material walk (null: not wanted)
+		uint2* Start;           // each operand on the stack: its first events (kMaxStack + 1)
+		int Cap;                // events a list holds
 	};
 
 	struct TapeCounts
@@ -412,38 +603,26 @@ namespace tg
 		int Value, Material;
 		bool Same;              // no difference was decided by its right operand: one list serves both
 		int Sign;               // 1 or -1: the program keeps that sign in the box; 0: it may not
+		float2 Distance;        // the program's values at this lane's two points,
+		float2 Error;           // and the part of their rounding that grows with the operands
 	};
 
-	// Builds the tape of the distance program of `quads` records at `code`, stop included, for
-	// a box, by all lanes of a warp: lane l's pair of points are centres of two balls, and the
-	// balls of all lanes cover the box.  `reach` is how far the difference of two operands can
-	// move inside a ball, with the fixed part of the rounding (TapeReach); the part that grows
-	// with the operands' own coordinates (brushes far from the box) is added here: each brush's
-	// float error is at most a few roundings of its local coordinates and sizes.  Returns false
-	// when a list outgrows its scratch.
-	//
-	// The records come through a window in shared memory, 32 quads at a time, the next 32 in
-	// flight: read one by one from memory, every record's first use waited for L2, and a
-	// program of some hundred records held its warp longer than all others took together.
-	__device__ __forceinline__ bool BuildTape(const float4* __restrict__ code, int quads, float2 px, float2 py, float2 pz, float reach,
-		const PairUnits& u, float2* spill, int stride, TapeScratch& ts, TapeCounts& out)
+	// Builds the tape of a program for a box, by all lanes of a warp: lane l's pair of points
+	// are centres of two balls, and the balls of all lanes cover the box.  `reach` is how far
+	// the difference of two operands can move inside a ball, with the fixed part of the
+	// rounding (TapeReach); the part that grows with the operands' own coordinates (brushes
+	// far from the box) is added here: each brush's float error is at most a few roundings of
+	// its local coordinates and sizes.  Returns false when a list outgrows its room.
+	template<bool Materials, typename Source>
+	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, const PairUnits& u, float2* spill,
+		int stride, const TapeLists& ts, TapeCounts& out)
 	{
-		const float2 x1[1] = { px }, y1[1] = { py }, z1[1] = { pz };
 		const int lane = (int)(threadIdx.x & 31);
 		float2 acc = make_float2(0.0f, 0.0f), left = acc;
 		float2 size = make_float2(0.0f, 0.0f);
-		int depth = 0, pc = 0, surface = 0;
+		int depth = 0;
 		int nv = 0, nm = 0;
 		bool same = true;
-		if (quads > 0xFFF0) return false;
-		// The window holds quads [32 * chunk, 32 * chunk + 64); `ahead` the 32 after those.
-		int chunk = 0;
-		auto fetch = [&](int q) { return __ldg(code + min(q, quads - 1)); };
-		ts.Window[lane] = fetch(lane);
-		ts.Window[lane + 32] = fetch(lane + 32);
-		float4 ahead = fetch(lane + 64);
-		__syncwarp();
-		auto load = [&](int q) { return ts.Window[q & 63]; };
 		// [from, to) of a list moves down to `down`.
 		auto move = [&](uint2* list, int down, int from, int to)
 		{
@@ -458,18 +637,9 @@ namespace tg
 		};
 		for (int guard = 0; guard < (1 << 24); ++guard)
 		{
-			if (nv + 4 > kTapeCap || nm + 4 > kTapeCap) return false;
-			if ((pc >> 5) != chunk)
-			{
-				__syncwarp();
-				ts.Window[(chunk & 1) * 32 + lane] = ahead;
-				++chunk;
-				ahead = fetch(32 * chunk + 64 + lane);
-				__syncwarp();
-			}
-			uint32_t head = ProgramHead(load(pc).x);
+			if (nv + 4 > ts.Cap || (Materials && nm + 4 > ts.Cap)) return false;
+			uint32_t head = src.Head();
 			uint32_t op = head & 0xFFu;
-			uint32_t event = ((uint32_t)pc << 16) | (head & ~RecThenSet);
 			int rv = nv, rm = nm;       // first events of the right operand
 			if (op >= OpSphere && op <= OpPlane)
 			{
@@ -481,21 +651,16 @@ namespace tg
 					ts.Start[depth] = make_uint2((uint32_t)nv, (uint32_t)nm);
 					++depth;
 				}
-				ts.Value[nv++] = make_uint2(event, (uint32_t)surface);
-				ts.Material[nm++] = make_uint2(event, (uint32_t)surface);
-				float2 qx[1], qy[1], qz[1], d[1];
-				float4 h;
-				BrushStep<1>(load, pc, head, x1, y1, z1, u, qx, qy, qz, h, d);
-				acc = d[0];
-				const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
-				size.x = fmaxf(size.x, fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(acc.x));
-				size.y = fmaxf(size.y, fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(acc.y));
-				pc += DistanceRecordQuads(head);
-				surface += 4;
+				const uint2 ev = src.Event(head);
+				ts.Value[nv++] = ev;
+				if (Materials) ts.Material[nm++] = ev;
+				float2 own;
+				acc = src.Brush(head, px, py, pz, u, own);
+				size = make_float2(fmaxf(size.x, own.x), fmaxf(size.y, own.y));
+				src.Advance(head);
 				if (!thenSet) continue;
-				head = ProgramHead(load(pc).x);
+				head = src.Head();
 				op = head & 0xFFu;
-				event = ((uint32_t)pc << 16) | head;
 			}
 			else if (op >= OpUnion && op <= OpBlendDiff)
 			{
@@ -504,20 +669,22 @@ namespace tg
 				rv = (int)r.x; rm = (int)r.y;
 				left = spill[(depth - 1) * stride];
 			}
-			else if (op == OpFlate)
+			else if (op == OpStop)
 			{
-				ts.Value[nv++] = make_uint2(event, (uint32_t)surface);
-				ts.Material[nm++] = make_uint2(event, (uint32_t)surface);
-				acc = Sub2(acc, Pair(load(pc).y), u);
-				++pc;
-				++surface;
-				continue;
+				break;
 			}
 			else
 			{
-				break;   // OpStop
+				// Flate, or what an earlier tape put in.
+				const uint2 ev = src.Event(head);
+				ts.Value[nv++] = ev;
+				if (Materials) ts.Material[nm++] = ev;
+				if (op == OpFlate) acc = Sub2(acc, Pair(src.Operand()), u);
+				else acc = op == OpTapeNegate ? make_float2(-acc.x, -acc.y) : make_float2(acc.x + 0.0f, acc.y + 0.0f);
+				src.Advance(head);
+				continue;
 			}
-			const float k = load(pc).y;
+			const float k = src.Operand();
 			const bool blend = op >= OpBlendUnion;
 			const bool diff = op == OpDiff || op == OpBlendDiff;
 			const bool unions = op == OpUnion || op == OpBlendUnion;
@@ -530,13 +697,17 @@ namespace tg
 			const bool leftWins = __all_sync(0xFFFFFFFFu, decides && s.x > t.x && s.y > t.y);
 			const bool rightWins = __all_sync(0xFFFFFFFFu, decides && s.x < -t.x && s.y < -t.y);
 			const uint2 l = ts.Start[depth - 1];
-			const uint2 set = make_uint2(event, (uint32_t)surface);
+			const uint2 set = src.Event(head);
 			const uint2 addZero = make_uint2(OpTapeAddZero, 0u);
 			if (leftWins)
 			{
 				nv = rv;
 				nm = rm;
-				if (blend && !unions) { ts.Value[nv++] = addZero; ts.Material[nm++] = addZero; }
+				if (blend && !unions)
+				{
+					ts.Value[nv++] = addZero;
+					if (Materials) ts.Material[nm++] = addZero;
+				}
 			}
 			else
 			{
@@ -553,29 +724,33 @@ namespace tg
 					if (nv - rv == 1 && (ts.Value[rv].x & 0xFFu) <= OpPlane) ts.Value[rv].x |= RecThenSet;
 					ts.Value[nv++] = set;
 				}
-				if (rightWins && !diff)
+				if (Materials)
 				{
-					move(ts.Material, (int)l.y, rm, nm);
-					nm -= rm - (int)l.y;
-					if (blend && !unions) ts.Material[nm++] = addZero;
-				}
-				else
-				{
-					if (rightWins) same = false;
-					if (nm - rm == 1 && (ts.Material[rm].x & 0xFFu) <= OpPlane) ts.Material[rm].x |= RecThenSet;
-					ts.Material[nm++] = set;
+					if (rightWins && !diff)
+					{
+						move(ts.Material, (int)l.y, rm, nm);
+						nm -= rm - (int)l.y;
+						if (blend && !unions) ts.Material[nm++] = addZero;
+					}
+					else
+					{
+						if (rightWins) same = false;
+						if (nm - rm == 1 && (ts.Material[rm].x & 0xFFu) <= OpPlane) ts.Material[rm].x |= RecThenSet;
+						ts.Material[nm++] = set;
+					}
 				}
 			}
 			acc = TapeSet2(op, left, acc, k);
-			++pc;
-			++surface;
+			src.Advance(head);
 		}
 		__syncwarp();
 		out.Value = nv;
 		out.Material = nm;
 		out.Same = same;
+		out.Distance = acc;
+		out.Error = make_float2(2e-5f * size.x, 2e-5f * size.y);
 		// |f| beyond a ball's radius (half the reach covers it) at every centre: no sign change.
-		const float2 far = make_float2(0.5f * reach + 2e-5f * size.x, 0.5f * reach + 2e-5f * size.y);
+		const float2 far = make_float2(0.5f * reach + out.Error.x, 0.5f * reach + out.Error.y);
 		out.Sign = __all_sync(0xFFFFFFFFu, acc.x > far.x && acc.y > far.y) ? 1
 			: __all_sync(0xFFFFFFFFu, acc.x < -far.x && acc.y < -far.y) ? -1 : 0;
 		return true;

@@ -219,15 +219,15 @@ def last_export_timing():
 
 
 class _HostBlocks:
-    """Owns the host blocks of one tg_mesh (pinned memory the library reuses): they go back
-    to the library with tg_mesh_free once no array views them."""
+    """Owns the host blocks of one tg_mesh or tg_voxels (pinned memory the library reuses):
+    they go back to the library with its free function once no array views them."""
 
-    def __init__(self, hm: _lib.HostMesh):
-        self.hm = hm
+    def __init__(self, blocks, free="tg_mesh_free"):
+        self.blocks, self.free = blocks, free
 
     def __del__(self):
         try:
-            load().tg_mesh_free(C.byref(self.hm))
+            getattr(load(), self.free)(C.byref(self.blocks))
         except Exception:   # interpreter shutdown
             pass
 
@@ -321,15 +321,15 @@ class Program:
 
     def export_voxels(self, grid_size, color_index=0, stream=None):
         """VoxExport's voxels on the GPU: ((n, 4) int32 x y z colour, size, radius)."""
-        lib = load()
         v = _lib.Voxels()
-        check(lib.tg_export_voxels(self.ptr, float(grid_size), int(color_index), C.byref(v), stream), "tg_export_voxels")
-        try:
-            n = int(v.count)
-            vox = (np.ctypeslib.as_array(v.voxels, shape=(n * 4,)).reshape(n, 4).copy() if n else np.zeros((0, 4), np.int32))
-            return vox, tuple(v.size), float(v.radius)
-        finally:
-            lib.tg_voxels_free(C.byref(v))
+        check(load().tg_export_voxels(self.ptr, float(grid_size), int(color_index), C.byref(v), stream), "tg_export_voxels")
+        n = int(v.count)
+        owner = _HostBlocks(v, "tg_voxels_free")
+        if not n:
+            return np.zeros((0, 4), np.int32), tuple(v.size), float(v.radius)
+        buf = (C.c_int32 * (n * 4)).from_address(C.addressof(v.voxels.contents))
+        buf._owner = owner
+        return np.frombuffer(buf, np.int32).reshape(n, 4), tuple(v.size), float(v.radius)
 
 
 def write_drawables(drawables, path, frames=None, fmt="ply", scale=1.0):

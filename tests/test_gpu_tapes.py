@@ -73,3 +73,21 @@ def test_brick_tapes_far_large_and_stretched_operands(lib):
             whole = prog.export_mesh(grid, brick=6)
             assert whole.vertices.shape[0] > 1000
             _same(whole, prog.export_mesh(grid, tapes=True))
+
+
+@pytest.mark.parametrize("prims,ops,grid", [(1, ALL_OPS, 1.0), (30, ALL_OPS, 5.0), (30, ALL_OPS, 16.0), (120, W.OPS_60_20_10_10, 17.0),
+                                            (200, ALL_OPS, 33.0)])
+def test_voxel_blocks_match_oracle(lib, port, prims, ops, grid):
+    """Lattices smaller than a 4^3 box, of whole and of cut 16^3 and 64^3 blocks."""
+    seed = 11
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops))):
+        seed += 1
+    h = port.build(spec)
+    try:
+        want, size, _ = port.vox(h, grid, 3)
+    finally:
+        port.free(h)
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        vox, gsize, _ = prog.export_voxels(grid, 3)
+    np.testing.assert_array_equal(vox, want)
+    assert gsize == size
