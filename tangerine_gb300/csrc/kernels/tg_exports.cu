@@ -248,7 +248,14 @@ namespace tg
 		// block runs the program it was given at its 64 parts' centres.
 		constexpr int kVoxCoarse = 64, kVoxBlock = 16, kVoxFine = 4;
 		constexpr int kVoxCoarseCap = 2048, kVoxBlockCap = 192;
-		constexpr int kVoxWarps = 4, kVoxCtasPerSm = 6;
+		constexpr int kVoxWarps = 4, kVoxCtasPerSm = 6, kVoxEvalCtasPerSm = 8;
+
+		// A warp's scratch while it builds a 16^3 block's tape.
+		struct VoxScratch
+		{
+			float4 Window[64];
+			uint2 Heads[16], Value[kVoxBlockCap], Start[kMaxStack + 2];
+		};
 
 		struct VoxGrid
 		{
@@ -257,11 +264,24 @@ namespace tg
 
 		struct VoxState
 		{
-			uint2* Events;          // kVoxCoarseCap per 64^3 block: its tape
-			uint32_t* Counts;       // its length (kNoTape: none)
+			uint2* Events;          // kVoxCoarseCap per 64^3 block: its tape; then the 16^3 blocks' tapes
+			uint32_t* Counts;       // per 64^3 block: its tape's length (kNoTape: none)
 			uint32_t* List;         // 16^3 blocks to look at: 64^3 block * 64 + part
-			uint32_t* Counters;     // their number, and how many are taken
+			uint2* Tapes;           // per listed 16^3 block: first event and length of the tape it goes by
+			uint32_t* Boxes;        // 4^3 boxes to test: listed block * 64 + part
+			uint32_t* Counters;     // blocks listed, blocks taken, events of the 16^3 blocks, boxes listed, boxes taken
+			uint32_t EventBase, EventCap;   // where the 16^3 blocks' events begin, and how many fit
 		};
+		constexpr int kVoxCounters = 5;
+
+		// The first voxel of a listed 16^3 block.
+		__device__ __forceinline__ void VoxBlockStart(const VoxGrid& vg, uint32_t entry, int (&from)[3])
+		{
+			const int b = (int)(entry >> 6), part = (int)(entry & 63u);
+			from[0] = (b % vg.NX) * kVoxCoarse + (part & 3) * kVoxBlock;
+			from[1] = ((b / vg.NX) % vg.NY) * kVoxCoarse + ((part >> 2) & 3) * kVoxBlock;
+			from[2] = (b / (vg.NX * vg.NY)) * kVoxCoarse + (part >> 4) * kVoxBlock;
+		}
 
 		// Part `part` (0..63, x fastest) of a block that starts at voxel `from` and has 4 x 4 x 4
 		// parts of `edge` voxels an axis; false when it lies outside the lattice (the box is then
@@ -348,25 +368,16 @@ namespace tg
 		}
 
 		// One warp per listed 16^3 block, drawn from a counter: its tape from its 64^3 block's,
-		// then the voxels of the 4^3 boxes that may hold a kept one, two a lane.
-		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxCtasPerSm) VoxFineKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
-			uint32_t* __restrict__ words, int spill_pairs)
+		// and the 4^3 boxes in it that may hold a kept voxel.
+		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxCtasPerSm) VoxBlockKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
+			int spill_pairs)
 		{
 			extern __shared__ __align__(16) uint8_t shared[];
-			struct Scratch
-			{
-				float4 Window[64];
-				uint2 Heads[16], Value[kVoxBlockCap], Start[kMaxStack + 2];
-				float Axis[3][kVoxBlock];
-			};
 			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-			Scratch& sc = reinterpret_cast<Scratch*>(shared)[warp];
-			float2* spill = reinterpret_cast<float2*>(shared + kVoxWarps * sizeof(Scratch)) + warp * spill_pairs * 32 + lane;
-			const float4* code = prog.Code + prog.FullSurfaceCode;
-			auto load = [&](int q) { return __ldg(code + q); };
+			VoxScratch& sc = reinterpret_cast<VoxScratch*>(shared)[warp];
+			float2* spill = reinterpret_cast<float2*>(shared + kVoxWarps * sizeof(VoxScratch)) + warp * spill_pairs * 32 + lane;
 			const float rootClip = fabsf(__ldg(&prog.Nodes[0].ClipRadius));
 			const PairUnits units = LoadPairUnits();
-			const int size[3] = { s.SX, s.SY, s.SZ };
 			const uint32_t n = st.Counters[0];
 			for (;;)
 			{
@@ -375,65 +386,97 @@ namespace tg
 				item = __shfl_sync(0xFFFFFFFFu, item, 0);
 				if (item >= n) break;
 				const uint32_t entry = __ldg(st.List + item);
-				const int b = (int)(entry >> 6), part = (int)(entry & 63u);
-				const int from[3] = { (b % vg.NX) * kVoxCoarse + (part & 3) * kVoxBlock, ((b / vg.NX) % vg.NY) * kVoxCoarse + ((part >> 2) & 3) * kVoxBlock,
-					(b / (vg.NX * vg.NY)) * kVoxCoarse + (part >> 4) * kVoxBlock };
-				const uint32_t given = __ldg(st.Counts + b);
-				const uint2* events = st.Events + (int64_t)b * kVoxCoarseCap;
-				__syncwarp();       // the previous block is done with the scratch
-				for (int i = lane; i < 3 * kVoxBlock; i += 32)
-				{
-					const int a = i / kVoxBlock, q = i % kVoxBlock;
-					sc.Axis[a][q] = VoxCentre(s.Min[a], s.Max[a], min(from[a] + q, size[a] - 1), size[a]);
-				}
+				int from[3];
+				VoxBlockStart(vg, entry, from);
+				const uint32_t given = __ldg(st.Counts + (entry >> 6));
+				const uint32_t first = (entry >> 6) * (uint32_t)kVoxCoarseCap;
 				const VoxLane l = VoxLaneOf(s, from, kVoxFine, rootClip);
 				bool ok = false;
 				TapeCounts counts;
 				if (given != kNoTape)
 				{
+					__syncwarp();       // the previous block's events have been copied out
 					SurfaceEventSource src;
-					src.Open(code, events, (int)given, sc.Window, sc.Heads);
+					src.Open(prog.Code + prog.FullSurfaceCode, st.Events + first, (int)given, sc.Window, sc.Heads);
 					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32,
 						TapeLists{ sc.Value, nullptr, sc.Start, kVoxBlockCap }, counts);
 				}
-				__syncwarp();
-				unsigned kept[2];
+				// The box goes by its own tape, where there is room for it.
+				uint2 tape = make_uint2(first, given);
+				if (ok)
+				{
+					uint32_t at = 0;
+					if (lane == 0) at = atomicAdd(st.Counters + 2, (uint32_t)counts.Value);
+					at = __shfl_sync(0xFFFFFFFFu, at, 0);
+					if (at <= st.EventCap && st.EventCap - at >= (uint32_t)counts.Value)
+					{
+						tape = make_uint2(st.EventBase + at, (uint32_t)counts.Value);
+						for (int i = lane; i < counts.Value; i += 32) st.Events[tape.x + i] = sc.Value[i];
+					}
+				}
+				if (lane == 0) st.Tapes[item] = tape;
 #pragma unroll
 				for (int j = 0; j < 2; ++j)
 				{
 					const float d = j ? counts.Distance.y : counts.Distance.x, r = j ? l.R.y : l.R.x;
 					const float margin = (j ? l.Margin.y : l.Margin.x) + (j ? counts.Error.y : counts.Error.x);
-					kept[j] = __ballot_sync(0xFFFFFFFFu, l.In[j] && !(ok && fabsf(d) > r + s.Radius + margin));
+					const bool keep = l.In[j] && !(ok && fabsf(d) > r + s.Radius + margin);
+					const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+					uint32_t at = 0;
+					if (lane == 0 && kept) at = atomicAdd(st.Counters + 3, (uint32_t)__popc(kept));
+					at = __shfl_sync(0xFFFFFFFFu, at, 0);
+					if (keep) st.Boxes[at + (uint32_t)__popc(kept & ((1u << lane) - 1u))] = item * 64u + (uint32_t)(lane + 32 * j);
 				}
-				const int vx = lane & 3, vy = (lane >> 2) & 3, vz = lane >> 4;
-				while (kept[0] | kept[1])
-				{
-					const int half = kept[0] ? 0 : 1;
-					const int box = __ffs((int)kept[half]) - 1 + 32 * half;
-					kept[half] &= kept[half] - 1u;
-					const int ox = (box & 3) * kVoxFine + vx, oy = ((box >> 2) & 3) * kVoxFine + vy, oz = (box >> 4) * kVoxFine + vz;
-					const float2 px[1] = { make_float2(sc.Axis[0][ox], sc.Axis[0][ox]) }, py[1] = { make_float2(sc.Axis[1][oy], sc.Axis[1][oy]) };
-					const float2 pz[1] = { make_float2(sc.Axis[2][oz], sc.Axis[2][oz + 2]) };
-					float2 d[1];
-					if (given == kNoTape) d[0] = RunWholeSurfacePair(prog.Code, prog.FullSurfaceCode, px[0], py[0], pz[0], spill, 32);
-					else
-						RunSurfaceTapePairs<1>(load, 0, [&](uint32_t e) { return ok ? sc.Value[e] : __ldg(events + e); },
-							ok ? (uint32_t)counts.Value : given, px, py, pz, units, d, spill, 32);
+			}
+		}
+
+		// One warp per listed 4^3 box, drawn from a counter: its voxels, two a lane.
+		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxEvalCtasPerSm) VoxBoxKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
+			uint32_t* __restrict__ words)
+		{
+			extern __shared__ __align__(16) float2 spill2[];
+			const int lane = (int)(threadIdx.x & 31);
+			const float4* code = prog.Code + prog.FullSurfaceCode;
+			auto load = [&](int q) { return __ldg(code + q); };
+			const PairUnits units = LoadPairUnits();
+			const uint32_t n = st.Counters[3];
+			for (;;)
+			{
+				uint32_t item = 0;
+				if (lane == 0) item = atomicAdd(st.Counters + 4, 1u);
+				item = __shfl_sync(0xFFFFFFFFu, item, 0);
+				if (item >= n) break;
+				const uint32_t entry = __ldg(st.Boxes + item);
+				const uint32_t block = __ldg(st.List + (entry >> 6));
+				const uint2 tape = __ldg(st.Tapes + (entry >> 6));
+				int from[3];
+				VoxBlockStart(vg, block, from);
+				const int part = (int)(entry & 63u);
+				const int vx = lane & 3;
+				const int x = from[0] + (part & 3) * kVoxFine + vx, y = from[1] + ((part >> 2) & 3) * kVoxFine + ((lane >> 2) & 3);
+				const int z = from[2] + (part >> 4) * kVoxFine + (lane >> 4);
+				const float cx = VoxCentre(s.Min[0], s.Max[0], x, s.SX), cy = VoxCentre(s.Min[1], s.Max[1], y, s.SY);
+				const float2 px[1] = { make_float2(cx, cx) }, py[1] = { make_float2(cy, cy) };
+				const float2 pz[1] = { make_float2(VoxCentre(s.Min[2], s.Max[2], z, s.SZ), VoxCentre(s.Min[2], s.Max[2], z + 2, s.SZ)) };
+				float2 d[1];
+				const uint2* events = st.Events + tape.x;
+				if (tape.y == kNoTape) d[0] = RunWholeSurfacePair(prog.Code, prog.FullSurfaceCode, px[0], py[0], pz[0], spill2 + threadIdx.x, kVoxWarps * 32);
+				else
+					RunSurfaceTapePairs<1>(load, 0, [&](uint32_t e) { return __ldg(events + e); }, tape.y, px, py, pz, units, d, spill2 + threadIdx.x,
+						kVoxWarps * 32);
 #pragma unroll
-					for (int j = 0; j < 2; ++j)
+				for (int j = 0; j < 2; ++j)
+				{
+					const bool keep = x < s.SX && y < s.SY && z + 2 * j < s.SZ && fabsf(j ? d[0].y : d[0].x) <= s.Radius;
+					const unsigned bits = __ballot_sync(0xFFFFFFFFu, keep);
+					// A row of four voxels of the box is four neighbouring lanes.
+					const uint32_t row = (bits >> (lane & 28)) & 15u;
+					if (vx == 0 && row)
 					{
-						const int x = from[0] + ox, y = from[1] + oy, z = from[2] + oz + 2 * j;
-						const bool keep = x < s.SX && y < s.SY && z < s.SZ && fabsf(j ? d[0].y : d[0].x) <= s.Radius;
-						const unsigned bits = __ballot_sync(0xFFFFFFFFu, keep);
-						// A row of four voxels of the box is four neighbouring lanes.
-						const uint32_t row = (bits >> (lane & 28)) & 15u;
-						if (vx == 0 && row)
-						{
-							const int64_t t = x + (int64_t)s.SX * (y + (int64_t)s.SY * z);
-							const int shift = (int)(t & 31);
-							atomicOr(words + (t >> 5), row << shift);
-							if (shift > 28 && (row >> (32 - shift))) atomicOr(words + (t >> 5) + 1, row >> (32 - shift));
-						}
+						const int64_t t = x + (int64_t)s.SX * (y + (int64_t)s.SY * (z + 2 * j));
+						const int shift = (int)(t & 31);
+						atomicOr(words + (t >> 5), row << shift);
+						if (shift > 28 && (row >> (32 - shift))) atomicOr(words + (t >> 5) + 1, row >> (32 - shift));
 					}
 				}
 			}
@@ -588,22 +631,46 @@ namespace tg
 		return { (s.SX + kVoxCoarse - 1) / kVoxCoarse, (s.SY + kVoxCoarse - 1) / kVoxCoarse, (s.SZ + kVoxCoarse - 1) / kVoxCoarse };
 	}
 
-	static bool VoxByBlocks(const DeviceProgram& prog) { return prog.Lipschitz && (prog.Form & kFormPrunable); }
+	// Lattices so thin that most of their blocks lie outside keep the general path: the blocks'
+	// scratch would outgrow the lattice's own.
+	static bool VoxByBlocks(const DeviceProgram& prog, const VoxSpec& s)
+	{
+		const VoxGrid vg = VoxGridOf(s);
+		return prog.Lipschitz && (prog.Form & kFormPrunable) && (int64_t)vg.NX * vg.NY * vg.NZ <= 64 + s.Total / 16384;
+	}
+
+	// The scratch's parts, 16-byte aligned one after the other; the bytes they take.
+	static size_t VoxLayout(const VoxSpec& s, void* scratch, VoxState& st)
+	{
+		const VoxGrid vg = VoxGridOf(s);
+		const size_t blocks = (size_t)vg.NX * vg.NY * vg.NZ, boxes = blocks * 64;
+		size_t at = 0;
+		auto take = [&](size_t bytes) { uint8_t* p = static_cast<uint8_t*>(scratch) + at; at += (bytes + 15) / 16 * 16; return p; };
+		// Events of the 16^3 blocks' own tapes: 16 on average, one block in four or five listed.
+		st.EventBase = (uint32_t)(blocks * kVoxCoarseCap);
+		st.EventCap = (uint32_t)(boxes * 16);
+		st.Events = reinterpret_cast<uint2*>(take(((size_t)st.EventBase + st.EventCap) * sizeof(uint2)));
+		st.Counts = reinterpret_cast<uint32_t*>(take(blocks * sizeof(uint32_t)));
+		st.List = reinterpret_cast<uint32_t*>(take(boxes * sizeof(uint32_t)));
+		st.Tapes = reinterpret_cast<uint2*>(take(boxes * sizeof(uint2)));
+		st.Boxes = reinterpret_cast<uint32_t*>(take(boxes * 64 * sizeof(uint32_t)));
+		st.Counters = reinterpret_cast<uint32_t*>(take(kVoxCounters * sizeof(uint32_t)));
+		return at;
+	}
 
 	size_t VoxScratchBytes(const DeviceProgram& prog, const VoxSpec& s)
 	{
 		if (s.Total <= 0) return 16;
-		if (!VoxByBlocks(prog)) return VoxelBrickWords(s.SX, s.SY, s.SZ) * sizeof(uint32_t);
-		const VoxGrid vg = VoxGridOf(s);
-		const size_t blocks = (size_t)vg.NX * vg.NY * vg.NZ;
-		return blocks * (kVoxCoarseCap * sizeof(uint2) + sizeof(uint32_t) + 64 * sizeof(uint32_t)) + 4 * sizeof(uint32_t);
+		if (!VoxByBlocks(prog, s)) return VoxelBrickWords(s.SX, s.SY, s.SZ) * sizeof(uint32_t);
+		VoxState st;
+		return VoxLayout(s, nullptr, st);
 	}
 
 	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream)
 	{
 		if (s.Total <= 0) return cudaSuccess;
 		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
-		if (!VoxByBlocks(prog))
+		if (!VoxByBlocks(prog, s))
 		{
 			uint32_t* brick_bits = static_cast<uint32_t*>(scratch);
 			const VoxelBricks vb = BricksOf(s.SX, s.SY, s.SZ);
@@ -624,26 +691,24 @@ namespace tg
 			return cudaGetLastError();
 		}
 		const VoxGrid vg = VoxGridOf(s);
-		const int64_t blocks = (int64_t)vg.NX * vg.NY * vg.NZ;
 		VoxState st;
-		st.Events = static_cast<uint2*>(scratch);
-		st.Counts = reinterpret_cast<uint32_t*>(st.Events + blocks * kVoxCoarseCap);
-		st.List = st.Counts + blocks;
-		st.Counters = st.List + blocks * 64;
+		VoxLayout(s, scratch, st);
 		cudaError_t e = cudaMemsetAsync(words, 0, (size_t)((s.Total + 31) / 32) * 4, stream);
-		if (e == cudaSuccess) e = cudaMemsetAsync(st.Counters, 0, 2 * sizeof(uint32_t), stream);
+		if (e == cudaSuccess) e = cudaMemsetAsync(st.Counters, 0, kVoxCounters * sizeof(uint32_t), stream);
 		if (e != cudaSuccess) return e;
 		const size_t coarse = 64 * sizeof(float4) + (kVoxCoarseCap + kMaxStack + 2) * sizeof(uint2) + (size_t)depth * 32 * sizeof(float2);
-		// The kernel's own scratch struct: window, events' heads, tape, stack starts, axes.
-		const size_t warp = 64 * sizeof(float4) + (16 + kVoxBlockCap + kMaxStack + 2) * sizeof(uint2) + 3 * kVoxBlock * sizeof(float);
-		const size_t fine = kVoxWarps * (warp + (size_t)depth * 32 * sizeof(float2));
+		const size_t fine = kVoxWarps * (sizeof(VoxScratch) + (size_t)depth * 32 * sizeof(float2));
+		const size_t eval = kVoxWarps * (size_t)depth * 32 * sizeof(float2);
 		if (coarse > 48 * 1024) e = cudaFuncSetAttribute(VoxCoarseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coarse);
-		if (e == cudaSuccess && fine > 48 * 1024) e = cudaFuncSetAttribute(VoxFineKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fine);
+		if (e == cudaSuccess && fine > 48 * 1024) e = cudaFuncSetAttribute(VoxBlockKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fine);
 		if (e != cudaSuccess) return e;
-		VoxCoarseKernel<<<(unsigned)blocks, 32, coarse, stream>>>(prog, s, vg, st, depth);
+		VoxCoarseKernel<<<(unsigned)(vg.NX * vg.NY * vg.NZ), 32, coarse, stream>>>(prog, s, vg, st, depth);
 		e = cudaGetLastError();
 		if (e != cudaSuccess) return e;
-		VoxFineKernel<<<sms * kVoxCtasPerSm, kVoxWarps * 32, fine, stream>>>(prog, s, vg, st, words, depth);
+		VoxBlockKernel<<<sms * kVoxCtasPerSm, kVoxWarps * 32, fine, stream>>>(prog, s, vg, st, depth);
+		e = cudaGetLastError();
+		if (e != cudaSuccess) return e;
+		VoxBoxKernel<<<sms * kVoxEvalCtasPerSm, kVoxWarps * 32, eval, stream>>>(prog, s, vg, st, words);
 		return cudaGetLastError();
 	}
 
