@@ -339,8 +339,7 @@ namespace tg
 	// 512^3 861 / 1062, and 128^3 721 / 653.
 	static bool TapesPay(const Program& p, int64_t bricks)
 	{
-		const double quads = (double)p.Host.DistanceQuadsTotal / std::max(1, p.Host.Header.NodeCount);
-		return (double)bricks * (quads - 12.0) >= 3.5e6;
+		return (double)bricks * (CellQuads(p) - 12.0) >= 3.5e6;
 	}
 
 	cudaError_t Engine::ReadSmCount()

@@ -65,6 +65,12 @@ namespace tg
 	};
 	void FreeHostMesh(HostMeshOut& m);
 
+	// Quads of an octree cell's distance program, on average.
+	inline double CellQuads(const Program& p)
+	{
+		return (double)p.Host.DistanceQuadsTotal / (p.Host.Header.NodeCount > 0 ? p.Host.Header.NodeCount : 1);
+	}
+
 	struct ExportOptions
 	{
 		bool Attributes = true;     // gradient normals and colours

@@ -100,17 +100,39 @@ namespace tg
 		TG_TRY(WordBase.Reserve((size_t)(words ? words : 1) * 4));
 		TG_TRY(Counts.Reserve(4 * sizeof(uint32_t)));
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4 + 4));
-		PreValid = false;   // these bits replace a pending PreClassify's
-		TG_TRY(BrickBits.Reserve(VoxelBrickWords(s.IX, s.IY, s.IZ) * 4));
-		Begin("cloud_flags", st);
-		TG_TRY(LaunchCloudFlags(p.View, s, BrickBits.As<uint32_t>(), Words.As<uint32_t>(), st));
-		End(st);
-		// The kept voxels' numbers in increasing order (bitmask -> scan -> list).
-		TG_TRY(Cubes.Reserve((size_t)(words ? words : 1) * 32 * 4));
-		Begin("list_cells", st);
-		TG_TRY(LaunchListBricks(Words.As<uint32_t>(), s.Total, WordBase.As<uint32_t>(), Scratch.As<uint32_t>(), Cubes.As<uint32_t>(),
-			Counts.As<uint32_t>(), st));
-		End(st);
+		const bool byTapes = CloudByTapes(p.View, s, CellQuads(p));
+		BrickTapes tapes{};
+		if (byTapes)
+		{
+			const int64_t bricks = CloudBricks(s);
+			TG_TRY(ReadSmCount());
+			TG_TRY(ReserveTapes(bricks, tapes));
+			TG_TRY(VoxScratch.Reserve((size_t)bricks * 8));
+			uint32_t* list = VoxScratch.As<uint32_t>();
+			TG_TRY(ActiveCells.Reserve((size_t)s.Total * 4));
+			Begin("cloud_flags", st);
+			TG_TRY(LaunchCloudVoxels(p.View, s, list, list + bricks, tapes, Words.As<uint32_t>(),
+				ActiveCells.As<uint32_t>(), Counts.As<uint32_t>() + 1, SmCount, st));
+			End(st);
+			Begin("list_cells", st);
+			TG_TRY(LaunchExclusiveScan(Words.As<uint32_t>(), words, true, WordBase.As<uint32_t>(), Counts.As<uint32_t>(),
+				Scratch.As<uint32_t>(), st));
+			End(st);
+		}
+		else
+		{
+			PreValid = false;   // these bits replace a pending PreClassify's
+			TG_TRY(BrickBits.Reserve(VoxelBrickWords(s.IX, s.IY, s.IZ) * 4));
+			Begin("cloud_flags", st);
+			TG_TRY(LaunchCloudFlags(p.View, s, BrickBits.As<uint32_t>(), Words.As<uint32_t>(), st));
+			End(st);
+			// The kept voxels' numbers in increasing order (bitmask -> scan -> list).
+			TG_TRY(Cubes.Reserve((size_t)(words ? words : 1) * 32 * 4));
+			Begin("list_cells", st);
+			TG_TRY(LaunchListBricks(Words.As<uint32_t>(), s.Total, WordBase.As<uint32_t>(), Scratch.As<uint32_t>(), Cubes.As<uint32_t>(),
+				Counts.As<uint32_t>(), st));
+			End(st);
+		}
 		TG_TRY(cudaMemcpyAsync(HostCounts, Counts.Ptr, 4, cudaMemcpyDeviceToHost, st));
 		TG_TRY(cudaStreamSynchronize(st));
 		const uint32_t n = HostCounts[0];
@@ -128,25 +150,39 @@ namespace tg
 			if (control->Stage && control->Stage->load() > 2) refine = 0;
 		}
 		TG_TRY(Vertices.Reserve((size_t)n * 12 + 12));
+		float* normals = nullptr;
+		uint8_t* colors = nullptr;
+		if (attributes)
+		{
+			TG_TRY(Normals.Reserve((size_t)n * 12 + 12));
+			normals = Normals.As<float>();
+			if (p.Host.Header.HasPaint)
+			{
+				TG_TRY(Colors.Reserve((size_t)n * 3 + 3));
+				colors = Colors.As<uint8_t>();
+			}
+		}
 		Begin("cloud_refine", st);
-		TG_TRY(LaunchCloudRefine(p.View, s, Cubes.As<uint32_t>(), Counts.As<uint32_t>(), n, refine, Vertices.As<float>(), st));
+		if (byTapes)
+		{
+			TG_TRY(Cubes.Reserve((size_t)n * 4 + 4));
+			TG_TRY(LaunchCloudPoints(p.View, s, tapes, ActiveCells.As<uint32_t>(), n, Words.As<uint32_t>(), WordBase.As<uint32_t>(), refine,
+				Cubes.As<uint32_t>(), Vertices.As<float>(), normals, colors, st));
+		}
+		else TG_TRY(LaunchCloudRefine(p.View, s, Cubes.As<uint32_t>(), Counts.As<uint32_t>(), n, refine, Vertices.As<float>(), st));
 		End(st);
 		out.VertexCount = n;
 		out.Vertices = Vertices.As<float>();
 		out.Cubes = Cubes.As<uint32_t>();
 		if (attributes)
 		{
-			TG_TRY(Normals.Reserve((size_t)n * 12 + 12));
-			uint8_t* colors = nullptr;
-			if (p.Host.Header.HasPaint)
+			if (!byTapes)
 			{
-				TG_TRY(Colors.Reserve((size_t)n * 3 + 3));
-				colors = Colors.As<uint8_t>();
+				Begin("attributes", st);
+				TG_TRY(LaunchVertexAttributes(p.View, Vertices.As<float>(), n, normals, colors, st));
+				End(st);
 			}
-			Begin("attributes", st);
-			TG_TRY(LaunchVertexAttributes(p.View, Vertices.As<float>(), n, Normals.As<float>(), colors, st));
-			End(st);
-			out.Normals = Normals.As<float>();
+			out.Normals = normals;
 			out.Colors = colors;
 		}
 		TG_TRY(cudaStreamSynchronize(st));

@@ -103,37 +103,6 @@ namespace tg
 		}
 	}
 
-	// The box of a part's corner points (LaunchBrickTapes), `grow` lattice steps wider towards
-	// the rest of its brick.
-	__device__ __forceinline__ void PartBox(const GridSpec& g, const BrickGrid& bg, uint32_t b, uint32_t box, int grow, float (&lo)[3],
-		float (&hi)[3])
-	{
-		const uint32_t row = b / (uint32_t)bg.NBX, bz = row / (uint32_t)bg.NBY;
-		const int first[3] = { (int)(b - row * (uint32_t)bg.NBX) * bg.B, (int)(row - bz * (uint32_t)bg.NBY) * bg.B, (int)bz * bg.B };
-		const int last[3] = { min(first[0] + bg.B, g.NX - 1), min(first[1] + bg.B, g.NY - 1), min(first[2] + bg.B, g.NZ - 1) };
-		const float origin[3] = { g.X0, g.Y0, g.Z0 }, step[3] = { g.DX, g.DY, g.DZ };
-#pragma unroll
-		for (int a = 0; a < 3; ++a)
-		{
-			const int x0 = first[a] + (int)((box >> (8 * a)) & 15u), x1 = first[a] + (int)((box >> (8 * a + 4)) & 15u);
-			lo[a] = LatticeCoord(origin[a], max(x0 - grow, first[a]), step[a]);
-			hi[a] = LatticeCoord(origin[a], min(x1 + grow, last[a]), step[a]);
-		}
-	}
-
-	__device__ __forceinline__ void PartCorners(const GridSpec& g, const BrickGrid& bg, uint32_t b, uint32_t box, float (&lo)[3], float (&hi)[3])
-	{
-		PartBox(g, bg, b, box, 0, lo, hi);
-	}
-
-	// The space a part's tape is built for: one step more than its points towards the rest of
-	// the brick (the next part's points begin there, and a vertex between the two may descend
-	// to either part's cell).
-	__device__ __forceinline__ void PartRegion(const GridSpec& g, const BrickGrid& bg, uint32_t b, uint32_t box, float (&lo)[3], float (&hi)[3])
-	{
-		PartBox(g, bg, b, box, 1, lo, hi);
-	}
-
 	inline BrickGrid MakeBrickGrid(const GridSpec& g, int B)
 	{
 		return { B, (g.NX - 1 + B - 1) / B, (g.NY - 1 + B - 1) / B, (g.NZ - 1 + B - 1) / B };

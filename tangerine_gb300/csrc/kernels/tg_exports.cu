@@ -11,6 +11,7 @@
 #include "tg_kernels.hpp"
 #include "tg_surface.cuh"
 #include "tg_tape.cuh"
+#include "tg_parts.cuh"
 
 namespace tg
 {
@@ -208,6 +209,190 @@ namespace tg
 			points[(int64_t)v * 3 + 2] = cursor.z;
 		}
 
+		// The point cloud by shortened programs (tg_parts.cuh): bricks of 8^3 voxel centres.  A
+		// voxel's refined point may leave its brick by half a voxel.
+		struct CloudLattice
+		{
+			static constexpr int kStride = parts::kBox;
+			static constexpr bool kOutside = true;
+			CloudSpec Spec;
+			__device__ __forceinline__ float Coord(int a, int i) const { return ((float)i * Spec.Step[a] + Spec.Start[a]) + Spec.Half[a]; }
+			__host__ __device__ __forceinline__ int Points(int a) const { return a == 0 ? Spec.IX : a == 1 ? Spec.IY : Spec.IZ; }
+			__host__ __device__ __forceinline__ int Bricks(int a) const { return (Points(a) + parts::kBox - 1) / parts::kBox; }
+			__device__ __forceinline__ float Keep() const { return Spec.Diagonal; }
+			__device__ __forceinline__ int IndexAt(int a, float p) const
+			{
+				// In float until clamped: a wandering point may be far away, or not a number.
+				return (int)fminf(fmaxf((p - Coord(a, 0)) / Spec.Step[a], 0.0f), (float)(Points(a) - 1)) / parts::kBox;
+			}
+			__device__ __forceinline__ uint32_t BrickAt(Vec3 p) const
+			{
+				return (uint32_t)min(IndexAt(0, p.x), Bricks(0) - 1) + (uint32_t)Bricks(0) * ((uint32_t)min(IndexAt(1, p.y), Bricks(1) - 1) +
+					(uint32_t)Bricks(1) * (uint32_t)min(IndexAt(2, p.z), Bricks(2) - 1));
+			}
+		};
+
+		// CloudBricksKernel's test, with the kept bricks listed and their descents stored.
+		__global__ void __launch_bounds__(128) CloudListKernel(DeviceProgram prog, CloudLattice lat, uint32_t* __restrict__ list,
+			uint32_t* __restrict__ count, uint32_t* __restrict__ tops)
+		{
+			extern __shared__ float spill[];
+			const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+			const int lane = (int)(threadIdx.x & 31);
+			bool keep = false;
+			if (b < (int64_t)lat.Bricks(0) * lat.Bricks(1) * lat.Bricks(2))
+			{
+				int first[3], extent[3];
+				parts::BrickSpan(lat, (uint32_t)b, first, extent);
+				const uint32_t packed = parts::DescendBrick(prog, lat, first, extent);
+				const int cell = (int)(packed & 0x7FFFFFFFu);
+				keep = true;
+				if ((packed >> 31) && __ldg(&prog.Nodes[cell].ClipRadius) >= 0.0f)
+				{
+					float lo[3], hi[3], c[3], r, margin;
+#pragma unroll
+					for (int a = 0; a < 3; ++a) { lo[a] = lat.Coord(a, first[a]); hi[a] = lat.Coord(a, first[a] + extent[a]); }
+					BallOf(lo, hi, c, r, margin, fabsf(__ldg(&prog.Nodes[0].ClipRadius)));
+					const float px[1] = { c[0] }, py[1] = { c[1] }, pz[1] = { c[2] };
+					float f[1];
+					RunDistance<1>(prog.Code, __ldg(&prog.Nodes[cell].DistanceCode), px, py, pz, f, spill + threadIdx.x, 128);
+					keep = !(fabsf(f[0]) > r + lat.Spec.Diagonal + margin);
+				}
+				if (keep) tops[b] = packed;
+			}
+			const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
+			uint32_t at = 0;
+			if (lane == 0 && kept) at = atomicAdd(count, (uint32_t)__popc(kept));
+			at = __shfl_sync(0xFFFFFFFFu, at, 0);
+			if (keep) list[at + (uint32_t)__popc(kept & ((1u << lane) - 1u))] = (uint32_t)b;
+		}
+
+		// abs(Octree->Eval(Cursor)) < Diagonal for the voxels of the listed bricks, a warp per
+		// brick; the kept ones set their bits and are listed by brick and part, so that points
+		// running one tape follow each other.
+		__global__ void __launch_bounds__(parts::kThreads, 8) CloudVoxelsKernel(DeviceProgram prog, CloudLattice lat, const uint32_t* __restrict__ list,
+			const uint32_t* __restrict__ count, BrickTapes tapes, uint32_t* __restrict__ words, uint32_t* __restrict__ voxels,
+			uint32_t* __restrict__ voxel_count)
+		{
+			using namespace parts;
+			extern __shared__ __align__(16) float2 spill2[];
+			__shared__ uint16_t found[kWarps][kBox * kBox * kBox];
+			__shared__ float axes[kWarps][3][kBox];
+			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+			float (*axis)[kBox] = axes[warp];
+			uint16_t* kept = found[warp];
+			const PairUnits units = LoadPairUnits();
+			const uint32_t n = *count;
+			for (;;)
+			{
+				uint32_t item = 0;
+				if (lane == 0) item = atomicAdd(tapes.Counters + 3, 1u);
+				item = __shfl_sync(0xFFFFFFFFu, item, 0);
+				if (item >= n) break;
+				const uint32_t b = __ldg(list + item);
+				const uint2 own = __ldg(tapes.Bricks + b);
+				bool far = own.y != 0;
+				for (uint32_t p = 0; p < own.y; ++p) far = far && (__ldg(&tapes.Parts[own.x + p].Box) & (kBoxPositive | kBoxNegative));
+				if (far) continue;
+				int first[3], extent[3];
+				BrickSpan(lat, b, first, extent);
+				__syncwarp();       // the previous brick is done with the axes and the list
+				if (lane < 24) axis[lane >> 3][lane & 7] = lat.Coord(lane >> 3, first[lane >> 3] + (lane & 7));
+				__syncwarp();
+				uint32_t total = 0;
+				BrickPoints<true>(prog, tapes, own, extent, axis, units, spill2 + threadIdx.x, [&](int at, float v, bool live)
+				{
+					const unsigned keep = __ballot_sync(0xFFFFFFFFu, live && fabsf(v) < lat.Spec.Diagonal);
+					if ((keep >> lane) & 1u) kept[total + (uint32_t)__popc(keep & ((1u << lane) - 1u))] = (uint16_t)at;
+					total += (uint32_t)__popc(keep);
+				});
+				uint32_t to = 0;
+				if (lane == 0 && total) to = atomicAdd(voxel_count, total);
+				to = __shfl_sync(0xFFFFFFFFu, to, 0);
+				__syncwarp();
+				for (uint32_t i = (uint32_t)lane; i < total; i += 32)
+				{
+					const int at = kept[i];
+					const int64_t t = first[0] + (at & 7) + (int64_t)lat.Spec.IX * ((first[1] + ((at >> 3) & 7)) + (int64_t)lat.Spec.IY * (first[2] + (at >> 6)));
+					atomicOr(words + (t >> 5), 1u << (t & 31));
+					voxels[to + i] = (uint32_t)t;
+				}
+			}
+		}
+
+		// The refinement (export.cpp:434-465): `iterations` steps of Cursor += Gradient * -Eval,
+		// clamped to the voxel (the point moves only if it stays within the diagonal), then the
+		// point's normal and colour; a thread per voxel in the bricks' order, each point by its
+		// part's tape while it is in the part's box.
+		__global__ void __launch_bounds__(parts::kThreads, 6) CloudPointsKernel(DeviceProgram prog, CloudLattice lat, BrickTapes tapes,
+			const uint32_t* __restrict__ voxels, uint32_t n, const uint32_t* __restrict__ words, const uint32_t* __restrict__ word_base, int iterations,
+			uint32_t* __restrict__ cubes, float* __restrict__ points, float* __restrict__ normals, uint8_t* __restrict__ colors)
+		{
+			using namespace parts;
+			extern __shared__ __align__(16) float2 spill2[];
+			const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+			if (t >= n) return;
+			const CloudSpec& s = lat.Spec;
+			const uint32_t c = __ldg(voxels + t);
+			const uint32_t w = __ldg(words + (c >> 5));
+			const uint32_t v = __ldg(word_base + (c >> 5)) + __popc(w & ((1u << (c & 31)) - 1u));
+			const uint32_t row = c / (uint32_t)s.IX, k = row / (uint32_t)s.IY, i = c - row * (uint32_t)s.IX, j = row - k * (uint32_t)s.IY;
+			const uint2 own = __ldg(tapes.Bricks + i / kBox + (uint32_t)lat.Bricks(0) * (j / kBox + (uint32_t)lat.Bricks(1) * (k / kBox)));
+			const Vec3 vertex = CloudCentre(s, (int)c);
+			const PairUnits units = LoadPairUnits();
+			float2* spill = spill2 + threadIdx.x;
+			Vec3 cursor = vertex;
+			PointRun run;
+			run.Lo[0] = 1.0f; run.Hi[0] = 0.0f;
+			Vec3 normal(0.0f, 0.0f, 0.0f);
+			for (int r = 0; r <= iterations; ++r)
+			{
+				if (r == iterations)
+				{
+					if (iterations > 0)
+					{
+						const Vec3 half(s.Half[0], s.Half[1], s.Half[2]);
+						const Vec3 low = vertex - half, high = vertex + half;
+						cursor = TernaryMin(TernaryMax(cursor, low), high);
+						const Vec3 d = vertex - cursor;
+						if (!(sqrtf(Dot(d, d)) <= s.Diagonal)) cursor = vertex;
+					}
+					if (!normals) break;
+				}
+				if (!InRun(run, cursor))
+				{
+					// The voxel's own brick, then the one the point is in now (one that was not kept
+					// has no parts).  A point that runs whole programs holds up its warp: looked for in
+					// its own brick alone, a few in a hundred did, and two warps in three.
+					bool found = FindPart(tapes, own, cursor, run);
+					if (!found)
+					{
+						const uint32_t b = lat.BrickAt(cursor);
+						found = FindPart(tapes, __ldg(tapes.Bricks + b), cursor, run);
+					}
+					if (!found) RunWhole(prog, cursor, run);
+				}
+				float d = 0.0f;
+				normal = RunGradient<true>(prog, tapes, run, cursor, units, spill, r < iterations, d);
+				if (r == iterations) break;
+				// Octree->Eval(Cursor) * -1.0 rounds back to float exactly: a negation.
+				cursor = cursor + normal * -d;
+			}
+			cubes[v] = c;
+			points[(int64_t)v * 3 + 0] = cursor.x;
+			points[(int64_t)v * 3 + 1] = cursor.y;
+			points[(int64_t)v * 3 + 2] = cursor.z;
+			if (!normals) return;
+			normals[(int64_t)v * 3 + 0] = normal.x;
+			normals[(int64_t)v * 3 + 1] = normal.y;
+			normals[(int64_t)v * 3 + 2] = normal.z;
+			if (!colors) return;
+			const uchar4 color = RunColor(prog, tapes, run, cursor, units, spill);
+			colors[(int64_t)v * 3 + 0] = color.x;
+			colors[(int64_t)v * 3 + 1] = color.y;
+			colors[(int64_t)v * 3 + 2] = color.z;
+		}
+
 		// glm::mix(x, y, a) = x * (1 - a) + y * a, per component.
 		__device__ __forceinline__ float Mix(float x, float y, float a)
 		{
@@ -249,6 +434,7 @@ namespace tg
 		constexpr int kVoxCoarse = 64, kVoxBlock = 16, kVoxFine = 4;
 		constexpr int kVoxCoarseCap = 2048, kVoxBlockCap = 192;
 		constexpr int kVoxWarps = 4, kVoxCtasPerSm = 6, kVoxEvalCtasPerSm = 8;
+		constexpr int kVoxDirectBlocks = 1000;
 
 		// A warp's scratch while it builds a 16^3 block's tape.
 		struct VoxScratch
@@ -368,7 +554,9 @@ namespace tg
 		}
 
 		// One warp per listed 16^3 block, drawn from a counter: its tape from its 64^3 block's,
-		// and the 4^3 boxes in it that may hold a kept voxel.
+		// and the 4^3 boxes in it that may hold a kept voxel.  Direct: every 16^3 block, from the
+		// whole tree's program.
+		template<bool Direct>
 		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxCtasPerSm) VoxBlockKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
 			int spill_pairs)
 		{
@@ -378,28 +566,35 @@ namespace tg
 			float2* spill = reinterpret_cast<float2*>(shared + kVoxWarps * sizeof(VoxScratch)) + warp * spill_pairs * 32 + lane;
 			const float rootClip = fabsf(__ldg(&prog.Nodes[0].ClipRadius));
 			const PairUnits units = LoadPairUnits();
-			const uint32_t n = st.Counters[0];
+			const uint32_t n = Direct ? (uint32_t)(vg.NX * vg.NY * vg.NZ) * 64u : st.Counters[0];
 			for (;;)
 			{
 				uint32_t item = 0;
 				if (lane == 0) item = atomicAdd(st.Counters + 1, 1u);
 				item = __shfl_sync(0xFFFFFFFFu, item, 0);
 				if (item >= n) break;
-				const uint32_t entry = __ldg(st.List + item);
+				const uint32_t entry = Direct ? item : __ldg(st.List + item);
 				int from[3];
 				VoxBlockStart(vg, entry, from);
-				const uint32_t given = __ldg(st.Counts + (entry >> 6));
-				const uint32_t first = (entry >> 6) * (uint32_t)kVoxCoarseCap;
+				if (Direct && (from[0] >= s.SX || from[1] >= s.SY || from[2] >= s.SZ)) continue;
+				const uint32_t given = Direct ? kNoTape : __ldg(st.Counts + (entry >> 6));
+				const uint32_t first = Direct ? 0u : (entry >> 6) * (uint32_t)kVoxCoarseCap;
 				const VoxLane l = VoxLaneOf(s, from, kVoxFine, rootClip);
+				const TapeLists lists{ sc.Value, nullptr, sc.Start, kVoxBlockCap };
 				bool ok = false;
 				TapeCounts counts;
-				if (given != kNoTape)
+				__syncwarp();       // the previous block's events have been copied out
+				if (Direct)
 				{
-					__syncwarp();       // the previous block's events have been copied out
+					SurfaceSource src;
+					src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, sc.Window);
+					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32, lists, counts);
+				}
+				else if (given != kNoTape)
+				{
 					SurfaceEventSource src;
 					src.Open(prog.Code + prog.FullSurfaceCode, st.Events + first, (int)given, sc.Window, sc.Heads);
-					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32,
-						TapeLists{ sc.Value, nullptr, sc.Start, kVoxBlockCap }, counts);
+					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32, lists, counts);
 				}
 				// The box goes by its own tape, where there is room for it.
 				uint2 tape = make_uint2(first, given);
@@ -432,7 +627,7 @@ namespace tg
 
 		// One warp per listed 4^3 box, drawn from a counter: its voxels, two a lane.
 		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxEvalCtasPerSm) VoxBoxKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
-			uint32_t* __restrict__ words)
+			bool direct, uint32_t* __restrict__ words)
 		{
 			extern __shared__ __align__(16) float2 spill2[];
 			const int lane = (int)(threadIdx.x & 31);
@@ -447,7 +642,7 @@ namespace tg
 				item = __shfl_sync(0xFFFFFFFFu, item, 0);
 				if (item >= n) break;
 				const uint32_t entry = __ldg(st.Boxes + item);
-				const uint32_t block = __ldg(st.List + (entry >> 6));
+				const uint32_t block = direct ? entry >> 6 : __ldg(st.List + (entry >> 6));
 				const uint2 tape = __ldg(st.Tapes + (entry >> 6));
 				int from[3];
 				VoxBlockStart(vg, block, from);
@@ -609,6 +804,68 @@ namespace tg
 		return cudaGetLastError();
 	}
 
+	int64_t CloudBricks(const CloudSpec& s)
+	{
+		const CloudLattice lat{ s };
+		return (int64_t)lat.Bricks(0) * lat.Bricks(1) * lat.Bricks(2);
+	}
+
+	// Short programs and few bricks keep the direct tests (two launches and a pass of the whole
+	// programs cost more there).  Measured on a GB300, tapes against direct, us a call: 16
+	// primitives (16 quads a cell) 0.04 voxels 203 / 193, 0.02 222 / 275; 64 (23 quads) 556 /
+	// 429 and 470 / 634; 256 (54 quads) 0.08 voxels 1971 / 1188, 0.04 1549 / 1527, 0.02 1108 /
+	// 2295.  quads: those of an octree cell's distance program, on average.
+	bool CloudByTapes(const DeviceProgram& prog, const CloudSpec& s, double quads)
+	{
+		return s.Total > 0 && prog.Lipschitz && (prog.Form & kFormPrunable) && (double)CloudBricks(s) * (quads - 12.0) >= 45000.0;
+	}
+
+	cudaError_t LaunchCloudVoxels(const DeviceProgram& prog, const CloudSpec& s, uint32_t* list, uint32_t* tops, const BrickTapes& tapes,
+		uint32_t* words, uint32_t* voxels, uint32_t* counts, int sms, cudaStream_t stream)
+	{
+		const CloudLattice lat{ s };
+		cudaError_t e = cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), stream);
+		if (e == cudaSuccess) e = cudaMemsetAsync(words, 0, (size_t)((s.Total + 31) / 32) * 4, stream);
+		// Bricks that are not listed are looked up too, by points that wander: no parts there.
+		if (e == cudaSuccess) e = cudaMemsetAsync(tapes.Bricks, 0, (size_t)CloudBricks(s) * sizeof(uint2), stream);
+		if (e != cudaSuccess) return e;
+		size_t smem = DistanceSpillBytes(prog, 128);
+		if (smem > 48 * 1024)
+		{
+			e = cudaFuncSetAttribute(CloudListKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			if (e != cudaSuccess) return e;
+		}
+		CloudListKernel<<<Blocks(CloudBricks(s), 128), 128, smem, stream>>>(prog, lat, list, counts, tops);
+		e = cudaGetLastError();
+		if (e == cudaSuccess) e = parts::LaunchParts(prog, lat, list, counts, tops, tapes, sms, stream);
+		if (e != cudaSuccess) return e;
+		smem = parts::SpillPairs(prog, 1) * parts::kThreads * sizeof(float2);
+		if (smem > 39 * 1024)
+		{
+			e = cudaFuncSetAttribute(CloudVoxelsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			if (e != cudaSuccess) return e;
+		}
+		CloudVoxelsKernel<<<sms * 8, parts::kThreads, smem, stream>>>(prog, lat, list, counts, tapes, words, voxels, counts + 1);
+		return cudaGetLastError();
+	}
+
+	cudaError_t LaunchCloudPoints(const DeviceProgram& prog, const CloudSpec& s, const BrickTapes& tapes, const uint32_t* voxels, uint32_t n,
+		const uint32_t* words, const uint32_t* word_base, int iterations, uint32_t* cubes, float* points, float* normals, uint8_t* colors,
+		cudaStream_t stream)
+	{
+		if (n == 0) return cudaSuccess;
+		// The colour's walk takes two words a level, the gradient one pair.
+		const size_t smem = parts::SpillPairs(prog, 2) * parts::kThreads * sizeof(float2);
+		if (smem > 48 * 1024)
+		{
+			const cudaError_t e = cudaFuncSetAttribute(CloudPointsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			if (e != cudaSuccess) return e;
+		}
+		CloudPointsKernel<<<Blocks(n, parts::kThreads), parts::kThreads, smem, stream>>>(prog, CloudLattice{ s }, tapes, voxels, n, words, word_base,
+			iterations, cubes, points, normals, colors);
+		return cudaGetLastError();
+	}
+
 	cudaError_t LaunchCloudRefine(const DeviceProgram& prog, const CloudSpec& s, const uint32_t* cells, const uint32_t* count,
 		uint32_t capacity, int iterations, float* points, cudaStream_t stream)
 	{
@@ -699,16 +956,24 @@ namespace tg
 		const size_t coarse = 64 * sizeof(float4) + (kVoxCoarseCap + kMaxStack + 2) * sizeof(uint2) + (size_t)depth * 32 * sizeof(float2);
 		const size_t fine = kVoxWarps * (sizeof(VoxScratch) + (size_t)depth * 32 * sizeof(float2));
 		const size_t eval = kVoxWarps * (size_t)depth * 32 * sizeof(float2);
+		// The first level costs a pass over the whole tree by itself: lattices whose 16^3 blocks
+		// the GPU runs at once go without it.
+		const int64_t small = (int64_t)((s.SX + kVoxBlock - 1) / kVoxBlock) * ((s.SY + kVoxBlock - 1) / kVoxBlock) * ((s.SZ + kVoxBlock - 1) / kVoxBlock);
+		const bool direct = small <= kVoxDirectBlocks;
+		auto* block = direct ? VoxBlockKernel<true> : VoxBlockKernel<false>;
 		if (coarse > 48 * 1024) e = cudaFuncSetAttribute(VoxCoarseKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coarse);
-		if (e == cudaSuccess && fine > 48 * 1024) e = cudaFuncSetAttribute(VoxBlockKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fine);
+		if (e == cudaSuccess && fine > 48 * 1024) e = cudaFuncSetAttribute(block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fine);
 		if (e != cudaSuccess) return e;
-		VoxCoarseKernel<<<(unsigned)(vg.NX * vg.NY * vg.NZ), 32, coarse, stream>>>(prog, s, vg, st, depth);
+		if (!direct)
+		{
+			VoxCoarseKernel<<<(unsigned)(vg.NX * vg.NY * vg.NZ), 32, coarse, stream>>>(prog, s, vg, st, depth);
+			e = cudaGetLastError();
+			if (e != cudaSuccess) return e;
+		}
+		block<<<sms * kVoxCtasPerSm, kVoxWarps * 32, fine, stream>>>(prog, s, vg, st, depth);
 		e = cudaGetLastError();
 		if (e != cudaSuccess) return e;
-		VoxBlockKernel<<<sms * kVoxCtasPerSm, kVoxWarps * 32, fine, stream>>>(prog, s, vg, st, depth);
-		e = cudaGetLastError();
-		if (e != cudaSuccess) return e;
-		VoxBoxKernel<<<sms * kVoxEvalCtasPerSm, kVoxWarps * 32, eval, stream>>>(prog, s, vg, st, words);
+		VoxBoxKernel<<<sms * kVoxEvalCtasPerSm, kVoxWarps * 32, eval, stream>>>(prog, s, vg, st, direct, words);
 		return cudaGetLastError();
 	}
 

@@ -111,6 +111,11 @@ namespace tg
 		int Distance, Surface;  // first quads of the cell's two programs
 		uint32_t Material;      // first event of the material list
 		uint32_t Brick;
+		// The space the part stands for: all of it descends to its cell, and its tape holds there.
+		// Its points' box and one lattice step more, towards the rest of the brick at least (a
+		// vertex may lie between two parts' points), as far as the cell goes.
+		float Lo[3], Hi[3];
+		uint32_t Pad[2];
 	};
 	constexpr int kBrickTapeCounters = 5;   // parts, parts taken for building, events, bricks evaluated, long parts
 	struct BrickTapes
@@ -264,6 +269,18 @@ namespace tg
 	size_t VoxelBrickWords(int sx, int sy, int sz);
 	// One bit per voxel (cell number order): |octree distance at the centre| < Diagonal.
 	cudaError_t LaunchCloudFlags(const DeviceProgram& prog, const CloudSpec& s, uint32_t* brick_bits, uint32_t* words, cudaStream_t stream);
+	// The same by shortened programs (tg_parts.cuh), where the tree's can be (CloudByTapes):
+	// one bit per kept voxel and the voxels listed by brick; counts: bricks, voxels.  Scratch:
+	// list and tops hold a word per brick (CloudBricks), voxels one per voxel.
+	bool CloudByTapes(const DeviceProgram& prog, const CloudSpec& s, double quads);
+	int64_t CloudBricks(const CloudSpec& s);
+	cudaError_t LaunchCloudVoxels(const DeviceProgram& prog, const CloudSpec& s, uint32_t* list, uint32_t* tops, const BrickTapes& tapes,
+		uint32_t* words, uint32_t* voxels, uint32_t* counts, int sms, cudaStream_t stream);
+	// Those n voxels' numbers, refined points and (where not null) normals and colours, each at
+	// its rank in the bits.
+	cudaError_t LaunchCloudPoints(const DeviceProgram& prog, const CloudSpec& s, const BrickTapes& tapes, const uint32_t* voxels, uint32_t n,
+		const uint32_t* words, const uint32_t* word_base, int iterations, uint32_t* cubes, float* points, float* normals, uint8_t* colors,
+		cudaStream_t stream);
 	// Refined point of each listed cell (*count of them, at most `capacity`).
 	cudaError_t LaunchCloudRefine(const DeviceProgram& prog, const CloudSpec& s, const uint32_t* cells, const uint32_t* count,
 		uint32_t capacity, int iterations, float* points, cudaStream_t stream);

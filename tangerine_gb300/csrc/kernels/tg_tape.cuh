@@ -52,41 +52,69 @@ namespace tg
 		return BrushDistance(op, prm, Vec3(x, y, z));
 	}
 
-	__device__ __forceinline__ float CommonBrushDistance(uint32_t op, const float (&prm)[3], Vec3 p)
-	{
-		switch (op)
-		{
-		case OpSphere: return SdSphere(p, prm[0]);
-		case OpBox: return SdBox(p, Vec3(prm[0], prm[1], prm[2]));
-		case OpTorus: return SdTorus(p, prm[0], prm[1]);
-		default: return SdCylinder(p, prm[0], prm[1]);
-		}
-	}
-
 	// BrushDistance2 and SetDistance2 (tg_pair.cuh), the same values from less code: the
 	// evaluations by tapes are short, and a kernel that holds several interpreters waited for
-	// instructions more than for anything else (10 of 18 stall cycles an issue in the vertex
-	// attributes with the three blends and three rare brushes expanded for every lane).
+	// instructions more than for anything else (10 to 12 of 17 stall cycles an issue in the
+	// vertex attributes and the point cloud's refinement with the formulas expanded one by one).
+	// The common brushes share their squares and roots: a sphere and a box end with the length
+	// of a 3-vector, a torus and a cylinder with that of a 2-vector made from one.  Kernels with
+	// one interpreter, whose warps run it in step, take the formulas one by one instead
+	// (Compact = false: the builds and the brick evaluation 4 to 5 % faster so, the refinement
+	// 20 % slower).
+	template<bool Compact = true>
 	__device__ __forceinline__ float2 TapeBrush2(uint32_t op, const float4& h, float2 x, float2 y, float2 z, const PairUnits& u)
 	{
-		switch (op)
-		{
-		case OpSphere: return SdSphere2(x, y, z, h.y, u);
-		case OpBox: return SdBox2(x, y, z, h.y, h.z, h.w, u);
-		case OpTorus: return SdTorus2(x, y, z, h.y, h.z, u);
-		case OpCylinder: return SdCylinder2(x, y, z, h.y, h.z, u);
-		case OpPlane: return SdPlane2(x, y, z, h.y, h.z, h.w, u);
-		default:
+		const bool round = op == OpTorus || op == OpCylinder;
+		if (op != OpSphere && op != OpBox && !round)
 			return make_float2(RareBrushDistance(op, h.y, h.z, h.w, x.x, y.x, z.x), RareBrushDistance(op, h.y, h.z, h.w, x.y, y.y, z.y));
+		if (!Compact)
+		{
+			if (op == OpSphere) return SdSphere2(x, y, z, h.y, u);
+			if (op == OpBox) return SdBox2(x, y, z, h.y, h.z, h.w, u);
+			return op == OpTorus ? SdTorus2(x, y, z, h.y, h.z, u) : SdCylinder2(x, y, z, h.y, h.z, u);
+		}
+		float2 last = Pair(-h.y), zz = z;
+		if (op == OpBox)
+		{
+			x = Sub2(Abs2(x), Pair(h.y), u);
+			y = Sub2(Abs2(y), Pair(h.z), u);
+			zz = Sub2(Abs2(z), Pair(h.w), u);
+			last = make_float2(fminf(fmaxf(fmaxf(x.x, y.x), zz.x), 0.0f), fminf(fmaxf(fmaxf(x.y, y.y), zz.y), 0.0f));
+			x = TernaryMax2(x, 0.0f);
+			y = TernaryMax2(y, 0.0f);
+			zz = TernaryMax2(zz, 0.0f);
+		}
+		float2 s = Add2(Mul2(x, x, u), Mul2(y, y, u), u);
+		if (!round) s = Add2(s, Mul2(zz, zz, u), u);
+#pragma unroll 1
+		for (int root = 0; ; ++root)
+		{
+			const float2 length = Sqrt2(s);
+			if (!round || root == 1) return Add2(length, last, u);
+			// The distance from the axis less the major radius (a cylinder's radius).
+			float2 a = Add2(length, Pair(-h.y), u), b = z;
+			last = Pair(-h.z);
+			if (op == OpCylinder)
+			{
+				b = Sub2(Abs2(z), Pair(h.z), u);
+				last = make_float2(fminf(fmaxf(a.x, b.x), 0.0f), fminf(fmaxf(a.y, b.y), 0.0f));
+				a = TernaryMax2(a, 0.0f);
+				b = TernaryMax2(b, 0.0f);
+			}
+			s = Add2(Mul2(a, a, u), Mul2(b, b, u), u);
 		}
 	}
 
-	// The blends share one term: the difference blends as the intersection with its right
-	// operand negated (|l + r| is |l - -r|).
+	static __device__ __noinline__ float TapeBlendTerm(float m, float h, float k, bool subtract) { return BlendTerm(m, h, k, subtract); }
+
+	// The blends share one term, out of line where it is not zero: the difference blends as the
+	// intersection with its right operand negated (|l + r| is |l - -r|).
 	__device__ __forceinline__ float TapeBlend(bool unions, float l, float r, float k)
 	{
 		const float m = unions ? fminf(l, r) : fmaxf(l, r);
-		return BlendTerm(m, fmaxf(k - fabsf(l - r), 0.0f), k, unions);
+		const float h = fmaxf(k - fabsf(l - r), 0.0f);
+		if (h == 0.0f && k > 0.0f) return unions ? m - 0.0f : m + 0.0f;
+		return TapeBlendTerm(m, h, k, unions);
 	}
 
 	__device__ __forceinline__ float2 TapeSet2(uint32_t op, float2 l, float2 r, float k)
@@ -101,9 +129,12 @@ namespace tg
 		return make_float2(fmaxf(l.x, r.x), fmaxf(l.y, r.y));
 	}
 
+	// Transform::ApplyInv's division by a brush's scale, out of line: most brushes have none.
+	static __device__ __noinline__ float2 DividePair(float2 a, float s) { return make_float2(a.x / s, a.y / s); }
+
 	// A brush's distance (RunDistancePairs' step) from its record at `pc`, whose head is known;
 	// q is left at the points in the brush's own frame, h at the record's first quad.
-	template<int NP, typename Load>
+	template<int NP, bool Compact = true, typename Load>
 	__device__ __forceinline__ void BrushStep(Load load, int pc, uint32_t head, const float2 (&px)[NP], const float2 (&py)[NP],
 		const float2 (&pz)[NP], const PairUnits& u, float2 (&qx)[NP], float2 (&qy)[NP], float2 (&qz)[NP], float4& h, float2 (&d)[NP])
 	{
@@ -135,7 +166,7 @@ namespace tg
 			}
 		}
 #pragma unroll
-		for (int j = 0; j < NP; ++j) d[j] = TapeBrush2(head & 0xFFu, h, qx[j], qy[j], qz[j], u);
+		for (int j = 0; j < NP; ++j) d[j] = TapeBrush2<Compact>(head & 0xFFu, h, qx[j], qy[j], qz[j], u);
 		if (head & RecScale)
 		{
 			const float4 S = load(at);
@@ -148,7 +179,7 @@ namespace tg
 	// program at `base`; `event(i)` returns event i (from global or shared memory).  Operands
 	// below the top of the stack are at spill[(depth * NP + pair) * stride].  The set
 	// operator's code appears once: a brush that is its right operand falls through to it.
-	template<int NP, typename Load, typename Event>
+	template<int NP, bool Compact = true, typename Load, typename Event>
 	__device__ __forceinline__ void RunTapePairs(Load load, int base, Event event, uint32_t count, const float2 (&px)[NP],
 		const float2 (&py)[NP], const float2 (&pz)[NP], const PairUnits& u, float2 (&acc)[NP], float2* spill, int stride)
 	{
@@ -178,7 +209,7 @@ namespace tg
 				for (int j = 0; j < NP; ++j) left[j] = acc[j];
 				float2 qx[NP], qy[NP], qz[NP];
 				float4 h;
-				BrushStep<NP>(load, at, head, px, py, pz, u, qx, qy, qz, h, acc);
+				BrushStep<NP, Compact>(load, at, head, px, py, pz, u, qx, qy, qz, h, acc);
 				if (e >= count) break;
 				if (!(head & RecThenSet)) continue;
 				op = x & 0xFFu;
@@ -226,6 +257,7 @@ namespace tg
 
 	// A brush's distance in a surface program (RunSurfacePair's step): T the translation and
 	// scale, Q the inverse quaternion as (w, x, y, z).
+	template<bool Compact = true>
 	__device__ __forceinline__ float2 SurfaceBrushStep(uint32_t op, const float4& h, const float4& Q, const float4& T, float2 px, float2 py,
 		float2 pz, const PairUnits& u)
 	{
@@ -239,11 +271,11 @@ namespace tg
 		const bool scaled = T.w != 1.0f;    // x / 1 and x * 1 are x exactly
 		if (scaled)
 		{
-			lx = make_float2(lx.x / T.w, lx.y / T.w);
-			ly = make_float2(ly.x / T.w, ly.y / T.w);
-			lz = make_float2(lz.x / T.w, lz.y / T.w);
+			lx = DividePair(lx, T.w);
+			ly = DividePair(ly, T.w);
+			lz = DividePair(lz, T.w);
 		}
-		const float2 d = TapeBrush2(op, h, lx, ly, lz, u);
+		const float2 d = TapeBrush2<Compact>(op, h, lx, ly, lz, u);
 		return scaled ? Mul2(d, Pair(T.w), u) : d;
 	}
 
@@ -317,6 +349,93 @@ namespace tg
 		}
 	}
 
+	// RunTapePairs<1> (surface = false) or RunSurfaceTapePairs<1> (surface = true) from one copy
+	// of code, for a kernel that runs both.
+	template<typename Load, typename Event>
+	__device__ __forceinline__ float2 RunEitherTapePair(bool surface, Load load, int base, Event event, uint32_t count, float2 px, float2 py,
+		float2 pz, const PairUnits& u, float2* spill, int stride)
+	{
+		float2 acc = make_float2(0.0f, 0.0f), left = acc;
+		int depth = 0;
+		uint32_t e = 0;
+		uint2 ev = event(0u);
+		for (;;)
+		{
+			uint32_t op = ev.x & 0xFFu;
+			int at = base + (surface ? (int)ev.y : (int)(ev.x >> 16));
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const uint32_t head = ev.x;
+				if (++e < count) ev = event(e);
+				if (!(head & RecThenSet))
+				{
+					if (depth > 0) spill[(depth - 1) * stride] = acc;
+					++depth;
+				}
+				left = acc;
+				const float4 h = load(at);
+				float2 qx = px, qy = py, qz = pz;
+				float scale = 1.0f;
+				if (surface)
+				{
+					const float4 Q = load(at + 1), T = load(at + 2);
+					const float2 vx = Sub2(px, Pair(T.x), u), vy = Sub2(py, Pair(T.y), u), vz = Sub2(pz, Pair(T.z), u);
+					float2 ux, uy, uz, wx, wy, wz;
+					CrossPair(Q.y, Q.z, Q.w, vx, vy, vz, ux, uy, uz, u);
+					CrossPair(Q.y, Q.z, Q.w, ux, uy, uz, wx, wy, wz, u);
+					qx = Add2(vx, Mul2(Add2(Mul2(ux, Pair(Q.x), u), wx, u), Pair(2.0f), u), u);
+					qy = Add2(vy, Mul2(Add2(Mul2(uy, Pair(Q.x), u), wy, u), Pair(2.0f), u), u);
+					qz = Add2(vz, Mul2(Add2(Mul2(uz, Pair(Q.x), u), wz, u), Pair(2.0f), u), u);
+					scale = T.w;
+					if (scale != 1.0f)
+					{
+						qx = DividePair(qx, scale);
+						qy = DividePair(qy, scale);
+						qz = DividePair(qz, scale);
+					}
+				}
+				else
+				{
+					++at;
+					if (head & RecMatrix)
+					{
+						const float4 X = load(at), Y = load(at + 1), Z = load(at + 2);
+						at += 3;
+						qx = AffineRow2(X, px, py, pz, u);
+						qy = AffineRow2(Y, px, py, pz, u);
+						qz = AffineRow2(Z, px, py, pz, u);
+					}
+					else if (head & RecOffset)
+					{
+						const float4 O = load(at++);
+						qx = Add2(px, Pair(O.x), u);
+						qy = Add2(py, Pair(O.y), u);
+						qz = Add2(pz, Pair(O.z), u);
+					}
+					if (head & RecScale) scale = load(at).x;
+				}
+				acc = TapeBrush2(op, h, qx, qy, qz, u);
+				// x * 1 is x exactly; a scale record of 1 multiplies the same.
+				if (scale != 1.0f) acc = Mul2(acc, Pair(scale), u);
+				if (e >= count) break;
+				if (!(head & RecThenSet)) continue;
+				op = ev.x & 0xFFu;
+				at = base + (surface ? (int)ev.y : (int)(ev.x >> 16));
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+				left = spill[(depth - 1) * stride];
+			}
+			if (op >= OpUnion && op <= OpBlendDiff) acc = TapeSet2(op, left, acc, op >= OpBlendUnion ? load(at).y : 0.0f);
+			else if (op == OpFlate) acc = Sub2(acc, Pair(load(at).y), u);
+			else acc = op == OpTapeNegate ? make_float2(-acc.x, -acc.y) : make_float2(acc.x + 0.0f, acc.y + 0.0f);
+			if (++e >= count) break;
+			ev = event(e);
+		}
+		return acc;
+	}
+
 	// The whole surface program at one pair of points, and GetMaterial's walk of it at one
 	// point: where there is no tape.
 	static __device__ __noinline__ float2 RunWholeSurfacePair(const float4* __restrict__ code, int pc, float2 px, float2 py, float2 pz,
@@ -338,7 +457,8 @@ namespace tg
 	// material, so intersections and blends choose by distance): the material list of a tape.
 	// `spill` as RunSurfaceBatch<1>'s, which other threads of the block may run meanwhile.
 	template<typename Load, typename Event>
-	__device__ __forceinline__ int RunMaterialTape(Load load, int base, Event event, uint32_t count, Vec3 p, float* spill, int stride)
+	__device__ __forceinline__ int RunMaterialTape(Load load, int base, Event event, uint32_t count, Vec3 p, const PairUnits& u, float* spill,
+		int stride)
 	{
 		// One brush left: its material, whatever its distance.
 		if (count == 1) return __float_as_int(load(base + (int)event(0u).y + 3).x);
@@ -365,14 +485,7 @@ namespace tg
 					++depth;
 				}
 				const float4 h = load(at), Q = load(at + 1), T = load(at + 2), M = load(at + 3);
-				const Quat qi{ Q.x, Q.y, Q.z, Q.w };
-				Vec3 local = Rotate(qi, p - Vec3(T.x, T.y, T.z));
-				const bool scaled = T.w != 1.0f;
-				if (scaled) local = local / T.w;
-				const float prm[3] = { h.y, h.z, h.w };
-				acc = op == OpSphere || op == OpBox || op == OpTorus || op == OpCylinder ? CommonBrushDistance(op, prm, local)
-					: RareBrushDistance(op, h.y, h.z, h.w, local.x, local.y, local.z);
-				if (scaled) acc = acc * T.w;
+				acc = SurfaceBrushStep(op, h, Q, T, Pair(p.x), Pair(p.y), Pair(p.z), u).x;
 				macc = __float_as_int(M.x);
 				if (!thenSet) continue;
 				if (e >= count) break;
@@ -393,8 +506,7 @@ namespace tg
 				continue;
 			}
 			const float k = op >= OpBlendUnion ? load(at).y : 0.0f;
-			const float2 both = TapeSet2(op, make_float2(left, left), make_float2(acc, acc), k);
-			const float d = both.x;
+			const float d = TapeSet2(op, Pair(left), Pair(acc), k).x;
 			// SetNode::GetMaterial (sdf_evaluator.cpp:957-1012).
 			const bool blend = op == OpBlendUnion || op == OpBlendInter;
 			const bool takeLeft = (op == OpDiff || op == OpBlendDiff) || (blend ? (fabsf(left - d) <= fabsf(acc - d)) : (d == left));
@@ -472,7 +584,7 @@ namespace tg
 			const float2 x[1] = { px }, y[1] = { py }, z[1] = { pz };
 			float2 qx[1], qy[1], qz[1], d[1];
 			float4 h;
-			BrushStep<1>([&](int q) { return In.Load(q); }, Pc, head, x, y, z, u, qx, qy, qz, h, d);
+			BrushStep<1, false>([&](int q) { return In.Load(q); }, Pc, head, x, y, z, u, qx, qy, qz, h, d);
 			const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
 			size = make_float2(fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(d[0].x),
 				fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(d[0].y));
@@ -510,7 +622,7 @@ namespace tg
 		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
 		{
 			const float4 h = In.Load(Pc), T = In.Load(Pc + 2);
-			const float2 d = SurfaceBrushStep(head & 0xFFu, h, In.Load(Pc + 1), T, px, py, pz, u);
+			const float2 d = SurfaceBrushStep<false>(head & 0xFFu, h, In.Load(Pc + 1), T, px, py, pz, u);
 			size = SurfaceBrushSize(h, T, px, py, pz, d);
 			return d;
 		}
@@ -583,7 +695,7 @@ namespace tg
 		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
 		{
 			const float4 h = Quad(0), T = Quad(2);
-			const float2 d = SurfaceBrushStep(head & 0xFFu, h, Quad(1), T, px, py, pz, u);
+			const float2 d = SurfaceBrushStep<false>(head & 0xFFu, h, Quad(1), T, px, py, pz, u);
 			size = SurfaceBrushSize(h, T, px, py, pz, d);
 			return d;
 		}
@@ -602,7 +714,6 @@ namespace tg
 	{
 		int Value, Material;
 		bool Same;              // no difference was decided by its right operand: one list serves both
-		int Sign;               // 1 or -1: the program keeps that sign in the box; 0: it may not
 		float2 Distance;        // the program's values at this lane's two points,
 		float2 Error;           // and the part of their rounding that grows with the operands
 	};
@@ -749,10 +860,6 @@ namespace tg
 		out.Same = same;
 		out.Distance = acc;
 		out.Error = make_float2(2e-5f * size.x, 2e-5f * size.y);
-		// |f| beyond a ball's radius (half the reach covers it) at every centre: no sign change.
-		const float2 far = make_float2(0.5f * reach + out.Error.x, 0.5f * reach + out.Error.y);
-		out.Sign = __all_sync(0xFFFFFFFFu, acc.x > far.x && acc.y > far.y) ? 1
-			: __all_sync(0xFFFFFFFFu, acc.x < -far.x && acc.y < -far.y) ? -1 : 0;
 		return true;
 	}
 

@@ -91,3 +91,35 @@ def test_voxel_blocks_match_oracle(lib, port, prims, ops, grid):
         vox, gsize, _ = prog.export_voxels(grid, 3)
     np.testing.assert_array_equal(vox, want)
     assert gsize == size
+
+
+@pytest.mark.parametrize("prims,ops,paint,step,refine", [(200, ALL_OPS, True, (0.021, 0.027, 0.019), 4), (200, W.OPS_60_20_10_10, False, 0.021, 0),
+                                                         (100, ALL_OPS, True, 0.02, 1)])
+def test_point_cloud_tapes_match_oracle(lib, port, prims, ops, paint, step, refine):
+    """Lattices past the size from which the cloud goes by tapes, bricks cut on every axis;
+    refined points leave their voxel's brick and its parts on the way."""
+    seed = 21
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops, paint=paint))):
+        seed += 1
+    h = port.build(spec)
+    o = port.octree(h)
+    try:
+        b = port.bounds(h)
+        points, cells = port.point_cloud(o, b[:3], b[3:], step, refine)
+        normals, colors = port.vertex_attributes(o, points)
+    finally:
+        port.octree_free(o)
+        port.free(h)
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        bricks = np.prod(np.ceil((b[3:] - b[:3]) / np.asarray(step) / 8))
+        quads = prog.info().distance_quads / prog.info().octree_cells
+        assert bricks * (quads - 12) > 45000
+        m = prog.export_point_cloud(b[:3], b[3:], step, refine)
+    assert points.shape[0] > 1000
+    np.testing.assert_array_equal(m.cubes, cells.astype(np.uint32))
+    np.testing.assert_array_equal(m.vertices, points)
+    np.testing.assert_array_equal(m.normals, normals)
+    if paint:
+        np.testing.assert_array_equal(m.colors, colors)
+    else:
+        assert m.colors is None
