@@ -759,8 +759,19 @@ namespace tg
 		}
 		else
 		{
+			const OctNode& root = p.Host.Nodes[0];
+			const int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px);
+			BrickTapes tapes{};
+			if (bricks)
+			{
+				TG_TRY(ReadSmCount());
+				TG_TRY(ReserveTapes((int64_t)bricks * bricks * bricks, tapes));
+			}
 			Begin("render", s);
-			TG_TRY(LaunchRender(p.View, Cameras.As<CameraBasis>(), count, width, height, steps, epsilon, exact, dDepth, dNormals, dColors, s));
+			if (bricks)
+				TG_TRY(LaunchRenderTapes(p.View, root.Pivot, root.ClipRadius, bricks, tapes, Cameras.As<CameraBasis>(), count, width, height, steps,
+					epsilon, dDepth, dNormals, dColors, SmCount, s));
+			else TG_TRY(LaunchRender(p.View, Cameras.As<CameraBasis>(), count, width, height, steps, epsilon, exact, dDepth, dNormals, dColors, s));
 			End(s);
 		}
 		if (!out_is_device)

@@ -190,6 +190,14 @@ namespace tg
 	// Achieved FP32 fused-multiply-add throughput of this GPU (TFLOP/s, 2 flops per FMA).
 	cudaError_t MeasureFp32Peak(double* tflops, cudaStream_t stream);
 
+	// LaunchRender's octree-bounded form by tapes of the root cube's bricks (the same steps and
+	// images): how many bricks per axis pay for that many pixels (0: none), and the launch, with
+	// the tapes' buffers for bricks^3 bricks.  pivot, root_clip: the root cell's.
+	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels);
+	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes,
+		const CameraBasis* cameras, int count, int width, int height, int max_steps, float epsilon, float* depth, float* normals,
+		uint8_t* colors, int sms, cudaStream_t stream);
+
 	// The order the attribute passes visit the vertices in.  Cells == nullptr: vertex order.
 	// Otherwise the active-cell list of the culled export (its cells grouped by brick): entry t
 	// is the vertex of cell Cells[t], numbered as the cell passes number it (rank of the

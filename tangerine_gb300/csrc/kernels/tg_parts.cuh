@@ -200,13 +200,13 @@ namespace tg
 		__global__ void __launch_bounds__(kThreads) BrickPartsKernel(DeviceProgram prog, L lat, const uint32_t* __restrict__ list,
 			const uint32_t* __restrict__ count, const uint32_t* __restrict__ tops, BrickTapes tapes)
 		{
-			const uint32_t n = *count;
+			const uint32_t n = count ? *count : (uint32_t)lat.Bricks(0) * (uint32_t)lat.Bricks(1) * (uint32_t)lat.Bricks(2);
 			const int lane = (int)(threadIdx.x & 31), corner = lane & 7;
 			for (uint32_t base = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * 4u; base < n; base += gridDim.x * kWarps * 4u)
 			{
 				const uint32_t item = base + (uint32_t)(lane >> 3);
 				const bool live = item < n;
-				const uint32_t b = live ? __ldg(list + item) : 0u;
+				const uint32_t b = live ? (list ? __ldg(list + item) : item) : 0u;
 				int first3[3], extent[3];
 				BrickSpan(lat, b, first3, extent);
 				const int i0 = first3[0], j0 = first3[1], k0 = first3[2], ex = extent[0], ey = extent[1], ez = extent[2];
@@ -421,6 +421,7 @@ namespace tg
 		// What a point runs: its part's lists over its cell's surface and distance programs.
 		struct PointRun
 		{
+			int Cell;
 			int Surface, Distance;          // first quads
 			uint32_t Value, Material;       // first events
 			uint32_t Events, Walk;          // events of the two lists (kNoTape: the whole program)
@@ -443,6 +444,7 @@ namespace tg
 				run.Hi[0] = __uint_as_float(a.w); run.Hi[1] = __uint_as_float(b.x); run.Hi[2] = __uint_as_float(b.y);
 				if (!InRun(run, p)) continue;
 				const uint4 c = __ldg(part), d = __ldg(part + 1);
+				run.Cell = (int)c.x;
 				run.Value = c.z;
 				run.Events = c.w & 0xFFFFu;
 				run.Walk = c.w >> 16;
@@ -458,6 +460,7 @@ namespace tg
 		__device__ __forceinline__ void RunWhole(const DeviceProgram& prog, Vec3 p, PointRun& run)
 		{
 			const int cell = DescendOctree(prog.Nodes, p.x, p.y, p.z);
+			run.Cell = cell;
 			run.Surface = __ldg(&prog.Nodes[cell].SurfaceCode);
 			run.Distance = __ldg(&prog.Nodes[cell].DistanceCode);
 			run.Events = run.Walk = kNoTape;
@@ -533,7 +536,7 @@ namespace tg
 			return (size_t)(prog.MaxStack > 1 ? prog.MaxStack - 1 : 1) * pairs;
 		}
 
-		// Parts and tapes of the listed bricks of a lattice.
+		// Parts and tapes of the listed bricks of a lattice (list and count null: of all bricks).
 		template<typename L>
 		inline cudaError_t LaunchParts(const DeviceProgram& prog, const L& lat, const uint32_t* list, const uint32_t* count, const uint32_t* tops,
 			const BrickTapes& tapes, int sms, cudaStream_t stream)

@@ -244,6 +244,84 @@ namespace tg
 		}
 	}
 
+	// The distance at one point by a tape (RunTapePairs, one lane).  Operands below the top of
+	// the stack are at spill[depth * stride].
+	template<typename Load, typename Event>
+	__device__ __forceinline__ float RunTapePoint(Load load, int base, Event event, uint32_t count, float px, float py, float pz, float* spill,
+		int stride)
+	{
+		float acc = 0.0f, left = 0.0f;
+		int depth = 0;
+		uint32_t e = 0, x = event(0u).x;
+		for (;;)
+		{
+			uint32_t op = x & 0xFFu;
+			int at = base + (int)(x >> 16);
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const uint32_t head = x;
+				if (++e < count) x = event(e).x;
+				if (!(head & RecThenSet))
+				{
+					if (depth > 0) spill[(depth - 1) * stride] = acc;
+					++depth;
+				}
+				left = acc;
+				const float4 h = load(at++);
+				float qx = px, qy = py, qz = pz;
+				if (head & RecMatrix)
+				{
+					const float4 X = load(at), Y = load(at + 1), Z = load(at + 2);
+					at += 3;
+					qx = (X.x * px + X.y * py) + (X.z * pz + X.w);
+					qy = (Y.x * px + Y.y * py) + (Y.z * pz + Y.w);
+					qz = (Z.x * px + Z.y * py) + (Z.z * pz + Z.w);
+				}
+				else if (head & RecOffset)
+				{
+					const float4 O = load(at++);
+					qx = px + O.x; qy = py + O.y; qz = pz + O.z;
+				}
+				const Vec3 q(qx, qy, qz);
+				if (op == OpSphere) acc = SdSphere(q, h.y);
+				else if (op == OpBox) acc = SdBox(q, Vec3(h.y, h.z, h.w));
+				else if (op == OpTorus) acc = SdTorus(q, h.y, h.z);
+				else if (op == OpCylinder) acc = SdCylinder(q, h.y, h.z);
+				else acc = RareBrushDistance(op, h.y, h.z, h.w, qx, qy, qz);
+				if (head & RecScale) acc = acc * load(at).x;
+				if (e >= count) break;
+				if (!(head & RecThenSet)) continue;
+				op = x & 0xFFu;
+				at = base + (int)(x >> 16);
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+				left = spill[(depth - 1) * stride];
+			}
+			if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				const float r = op == OpDiff || op == OpBlendDiff ? -acc : acc;
+				if (op >= OpBlendUnion) acc = TapeBlend(op == OpBlendUnion, left, r, load(at).y);
+				else acc = op == OpUnion ? fminf(left, r) : fmaxf(left, r);
+			}
+			else if (op == OpFlate) acc = acc - load(at).y;
+			else acc = op == OpTapeNegate ? -acc : acc + 0.0f;
+			if (++e >= count) break;
+			x = event(e).x;
+		}
+		return acc;
+	}
+
+	// The whole distance program at one point.
+	static __device__ __noinline__ float RunWholePoint(const float4* __restrict__ code, int pc, float x, float y, float z, float* spill, int stride)
+	{
+		const float px[1] = { x }, py[1] = { y }, pz[1] = { z };
+		float d[1];
+		RunDistance<1>(code, pc, px, py, pz, d, spill, stride);
+		return d[0];
+	}
+
 	// The whole distance program at one pair of points, where there is no tape.  Out of line:
 	// rare beside the tapes, and the callers' code stays small.
 	static __device__ __noinline__ float2 RunWholePair(const float4* __restrict__ code, int pc, float2 px, float2 py, float2 pz, float2* spill,

@@ -18,12 +18,14 @@
 #include "tg_device.cuh"
 #include "tg_kernels.hpp"
 #include "tg_trace.cuh"
+#include "tg_parts.cuh"
 
 namespace tg
 {
 	namespace
 	{
 		constexpr int kTraceThreads = 128;
+		constexpr int kTileX = 16, kTileY = 8;     // pixels of a block
 
 		// SDFNode::RayMarch on the whole tree.
 		__device__ __forceinline__ March MarchExact(const DeviceProgram& prog, Vec3 start, Vec3 dir_in, int iterations, float epsilon,
@@ -187,6 +189,130 @@ namespace tg
 			}
 		}
 
+		// The root cube in bricks for the renderer's tapes: 8^3 points a brick at the centres of
+		// the cube's (8 N)^3 cells.  The octree halves the cube, so a brick lies in one cell where
+		// the cells are no smaller.
+		struct RenderLattice
+		{
+			static constexpr int kStride = parts::kBox;
+			static constexpr bool kOutside = true;
+			float Origin[3];
+			float Step;
+			int N;
+			__device__ __forceinline__ float Coord(int a, int i) const { return Origin[a] + ((float)i + 0.5f) * Step; }
+			__host__ __device__ __forceinline__ int Points(int) const { return N * parts::kBox; }
+			__host__ __device__ __forceinline__ int Bricks(int) const { return N; }
+			__device__ __forceinline__ float Keep() const { return INFINITY; }
+			__device__ __forceinline__ uint32_t BrickAt(Vec3 p) const
+			{
+				const float over = 1.0f / (Step * (float)parts::kBox);
+				const float most = (float)(N - 1);
+				const uint32_t x = (uint32_t)fminf(fmaxf((p.x - Origin[0]) * over, 0.0f), most);
+				const uint32_t y = (uint32_t)fminf(fmaxf((p.y - Origin[1]) * over, 0.0f), most);
+				const uint32_t z = (uint32_t)fminf(fmaxf((p.z - Origin[2]) * over, 0.0f), most);
+				return x + (uint32_t)N * (y + (uint32_t)N * z);
+			}
+		};
+
+		// MarchBounded by the bricks' tapes: the same distances, and so the same steps.
+		__device__ __forceinline__ March MarchTapes(const DeviceProgram& prog, const RenderLattice& lat, const BrickTapes& tapes, Vec3 start,
+			Vec3 dir_in, int iterations, float epsilon, float* spill, parts::PointRun& run)
+		{
+			const Vec3 dir = Normalize(dir_in);
+			const float rootClip = fabsf(__ldg(&prog.Nodes[0].ClipRadius));
+			const Vec3 root(__ldg(&prog.Nodes[0].Pivot[0]), __ldg(&prog.Nodes[0].Pivot[1]), __ldg(&prog.Nodes[0].Pivot[2]));
+			const float half = rootClip * 0.57735f;               // root cube half-width
+			// Leaving the root sphere along the ray ends the march: nothing lies beyond.
+			const Vec3 oc = start - root;
+			const float b = Dot(oc, dir);
+			const float c = Dot(oc, oc) - rootClip * rootClip;
+			const float disc = b * b - c;
+			if (disc < 0.0f) return { false, INFINITY, start };
+			const float exitTravel = -b + sqrtf(disc);
+			if (exitTravel < 0.0f) return { false, INFINITY, start };
+			const float4* code = prog.Code;
+			Vec3 pos = start;
+			float travel = 0.0f;
+			run.Lo[0] = 1.0f; run.Hi[0] = 0.0f;
+			for (int i = 0; i < iterations; ++i)
+			{
+				const Vec3 off = pos - root;
+				const float ox = fmaxf(fabsf(off.x) - half, 0.0f), oy = fmaxf(fabsf(off.y) - half, 0.0f), oz = fmaxf(fabsf(off.z) - half, 0.0f);
+				float step = sqrtf(ox * ox + oy * oy + oz * oz);
+				if (!(step > epsilon))
+				{
+					if (!parts::InRun(run, pos) && !parts::FindPart(tapes, __ldg(tapes.Bricks + lat.BrickAt(pos)), pos, run))
+						parts::RunWhole(prog, pos, run);
+					float f;
+					if (run.Events != kNoTape)
+					{
+						const uint2* ev = tapes.Events + run.Value;
+						f = RunTapePoint([&](int q) { return __ldg(code + q); }, run.Distance, [&](uint32_t e) { return __ldg(ev + e); }, run.Events,
+							pos.x, pos.y, pos.z, spill, 2 * kTraceThreads);
+					}
+					else f = RunWholePoint(code, run.Distance, pos.x, pos.y, pos.z, spill, 2 * kTraceThreads);
+					if (f <= epsilon) return { true, travel, pos };
+					const OctNode* n = prog.Nodes + run.Cell;
+					const Vec3 dp = pos - Vec3(__ldg(&n->Pivot[0]), __ldg(&n->Pivot[1]), __ldg(&n->Pivot[2]));
+					const float room = __ldg(&n->ClipRadius) - Length(dp);
+					step = fminf(f, fmaxf(room, epsilon));
+				}
+				travel = travel + step;
+				if (travel > exitTravel) break;
+				pos = dir * travel + start;
+			}
+			return { false, INFINITY, pos };
+		}
+
+		__device__ __forceinline__ Vec3 PixelRay(const CameraBasis& cam, int x, int y, int width, int height)
+		{
+			const float u = ((2.0f * ((float)x + 0.5f) / (float)width) - 1.0f) * cam.TanHalfFov * cam.Aspect;
+			const float v = (1.0f - 2.0f * ((float)y + 0.5f) / (float)height) * cam.TanHalfFov;
+			const Vec3 fwd(cam.Forward[0], cam.Forward[1], cam.Forward[2]);
+			const Vec3 right(cam.Right[0], cam.Right[1], cam.Right[2]);
+			const Vec3 up(cam.Up[0], cam.Up[1], cam.Up[2]);
+			return (fwd + right * u) + up * v;
+		}
+
+		// RenderKernel's octree-bounded form by tapes.  A warp takes 8 x 4 pixels: neighbouring
+		// rays mostly share bricks, in a row of 32 they part sooner.
+		__global__ void __launch_bounds__(kTraceThreads, 8) RenderTapesKernel(DeviceProgram prog, RenderLattice lat, BrickTapes tapes,
+			const CameraBasis* __restrict__ cams, int count, int width, int height, int steps, float epsilon, float* __restrict__ depth,
+			float* __restrict__ normals, uint8_t* __restrict__ colors)
+		{
+			extern __shared__ __align__(16) float2 spill2[];
+			const int tilesX = (width + kTileX - 1) / kTileX, tilesY = (height + kTileY - 1) / kTileY;
+			const int tile = (int)(blockIdx.x % (unsigned)(tilesX * tilesY)), c = (int)(blockIdx.x / (unsigned)(tilesX * tilesY));
+			const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+			const int x = (tile % tilesX) * kTileX + (warp & 1) * 8 + (lane & 7), y = (tile / tilesX) * kTileY + (warp >> 1) * 4 + (lane >> 3);
+			if (x >= width || y >= height || c >= count) return;
+			const int64_t t = ((int64_t)c * height + y) * width + x;
+			const CameraBasis& cam = cams[c];
+			float2* spill = spill2 + threadIdx.x;
+			parts::PointRun run;
+			const March m = MarchTapes(prog, lat, tapes, Vec3(cam.Position[0], cam.Position[1], cam.Position[2]), PixelRay(cam, x, y, width, height),
+				steps, epsilon, reinterpret_cast<float*>(spill), run);
+			depth[t] = m.Travel;
+			Vec3 n(0.0f, 0.0f, 0.0f);
+			uchar4 col = make_uchar4(0, 0, 0, 0);
+			if (m.Hit)
+			{
+				const PairUnits units = LoadPairUnits();
+				float none;
+				n = parts::RunGradient<false>(prog, tapes, run, m.Position, units, spill, false, none);
+				if (colors) col = parts::RunColor(prog, tapes, run, m.Position, units, spill);
+			}
+			normals[t * 3] = n.x;
+			normals[t * 3 + 1] = n.y;
+			normals[t * 3 + 2] = n.z;
+			if (colors)
+			{
+				colors[t * 3] = col.x;
+				colors[t * 3 + 1] = col.y;
+				colors[t * 3 + 2] = col.z;
+			}
+		}
+
 		size_t TraceSpillBytes(const DeviceProgram& prog)
 		{
 			const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
@@ -244,6 +370,44 @@ namespace tg
 		if (smem > 48 * 1024) cudaFuncSetAttribute(RenderKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 		RenderKernel<<<(unsigned)((total + kTraceThreads - 1) / kTraceThreads), kTraceThreads, smem, stream>>>(
 			prog, cameras, count, width, height, max_steps, epsilon, exact || !prog.Lipschitz, depth, normals, colors);
+		return cudaGetLastError();
+	}
+
+	// Bricks per axis for the renderer's tapes, 0 for none.  A tape costs a pass of its cell's
+	// program at 64 points; a pixel takes some fifteen, thirty-two pixels at a time.
+	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels)
+	{
+		if (!prog.Lipschitz || !(prog.Form & kFormPrunable)) return 0;
+		const float span = 2.0f * fabsf(root_clip) * 0.57735f;
+		// The cells' edge: the cube halved until no more than the octree's target.
+		int cells = 1;
+		while (cells < 128 && span / (float)cells > 0.25f) cells *= 2;
+		const int n = cells < 32 ? 32 : cells;
+		return n <= 64 && pixels >= 16 * (int64_t)n * n * n ? n : 0;
+	}
+
+	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes,
+		const CameraBasis* cameras, int count, int width, int height, int max_steps, float epsilon, float* depth, float* normals,
+		uint8_t* colors, int sms, cudaStream_t stream)
+	{
+		RenderLattice lat;
+		const float half = fabsf(root_clip) * 0.57735f;
+		lat.N = bricks;
+		lat.Step = 2.0f * half / (float)(bricks * parts::kBox);
+		for (int a = 0; a < 3; ++a) lat.Origin[a] = pivot[a] - half;
+		cudaError_t e = parts::LaunchParts(prog, lat, nullptr, nullptr, nullptr, tapes, sms, stream);
+		if (e != cudaSuccess) return e;
+		// The colour's walk takes two words a level, the gradient one pair.
+		const size_t smem = parts::SpillPairs(prog, 2) * kTraceThreads * sizeof(float2);
+		if (smem > 48 * 1024)
+		{
+			e = cudaFuncSetAttribute(RenderTapesKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			if (e != cudaSuccess) return e;
+		}
+		const int64_t blocks = (int64_t)((width + kTileX - 1) / kTileX) * ((height + kTileY - 1) / kTileY) * count;
+		if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
+		RenderTapesKernel<<<(unsigned)blocks, kTraceThreads, smem, stream>>>(prog, lat, tapes, cameras, count, width, height, max_steps, epsilon,
+			depth, normals, colors);
 		return cudaGetLastError();
 	}
 }

@@ -123,3 +123,21 @@ def test_point_cloud_tapes_match_oracle(lib, port, prims, ops, paint, step, refi
         np.testing.assert_array_equal(m.colors, colors)
     else:
         assert m.colors is None
+
+
+@pytest.mark.parametrize("prims,ops", [(3, ALL_OPS), (150, ALL_OPS), (600, W.OPS_60_20_10_10)])
+def test_render_by_tapes_equals_render_without(lib, prims, ops):
+    """Enough pixels together go by the root cube's tapes; the same poses one by one do not.
+    Odd image sides, a camera inside the root cube, one that misses it."""
+    seed = 31
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops))):
+        seed += 1
+    poses = np.concatenate([W.camera_poses(7, 7), [[0.3, 0.2, 0.1], [60.0, 50.0, 70.0]]]).astype(np.float32)
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        depth, normals, colors = prog.render(sdf.cameras(poses), 333, 241)
+        assert poses.shape[0] * 333 * 241 >= 16 * 32 ** 3 and np.isfinite(depth).any()
+        for i, p in enumerate(poses):
+            d, n, c = prog.render(sdf.cameras(p[None]), 333, 241)
+            np.testing.assert_array_equal(d[0], depth[i])
+            np.testing.assert_array_equal(n[0], normals[i])
+            np.testing.assert_array_equal(c[0], colors[i])
