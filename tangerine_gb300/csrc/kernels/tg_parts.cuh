@@ -469,8 +469,9 @@ namespace tg
 		}
 
 		// SDFNode::Gradient at p (the four points as two pairs) and, with Distance, the cell's
-		// distance program there.  `spill`: this thread's column, kThreads pairs apart.
-		template<bool Distance>
+		// distance program there.  `spill`: this thread's column, Stride
+		// pairs apart.
+		template<bool Distance, int Stride = kThreads>
 		__device__ __forceinline__ Vec3 RunGradient(const DeviceProgram& prog, const BrickTapes& tapes, const PointRun& run, Vec3 p,
 			const PairUnits& units, float2* spill, bool wanted, float& distance)
 		{
@@ -491,11 +492,11 @@ namespace tg
 				{
 					if constexpr (Distance)
 						r[0] = RunEitherTapePair(surface, load, surface ? run.Surface : run.Distance, event, run.Events, px[0], py[0], pz[0], units, spill,
-							kThreads);
-					else RunSurfaceTapePairs<1>(load, run.Surface, event, run.Events, px, py, pz, units, r, spill, kThreads);
+							Stride);
+					else RunSurfaceTapePairs<1>(load, run.Surface, event, run.Events, px, py, pz, units, r, spill, Stride);
 				}
-				else if (surface) r[0] = RunWholeSurfacePair(code, run.Surface, px[0], py[0], pz[0], spill, kThreads);
-				else r[0] = RunWholePair(code, run.Distance, px[0], py[0], pz[0], spill, kThreads);
+				else if (surface) r[0] = RunWholeSurfacePair(code, run.Surface, px[0], py[0], pz[0], spill, Stride);
+				else r[0] = RunWholePair(code, run.Distance, px[0], py[0], pz[0], spill, Stride);
 				if (q == 0) d[0] = r[0]; else if (q == 1) d[1] = r[0]; else distance = r[0].x;
 			}
 			float e[5] = { d[0].x, d[0].y, d[1].x, d[1].y, 0.0f };
@@ -506,11 +507,12 @@ namespace tg
 			sum = sum + yxy * e[2];
 			sum = sum + xxx * e[3];
 			if ((sum.x * sum.x + sum.y * sum.y) + sum.z * sum.z == 0.0f)
-				e[4] = RunWholeSurfacePair(code, run.Surface, make_float2(p.x, p.x), make_float2(p.y, p.y), make_float2(p.z, p.z), spill, kThreads).x;
+				e[4] = RunWholeSurfacePair(code, run.Surface, make_float2(p.x, p.x), make_float2(p.y, p.y), make_float2(p.z, p.z), spill, Stride).x;
 			return GradientOf(e);
 		}
 
 		// The vertex's colour bytes (GetMaterial), white where it has no material.
+		template<int Stride = kThreads>
 		__device__ __forceinline__ uchar4 RunColor(const DeviceProgram& prog, const BrickTapes& tapes, const PointRun& run, Vec3 p,
 			const PairUnits& units, float2* spill)
 		{
@@ -524,9 +526,9 @@ namespace tg
 			{
 				const uint2* ev = tapes.Events + run.Material;
 				m = RunMaterialTape([&](int q) { return __ldg(code + q); }, run.Surface, [&](uint32_t q) { return __ldg(ev + q); }, run.Walk, p,
-					units, walk, 2 * kThreads);
+					units, walk, 2 * Stride);
 			}
-			else m = RunWholeMaterial(code, run.Surface, p, walk, 2 * kThreads);
+			else m = RunWholeMaterial(code, run.Surface, p, walk, 2 * Stride);
 			return m >= 0 ? prog.Colors[m] : make_uchar4(255, 255, 255, 255);
 		}
 

@@ -105,6 +105,28 @@ namespace tg
 		}
 	}
 
+	// TapeBrush2 for one point; the kinds of brush are told apart by selection, so that lanes on
+	// different tapes stay together.
+	__device__ __forceinline__ float TapeBrush(uint32_t op, const float4& h, float x, float y, float z)
+	{
+		const bool box = op == OpBox, cylinder = op == OpCylinder, round = op == OpTorus || cylinder;
+		if (!box && !round && op != OpSphere) return RareBrushDistance(op, h.y, h.z, h.w, x, y, z);
+		const float ax = box ? fabsf(x) - h.y : x, ay = box ? fabsf(y) - h.z : y, az = box ? fabsf(z) - h.w : z;
+		float last = box ? fminf(fmaxf(fmaxf(ax, ay), az), 0.0f) : -h.y;
+		const float vx = box ? TernaryMax(ax, 0.0f) : ax, vy = box ? TernaryMax(ay, 0.0f) : ay, vz = box ? TernaryMax(az, 0.0f) : az;
+		const float s = vx * vx + vy * vy;
+		float length = sqrtf(round ? s : s + vz * vz);
+		if (round)
+		{
+			// The distance from the axis less the major radius (a cylinder's radius).
+			const float a = length + -h.y, b = cylinder ? fabsf(z) - h.z : z;
+			last = cylinder ? fminf(fmaxf(a, b), 0.0f) : -h.z;
+			const float va = cylinder ? TernaryMax(a, 0.0f) : a, vb = cylinder ? TernaryMax(b, 0.0f) : b;
+			length = sqrtf(va * va + vb * vb);
+		}
+		return length + last;
+	}
+
 	static __device__ __noinline__ float TapeBlendTerm(float m, float h, float k, bool subtract) { return BlendTerm(m, h, k, subtract); }
 
 	// The blends share one term, out of line where it is not zero: the difference blends as the
@@ -282,12 +304,7 @@ namespace tg
 					const float4 O = load(at++);
 					qx = px + O.x; qy = py + O.y; qz = pz + O.z;
 				}
-				const Vec3 q(qx, qy, qz);
-				if (op == OpSphere) acc = SdSphere(q, h.y);
-				else if (op == OpBox) acc = SdBox(q, Vec3(h.y, h.z, h.w));
-				else if (op == OpTorus) acc = SdTorus(q, h.y, h.z);
-				else if (op == OpCylinder) acc = SdCylinder(q, h.y, h.z);
-				else acc = RareBrushDistance(op, h.y, h.z, h.w, qx, qy, qz);
+				acc = TapeBrush(op, h, qx, qy, qz);
 				if (head & RecScale) acc = acc * load(at).x;
 				if (e >= count) break;
 				if (!(head & RecThenSet)) continue;

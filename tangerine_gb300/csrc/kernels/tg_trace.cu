@@ -25,7 +25,7 @@ namespace tg
 	namespace
 	{
 		constexpr int kTraceThreads = 128;
-		constexpr int kTileX = 16, kTileY = 8;     // pixels of a block
+		constexpr int kTileX = 8, kTileY = 4;      // pixels of a warp
 
 		// SDFNode::RayMarch on the whole tree.
 		__device__ __forceinline__ March MarchExact(const DeviceProgram& prog, Vec3 start, Vec3 dir_in, int iterations, float epsilon,
@@ -234,6 +234,8 @@ namespace tg
 			Vec3 pos = start;
 			float travel = 0.0f;
 			run.Lo[0] = 1.0f; run.Hi[0] = 0.0f;
+			Vec3 pivot(0.0f, 0.0f, 0.0f);
+			float clip = 0.0f;
 			for (int i = 0; i < iterations; ++i)
 			{
 				const Vec3 off = pos - root;
@@ -241,20 +243,23 @@ namespace tg
 				float step = sqrtf(ox * ox + oy * oy + oz * oz);
 				if (!(step > epsilon))
 				{
-					if (!parts::InRun(run, pos) && !parts::FindPart(tapes, __ldg(tapes.Bricks + lat.BrickAt(pos)), pos, run))
-						parts::RunWhole(prog, pos, run);
+					if (!parts::InRun(run, pos))
+					{
+						if (!parts::FindPart(tapes, __ldg(tapes.Bricks + lat.BrickAt(pos)), pos, run)) parts::RunWhole(prog, pos, run);
+						const OctNode* n = prog.Nodes + run.Cell;
+						pivot = Vec3(__ldg(&n->Pivot[0]), __ldg(&n->Pivot[1]), __ldg(&n->Pivot[2]));
+						clip = __ldg(&n->ClipRadius);
+					}
 					float f;
 					if (run.Events != kNoTape)
 					{
 						const uint2* ev = tapes.Events + run.Value;
 						f = RunTapePoint([&](int q) { return __ldg(code + q); }, run.Distance, [&](uint32_t e) { return __ldg(ev + e); }, run.Events,
-							pos.x, pos.y, pos.z, spill, 2 * kTraceThreads);
+							pos.x, pos.y, pos.z, spill, 2 * 32);
 					}
-					else f = RunWholePoint(code, run.Distance, pos.x, pos.y, pos.z, spill, 2 * kTraceThreads);
+					else f = RunWholePoint(code, run.Distance, pos.x, pos.y, pos.z, spill, 2 * 32);
 					if (f <= epsilon) return { true, travel, pos };
-					const OctNode* n = prog.Nodes + run.Cell;
-					const Vec3 dp = pos - Vec3(__ldg(&n->Pivot[0]), __ldg(&n->Pivot[1]), __ldg(&n->Pivot[2]));
-					const float room = __ldg(&n->ClipRadius) - Length(dp);
+					const float room = clip - Length(pos - pivot);
 					step = fminf(f, fmaxf(room, epsilon));
 				}
 				travel = travel + step;
@@ -274,17 +279,17 @@ namespace tg
 			return (fwd + right * u) + up * v;
 		}
 
-		// RenderKernel's octree-bounded form by tapes.  A warp takes 8 x 4 pixels: neighbouring
-		// rays mostly share bricks, in a row of 32 they part sooner.
-		__global__ void __launch_bounds__(kTraceThreads, 8) RenderTapesKernel(DeviceProgram prog, RenderLattice lat, BrickTapes tapes,
+		// RenderKernel's octree-bounded form by tapes.  A block is one warp of 8 x 4 pixels:
+		// neighbouring rays mostly share bricks (in a row of 32 they part sooner), and rays that
+		// graze the surface for a hundred steps and more hold up no other warp's place.
+		__global__ void __launch_bounds__(32, 32) RenderTapesKernel(DeviceProgram prog, RenderLattice lat, BrickTapes tapes,
 			const CameraBasis* __restrict__ cams, int count, int width, int height, int steps, float epsilon, float* __restrict__ depth,
 			float* __restrict__ normals, uint8_t* __restrict__ colors)
 		{
 			extern __shared__ __align__(16) float2 spill2[];
 			const int tilesX = (width + kTileX - 1) / kTileX, tilesY = (height + kTileY - 1) / kTileY;
 			const int tile = (int)(blockIdx.x % (unsigned)(tilesX * tilesY)), c = (int)(blockIdx.x / (unsigned)(tilesX * tilesY));
-			const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
-			const int x = (tile % tilesX) * kTileX + (warp & 1) * 8 + (lane & 7), y = (tile / tilesX) * kTileY + (warp >> 1) * 4 + (lane >> 3);
+			const int x = (tile % tilesX) * kTileX + (int)(threadIdx.x & 7), y = (tile / tilesX) * kTileY + (int)(threadIdx.x >> 3);
 			if (x >= width || y >= height || c >= count) return;
 			const int64_t t = ((int64_t)c * height + y) * width + x;
 			const CameraBasis& cam = cams[c];
@@ -299,8 +304,8 @@ namespace tg
 			{
 				const PairUnits units = LoadPairUnits();
 				float none;
-				n = parts::RunGradient<false>(prog, tapes, run, m.Position, units, spill, false, none);
-				if (colors) col = parts::RunColor(prog, tapes, run, m.Position, units, spill);
+				n = parts::RunGradient<false, 32>(prog, tapes, run, m.Position, units, spill, false, none);
+				if (colors) col = parts::RunColor<32>(prog, tapes, run, m.Position, units, spill);
 			}
 			normals[t * 3] = n.x;
 			normals[t * 3 + 1] = n.y;
@@ -374,7 +379,11 @@ namespace tg
 	}
 
 	// Bricks per axis for the renderer's tapes, 0 for none.  A tape costs a pass of its cell's
-	// program at 64 points; a pixel takes some fifteen, thirty-two pixels at a time.
+	// program by one warp; without, a render of any size lasts as long as the ray that grazes
+	// the surface longest, some hundred whole programs one after the other.  Measured on a
+	// GB300, tapes against none, us an image: 16 primitives 64 x 48 238 / 184, 200 x 150 287 /
+	// 330; 64 primitives 422 / 352 and 429 / 675; 512 primitives 780 / 1349 and 1291 / 2170;
+	// 1024 primitives two of 1920 x 1080 2.39 / 6.2 ms.
 	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels)
 	{
 		if (!prog.Lipschitz || !(prog.Form & kFormPrunable)) return 0;
@@ -383,7 +392,7 @@ namespace tg
 		int cells = 1;
 		while (cells < 128 && span / (float)cells > 0.25f) cells *= 2;
 		const int n = cells < 32 ? 32 : cells;
-		return n <= 64 && pixels >= 16 * (int64_t)n * n * n ? n : 0;
+		return n <= 64 && pixels >= (int64_t)n * n * n / 4 ? n : 0;
 	}
 
 	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes,
@@ -398,7 +407,7 @@ namespace tg
 		cudaError_t e = parts::LaunchParts(prog, lat, nullptr, nullptr, nullptr, tapes, sms, stream);
 		if (e != cudaSuccess) return e;
 		// The colour's walk takes two words a level, the gradient one pair.
-		const size_t smem = parts::SpillPairs(prog, 2) * kTraceThreads * sizeof(float2);
+		const size_t smem = parts::SpillPairs(prog, 2) * 32 * sizeof(float2);
 		if (smem > 48 * 1024)
 		{
 			e = cudaFuncSetAttribute(RenderTapesKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -406,7 +415,7 @@ namespace tg
 		}
 		const int64_t blocks = (int64_t)((width + kTileX - 1) / kTileX) * ((height + kTileY - 1) / kTileY) * count;
 		if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
-		RenderTapesKernel<<<(unsigned)blocks, kTraceThreads, smem, stream>>>(prog, lat, tapes, cameras, count, width, height, max_steps, epsilon,
+		RenderTapesKernel<<<(unsigned)blocks, 32, smem, stream>>>(prog, lat, tapes, cameras, count, width, height, max_steps, epsilon,
 			depth, normals, colors);
 		return cudaGetLastError();
 	}

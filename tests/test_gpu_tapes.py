@@ -134,10 +134,10 @@ def test_render_by_tapes_equals_render_without(lib, prims, ops):
         seed += 1
     poses = np.concatenate([W.camera_poses(7, 7), [[0.3, 0.2, 0.1], [60.0, 50.0, 70.0]]]).astype(np.float32)
     with sdf.compile(sdf.from_spec(spec)) as prog:
-        depth, normals, colors = prog.render(sdf.cameras(poses), 333, 241)
-        assert poses.shape[0] * 333 * 241 >= 16 * 32 ** 3 and np.isfinite(depth).any()
+        depth, normals, colors = prog.render(sdf.cameras(poses), 83, 61)
+        assert poses.shape[0] * 83 * 61 >= 32 ** 3 / 4 > 83 * 61 and np.isfinite(depth).any()
         for i, p in enumerate(poses):
-            d, n, c = prog.render(sdf.cameras(p[None]), 333, 241)
+            d, n, c = prog.render(sdf.cameras(p[None]), 83, 61)
             np.testing.assert_array_equal(d[0], depth[i])
             np.testing.assert_array_equal(n[0], normals[i])
             np.testing.assert_array_equal(c[0], colors[i])
