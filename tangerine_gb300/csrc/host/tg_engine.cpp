@@ -147,6 +147,8 @@ namespace tg
 			p.View.Lipschitz = p.Host.Header.Lipschitz;
 			p.View.Form = p.Host.Header.Form;
 			p.View.CodeQuads = p.Host.Header.CodeQuads;
+			p.View.FullBrushes = p.Host.Header.FullBrushes;
+			p.View.FullOps = p.Host.Header.FullOps;
 		}
 	}
 
@@ -699,7 +701,10 @@ namespace tg
 		TG_TRY(cudaMemcpyAsync(dOrig, origins, in, cudaMemcpyHostToDevice, s));
 		TG_TRY(cudaMemcpyAsync(dDir, dirs, in, cudaMemcpyHostToDevice, s));
 		Begin("ray_march", s);
-		if (frame && frame->Mode != 0) TG_TRY(LaunchRayQuery(p.View, *frame, dOrig, dDir, n, iterations, epsilon, dHit, dTravel, dPos, s));
+		TG_TRY(ReadSmCount());
+		const int team = TeamForm(p.View, n, TeamWork::Ray, SmCount);
+		if (team) TG_TRY(LaunchTeamRays(p.View, frame ? *frame : RayFrame{}, dOrig, dDir, n, iterations, epsilon, dHit, dTravel, dPos, team, SmCount, s));
+		else if (frame && frame->Mode != 0) TG_TRY(LaunchRayQuery(p.View, *frame, dOrig, dDir, n, iterations, epsilon, dHit, dTravel, dPos, s));
 		else TG_TRY(LaunchRayMarch(p.View, dOrig, dDir, n, iterations, epsilon, dHit, dTravel, dPos, s));
 		End(s);
 		TG_TRY(cudaMemcpyAsync(hit, dHit, (size_t)n, cudaMemcpyDeviceToHost, s));
@@ -718,7 +723,10 @@ namespace tg
 		TG_TRY(RayOut.Reserve(outBytes));
 		TG_TRY(cudaMemcpyAsync(RayIn.Ptr, points, in, cudaMemcpyHostToDevice, s));
 		Begin(gradient ? "tree_gradient" : "tree_eval", s);
-		TG_TRY(LaunchPointQuery(p.View, RayIn.As<float>(), n, gradient, RayOut.As<float>(), s));
+		TG_TRY(ReadSmCount());
+		const int team = TeamForm(p.View, n, gradient ? TeamWork::Gradient : TeamWork::Eval, SmCount);
+		if (team) TG_TRY(LaunchTeamPoints(p.View, RayIn.As<float>(), n, gradient, RayOut.As<float>(), team, SmCount, s));
+		else TG_TRY(LaunchPointQuery(p.View, RayIn.As<float>(), n, gradient, RayOut.As<float>(), s));
 		End(s);
 		TG_TRY(cudaMemcpyAsync(out, RayOut.Ptr, outBytes, cudaMemcpyDeviceToHost, s));
 		TG_TRY(cudaStreamSynchronize(s));

@@ -77,6 +77,8 @@ namespace tg
 		int32_t FullSurfaceCode;    // quad offset of the whole tree's surface program
 		int32_t Lipschitz;          // 1 when every brush is 1-Lipschitz (no ellipsoid)
 		int32_t Form;               // kForm* below
+		int32_t FullBrushes;        // brushes and operators of the whole tree, stencils' masks left out
+		int32_t FullOps;
 	};
 
 	// What the shortened programs (kernels/tg_tape.cuh) may assume of the whole tree.

@@ -859,6 +859,18 @@ namespace tg
 		return 0;
 	}
 
+	// Brushes and operators the tree's distance takes (a stencil's mask changes none).
+	static void CountNodes(const Node& n, int32_t& brushes, int32_t& ops)
+	{
+		switch (n.Kind)
+		{
+		case NodeKind::Brush: ++brushes; break;
+		case NodeKind::Set: ++ops; CountNodes(*n.Lhs, brushes, ops); CountNodes(*n.Rhs, brushes, ops); break;
+		case NodeKind::Flate: ++ops; CountNodes(*n.Lhs, brushes, ops); break;
+		case NodeKind::Stencil: CountNodes(*n.Lhs, brushes, ops); break;
+		}
+	}
+
 	std::vector<uint32_t> CompileReferenceWords(const Node& tree)
 	{
 		std::vector<uint32_t> w;
@@ -1148,6 +1160,7 @@ namespace tg
 		out.Header.FullSurfaceCode = full;
 		out.Header.Lipschitz = HasNonLipschitzBrush(*root) ? 0 : 1;
 		out.Header.Form = FormOf(*root);
+		CountNodes(*root, out.Header.FullBrushes, out.Header.FullOps);
 		if (maxStack > kMaxStack)
 		{
 			error = "tree needs a deeper evaluation stack than the kernels hold";

@@ -20,6 +20,7 @@ namespace tg
 		int Lipschitz;          // every brush 1-Lipschitz
 		int Form;               // kForm* (tg_layout.hpp): what may be left out of its programs
 		int CodeQuads;          // quads of Code; the whole tree's surface program is the last in it
+		int FullBrushes, FullOps;   // brushes and operators of that program (stencils' masks left out)
 	};
 
 	// Pinhole camera: pixel (x, y) looks along forward + right*u + up*v with
@@ -51,6 +52,14 @@ namespace tg
 	};
 	cudaError_t LaunchRayQuery(const DeviceProgram& prog, const RayFrame& frame, const float* origins, const float* dirs, int64_t n,
 		int max_iterations, float epsilon, uint8_t* hit, float* travel, float* position, cudaStream_t stream);
+	// The same by teams of threads (tg_team.cu), for counts that leave the GPU mostly idle with a
+	// thread each.  TeamForm: 0 a thread each, 1 a warp, 2 a block, which the launches then take.
+	enum class TeamWork { Eval, Gradient, Ray };
+	int TeamForm(const DeviceProgram& prog, int64_t n, TeamWork work, int sms);
+	cudaError_t LaunchTeamRays(const DeviceProgram& prog, const RayFrame& frame, const float* origins, const float* dirs, int64_t n,
+		int max_iterations, float epsilon, uint8_t* hit, float* travel, float* position, int form, int sms, cudaStream_t stream);
+	cudaError_t LaunchTeamPoints(const DeviceProgram& prog, const float* points, int64_t n, bool gradient, float* out, int form, int sms,
+		cudaStream_t stream);
 	// SDFNode::Eval (1 float per point) or SDFNode::Gradient (3) on the whole tree.
 	cudaError_t LaunchPointQuery(const DeviceProgram& prog, const float* points, int64_t n, bool gradient, float* out,
 		cudaStream_t stream);

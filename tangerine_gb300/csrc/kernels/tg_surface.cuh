@@ -3,6 +3,7 @@
 #pragma once
 
 #include "tg_device.cuh"
+#include "tg_kernels.hpp"
 
 namespace tg
 {
@@ -132,5 +133,23 @@ namespace tg
 			return Normalize(Vec3(e[0] - d, e[2] - d, e[1] - d));
 		}
 		return g / sqrtf(ls);
+	}
+
+	// The app's framed casts: mode 1 is Lua's magnet cast (lua_sdf.cpp:410-417, the direction is
+	// normalize(target - origin)); mode 2 is SDFModel::RayMarch (sdf_model.cpp:261-266): origin
+	// = Transform::ApplyInv (rotate by the inverse rotation after removing the translation, then
+	// divide by the scale), direction rotated by the inverse rotation.  Mode 0: as they are.
+	__device__ __forceinline__ void FrameRay(const RayFrame& f, Vec3& o, Vec3& d)
+	{
+		if (f.Mode == 1)
+		{
+			d = Normalize(d - o);
+		}
+		else if (f.Mode == 2)
+		{
+			const Quat qi = Inverse(Quat{ f.Rotation[0], f.Rotation[1], f.Rotation[2], f.Rotation[3] });
+			o = Rotate(qi, o - Vec3(f.Translation[0], f.Translation[1], f.Translation[2])) / f.Scale;
+			d = Rotate(qi, d);
+		}
 	}
 }

@@ -139,6 +139,13 @@ namespace tg
 		return TapeBlendTerm(m, h, k, unions);
 	}
 
+	__device__ __forceinline__ float TapeSet(uint32_t op, float l, float r, float k)
+	{
+		if (op == OpDiff || op == OpBlendDiff) r = -r;
+		if (op >= OpBlendUnion) return TapeBlend(op == OpBlendUnion, l, r, k);
+		return op == OpUnion ? fminf(l, r) : fmaxf(l, r);
+	}
+
 	__device__ __forceinline__ float2 TapeSet2(uint32_t op, float2 l, float2 r, float k)
 	{
 		if (op == OpDiff || op == OpBlendDiff) r = make_float2(-r.x, -r.y);
@@ -316,12 +323,7 @@ namespace tg
 				--depth;
 				left = spill[(depth - 1) * stride];
 			}
-			if (op >= OpUnion && op <= OpBlendDiff)
-			{
-				const float r = op == OpDiff || op == OpBlendDiff ? -acc : acc;
-				if (op >= OpBlendUnion) acc = TapeBlend(op == OpBlendUnion, left, r, load(at).y);
-				else acc = op == OpUnion ? fminf(left, r) : fmaxf(left, r);
-			}
+			if (op >= OpUnion && op <= OpBlendDiff) acc = TapeSet(op, left, acc, op >= OpBlendUnion ? load(at).y : 0.0f);
 			else if (op == OpFlate) acc = acc - load(at).y;
 			else acc = op == OpTapeNegate ? -acc : acc + 0.0f;
 			if (++e >= count) break;

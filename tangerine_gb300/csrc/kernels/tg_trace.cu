@@ -90,11 +90,7 @@ namespace tg
 			position[r * 3 + 2] = m.Position.z;
 		}
 
-		// The app's framed casts: mode 1 is Lua's magnet cast (lua_sdf.cpp:410-417, the
-		// direction is normalize(target - origin)); mode 2 is SDFModel::RayMarch
-		// (sdf_model.cpp:261-266): origin = Transform::ApplyInv (rotate by the inverse
-		// rotation after removing the translation, then divide by the scale), direction
-		// rotated by the inverse rotation.
+		// The app's framed casts (FrameRay).
 		__global__ void __launch_bounds__(kTraceThreads) RayQueryKernel(DeviceProgram prog, RayFrame f, const float* __restrict__ origins,
 			const float* __restrict__ dirs, int64_t n, int iterations, float epsilon, uint8_t* __restrict__ hit,
 			float* __restrict__ travel, float* __restrict__ position)
@@ -104,16 +100,7 @@ namespace tg
 			if (r >= n) return;
 			Vec3 o(origins[r * 3], origins[r * 3 + 1], origins[r * 3 + 2]);
 			Vec3 d(dirs[r * 3], dirs[r * 3 + 1], dirs[r * 3 + 2]);
-			if (f.Mode == 1)
-			{
-				d = Normalize(d - o);
-			}
-			else if (f.Mode == 2)
-			{
-				const Quat qi = Inverse(Quat{ f.Rotation[0], f.Rotation[1], f.Rotation[2], f.Rotation[3] });
-				o = Rotate(qi, o - Vec3(f.Translation[0], f.Translation[1], f.Translation[2])) / f.Scale;
-				d = Rotate(qi, d);
-			}
+			FrameRay(f, o, d);
 			const March m = MarchExact(prog, o, d, iterations, epsilon, spill + threadIdx.x);
 			hit[r] = m.Hit ? 1 : 0;
 			travel[r] = m.Travel;

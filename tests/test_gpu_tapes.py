@@ -141,3 +141,38 @@ def test_render_by_tapes_equals_render_without(lib, prims, ops):
             np.testing.assert_array_equal(d[0], depth[i])
             np.testing.assert_array_equal(n[0], normals[i])
             np.testing.assert_array_equal(c[0], colors[i])
+
+
+def _chain(seed, prims):
+    """A left-deep tree (a script's n-ary operators fold left): one operator a level."""
+    words = []
+    rng = W._Words(seed)
+    for i in range(prims):
+        W._emit_primitive(rng, words, True)
+        if i:
+            words += [W.UNION] if i % 5 else [W.BLEND_UNION, 0.05]
+        if i % 7 == 6:
+            words += [W.FLATE, 0.01]
+    return np.asarray(words, np.float32)
+
+
+@pytest.mark.parametrize("spec", [W.random_tree(5, 1), W.random_tree(6, 2), W.random_tree(8, 33, ops=ALL_OPS), W.random_tree(9, 257, ops=ALL_OPS),
+                                  _chain(3, 90)], ids=["1", "2", "33", "257", "chain"])
+def test_teams_equal_a_thread_each(lib, spec):
+    """Whole-tree queries by a block, a warp and a thread each: counts of one, around the
+    teams' sizes, and past their limit give the same bits."""
+    rng = np.random.default_rng(4)
+    many = 70000
+    points = rng.uniform(-1.3, 1.3, (many, 3)).astype(np.float32)
+    origins = rng.normal(size=(many, 3))
+    origins = (4.0 * origins / np.linalg.norm(origins, axis=1, keepdims=True)).astype(np.float32)
+    dirs = (rng.uniform(-1, 1, origins.shape) - origins).astype(np.float32)
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        values, gradients, (hit, travel, position) = prog.eval_tree(points), prog.gradient_tree(points), prog.ray_march(origins, dirs)
+        for n in (1, 2, 31, 160, 1500):
+            np.testing.assert_array_equal(prog.eval_tree(points[:n]), values[:n])
+            np.testing.assert_array_equal(prog.gradient_tree(points[:n]), gradients[:n])
+            h, t, p = prog.ray_march(origins[:n], dirs[:n])
+            np.testing.assert_array_equal(h, hit[:n])
+            np.testing.assert_array_equal(t, travel[:n])
+            np.testing.assert_array_equal(p, position[:n])
