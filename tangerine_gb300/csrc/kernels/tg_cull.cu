@@ -27,7 +27,7 @@ namespace tg
 {
 	namespace
 	{
-		constexpr int kClassifyThreads = 128;
+		constexpr int kClassifyThreads = 32;
 		constexpr int kBrickThreads = 128;     // 8 x 8 columns x 2 z-groups of 4 points
 		// Resident CTAs per SM the brick evaluation is compiled for (48 registers a thread).
 		// 7^3-cell bricks, 512^3 export: 0.65 ms at 8 (64 registers), 0.58 at 9, 0.56 at 10,
@@ -37,32 +37,29 @@ namespace tg
 		constexpr int kCellPassCtasPerSm = 16;
 		constexpr int kListedCtasPerSm = 8;
 
-		// A CTA takes a tile of 8 x 4 x 4 bricks and each warp an 8 x 4 patch of it: the
-		// bricks of a warp are neighbours in space, so they mostly run the same holder
-		// program (a warp along a row of 32 bricks spans several octree cells and diverges).
-		// Kept bricks set their bit with atomicOr into the zeroed bit words.
-		constexpr int kTileX = 8, kTileY = 4, kTileZ = kClassifyThreads / (kTileX * kTileY);
-
-		__global__ void __launch_bounds__(kClassifyThreads) ClassifyBricksKernel(DeviceProgram prog, GridSpec g, BrickGrid bg,
-			const uint32_t* __restrict__ candidates, uint32_t* __restrict__ brick_bits, uint32_t* __restrict__ brick_tops)
+		// A warp per block of 4 x 4 x 4 bricks (ClassifyBrickBlock), each a CTA: with four warps to
+		// a CTA its slot waits for the longest of the four programs (256 primitives at 700^3: 1189
+		// us with a thread per brick, 1163 with CTAs of four warps, 1130 so).  Kept bricks set their bit with
+		// atomicOr into the zeroed bit words.
+		__global__ void __launch_bounds__(kClassifyThreads, 32) ClassifyBricksKernel(DeviceProgram prog, GridSpec g, BrickGrid bg,
+			const uint32_t* __restrict__ candidates, uint32_t* __restrict__ brick_bits, uint32_t* __restrict__ brick_tops, int spill_pairs)
 		{
-			extern __shared__ float spill[];
-			const int tilesX = (bg.NBX + kTileX - 1) / kTileX, tilesY = (bg.NBY + kTileY - 1) / kTileY;
-			const int tile = (int)blockIdx.x;
-			const int bx = (tile % tilesX) * kTileX + (int)(threadIdx.x % kTileX);
-			const int by = ((tile / tilesX) % tilesY) * kTileY + (int)((threadIdx.x / kTileX) % kTileY);
-			const int bz = (tile / (tilesX * tilesY)) * kTileZ + (int)(threadIdx.x / (kTileX * kTileY));
-			if (bx >= bg.NBX || by >= bg.NBY || bz >= bg.NBZ) return;
-			const int64_t b = bx + (int64_t)bg.NBX * (by + (int64_t)bg.NBY * bz);
-			if (candidates && !((__ldg(candidates + (b >> 5)) >> (b & 31)) & 1u)) return;
-			const int sx = g.NX - 1, sy = g.NY - 1, sz = g.NZ - 1;
-			const int i0 = bx * bg.B, j0 = by * bg.B, k0 = bz * bg.B;
-			const int i1 = min(i0 + bg.B, sx), j1 = min(j0 + bg.B, sy), k1 = min(k0 + bg.B, sz);
-			if (BoxMayHoldSurface(prog, g, i0, i1, j0, j1, k0, k1, spill + threadIdx.x, kClassifyThreads))
-			{
-				atomicOr(brick_bits + (b >> 5), 1u << (b & 31));
-				if (brick_tops) brick_tops[b] = BrickTop(prog, g, i0, i1, j0, j1, k0, k1);
-			}
+			extern __shared__ __align__(16) float4 shared4[];
+			constexpr int kWarps = kClassifyThreads / 32;
+			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+			const int nx = (bg.NBX + kBlockBricks - 1) / kBlockBricks, ny = (bg.NBY + kBlockBricks - 1) / kBlockBricks;
+			const int nz = (bg.NBZ + kBlockBricks - 1) / kBlockBricks;
+			const int64_t block = (int64_t)blockIdx.x * kWarps + warp;
+			if (block >= (int64_t)nx * ny * nz) return;
+			const int x0 = (int)(block % nx) * kBlockBricks, y0 = (int)((block / nx) % ny) * kBlockBricks, z0 = (int)(block / ((int64_t)nx * ny)) * kBlockBricks;
+			float2* spill = reinterpret_cast<float2*>(shared4 + kWarps * 64) + warp * spill_pairs * 32 + lane;
+			ClassifyBrickBlock(prog, g, bg.B, bg.NBX, bg.NBY, bg.NBZ, x0, y0, z0, shared4 + warp * 64, spill,
+				[&](int64_t b) { return !candidates || ((__ldg(candidates + (b >> 5)) >> (b & 31)) & 1u) != 0; },
+				[&](int64_t b, int i0, int i1, int j0, int j1, int k0, int k1)
+				{
+					atomicOr(brick_bits + (b >> 5), 1u << (b & 31));
+					if (brick_tops) brick_tops[b] = BrickTop(prog, g, i0, i1, j0, j1, k0, k1);
+				});
 		}
 
 		// Kept bricks by cost class, a thread per brick.  Place = false adds each class's
@@ -472,12 +469,14 @@ namespace tg
 		const int64_t nb = (int64_t)bg.NBX * bg.NBY * bg.NBZ;
 		if (nb <= 0) return cudaSuccess;
 		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
-		const size_t smem = (size_t)depth * kClassifyThreads * sizeof(float);
+		const size_t smem = kClassifyThreads / 32 * 64 * sizeof(float4) + (size_t)depth * kClassifyThreads * sizeof(float2);
 		if (smem > 48 * 1024) cudaFuncSetAttribute(ClassifyBricksKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 		cudaError_t e = cudaMemsetAsync(brick_bits, 0, (size_t)((nb + 31) / 32) * 4, stream);
 		if (e != cudaSuccess) return e;
-		const int64_t tiles = (int64_t)((bg.NBX + kTileX - 1) / kTileX) * ((bg.NBY + kTileY - 1) / kTileY) * ((bg.NBZ + kTileZ - 1) / kTileZ);
-		ClassifyBricksKernel<<<(unsigned)tiles, kClassifyThreads, smem, stream>>>(prog, g, bg, candidates, brick_bits, brick_tops);
+		const auto blocks = [](int n) { return (int64_t)((n + kBlockBricks - 1) / kBlockBricks); };
+		const int64_t warps = blocks(bg.NBX) * blocks(bg.NBY) * blocks(bg.NBZ);
+		ClassifyBricksKernel<<<(unsigned)((warps + kClassifyThreads / 32 - 1) / (kClassifyThreads / 32)), kClassifyThreads, smem, stream>>>(prog, g, bg,
+			candidates, brick_bits, brick_tops, depth);
 		return cudaGetLastError();
 	}
 

@@ -798,6 +798,53 @@ namespace tg
 		}
 	};
 
+	// The source's program at a pair of points a lane, by all lanes of a warp.
+	template<typename Source>
+	__device__ __forceinline__ float2 RunSourcePair(Source& src, float2 px, float2 py, float2 pz, const PairUnits& u, float2* spill, int stride)
+	{
+		float2 acc = make_float2(0.0f, 0.0f), left = acc;
+		int depth = 0;
+		for (int guard = 0; guard < (1 << 24); ++guard)
+		{
+			uint32_t head = src.Head();
+			uint32_t op = head & 0xFFu;
+			if (op >= OpSphere && op <= OpPlane)
+			{
+				const bool thenSet = (head & RecThenSet) != 0;
+				left = acc;
+				if (!thenSet)
+				{
+					if (depth > 0) spill[(depth - 1) * stride] = acc;
+					++depth;
+				}
+				float2 size;
+				acc = src.Brush(head, px, py, pz, u, size);
+				src.Advance(head);
+				if (!thenSet) continue;
+				head = src.Head();
+				op = head & 0xFFu;
+			}
+			else if (op >= OpUnion && op <= OpBlendDiff)
+			{
+				--depth;
+				left = spill[(depth - 1) * stride];
+			}
+			else if (op == OpFlate)
+			{
+				acc = Sub2(acc, Pair(src.Operand()), u);
+				src.Advance(head);
+				continue;
+			}
+			else
+			{
+				break;   // OpStop
+			}
+			acc = TapeSet2(op, left, acc, src.Operand());
+			src.Advance(head);
+		}
+		return acc;
+	}
+
 	// The lists a warp writes its tape to, in shared memory.
 	struct TapeLists
 	{
