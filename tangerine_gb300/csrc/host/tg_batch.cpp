@@ -132,8 +132,6 @@ namespace tg
 			bm.BrickWord0 = bw0[m] = bword;
 			bm.CellWord0 = cword;
 			bm.Cull = (m < (int)Fields.size() && Fields[m]) ? (FieldRefine ? 2 : 1) : 0;
-			t0[m] = tiles;
-			tiles += (int64_t)((bm.NBX + 7) / 8) * ((bm.NBY + 3) / 4) * bm.NBZ;
 			const int64_t sx = g.NX - 1, sy = g.NY - 1, sz = g.NZ - 1;
 			cw[m] = (sx * sy * sz + 31) / 32;
 			cb0[m] = (uint64_t)cword * 32u;
@@ -144,6 +142,17 @@ namespace tg
 			samples += (int64_t)g.NX * g.NY * g.NZ;
 			capV += 10.0 * (double)std::max({ sx * sy, sy * sz, sx * sz }) + 4096.0;
 			MaxStack = std::max(MaxStack, bm.Prog.MaxStack);
+		}
+		// The classification's 4^3-brick blocks, the models with the longest programs first.
+		std::vector<int> order((size_t)n);
+		for (int m = 0; m < n; ++m) order[m] = m;
+		std::stable_sort(order.begin(), order.end(), [&](int a, int b)
+			{ return Programs[a]->Host.Header.FullBrushes > Programs[b]->Host.Header.FullBrushes; });
+		for (int i = 0; i < n; ++i)
+		{
+			const BatchModel& bm = models[order[i]];
+			t0[i] = tiles;
+			tiles += (int64_t)((bm.NBX + 3) / 4) * ((bm.NBY + 3) / 4) * ((bm.NBZ + 3) / 4);
 		}
 		BrickWordHost = bw0;
 		if ((double)bword * 32.0 >= 4294967296.0) { SetError("batch too large: more than 2^32 bricks"); return cudaErrorInvalidValue; }
@@ -158,6 +167,7 @@ namespace tg
 		TG_TRY(CellBit0.Reserve(8 * (size_t)n));
 		TG_TRY(CellWords.Reserve(8 * (size_t)n));
 		TG_TRY(Tile0.Reserve(8 * (size_t)n));
+		TG_TRY(TileModel.Reserve(sizeof(int) * (size_t)n));
 		TG_TRY(BrickBits.Reserve(4 * (size_t)bword));
 		TG_TRY(BrickWordBase.Reserve(4 * (size_t)bword));
 		TG_TRY(BrickList.Reserve(4 * (size_t)bword * 32));
@@ -181,6 +191,7 @@ namespace tg
 		TG_TRY(cudaMemcpyAsync(CellBit0.Ptr, cb0.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, s));
 		TG_TRY(cudaMemcpyAsync(CellWords.Ptr, cw.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, s));
 		TG_TRY(cudaMemcpyAsync(Tile0.Ptr, t0.data(), 8 * (size_t)n, cudaMemcpyHostToDevice, s));
+		TG_TRY(cudaMemcpyAsync(TileModel.Ptr, order.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, s));
 		TG_TRY(cudaStreamSynchronize(s));
 
 		State = BatchState{};
@@ -192,6 +203,9 @@ namespace tg
 		State.CellWords = CellWords.As<int64_t>();
 		State.BrickWordsTotal = bword;
 		State.Tile0 = Tile0.As<int64_t>();
+		State.TileModel = TileModel.As<int>();
+		State.MaxStack = MaxStack;
+		State.LargeBricks = std::any_of(Bricks.begin(), Bricks.end(), [](int B) { return B > 7; }) ? 1 : 0;
 		State.TilesTotal = tiles;
 		State.CellWordsTotal = cword;
 		State.BrickBits = BrickBits.As<uint32_t>();

@@ -21,6 +21,8 @@
 #include "tg_device.cuh"
 #include "tg_kernels.hpp"
 #include "tg_surface.cuh"
+#include "tg_pair.cuh"
+#include "tg_cellpass.cuh"
 
 namespace tg
 {
@@ -191,8 +193,10 @@ namespace tg
 
 		// ---- per-item work ---------------------------------------------------------------
 
+		// Box: the values also go to `box`, the brick's 8^3 corner box in shared memory.
 		template<int K>
-		__device__ void EvalBrickK(const BatchModel& m, float* __restrict__ lattice, uint32_t b, uint32_t packed_top, float* spill)
+		__device__ __forceinline__ void EvalBrickK(const BatchModel& m, float* __restrict__ lattice, uint32_t b, uint32_t packed_top, float* spill,
+			float* box)
 		{
 			// The brick's descent from phase 2: every point below the cell reached by the whole
 			// box, and only where the box straddles a pivot a per-point descent from there.
@@ -235,7 +239,11 @@ namespace tg
 					for (int k = 0; k < K; ++k)
 						if (c < 0 && ((todo >> k) & 1u)) c = cell[k];
 					float r[K];
-					RunDistance<K, false>(prog.Code, __ldg(&prog.Nodes[c].DistanceCode), px, py, pz, r, spill + threadIdx.x, kThreads);
+					const float4* code = prog.Code;
+					if constexpr (K % 2 == 0)
+						RunDistancePaired<K>([&](int q) { return __ldg(code + q); }, __ldg(&prog.Nodes[c].DistanceCode), px, py, pz, r,
+							spill + 2 * threadIdx.x, kThreads);
+					else RunDistance<K>(code, __ldg(&prog.Nodes[c].DistanceCode), px, py, pz, r, spill + threadIdx.x, kThreads);
 #pragma unroll
 					for (int k = 0; k < K; ++k)
 					{
@@ -252,20 +260,82 @@ namespace tg
 					for (int k = 0; k < K; ++k)
 					{
 						const int iz = izb + k;
-						if (iz <= k1) lattice[((int64_t)iz * g.NY + iy) * g.NX + ix] = res[k];
+						if (iz > k1) continue;
+						lattice[((int64_t)iz * g.NY + iy) * g.NX + ix] = res[k];
+						if (box) box[((iz - k0) * 8 + (iy - j0)) * 8 + (ix - i0)] = res[k];
 					}
 				}
 			}
 		}
 
+		// The cell pass of a brick of at most 7^3 cells from its box in shared memory, by the whole
+		// block: bits, and its active cells appended with one atomic.
+		__device__ __forceinline__ void BatchCellFlags(const BatchState& s, const BatchModel& m, const float* box, const BrickCells& bc,
+			const CellGeom& cg, uint32_t* warpBase)
+		{
+			const int lane = threadIdx.x & 31;
+			const int total = bc.nx * bc.ny * bc.nz;
+			unsigned ballots[kTiledRounds];
+			uint64_t cellOf[kTiledRounds];
+			uint32_t count = 0;
+#pragma unroll
+			for (int r = 0; r < kTiledRounds; ++r)
+			{
+				const int t = r * kThreads + (int)threadIdx.x;
+				bool active = false;
+				cellOf[r] = 0;
+				if (t < total)
+				{
+					const int x = t % bc.nx, y = (t / bc.nx) % bc.ny, z = t / (bc.nx * bc.ny);
+					const float* q = box + (z * 8 + y) * 8 + x;
+					const float v[8] = { q[0], q[1], q[9], q[8], q[64], q[65], q[73], q[72] };
+					unsigned pos = 0;
+#pragma unroll
+					for (int k = 0; k < 8; ++k) pos |= (v[k] >= 0.0f ? 1u : 0u) << k;
+					active = pos != 0u && pos != 0xFFu;
+					const int64_t c = (bc.i0 + x) + (bc.j0 + y) * cg.sx + (bc.k0 + z) * cg.sx * cg.sy;
+					if (active) atomicOr(s.CellBits + m.CellWord0 + (c >> 5), 1u << (c & 31));
+					cellOf[r] = (uint64_t)m.CellWord0 * 32u + (uint64_t)c;
+				}
+				ballots[r] = __ballot_sync(0xFFFFFFFFu, active);
+				count += (uint32_t)__popc(ballots[r]);
+			}
+			if (lane == 0) warpBase[threadIdx.x >> 5] = count;
+			__syncthreads();
+			if (threadIdx.x == 0)
+			{
+				uint32_t counts[kThreads / 32], sum = 0;
+#pragma unroll
+				for (int w = 0; w < kThreads / 32; ++w) { counts[w] = warpBase[w]; sum += counts[w]; }
+				uint32_t at = sum ? atomicAdd(s.Counters + 1, sum) : 0u;
+#pragma unroll
+				for (int w = 0; w < kThreads / 32; ++w) { warpBase[w] = at; at += counts[w]; }
+			}
+			__syncthreads();
+			uint32_t at = warpBase[threadIdx.x >> 5];
+			const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+			for (int r = 0; r < kTiledRounds; ++r)
+			{
+				const uint32_t slot = at + (uint32_t)__popc(ballots[r] & below);
+				if (((ballots[r] >> lane) & 1u) && slot < s.CapVertices) s.ActiveCells[slot] = cellOf[r];
+				at += (uint32_t)__popc(ballots[r]);
+			}
+		}
+
 		// ---- the persistent kernel ---------------------------------------------------------
 
-		// Compiled for 8 resident CTAs per SM (64 registers): at the default 80 registers the
-		// interpreter loops spilled about 1.2 KB a thread and the 512-tree batch took 140 ms;
-		// at 64 it spills 0.16 KB, outside the record loops, and takes 124 ms.
+		// Bound by the interpreters' issue and by the phases' last blocks, not by memory.  32 models
+		// of up to 512 primitives at up to 256^3 (microseconds a phase): classification 460 (was
+		// 1370 as a program a thread, in turn), evaluation with the cell pass 820 (1270 + 207),
+		// scans and lists 200, vertices and faces 170, attributes 330 (600 with a lane a point, in
+		// order of cells): 1980 in all, 3710 before.  2 models of up to 16 at 64^3: 209 -> 202.
+		// Compiled for 8 resident CTAs per SM (64 registers; 0.3 KB a thread spilled, outside the
+		// record loops).
 		__global__ void __launch_bounds__(kThreads, 8) BatchExportKernel(BatchState s)
 		{
-			extern __shared__ float spill[];
+			extern __shared__ __align__(16) float shared[];
+			float* spill = shared + kThreads / 32 * 64 * 4;      // after the warps' program windows
 			const int warpsPerGrid = gridDim.x * (kThreads / 32);
 			const int warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
 			const int lane = threadIdx.x & 31;
@@ -282,9 +352,10 @@ namespace tg
 			}
 
 			// 1. Classify every brick of every model; clear the cell bits.  Exact models go by
-			//    8 x 4 patches of neighbouring bricks (a warp each, bits set with atomicOr into
-			//    words zeroed first), which keeps a warp on one holder program.  Models culled
-			//    by a learned bound arrive with their bits set by it (a warp per bit word):
+			//    blocks of 4 x 4 x 4 bricks (a warp each, bits set with atomicOr into words zeroed
+			//    first), drawn from a counter, the models with the longest programs first, since a
+			//    block is one chain of records and the longest would otherwise end last.  Models
+			//    culled by a learned bound arrive with their bits set by it (a warp per bit word):
 			//    those keep them (Cull 1) or put the kept bricks through the exact test (Cull 2).
 			for (int64_t w = gtid; w < s.BrickWordsTotal; w += gthreads)
 			{
@@ -292,26 +363,24 @@ namespace tg
 			}
 			for (int64_t w = gtid; w < s.CellWordsTotal; w += gthreads) s.CellBits[w] = 0u;
 			if (!GridSync(s)) return;
-			for (int64_t t = warp; t < s.TilesTotal; t += warpsPerGrid)
+			// Each warp spills to a region of its own here: the two loops lay it out differently.
+			float2* ownSpill = reinterpret_cast<float2*>(spill) + (threadIdx.x >> 5) * 32 * (s.MaxStack > 1 ? s.MaxStack - 1 : 1);
+			for (;;)
 			{
-				const int mi = ModelOf(s.Tile0, s.Count, t);
-				const BatchModel& m = s.Models[mi];
+				uint32_t t = 0;
+				if (lane == 0) t = atomicAdd(s.Counters + 5, 1u);
+				t = __shfl_sync(0xFFFFFFFFu, t, 0);
+				if ((int64_t)t >= s.TilesTotal) break;
+				const int order = ModelOf(s.Tile0, s.Count, (int64_t)t);
+				const BatchModel& m = s.Models[__ldg(s.TileModel + order)];
 				if (m.Cull != 0) continue;
-				const int64_t local = t - __ldg(s.Tile0 + mi);
-				const int tilesX = (m.NBX + 7) / 8, tilesY = (m.NBY + 3) / 4;
-				const int bx = (int)(local % tilesX) * 8 + (lane & 7);
-				const int by = (int)((local / tilesX) % tilesY) * 4 + (lane >> 3);
-				const int bz = (int)(local / ((int64_t)tilesX * tilesY));
-				if (bx < m.NBX && by < m.NBY)
-				{
-					const int i0 = bx * m.B, j0 = by * m.B, k0 = bz * m.B;
-					if (BoxMayHoldSurface<false>(m.Prog, m.Grid, i0, min(i0 + m.B, m.Grid.NX - 1), j0, min(j0 + m.B, m.Grid.NY - 1),
-						k0, min(k0 + m.B, m.Grid.NZ - 1), spill + threadIdx.x, kThreads))
-					{
-						const int64_t b = bx + (int64_t)m.NBX * (by + (int64_t)m.NBY * bz);
-						atomicOr(s.BrickBits + m.BrickWord0 + (b >> 5), 1u << (b & 31));
-					}
-				}
+				const int local = (int)((int64_t)t - __ldg(s.Tile0 + order));
+				const int nx = (m.NBX + kBlockBricks - 1) / kBlockBricks, ny = (m.NBY + kBlockBricks - 1) / kBlockBricks;
+				ClassifyBrickBlock(m.Prog, m.Grid, m.B, m.NBX, m.NBY, m.NBZ, local % nx * kBlockBricks, local / nx % ny * kBlockBricks,
+					local / (nx * ny) * kBlockBricks, reinterpret_cast<float4*>(shared) + (threadIdx.x >> 5) * 64,
+					ownSpill + lane,
+					[](int64_t) { return true; },
+					[&](int64_t b, int, int, int, int, int, int) { atomicOr(s.BrickBits + m.BrickWord0 + (b >> 5), 1u << (b & 31)); });
 			}
 			for (int64_t w = warp; w < s.BrickWordsTotal; w += warpsPerGrid)
 			{
@@ -330,7 +399,7 @@ namespace tg
 					const int bx = (int)(local % m.NBX), by = (int)((local / m.NBX) % m.NBY), bz = (int)(local / ((int64_t)m.NBX * m.NBY));
 					const int i0 = bx * m.B, j0 = by * m.B, k0 = bz * m.B;
 					active = BoxMayHoldSurface<false>(m.Prog, m.Grid, i0, min(i0 + m.B, m.Grid.NX - 1), j0, min(j0 + m.B, m.Grid.NY - 1),
-						k0, min(k0 + m.B, m.Grid.NZ - 1), spill + threadIdx.x, kThreads);
+						k0, min(k0 + m.B, m.Grid.NZ - 1), reinterpret_cast<float*>(ownSpill) + lane, 32);
 				}
 				const unsigned ballot = __ballot_sync(0xFFFFFFFFu, active);
 				if (lane == 0) s.BrickBits[w] = ballot;
@@ -411,32 +480,48 @@ namespace tg
 			if (!GridSync(s)) return;
 			const uint32_t kept = s.Counters[0];
 
-			// 3. Distances at the lattice points of every kept brick (a CTA per brick).
-			for (uint32_t item = blockIdx.x; item < kept; item += gridDim.x)
+			// 3. Distances at the lattice points of every kept brick, a CTA per brick drawn from a
+			//    counter.  Bricks of at most 7^3 cells keep their values in an 8^3 box in shared
+			//    memory too, and flag and list their active cells from it at once (bits, and an
+			//    append list of global cell bits).
 			{
-				const uint32_t gb = s.BrickList[item];
-				const int mi = ModelOf(s.BrickWord0, s.Count, (int64_t)(gb >> 5));
-				const BatchModel& m = s.Models[mi];
-				const uint32_t b = gb - (uint32_t)(m.BrickWord0 * 32);
-				float* lat = s.Lattice + m.Lattice;
-				const uint32_t top = s.BrickTops[gb];
-				if (m.Lanes == 1) EvalBrickK<1>(m, lat, b, top, spill);
-				else if (m.Lanes == 4) EvalBrickK<4>(m, lat, b, top, spill);
-				else EvalBrickK<2>(m, lat, b, top, spill);
+				__shared__ float box[kTiledBox * kTiledBox * kTiledBox];
+				__shared__ uint32_t warpBase[kThreads / 32];
+				__shared__ uint32_t itemSlot;
+				for (;;)
+				{
+					if (threadIdx.x == 0) itemSlot = atomicAdd(s.Counters + 6, 1u);
+					__syncthreads();   // also: the previous brick is done with the box and the bases
+					const uint32_t item = itemSlot;
+					__syncthreads();
+					if (item >= kept) break;
+					const uint32_t gb = s.BrickList[item];
+					const int mi = ModelOf(s.BrickWord0, s.Count, (int64_t)(gb >> 5));
+					const BatchModel& m = s.Models[mi];
+					const uint32_t b = gb - (uint32_t)(m.BrickWord0 * 32);
+					float* lat = s.Lattice + m.Lattice;
+					const uint32_t top = s.BrickTops[gb];
+					float* own = m.B + 1 <= kTiledBox ? box : nullptr;
+					if (m.Lanes == 1) EvalBrickK<1>(m, lat, b, top, spill, own);
+					else if (m.Lanes == 4) EvalBrickK<4>(m, lat, b, top, spill, own);
+					else EvalBrickK<2>(m, lat, b, top, spill, own);
+					if (!own) continue;
+					__syncthreads();
+					const CellGeom cg = Geom(m.Grid);
+					BatchCellFlags(s, m, box, CellsOf(b, BrickGrid{ m.B, m.NBX, m.NBY, m.NBZ }, cg), cg, warpBase);
+				}
 			}
 			if (!GridSync(s)) return;
 
-			// 4. Active cells of the kept bricks: bits, and an append list of global cell bits.
-			//    Bricks of at most 7^3 cells (every brick size the tuner picks) stage their
-			//    lattice box in shared memory and append their cells with one atomic.
+			// 4. Active cells of the larger bricks, from the lattice.
+			if (s.LargeBricks)
 			{
-				__shared__ float box[8 * 8 * 8];
-				__shared__ uint32_t warpBase[kThreads / 32];
 				for (uint32_t item = blockIdx.x; item < kept; item += gridDim.x)
 				{
 					const uint32_t gb = s.BrickList[item];
 					const int mi = ModelOf(s.BrickWord0, s.Count, (int64_t)(gb >> 5));
 					const BatchModel& m = s.Models[mi];
+					if (m.B + 1 <= kTiledBox) continue;
 					const uint32_t b = gb - (uint32_t)(m.BrickWord0 * 32);
 					const CellGeom cg = Geom(m.Grid);
 					const float* lat = s.Lattice + m.Lattice;
@@ -446,64 +531,6 @@ namespace tg
 					const int nx = (int)min((int64_t)m.B, cg.sx - ci0), ny = (int)min((int64_t)m.B, cg.sy - cj0);
 					const int nz = (int)min((int64_t)m.B, cg.sz - ck0);
 					const int total = nx * ny * nz;
-					if (m.B <= 7)
-					{
-						__syncthreads();   // the previous brick is done with the box and the bases
-						for (int t = (int)threadIdx.x; t < 512; t += kThreads)
-						{
-							const int x = t & 7, y = (t >> 3) & 7, z = t >> 6;
-							if (x <= nx && y <= ny && z <= nz) box[t] = __ldg(lat + ((ck0 + z) * cg.ny + cj0 + y) * cg.nx + ci0 + x);
-						}
-						__syncthreads();
-						constexpr int kRounds = 3;   // 7^3 = 343 cells <= 3 x 128
-						unsigned ballots[kRounds];
-						uint64_t cellOf[kRounds];
-						uint32_t count = 0;
-#pragma unroll
-						for (int r = 0; r < kRounds; ++r)
-						{
-							const int t = r * kThreads + (int)threadIdx.x;
-							bool active = false;
-							cellOf[r] = 0;
-							if (t < total)
-							{
-								const int x = t % nx, y = (t / nx) % ny, z = t / (nx * ny);
-								const float* q = box + (z * 8 + y) * 8 + x;
-								const float v[8] = { q[0], q[1], q[9], q[8], q[64], q[65], q[73], q[72] };
-								unsigned pos = 0;
-#pragma unroll
-								for (int k = 0; k < 8; ++k) pos |= (v[k] >= 0.0f ? 1u : 0u) << k;
-								active = pos != 0u && pos != 0xFFu;
-								const int64_t c = (ci0 + x) + (cj0 + y) * cg.sx + (ck0 + z) * cg.sx * cg.sy;
-								if (active) atomicOr(s.CellBits + m.CellWord0 + (c >> 5), 1u << (c & 31));
-								cellOf[r] = (uint64_t)m.CellWord0 * 32u + (uint64_t)c;
-							}
-							ballots[r] = __ballot_sync(0xFFFFFFFFu, active);
-							count += (uint32_t)__popc(ballots[r]);
-						}
-						if (lane == 0) warpBase[threadIdx.x >> 5] = count;
-						__syncthreads();
-						if (threadIdx.x == 0)
-						{
-							uint32_t counts[kThreads / 32], sum = 0;
-#pragma unroll
-							for (int w = 0; w < kThreads / 32; ++w) { counts[w] = warpBase[w]; sum += counts[w]; }
-							uint32_t at = sum ? atomicAdd(s.Counters + 1, sum) : 0u;
-#pragma unroll
-							for (int w = 0; w < kThreads / 32; ++w) { warpBase[w] = at; at += counts[w]; }
-						}
-						__syncthreads();
-						uint32_t at = warpBase[threadIdx.x >> 5];
-						const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-						for (int r = 0; r < kRounds; ++r)
-						{
-							const uint32_t slot = at + (uint32_t)__popc(ballots[r] & below);
-							if (((ballots[r] >> lane) & 1u) && slot < s.CapVertices) s.ActiveCells[slot] = cellOf[r];
-							at += (uint32_t)__popc(ballots[r]);
-						}
-						continue;
-					}
 					for (int r0 = 0; r0 < total; r0 += kThreads)
 					{
 						const int t = r0 + (int)threadIdx.x;
@@ -529,8 +556,8 @@ namespace tg
 						if (active && at < s.CapVertices) s.ActiveCells[at] = (uint64_t)m.CellWord0 * 32u + (uint64_t)c;
 					}
 				}
+				if (!GridSync(s)) return;
 			}
-			if (!GridSync(s)) return;
 
 			// 5. Vertex numbers: ranks in the global cell bitmask.
 			if (!GridScan(s, s.CellBits, s.CellWordsTotal, true, s.CellWordBase, s.Counters + 2)) return;
@@ -614,40 +641,51 @@ namespace tg
 				}
 			}
 
-			// 9. Gradient normals (four lanes per vertex, one tetrahedral offset each, all
-			//    running the same code; the vertex itself only when the four cancel), then
-			//    colours (one thread per vertex of a painted model, GetMaterial's walk).
+			// 9. Gradient normals (two lanes per vertex, a pair of tetrahedral points each; the
+			//    vertex itself only when the four cancel), then colours (one thread per vertex of a
+			//    painted model, GetMaterial's walk).  The vertices in the order of the active-cell
+			//    list, whose cells are grouped by brick, so that a warp mostly runs one program.
 			if (s.Attributes && vertexRoom)
 			{
-				constexpr int kNormalPoints = kThreads / 4;
-				const int localPoint = threadIdx.x >> 2, elane = threadIdx.x & 3;
-				const int groupFirst = (lane & ~3);
+				constexpr int kNormalPoints = kThreads / 2;
+				const int half = threadIdx.x & 1;
+				auto vertexAt = [&](int64_t t, int& mi) -> uint32_t
+				{
+					const uint64_t gc = s.ActiveCells[t];
+					mi = ModelOf(s.CellBit0, s.Count, gc);
+					const uint32_t w = s.CellBits[gc >> 5];
+					return s.CellWordBase[gc >> 5] + __popc(w & ((1u << (gc & 31)) - 1u));
+				};
+				float2* spill2 = reinterpret_cast<float2*>(spill) + threadIdx.x;
 				for (int64_t first = (int64_t)blockIdx.x * kNormalPoints; first < vertices; first += (int64_t)gridDim.x * kNormalPoints)
 				{
-					const int64_t v = first + localPoint;
-					const bool mine = v < vertices;
-					float e = 0.0f;
+					const int64_t t = first + (threadIdx.x >> 1);
+					const bool mine = t < vertices;
+					float2 e = make_float2(0.0f, 0.0f);
 					int mi = 0, pc = 0;
+					int64_t v = 0;
 					Vec3 p(0.0f, 0.0f, 0.0f);
+					const float4* code = nullptr;
+					auto load = [&](int q) { return __ldg(code + q); };
 					if (mine)
 					{
-						mi = ModelOf(s.VertexBase, s.Count, (uint32_t)v);
+						v = vertexAt(t, mi);
 						const BatchModel& m = s.Models[mi];
+						code = m.Prog.Code;
 						p = Vec3(s.Vertices[v * 3], s.Vertices[v * 3 + 1], s.Vertices[v * 3 + 2]);
 						const int cell = DescendOctree(m.Prog.Nodes, p.x, p.y, p.z);
 						pc = __ldg(&m.Prog.Nodes[cell].SurfaceCode);
-						const Vec3 q = TetraPoint(p, elane);
-						const float px[1] = { q.x }, py[1] = { q.y }, pz[1] = { q.z };
-						float r[1];
-						RunSurfaceBatch<1, false>(m.Prog.Code, pc, px, py, pz, r, -1, nullptr, spill + threadIdx.x, kThreads);
-						e = r[0];
+						const Vec3 a = TetraPoint(p, 2 * half), b = TetraPoint(p, 2 * half + 1);
+						e = RunSurfacePair(load, pc, make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), spill2, kThreads);
 					}
+					const int own = lane & ~1;
 					float ev[5];
-#pragma unroll
-					for (int j = 0; j < 4; ++j) ev[j] = __shfl_sync(0xFFFFFFFFu, e, groupFirst + j);
-					if (mine && elane == 0)
+					ev[0] = __shfl_sync(0xFFFFFFFFu, e.x, own);
+					ev[1] = __shfl_sync(0xFFFFFFFFu, e.y, own);
+					ev[2] = __shfl_sync(0xFFFFFFFFu, e.x, own + 1);
+					ev[3] = __shfl_sync(0xFFFFFFFFu, e.y, own + 1);
+					if (mine && half == 0)
 					{
-						const BatchModel& m = s.Models[mi];
 						ev[4] = 0.0f;
 						const float h = 0.0001f;
 						const Vec3 xyy(h, -h, -h), yyx(-h, -h, h), yxy(-h, h, -h), xxx(h, h, h);
@@ -656,21 +694,18 @@ namespace tg
 						g = g + yxy * ev[2];
 						g = g + xxx * ev[3];
 						if ((g.x * g.x + g.y * g.y) + g.z * g.z == 0.0f)
-						{
-							const float qx[1] = { p.x }, qy[1] = { p.y }, qz[1] = { p.z };
-							float r[1];
-							RunSurfaceBatch<1, false>(m.Prog.Code, pc, qx, qy, qz, r, -1, nullptr, spill + threadIdx.x, kThreads);
-							ev[4] = r[0];
-						}
+							ev[4] = RunWholeSurfacePair(code, pc, make_float2(p.x, p.x), make_float2(p.y, p.y), make_float2(p.z, p.z), spill2, kThreads).x;
 						const Vec3 n = GradientOf(ev);
 						s.Normals[v * 3 + 0] = n.x;
 						s.Normals[v * 3 + 1] = n.y;
 						s.Normals[v * 3 + 2] = n.z;
 					}
 				}
-				for (int64_t v = gtid; v < vertices; v += gthreads)
+				__syncthreads();   // the walk below lays its operands out by float
+				for (int64_t t = gtid; t < vertices; t += gthreads)
 				{
-					const int mi = ModelOf(s.VertexBase, s.Count, (uint32_t)v);
+					int mi;
+					const int64_t v = vertexAt(t, mi);
 					const BatchModel& m = s.Models[mi];
 					if (!m.HasPaint) continue;
 					const Vec3 p(s.Vertices[v * 3], s.Vertices[v * 3 + 1], s.Vertices[v * 3 + 2]);
@@ -679,7 +714,7 @@ namespace tg
 					const float px[1] = { p.x }, py[1] = { p.y }, pz[1] = { p.z };
 					float r[1];
 					int mt = -1;
-					RunSurfaceBatch<1, false>(m.Prog.Code, pc, px, py, pz, r, 0, &mt, spill + threadIdx.x, kThreads);
+					RunSurfaceBatch<1>(m.Prog.Code, pc, px, py, pz, r, 0, &mt, spill + threadIdx.x, kThreads);
 					const uchar4 c = mt >= 0 ? m.Prog.Colors[mt] : make_uchar4(255, 255, 255, 255);
 					s.Colors[v * 3 + 0] = c.x;
 					s.Colors[v * 3 + 1] = c.y;
@@ -692,7 +727,8 @@ namespace tg
 	size_t BatchSharedBytes(int max_stack)
 	{
 		const int depth = max_stack > 1 ? max_stack - 1 : 1;
-		return (size_t)depth * 4 * kThreads * sizeof(float);      // K = 4 lanes of distance spill
+		// The warps' program windows, then K = 4 lanes of distance spill.
+		return (size_t)kThreads / 32 * 64 * sizeof(float4) + (size_t)depth * 4 * kThreads * sizeof(float);
 	}
 
 	int BatchThreads() { return kThreads; }

@@ -410,7 +410,8 @@ namespace tg
 		int Count;
 		int Attributes;
 		const int64_t* BrickWord0;     // per model, ascending
-		const int64_t* Tile0;          // per model, ascending: first 8 x 4 brick patch of its classification
+		const int64_t* Tile0;          // ascending: first 4^3-brick block of each model's classification,
+		const int* TileModel;          // and whose it is: the models with the longest programs first
 		int64_t TilesTotal;
 		const uint64_t* CellBit0;      // per model: CellWord0 * 32
 		const int64_t* CellWords;      // per model
@@ -433,7 +434,10 @@ namespace tg
 		uint32_t* Faces;
 		uint32_t* VertexBase;          // per model + 1: first vertex (global numbering)
 		uint32_t* FaceBaseModel;       // per model + 1: first face
-		uint32_t* Counters;            // kept bricks, active cells, vertices, faces, overflow bits; [8..15]: cost
+		int MaxStack;
+		int LargeBricks;               // some model's bricks exceed 7^3 cells
+		uint32_t* Counters;            // kept bricks, active cells, vertices, faces, overflow bits, classification
+		                               // blocks taken, bricks taken; [8..15]: cost
 		                               // classes' brick counts and cursors
 		uint32_t* ScanPartials;        // blocks + 1
 		unsigned* Barrier;             // arrival count, generation

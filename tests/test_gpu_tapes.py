@@ -176,3 +176,25 @@ def test_teams_equal_a_thread_each(lib, spec):
             np.testing.assert_array_equal(h, hit[:n])
             np.testing.assert_array_equal(t, travel[:n])
             np.testing.assert_array_equal(p, position[:n])
+
+
+@pytest.mark.parametrize("bricks", [(7, 8), (1, 7), (2, 3), (15, 4)])
+def test_batch_of_fixture_trees_equals_dense_exports(lib, golden, bricks):
+    """Brick blocks and cell passes of every kind of tree (distorting ones are classified a
+    brick at a time), bricks with and without a box in shared memory in one batch."""
+    specs = [golden[n]["spec"] for n in golden_names() if "octree_nodes" in golden[n]]
+    programs = [sdf.compile(sdf.from_spec(s)) for s in specs]
+    grids = []
+    for i, prog in enumerate(programs):
+        info = prog.info()
+        lo, hi = np.asarray(info.bounds_min[:]), np.asarray(info.bounds_max[:])
+        step = float(np.max(hi - lo)) * 1.1 / (9 + 5 * (i % 7))
+        n = [int(np.ceil((h - l) * 1.1 / step)) + 3 for l, h in zip(lo, hi)]
+        grids.append(_lib.Grid(*[float(l - 0.05 * (h - l) - step) for l, h in zip(lo, hi)], step, *n))
+    with sdf.Batch(programs, grids) as b:
+        b.set_tuning([bricks[i % 2] for i in range(len(programs))], [(1, 2, 4)[i % 3] for i in range(len(programs))])
+        b.run()
+        for m, (prog, grid) in enumerate(zip(programs, grids)):
+            _same(b.mesh(m), prog.export_mesh(grid, dense=True))
+    for p in programs:
+        p.close()
