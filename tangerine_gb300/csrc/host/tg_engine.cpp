@@ -263,10 +263,48 @@ namespace tg
 
 #define TG_TRY(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
 
+	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
+	// A tape saves about what its cell's program has beyond a dozen quads (two brushes), on
+	// every pass over the brick, and costs one pass of the whole program and two launches: it
+	// pays from a number of bricks that falls as the programs get longer.  Measured on a
+	// GB300, export to the device, tapes against whole programs, in us: 64 primitives (23
+	// quads a cell) 384^3 356 / 333, 512^3 414 / 417, 700^3 596 / 660; 16 primitives (16
+	// quads) 512^3 256 / 241, 700^3 346 / 356; 256 primitives (54 quads) 256^3 695 / 735,
+	// 512^3 861 / 1062, and 128^3 721 / 653.
+	static bool TapesPay(const Program& p, int64_t bricks)
+	{
+		return p.View.Lipschitz && (p.View.Form & kFormPrunable) && (double)bricks * (CellQuads(p) - 12.0) >= 3.5e6;
+	}
+
+	// Whether a whole lattice goes by tapes, in bricks of 16^3 points (a quarter full at least).
+	// By whole programs it takes about 0.7 to 0.9 us per million quads that its points run
+	// together; by tapes 6 us per million points, and 100 to 350 us whatever the size, the more
+	// the larger the tree (the chains of splitting bricks and of the longest program's one pass).
+	// Whole programs / tapes in us by millions of quads: 8 primitives 89 / 111 at 89, 136 / 133 at
+	// 174, 433 / 253 at 713; 30 primitives 157 / 204 at 109, 261 / 229 at 213, 789 / 340 at 876; 64
+	// primitives 229 / 229 at 232, 405 / 260 at 455, 1415 / 257 at 1877; 128 primitives 296 / 202 at
+	// 294, 231 / 256 at 177; 256 primitives 372 / 422 at 270, 384 / 366 at 401, 5515 / 618 at 8900.
+	static bool GridTapesPay(const Program& p, const GridSpec& g)
+	{
+		if (!p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
+		const double points = (double)g.NX * g.NY * g.NZ;
+		const auto bricks = [](int n) { return (double)((n + 15) / 16); };
+		return points * p.Host.VolumeQuads >= 1e6 * (200.0 + p.Host.Header.FullBrushes) &&
+			points >= 1024.0 * bricks(g.NX) * bricks(g.NY) * bricks(g.NZ);
+	}
+
 	cudaError_t Engine::EvalGrid(const Program& p, const GridSpec& g, float* out, cudaStream_t s)
 	{
+		BrickTapes tapes{};
+		const bool byTapes = GridTapesPay(p, g);
+		if (byTapes)
+		{
+			const int64_t slab = DenseSlabBricks(g);
+			TG_TRY(ReadSmCount());
+			TG_TRY(ReserveTapes(slab, (size_t)slab * 16 + 4096, tapes));
+		}
 		Begin("eval_grid", s);
-		cudaError_t e = LaunchEvalGrid(p.View, g, out, s);
+		const cudaError_t e = byTapes ? LaunchEvalGridTapes(p.View, g, tapes, out, SmCount, s) : LaunchEvalGrid(p.View, g, out, s);
 		End(s);
 		return e;
 	}
@@ -331,19 +369,6 @@ namespace tg
 		return cudaSuccess;
 	}
 
-	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
-	// A tape saves about what its cell's program has beyond a dozen quads (two brushes), on
-	// every pass over the brick, and costs one pass of the whole program and two launches: it
-	// pays from a number of bricks that falls as the programs get longer.  Measured on a
-	// GB300, export to the device, tapes against whole programs, in us: 64 primitives (23
-	// quads a cell) 384^3 356 / 333, 512^3 414 / 417, 700^3 596 / 660; 16 primitives (16
-	// quads) 512^3 256 / 241, 700^3 346 / 356; 256 primitives (54 quads) 256^3 695 / 735,
-	// 512^3 861 / 1062, and 128^3 721 / 653.
-	static bool TapesPay(const Program& p, int64_t bricks)
-	{
-		return (double)bricks * (CellQuads(p) - 12.0) >= 3.5e6;
-	}
-
 	cudaError_t Engine::ReadSmCount()
 	{
 		if (SmCount) return cudaSuccess;
@@ -352,10 +377,10 @@ namespace tg
 		return cudaDeviceGetAttribute(&SmCount, cudaDevAttrMultiProcessorCount, dev);
 	}
 
-	cudaError_t Engine::ReserveTapes(int64_t bricks, BrickTapes& out)
+	cudaError_t Engine::ReserveTapes(int64_t bricks, size_t parts, BrickTapes& out)
 	{
-		out.PartCapacity = (uint32_t)std::min<size_t>(BrickPartCapacity(bricks), 0x7FFFFFFFu);
-		out.EventCapacity = (uint32_t)std::min<size_t>(BrickEventCapacity(bricks), 0x7FFFFFFFu);
+		out.PartCapacity = (uint32_t)std::min<size_t>(parts, 0x7FFFFFFFu);
+		out.EventCapacity = (uint32_t)std::min<size_t>(BrickEventCapacity(parts), 0x7FFFFFFFu);
 		TG_TRY(TapeBricks.Reserve((size_t)bricks * sizeof(uint2)));
 		TG_TRY(TapeParts.Reserve((size_t)out.PartCapacity * sizeof(BrickPart)));
 		TG_TRY(TapeEvents.Reserve((size_t)out.EventCapacity * sizeof(uint2)));
@@ -477,7 +502,7 @@ namespace tg
 			{
 				// Each brick's shortened programs, then the evaluation by them with the cell pass
 				// folded in, on each brick's values in shared memory.
-				TG_TRY(ReserveTapes(nb, tapes));
+				TG_TRY(ReserveTapes(nb, BrickPartCapacity(nb), tapes));
 				Begin("brick_tapes", s);
 				TG_TRY(LaunchBrickTapes(p.View, g, B, BrickList.As<uint32_t>(), brickCount, tops, tapes, SmCount, s));
 				End(s);
@@ -773,7 +798,7 @@ namespace tg
 			if (bricks)
 			{
 				TG_TRY(ReadSmCount());
-				TG_TRY(ReserveTapes((int64_t)bricks * bricks * bricks, tapes));
+				TG_TRY(ReserveTapes((int64_t)bricks * bricks * bricks, BrickPartCapacity((int64_t)bricks * bricks * bricks), tapes));
 			}
 			Begin("render", s);
 			if (bricks)

@@ -208,7 +208,7 @@ namespace tg
 		cudaStream_t Stream = nullptr;
 		cudaStream_t CopyStream = nullptr;          // early device-to-host copies of an export
 		// The buffers of a grid's brick tapes (LaunchBrickTapes), kept between exports.
-		cudaError_t ReserveTapes(int64_t bricks, BrickTapes& out);
+		cudaError_t ReserveTapes(int64_t bricks, size_t parts, BrickTapes& out);
 		cudaError_t ReadSmCount();
 		cudaEvent_t MeshReady = nullptr;
 		cudaEvent_t CodeReady = nullptr;            // RestageCode's copy of an export is done

@@ -106,7 +106,7 @@ namespace tg
 		{
 			const int64_t bricks = CloudBricks(s);
 			TG_TRY(ReadSmCount());
-			TG_TRY(ReserveTapes(bricks, tapes));
+			TG_TRY(ReserveTapes(bricks, BrickPartCapacity(bricks), tapes));
 			TG_TRY(VoxScratch.Reserve((size_t)bricks * 8));
 			uint32_t* list = VoxScratch.As<uint32_t>();
 			TG_TRY(ActiveCells.Reserve((size_t)s.Total * 4));

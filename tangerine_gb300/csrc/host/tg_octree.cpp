@@ -1128,6 +1128,7 @@ namespace tg
 			out.CodeChunks.push_back(std::move(chunkCode[(size_t)ch]));
 		}
 		int maxStack = 0;
+		double volume = 0.0;
 		out.Nodes.resize(octree.Cells.size());
 		for (size_t i = 0; i < octree.Cells.size(); ++i)
 		{
@@ -1154,7 +1155,14 @@ namespace tg
 			n.ClipRadius = e.NonLipschitz ? -c.ClipRadius : c.ClipRadius;
 			if (n.StackSize > maxStack) maxStack = n.StackSize;
 			out.DistanceQuadsTotal += e.Surface - e.Distance;
+			// The part of the cell's volume whose points run its program.
+			int own = c.Terminus ? 8 : 0;
+			for (int k = 0; k < 8 && !c.Terminus; ++k) own += c.Children[k] < 0 ? 1 : 0;
+			const double weight = own * (double)c.ClipRadius * c.ClipRadius * c.ClipRadius;
+			volume += weight;
+			out.VolumeQuads += weight * (e.Surface - e.Distance);
 		}
+		if (volume > 0.0) out.VolumeQuads /= volume;
 		const int full = programs[evaluators].Surface;
 		if (programs[evaluators].Stack > maxStack) maxStack = programs[evaluators].Stack;
 		out.Header.FullSurfaceCode = full;

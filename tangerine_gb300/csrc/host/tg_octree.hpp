@@ -74,6 +74,7 @@ namespace tg
 		double BuildSeconds = 0.0;
 		double OctreeSeconds = 0.0;       // of which the octree (clips, merges)
 		int64_t DistanceQuadsTotal = 0;
+		double VolumeQuads = 0.0;           // distance quads a point runs, on average over the octree's cube
 	};
 
 	// The export octree's root cell on its own, as a one-cell program image: Node is the

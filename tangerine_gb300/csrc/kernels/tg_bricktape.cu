@@ -20,7 +20,8 @@ namespace tg
 		struct MeshLattice
 		{
 			static constexpr int kStride = kCells;
-			static constexpr bool kOutside = false;
+			static constexpr int kBox = parts::kBox, kMost = 24;
+			static constexpr bool kOutside = false, kBetween = true;
 			GridSpec Grid;
 			__device__ __forceinline__ float Coord(int a, int i) const
 			{
@@ -189,7 +190,7 @@ namespace tg
 	// ten or twenty, with two or three parts each; a coarse one keeps more, with up to a dozen.
 	// What does not fit is evaluated without (BrickPartsKernel, BuildPartTapesKernel).
 	size_t BrickPartCapacity(int64_t bricks) { return (size_t)bricks / 2 + 65536; }
-	size_t BrickEventCapacity(int64_t bricks) { return BrickPartCapacity(bricks) * 12; }
+	size_t BrickEventCapacity(size_t parts) { return parts * 12; }
 
 	cudaError_t LaunchBrickTapes(const DeviceProgram& prog, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,
 		const uint32_t* tops, const BrickTapes& tapes, int sms, cudaStream_t stream)

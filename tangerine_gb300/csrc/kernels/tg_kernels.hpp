@@ -71,6 +71,13 @@ namespace tg
 	// `lanes` points per thread (1, 2 or 4) share one pass over the records.
 	cudaError_t LaunchEvalGrid(const DeviceProgram& prog, const GridSpec& grid, float* out, cudaStream_t stream, int lanes = 4);
 
+	// The same through shortened programs, a slab of the lattice after the other: the tapes'
+	// room is for DenseSlabBricks bricks.
+	struct BrickTapes;
+	int64_t DenseSlabBricks(const GridSpec& grid);
+	cudaError_t LaunchEvalGridTapes(const DeviceProgram& prog, const GridSpec& grid, const BrickTapes& tapes, float* out, int sms,
+		cudaStream_t stream);
+
 	// Surface nets, cell pass part 1: one bit per cell (x fastest) set when the cell's
 	// eight corners do not all share a sign.  `words` holds ceil(cells / 32) words.
 	cudaError_t LaunchCellFlags(const float* lattice, const GridSpec& grid, uint32_t* words, cudaStream_t stream);
@@ -138,7 +145,7 @@ namespace tg
 	};
 	constexpr uint32_t kLongParts = 16384;
 	size_t BrickPartCapacity(int64_t bricks);
-	size_t BrickEventCapacity(int64_t bricks);
+	size_t BrickEventCapacity(size_t parts);
 	// Parts and tapes of the listed bricks.  tops: as LaunchEvalBricks.
 	cudaError_t LaunchBrickTapes(const DeviceProgram& prog, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,
 		const uint32_t* tops, const BrickTapes& tapes, int sms, cudaStream_t stream);

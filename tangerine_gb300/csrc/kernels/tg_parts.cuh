@@ -6,8 +6,10 @@
 // which the part's points and the vertices in it then run.
 //
 // A lattice L says where its points lie: Coord(axis, index), Points(axis), Bricks(axis),
-// kStride (points from one brick to the next), kOutside (vertices may leave their brick by up
-// to a step), and Keep(): the distance beyond which a part's points are of no interest.
+// kStride (points from one brick to the next), kBox (points of a brick per axis, at most 16),
+// kMost (parts of a brick, at most), kOutside (vertices may leave their brick by up to a step),
+// kBetween (points between the lattice's look for their part, too), and Keep(): the distance
+// beyond which a part's points are of no interest.
 #pragma once
 
 #include "tg_device.cuh"
@@ -23,7 +25,7 @@ namespace tg
 		constexpr int kWarps = kThreads / 32;
 		constexpr int kPartCtasPerSm = 12;
 		constexpr int kBuildCtasPerSm = 8;
-		constexpr int kBox = 8;             // points of a brick per axis, at most
+		constexpr int kBox = 8;             // points per axis of most lattices' bricks
 		constexpr int kLongQuads = 96;      // programs from this long are built first
 
 		__device__ __forceinline__ uint32_t PackBox(int x0, int x1, int y0, int y1, int z0, int z1)
@@ -39,9 +41,16 @@ namespace tg
 		template<typename L>
 		__device__ __forceinline__ int LastAtMost(const L& lat, int a, int first, int lo, int hi, float pivot)
 		{
-			int i = lo - 1;
-			while (i < hi && !(lat.Coord(a, first + i + 1) > pivot)) ++i;
-			return i;
+			int in = lo - 1, out = hi + 1;
+#pragma unroll
+			for (int step = 0; step < (L::kBox > 8 ? 5 : 4); ++step)
+			{
+				const int mid = (in + out) >> 1;
+				if (out - in < 2) break;
+				if (!(lat.Coord(a, first + mid) > pivot)) in = mid;
+				else out = mid;
+			}
+			return in;
 		}
 
 		// The first point of brick b per axis, and how many points follow it in the brick.
@@ -54,7 +63,7 @@ namespace tg
 			first[1] = (int)(row - bz * ny) * L::kStride;
 			first[2] = (int)bz * L::kStride;
 #pragma unroll
-			for (int a = 0; a < 3; ++a) extent[a] = min(kBox - 1, lat.Points(a) - 1 - first[a]);
+			for (int a = 0; a < 3; ++a) extent[a] = min(L::kBox - 1, lat.Points(a) - 1 - first[a]);
 		}
 
 		// A brick's box as DescendBox's answer: the cell reached, bit 31 set when every point of
@@ -97,32 +106,44 @@ namespace tg
 				}
 				int first[3], extent[3];
 				BrickSpan(lat, b, first, extent);
-				float p[3];
-#pragma unroll
-				for (int a = 0; a < 3; ++a)
+				if constexpr (!L::kBetween)
 				{
-					const int x0 = (int)((box >> (8 * a)) & 15u), x1 = (int)((box >> (8 * a + 4)) & 15u);
-					p[a] = lat.Coord(a, first[a] + x0);
-					out.Lo[a] = lat.Coord(a, first[a] + (L::kOutside ? x0 - 1 : max(x0 - 1, 0)));
-					out.Hi[a] = lat.Coord(a, first[a] + (L::kOutside ? x1 + 1 : min(x1 + 1, extent[a])));
-				}
-				// The pivots passed on the way to the cell bound it (DescendOctree's `p > pivot`).
-				int at = 0;
-				for (int guard = 0; guard < 64; ++guard)
-				{
-					const float4 n = __ldg(reinterpret_cast<const float4*>(prog.Nodes + at));
-					if (__float_as_int(n.w) & kNodeTerminus) break;
-					const float pivot[3] = { n.x, n.y, n.z };
-					int octant = 0;
 #pragma unroll
 					for (int a = 0; a < 3; ++a)
 					{
-						if (p[a] > pivot[a]) { octant |= 1 << a; out.Lo[a] = fmaxf(out.Lo[a], nextafterf(pivot[a], INFINITY)); }
-						else out.Hi[a] = fminf(out.Hi[a], pivot[a]);
+						out.Lo[a] = lat.Coord(a, first[a] + (int)((box >> (8 * a)) & 15u));
+						out.Hi[a] = lat.Coord(a, first[a] + (int)((box >> (8 * a + 4)) & 15u));
 					}
-					const int child = __ldg(&prog.Nodes[at].Child[octant]);
-					if (child < 0) break;
-					at = child;
+				}
+				else
+				{
+					float p[3];
+#pragma unroll
+					for (int a = 0; a < 3; ++a)
+					{
+						const int x0 = (int)((box >> (8 * a)) & 15u), x1 = (int)((box >> (8 * a + 4)) & 15u);
+						p[a] = lat.Coord(a, first[a] + x0);
+						out.Lo[a] = lat.Coord(a, first[a] + (L::kOutside ? x0 - 1 : max(x0 - 1, 0)));
+						out.Hi[a] = lat.Coord(a, first[a] + (L::kOutside ? x1 + 1 : min(x1 + 1, extent[a])));
+					}
+					// The pivots passed on the way to the cell bound it (DescendOctree's `p > pivot`).
+					int at = 0;
+					for (int guard = 0; guard < 64; ++guard)
+					{
+						const float4 n = __ldg(reinterpret_cast<const float4*>(prog.Nodes + at));
+						if (__float_as_int(n.w) & kNodeTerminus) break;
+						const float pivot[3] = { n.x, n.y, n.z };
+						int octant = 0;
+#pragma unroll
+						for (int a = 0; a < 3; ++a)
+						{
+							if (p[a] > pivot[a]) { octant |= 1 << a; out.Lo[a] = fmaxf(out.Lo[a], nextafterf(pivot[a], INFINITY)); }
+							else out.Hi[a] = fminf(out.Hi[a], pivot[a]);
+						}
+						const int child = __ldg(&prog.Nodes[at].Child[octant]);
+						if (child < 0) break;
+						at = child;
+					}
 				}
 			}
 			const uint4* from = reinterpret_cast<const uint4*>(&out);
@@ -137,7 +158,7 @@ namespace tg
 		__device__ __noinline__ void SplitBrick(const DeviceProgram& prog, const L& lat, const BrickTapes& tapes, uint32_t b, int i0, int j0, int k0,
 			int top, uint32_t whole)
 		{
-			constexpr int kStack = 24, kMost = 24;
+			constexpr int kMost = L::kMost, kStack = kMost > 24 ? 48 : 24;
 			uint2 found[kMost], stack[kStack];
 			int parts = 0, depth = 0;
 			bool fits = true;
@@ -347,24 +368,22 @@ namespace tg
 			}
 		}
 
-		// n / d for n < 512 and 1 <= d <= 8, as a product and a shift.
-		__device__ __forceinline__ int SmallDivide(int n, int d)
-		{
-			constexpr uint32_t kOver[9] = { 0, 65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192 };
-			uint32_t over = kOver[1];
-#pragma unroll
-			for (int q = 2; q <= 8; ++q) over = d == q ? kOver[q] : over;
-			return (int)(((uint32_t)n * over) >> 16);
-		}
+		// n / d for n < 4096 and 1 <= d <= 16 as a product and a shift, from over = OverSixteenBits(d):
+		// over exceeds 65536 / d by less than 1, n over / 65536 exceeds n / d by less than 1 / 16.
+		__device__ __forceinline__ uint32_t OverSixteenBits(int d) { return 65535u / (uint32_t)d + 1u; }
+		__device__ __forceinline__ int SmallDivide(int n, uint32_t over) { return (int)(((uint32_t)n * over) >> 16); }
 
 		// The distances of one brick's points, by a warp: its parts in 64-point passes (a part's
 		// points numbered x fastest, two per lane, all lanes on one tape); the warp calls
-		// visit(at, value, live) with each lane's point, at = x + 8 y + 64 z in the brick.  `axis`:
-		// the points' coordinates per axis.  SkipFar: parts that stay beyond the lattice's Keep() are left out.
-		template<bool SkipFar, typename Visit>
+		// visit(at, value, live) with each lane's point, at = x + Box (y + Box z) in the brick.  `axis`:
+		// the points' coordinates per axis; levels [lowest, highest] only.  SkipFar: parts that stay
+		// beyond the lattice's Keep() are left out.
+		template<bool SkipFar, int Box = kBox, typename Visit>
 		__device__ __forceinline__ void BrickPoints(const DeviceProgram& prog, const BrickTapes& tapes, uint2 own, const int (&extent)[3],
-			const float (*axis)[kBox], const PairUnits& units, float2* spill, Visit visit)
+			const float (*axis)[Box], const PairUnits& units, float2* spill, Visit visit, int lowest = 0, int highest = Box - 1)
 		{
+			constexpr int kShift = Box == 16 ? 4 : 3;
+			static_assert(Box == 1 << kShift, "bricks of 8 or 16 points an axis");
 			const float4* code = prog.Code;
 			auto load = [&](int q) { return __ldg(code + q); };
 			const int lane = (int)(threadIdx.x & 31);
@@ -383,9 +402,11 @@ namespace tg
 					events = q.w & 0xFFFFu;
 				}
 				if (SkipFar && (span & (kBoxPositive | kBoxNegative))) continue;
-				const int x0 = (int)(span & 15u), y0 = (int)((span >> 8) & 15u), z0 = (int)((span >> 16) & 15u);
-				const int nx = (int)((span >> 4) & 15u) - x0 + 1, ny = (int)((span >> 12) & 15u) - y0 + 1, nz = (int)((span >> 20) & 15u) - z0 + 1;
+				const int x0 = (int)(span & 15u), y0 = (int)((span >> 8) & 15u), z0 = max((int)((span >> 16) & 15u), lowest);
+				const int nx = (int)((span >> 4) & 15u) - x0 + 1, ny = (int)((span >> 12) & 15u) - y0 + 1;
+				const int nz = min((int)((span >> 20) & 15u), highest) - z0 + 1;
 				const int points = nx * ny * nz;
+				const uint32_t overX = OverSixteenBits(nx), overY = OverSixteenBits(ny);
 				const uint2* ev = tapes.Events + tape;
 				for (int first = 0; first < points; first += 64)
 				{
@@ -395,10 +416,10 @@ namespace tg
 					for (int k = 0; k < 2; ++k)
 					{
 						const int t = min(first + lane + 32 * k, points - 1);
-						const int r = SmallDivide(t, nx);
-						const int z = SmallDivide(r, ny);
-						at[k] = x0 + (t - r * nx) + ((y0 + (r - z * ny)) << 3) + ((z0 + z) << 6);
-						const float x = axis[0][at[k] & 7], y = axis[1][(at[k] >> 3) & 7], zz = axis[2][at[k] >> 6];
+						const int r = SmallDivide(t, overX);
+						const int z = SmallDivide(r, overY);
+						at[k] = x0 + (t - r * nx) + ((y0 + (r - z * ny)) << kShift) + ((z0 + z) << (2 * kShift));
+						const float x = axis[0][at[k] & (Box - 1)], y = axis[1][(at[k] >> kShift) & (Box - 1)], zz = axis[2][at[k] >> (2 * kShift)];
 						if (k & 1) { px[0].y = x; py[0].y = y; pz[0].y = zz; }
 						else { px[0].x = x; py[0].x = y; pz[0].x = zz; }
 					}

@@ -182,7 +182,8 @@ namespace tg
 		struct RenderLattice
 		{
 			static constexpr int kStride = parts::kBox;
-			static constexpr bool kOutside = true;
+			static constexpr int kBox = parts::kBox, kMost = 24;
+			static constexpr bool kOutside = true, kBetween = true;
 			float Origin[3];
 			float Step;
 			int N;

@@ -198,3 +198,23 @@ def test_batch_of_fixture_trees_equals_dense_exports(lib, golden, bricks):
             _same(b.mesh(m), prog.export_mesh(grid, dense=True))
     for p in programs:
         p.close()
+
+
+@pytest.mark.parametrize("prims,ops,shape", [(64, ALL_OPS, (257, 193, 209)), (256, W.OPS_60_20_10_10, (241, 999, 50)), (30, ALL_OPS, (1025, 1025, 66)),
+                                             (1, ALL_OPS, (353, 320, 300))])
+def test_large_lattices_equal_their_pieces(lib, prims, ops, shape):
+    """A large lattice (by tapes, in slabs) against small ones cut out of it (by whole
+    programs): coordinates are multiples of 2^-7, the same in both, and so are the values."""
+    seed = 21
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops))):
+        seed += 1
+    step = 1.0 / 64.0 if max(shape) < 500 else 1.0 / 128.0
+    low = [-round(n * step / 2 / step) * step for n in shape]
+    rng = np.random.default_rng(8)
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        whole = prog.eval_grid(_lib.Grid(*low, step, *shape))
+        for cut in range(24):
+            size = [min(n, int(rng.integers(2, 70))) for n in shape]
+            at = [0 if cut == 0 else n - s if cut == 1 else int(rng.integers(0, n - s + 1)) for n, s in zip(shape, size)]
+            piece = prog.eval_grid(_lib.Grid(*[l + a * step for l, a in zip(low, at)], step, *size))
+            np.testing.assert_array_equal(piece, whole[at[2]:at[2] + size[2], at[1]:at[1] + size[1], at[0]:at[0] + size[0]])
