@@ -303,12 +303,14 @@ namespace tg
 		}
 	}
 
-	// A thread each takes about as long for one as for many (the program's records one after the
-	// other); a team's time grows with the count.  Measured on a GB300, teams against a thread
-	// each, us a call: rays through 8 primitives 3000 220 / 363, 9000 464 / 384; 64 primitives 30
-	// 288 / 2414, 16384 1298 / 2547; 128 primitives 16384 1584 / 4901; gradients of 16
-	// primitives 2000 33 / 48, 10000 56 / 58, 19000 69 / 60; of 256 primitives 100 108 / 419,
-	// 19000 269 / 442, 60000 about even.
+	// A thread per ray (two lanes or half a lane per point, PointQueryKernel) takes about as long
+	// for one as for many (the program's records one after the other); a team's time grows with
+	// the count.  Measured on a GB300, teams against that, us a call: rays through 8 primitives
+	// 3000 220 / 363, 9000 464 / 384; 64 primitives 30 288 / 2414, 16384 1298 / 2547; 128
+	// primitives 16384 1584 / 4901; gradients of 16 primitives 1000 31 / 32, 4000 37 / 34; of 64
+	// primitives 1000 56 / 60, 8000 76 / 69; of 256 primitives 200 119 / 173, 8000 179 / 189,
+	// 16000 239 / 202; values of 64 primitives 1000 47 / 59, 16000 68 / 68; of 256 primitives 1000
+	// 117 / 169, 30000 179 / 182.
 	int TeamForm(const DeviceProgram& prog, int64_t n, TeamWork work, int sms)
 	{
 		const int points = work == TeamWork::Gradient ? 4 : 1;
@@ -317,7 +319,7 @@ namespace tg
 		if (n <= sms && TeamSmem(prog, true, points)) return 2;
 		const double brushes = (double)prog.FullBrushes;
 		const double most = work == TeamWork::Ray ? 26.0 * brushes / (0.037 + 0.0004 * brushes)
-			: 1.2 * brushes / (0.0017 + 0.000022 * brushes) * (work == TeamWork::Gradient ? 1.0 : 0.5);
+			: work == TeamWork::Gradient ? 10000.0 * brushes / (brushes + 48.0) : 0.6 * brushes / (0.0017 + 0.000022 * brushes);
 		return (double)n <= most && TeamSmem(prog, false, points) ? 1 : 0;
 	}
 

@@ -109,25 +109,57 @@ namespace tg
 			position[r * 3 + 2] = m.Position.z;
 		}
 
-		// SDFNode::Eval (gradient = false) or SDFNode::Gradient on the whole tree per point,
-		// as Lua's eval / gradient and EvalTree compute them (lua_sdf.cpp:386-405).
-		__global__ void __launch_bounds__(kTraceThreads) PointQueryKernel(DeviceProgram prog, const float* __restrict__ points, int64_t n,
-			bool gradient, float* __restrict__ out)
+		// SDFNode::Eval or SDFNode::Gradient on the whole tree per point, as Lua's eval / gradient
+		// and EvalTree compute them (lua_sdf.cpp:386-405): a pair of evaluations a lane, two points
+		// or two of a point's four (two lanes a point), all lanes of a warp on the program's one
+		// walk, read through a window in shared memory.  Bound by issue.  Calls from and to the
+		// host, a thread a point (one evaluation after the other) against this: gradients of 64
+		// primitives 100 000 188 / 155, 30 000 142 / 84, of 256 primitives 200 000 1177 / 825, 30 000
+		// 455 / 231, of 8 primitives 1000 35 / 31; values of 256 primitives 200 000 376 / 293.
+		constexpr int kQueryThreads = 128;
+
+		template<bool Gradient>
+		__global__ void __launch_bounds__(kQueryThreads) PointQueryKernel(DeviceProgram prog, const float* __restrict__ points, int64_t n,
+			float* __restrict__ out, int spill_pairs)
 		{
-			extern __shared__ float spill[];
-			const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-			if (t >= n) return;
-			const Vec3 p(points[t * 3], points[t * 3 + 1], points[t * 3 + 2]);
-			if (gradient)
+			extern __shared__ __align__(16) float4 shared4[];
+			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+			float4* window = shared4 + warp * 64;
+			float2* spill = reinterpret_cast<float2*>(shared4 + kQueryThreads / 32 * 64) + warp * spill_pairs * 32 + lane;
+			const int64_t group = (int64_t)blockIdx.x * (kQueryThreads / 32) + warp;
+			const PairUnits units = LoadPairUnits();
+			const float4* code = prog.Code + prog.FullSurfaceCode;
+			auto at = [&](int64_t t) { t = min(t, n - 1); return Vec3(points[t * 3], points[t * 3 + 1], points[t * 3 + 2]); };
+			SurfaceSource src;
+			src.In.Open(code, prog.CodeQuads - prog.FullSurfaceCode, window);
+			if constexpr (!Gradient)
 			{
-				const Vec3 g = TraceShade(prog, prog.FullSurfaceCode, p, false, nullptr, spill + threadIdx.x, kTraceThreads);
-				out[t * 3] = g.x;
-				out[t * 3 + 1] = g.y;
-				out[t * 3 + 2] = g.z;
+				const int64_t t = group * 64 + lane;
+				const Vec3 a = at(t), b = at(t + 32);
+				const float2 d = RunSourcePair(src, make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), units, spill, 32);
+				if (t < n) out[t] = d.x;
+				if (t + 32 < n) out[t + 32] = d.y;
 			}
 			else
 			{
-				out[t] = TraceSurfaceAt(prog, prog.FullSurfaceCode, p, false, nullptr, spill + threadIdx.x, kTraceThreads);
+				const int64_t t = group * 16 + (lane >> 1);
+				const Vec3 p = at(t), a = TetraPoint(p, 2 * (lane & 1)), b = TetraPoint(p, 2 * (lane & 1) + 1);
+				const float2 d = RunSourcePair(src, make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), units, spill, 32);
+				float e[5] = { d.x, d.y, __shfl_down_sync(0xFFFFFFFFu, d.x, 1), __shfl_down_sync(0xFFFFFFFFu, d.y, 1), 0.0f };
+				if (t >= n || (lane & 1)) return;
+				const float h = 0.0001f;
+				const Vec3 xyy(h, -h, -h), yyx(-h, -h, h), yxy(-h, h, -h), xxx(h, h, h);
+				Vec3 g = xyy * e[0];
+				g = g + yyx * e[1];
+				g = g + yxy * e[2];
+				g = g + xxx * e[3];
+				if ((g.x * g.x + g.y * g.y) + g.z * g.z == 0.0f)
+					e[4] = RunWholeSurfacePair(prog.Code, prog.FullSurfaceCode, make_float2(p.x, p.x), make_float2(p.y, p.y), make_float2(p.z, p.z),
+						spill, 32).x;
+				const Vec3 v = GradientOf(e);
+				out[t * 3] = v.x;
+				out[t * 3 + 1] = v.y;
+				out[t * 3 + 2] = v.z;
 			}
 		}
 
@@ -343,14 +375,15 @@ namespace tg
 		cudaStream_t stream)
 	{
 		if (n <= 0) return cudaSuccess;
-		const size_t smem = TraceSpillBytes(prog);
+		const size_t pairs = parts::SpillPairs(prog, 1), smem = kQueryThreads / 32 * (64 * sizeof(float4) + pairs * 32 * sizeof(float2));
+		auto* kernel = gradient ? PointQueryKernel<true> : PointQueryKernel<false>;
 		if (smem > 48 * 1024)
 		{
-			cudaError_t e = cudaFuncSetAttribute(PointQueryKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 			if (e != cudaSuccess) return e;
 		}
-		PointQueryKernel<<<(unsigned)((n + kTraceThreads - 1) / kTraceThreads), kTraceThreads, smem, stream>>>(
-			prog, points, n, gradient, out);
+		const int64_t per = kQueryThreads / 32 * (gradient ? 16 : 64);
+		kernel<<<(unsigned)((n + per - 1) / per), kQueryThreads, smem, stream>>>(prog, points, n, out, (int)pairs);
 		return cudaGetLastError();
 	}
 

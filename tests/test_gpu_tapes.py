@@ -218,3 +218,23 @@ def test_large_lattices_equal_their_pieces(lib, prims, ops, shape):
             at = [0 if cut == 0 else n - s if cut == 1 else int(rng.integers(0, n - s + 1)) for n, s in zip(shape, size)]
             piece = prog.eval_grid(_lib.Grid(*[l + a * step for l, a in zip(low, at)], step, *size))
             np.testing.assert_array_equal(piece, whole[at[2]:at[2] + size[2], at[1]:at[1] + size[1], at[0]:at[0] + size[0]])
+
+
+@pytest.mark.parametrize("name", golden_names())
+def test_point_queries_match_oracle(lib, port, golden, name):
+    """Whole-tree values and gradients in counts around a warp's 64 and 16 points, for every
+    kind of tree."""
+    spec = golden[name]["spec"]
+    try:
+        prog = sdf.compile(sdf.from_spec(spec))
+    except Exception:
+        pytest.skip("no octree for this tree")
+    rng = np.random.default_rng(6)
+    points = rng.uniform(-1.5, 1.5, (20005, 3)).astype(np.float32)
+    points[5000:] = points[rng.integers(0, 1500, 15005)]
+    handle = port.build(spec)
+    values, gradients = port.eval(handle, points), port.gradient(handle, points)
+    with prog:
+        for n in (1, 15, 16, 17, 63, 65, 20005):
+            np.testing.assert_array_equal(prog.eval_tree(points[:n]), values[:n])
+            np.testing.assert_array_equal(prog.gradient_tree(points[:n]), gradients[:n])
