@@ -208,13 +208,15 @@ namespace tg
 		cudaStream_t Stream = nullptr;
 		cudaStream_t CopyStream = nullptr;          // early device-to-host copies of an export
 		// The buffers of a grid's brick tapes (LaunchBrickTapes), kept between exports.
-		cudaError_t ReserveTapes(int64_t bricks, size_t parts, BrickTapes& out);
+		struct TapeBuffers { DeviceBuffer Bricks, Parts, Events, Counters; };
+		cudaError_t ReserveTapes(int64_t bricks, size_t parts, BrickTapes& out) { return ReserveTapes(Tapes, bricks, parts, out); }
+		cudaError_t ReserveTapes(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out);
 		cudaError_t ReadSmCount();
 		cudaEvent_t MeshReady = nullptr;
 		cudaEvent_t CodeReady = nullptr;            // RestageCode's copy of an export is done
 		DeviceBuffer LatticeBuf, Words, WordBase, Scratch, Counts, Vertices, Cubes, FaceCounts, FaceBase, Faces, Normals, Colors;
 		DeviceBuffer Points, PointOut, BrickBits, BrickList, BrickTops, ClassCounts, ProgramScratch, ActiveCells;
-		DeviceBuffer TapeBricks, TapeParts, TapeEvents, TapeCounters;    // ReserveTapes
+		TapeBuffers Tapes, CoarseTapes;
 		DeviceBuffer RayIn, RayOut, Cameras, Image, RenderCounters;
 		DeviceBuffer SodaBoxes, SodaCache, SodaColors;
 		DeviceBuffer VoxScratch, VoxelsOut;

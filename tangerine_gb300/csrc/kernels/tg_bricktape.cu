@@ -21,7 +21,8 @@ namespace tg
 		{
 			static constexpr int kStride = kCells;
 			static constexpr int kBox = parts::kBox, kMost = 24;
-			static constexpr bool kOutside = false, kBetween = true;
+			static constexpr bool kOutside = false, kBetween = true, kAbove = false;
+			static constexpr int kShortest = 0;
 			GridSpec Grid;
 			__device__ __forceinline__ float Coord(int a, int i) const
 			{

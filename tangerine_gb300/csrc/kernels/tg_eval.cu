@@ -136,7 +136,8 @@ namespace tg
 		struct DenseLattice
 		{
 			static constexpr int kBox = 16, kStride = 16, kMost = 96;
-			static constexpr bool kOutside = false, kBetween = false;
+			static constexpr bool kOutside = false, kBetween = false, kAbove = false;
+			static constexpr int kShortest = 0;
 			GridSpec Grid;
 			int K0, Levels;
 			__device__ __forceinline__ float Coord(int a, int i) const

@@ -215,7 +215,8 @@ namespace tg
 		{
 			static constexpr int kStride = parts::kBox;
 			static constexpr int kBox = parts::kBox, kMost = 24;
-			static constexpr bool kOutside = true, kBetween = true;
+			static constexpr bool kOutside = true, kBetween = true, kAbove = false;
+			static constexpr int kShortest = 0;
 			CloudSpec Spec;
 			__device__ __forceinline__ float Coord(int a, int i) const { return ((float)i * Spec.Step[a] + Spec.Start[a]) + Spec.Half[a]; }
 			__host__ __device__ __forceinline__ int Points(int a) const { return a == 0 ? Spec.IX : a == 1 ? Spec.IY : Spec.IZ; }

@@ -131,7 +131,7 @@ namespace tg
 		// Its points' box and one lattice step more, towards the rest of the brick at least (a
 		// vertex may lie between two parts' points), as far as the cell goes.
 		float Lo[3], Hi[3];
-		uint32_t Pad[2];
+		uint2 First;            // the value list's first event: most have only one
 	};
 	constexpr int kBrickTapeCounters = 5;   // parts, parts taken for building, events, bricks evaluated, long parts
 	struct BrickTapes
@@ -210,7 +210,10 @@ namespace tg
 	// images): how many bricks per axis pay for that many pixels (0: none), and the launch, with
 	// the tapes' buffers for bricks^3 bricks.  pivot, root_clip: the root cell's.
 	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels);
+	// above: the buffers for tapes of the 4^3 times larger bricks first ((bricks / 4)^3), from which
+	// the others are then built (Bricks == nullptr: without).
 	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes,
+		const BrickTapes& above,
 		const CameraBasis* cameras, int count, int width, int height, int max_steps, float epsilon, float* depth, float* normals,
 		uint8_t* colors, int sms, cudaStream_t stream);
 

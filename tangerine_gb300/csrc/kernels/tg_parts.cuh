@@ -8,8 +8,10 @@
 // A lattice L says where its points lie: Coord(axis, index), Points(axis), Bricks(axis),
 // kStride (points from one brick to the next), kBox (points of a brick per axis, at most 16),
 // kMost (parts of a brick, at most), kOutside (vertices may leave their brick by up to a step),
-// kBetween (points between the lattice's look for their part, too), and Keep(): the distance
-// beyond which a part's points are of no interest.
+// kBetween (points between the lattice's look for their part, too), kShortest (quads of the
+// programs that get a tape, at least; not 0: the tapes are there to build finer ones from),
+// kAbove (there may be such coarser tapes: those of brick Above(b) for brick b), and Keep(): the
+// distance beyond which a part's points are of no interest.
 #pragma once
 
 #include "tg_device.cuh"
@@ -27,6 +29,7 @@ namespace tg
 		constexpr int kBuildCtasPerSm = 8;
 		constexpr int kBox = 8;             // points per axis of most lattices' bricks
 		constexpr int kLongQuads = 96;      // programs from this long are built first
+		constexpr int kAboveQuads = 48;     // and from this long by way of a coarser brick's tape
 
 		__device__ __forceinline__ uint32_t PackBox(int x0, int x1, int y0, int y1, int z0, int z1)
 		{
@@ -88,7 +91,7 @@ namespace tg
 			out.Counts = kNoTape | (kNoTape << 16);
 			out.Distance = out.Surface = 0;
 			out.Brick = b;
-			out.Pad[0] = out.Pad[1] = 0;
+			out.First = make_uint2(0u, 0u);
 #pragma unroll
 			for (int a = 0; a < 3; ++a) { out.Lo[a] = 1.0f; out.Hi[a] = 0.0f; }
 			if (cell >= 0)
@@ -289,25 +292,45 @@ namespace tg
 		}
 
 		// A warp's scratch while it builds a part's tape.
+		template<int Cap>
 		struct TapeScratch
 		{
-			uint2 Value[kTapeCap], Material[kTapeCap];
+			uint2 Value[Cap], Material[Cap];
 			uint2 Start[kMaxStack + 2];
+			uint2 Heads[8];
 			float4 Window[64];
 		};
+
+		// The part of a coarser lattice's brick that holds this one, with a material list: that
+		// list leaves out nothing that any point of it needs, for the distance or for the material.
+		__device__ __forceinline__ int PartAround(const BrickTapes& above, uint2 own, int cell, const float (&lo)[3], const float (&hi)[3])
+		{
+			const uint32_t q = threadIdx.x & 31;
+			bool mine = false;
+			if (q < own.y)
+			{
+				const BrickPart& p = above.Parts[own.x + q];
+				mine = p.Cell == cell && (p.Counts >> 16) != kNoTape;
+#pragma unroll
+				for (int a = 0; a < 3; ++a) mine = mine && p.Lo[a] <= lo[a] && p.Hi[a] >= hi[a];
+			}
+			const unsigned which = __ballot_sync(0xFFFFFFFFu, mine);
+			return which ? (int)own.x + __ffs((int)which) - 1 : -1;
+		}
 
 		// One warp per part, drawn from a counter, those with long programs first (a single one
 		// of several hundred records keeps a warp busy longer than the whole launch otherwise
 		// takes).  Bound by issue and by the latency of the one pass over the cell's program.
 		template<typename L>
 		__global__ void __launch_bounds__(kThreads, kBuildCtasPerSm) BuildPartTapesKernel(DeviceProgram prog, L lat, BrickTapes tapes,
-			int spill_pairs)
+			BrickTapes above, int spill_pairs)
 		{
 			extern __shared__ __align__(16) uint8_t shared[];
 			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-			TapeScratch& ts = reinterpret_cast<TapeScratch*>(shared)[warp];
-			const TapeLists lists{ ts.Value, ts.Material, ts.Start, kTapeCap };
-			float2* spill = reinterpret_cast<float2*>(shared + kWarps * sizeof(TapeScratch)) + warp * spill_pairs * 32 + lane;
+			using Scratch = TapeScratch<L::kShortest ? 2 * kTapeCap : kTapeCap>;
+			Scratch& ts = reinterpret_cast<Scratch*>(shared)[warp];
+			const TapeLists lists{ ts.Value, ts.Material, ts.Start, L::kShortest ? 2 * kTapeCap : kTapeCap };
+			float2* spill = reinterpret_cast<float2*>(shared + kWarps * sizeof(Scratch)) + warp * spill_pairs * 32 + lane;
 			const uint32_t n = min(tapes.Counters[0], tapes.PartCapacity), longs = min(tapes.Counters[4], kLongParts);
 			const float rootClip = __ldg(&prog.Nodes[0].ClipRadius);
 			const PairUnits units = LoadPairUnits();
@@ -324,7 +347,8 @@ namespace tg
 				const uint32_t box = part.Box;
 				if (cell < 0 || (item >= longs && (box & kBoxLong))) continue;
 				if (__ldg(&prog.Nodes[cell].ClipRadius) < 0.0f) continue;    // not 1-Lipschitz: no tape
-				const int base = part.Distance;
+				const int base = part.Distance, quads = part.Surface - base;
+				if (quads < L::kShortest) continue;
 				TapeCounts counts;
 				float reach;
 				__syncwarp();       // the previous part's lists have been copied out
@@ -339,11 +363,24 @@ namespace tg
 					const float r = 0.5f * sqrtf(wx * wx + wy * wy + wz * wz) + kTetraReach;
 					reach = TapeReach(r, fmaxf(fabsf(lo[0]), fabsf(hi[0])), fmaxf(fabsf(lo[1]), fabsf(hi[1])),
 						fmaxf(fabsf(lo[2]), fabsf(hi[2])), rootClip);
-					DistanceSource src;
-					const int quads = part.Surface - base;
-					src.In.Open(code + base, quads, ts.Window);
-					ok = quads <= 0xFFF0 && BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach,
-						units, spill, 32, lists, counts);
+					int around = -1;
+					if constexpr (L::kAbove)
+						if (above.Bricks && quads >= kAboveQuads) around = PartAround(above, above.Bricks[lat.Above(part.Brick)], cell, lo, hi);
+					if (L::kAbove && around >= 0)
+					{
+						const BrickPart& p = above.Parts[around];
+						DistanceEventSource src;
+						src.Open(code + base, above.Events + p.Material, (int)(p.Counts >> 16), ts.Window, ts.Heads);
+						ok = BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach, units, spill, 32,
+							lists, counts);
+					}
+					else
+					{
+						DistanceSource src;
+						src.In.Open(code + base, quads, ts.Window);
+						ok = quads <= 0xFFF0 && BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach,
+							units, spill, 32, lists, counts);
+					}
 				}
 				if (!ok) continue;
 				// |f| beyond a ball's radius (half the reach covers it) and Keep() at every centre.
@@ -361,9 +398,10 @@ namespace tg
 				if (lane == 0)
 				{
 					part.Value = at;
+					part.First = ts.Value[0];
 					part.Material = counts.Same ? at : at + (uint32_t)counts.Value;
 					part.Counts = (uint32_t)counts.Value |
-						((prog.Form & kFormPainted) ? (uint32_t)(counts.Same ? counts.Value : counts.Material) << 16 : kNoTape << 16);
+						((prog.Form & kFormPainted) || L::kShortest ? (uint32_t)(counts.Same ? counts.Value : counts.Material) << 16 : kNoTape << 16);
 				}
 			}
 		}
@@ -446,6 +484,7 @@ namespace tg
 			int Surface, Distance;          // first quads
 			uint32_t Value, Material;       // first events
 			uint32_t Events, Walk;          // events of the two lists (kNoTape: the whole program)
+			uint2 First;                    // the first list's first event
 			float Lo[3], Hi[3];             // the points known to run the same
 		};
 
@@ -460,11 +499,11 @@ namespace tg
 			for (uint32_t q = 0; q < own.y; ++q)
 			{
 				const uint4* part = reinterpret_cast<const uint4*>(tapes.Parts + own.x + q);
-				const uint4 a = __ldg(part + 2), b = __ldg(part + 3);
+				// The whole part at once: a march is a chain of such loads.
+				const uint4 c = __ldg(part), d = __ldg(part + 1), a = __ldg(part + 2), b = __ldg(part + 3);
 				run.Lo[0] = __uint_as_float(a.x); run.Lo[1] = __uint_as_float(a.y); run.Lo[2] = __uint_as_float(a.z);
 				run.Hi[0] = __uint_as_float(a.w); run.Hi[1] = __uint_as_float(b.x); run.Hi[2] = __uint_as_float(b.y);
 				if (!InRun(run, p)) continue;
-				const uint4 c = __ldg(part), d = __ldg(part + 1);
 				run.Cell = (int)c.x;
 				run.Value = c.z;
 				run.Events = c.w & 0xFFFFu;
@@ -472,6 +511,7 @@ namespace tg
 				run.Distance = (int)d.x;
 				run.Surface = (int)d.y;
 				run.Material = d.z;
+				run.First = make_uint2(b.z, b.w);
 				return true;
 			}
 			return false;
@@ -562,7 +602,7 @@ namespace tg
 		// Parts and tapes of the listed bricks of a lattice (list and count null: of all bricks).
 		template<typename L>
 		inline cudaError_t LaunchParts(const DeviceProgram& prog, const L& lat, const uint32_t* list, const uint32_t* count, const uint32_t* tops,
-			const BrickTapes& tapes, int sms, cudaStream_t stream)
+			const BrickTapes& tapes, int sms, cudaStream_t stream, const BrickTapes& above = BrickTapes{})
 		{
 			cudaError_t e = cudaMemsetAsync(tapes.Counters, 0, kBrickTapeCounters * sizeof(uint32_t), stream);
 			if (e != cudaSuccess) return e;
@@ -572,13 +612,13 @@ namespace tg
 			e = cudaGetLastError();
 			if (e != cudaSuccess || !(prog.Form & kFormPrunable)) return e;
 			const size_t pairs = SpillPairs(prog, 1);
-			const size_t smem = kWarps * (sizeof(TapeScratch) + pairs * 32 * sizeof(float2));
+			const size_t smem = kWarps * (sizeof(TapeScratch<L::kShortest ? 2 * kTapeCap : kTapeCap>) + pairs * 32 * sizeof(float2));
 			if (smem > 48 * 1024)
 			{
 				e = cudaFuncSetAttribute(BuildPartTapesKernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 				if (e != cudaSuccess) return e;
 			}
-			BuildPartTapesKernel<L><<<sms * kBuildCtasPerSm, kThreads, smem, stream>>>(prog, lat, tapes, (int)pairs);
+			BuildPartTapesKernel<L><<<sms * kBuildCtasPerSm, kThreads, smem, stream>>>(prog, lat, tapes, above, (int)pairs);
 			return cudaGetLastError();
 		}
 	}

@@ -273,15 +273,15 @@ namespace tg
 		}
 	}
 
-	// The distance at one point by a tape (RunTapePairs, one lane).  Operands below the top of
-	// the stack are at spill[depth * stride].
+	// The distance at one point by a tape (RunTapePairs, one lane) whose first event is x.
+	// Operands below the top of the stack are at spill[depth * stride].
 	template<typename Load, typename Event>
-	__device__ __forceinline__ float RunTapePoint(Load load, int base, Event event, uint32_t count, float px, float py, float pz, float* spill,
-		int stride)
+	__device__ __forceinline__ float RunTapePoint(Load load, int base, uint32_t x, Event event, uint32_t count, float px, float py, float pz,
+		float* spill, int stride)
 	{
 		float acc = 0.0f, left = 0.0f;
 		int depth = 0;
-		uint32_t e = 0, x = event(0u).x;
+		uint32_t e = 0;
 		for (;;)
 		{
 			uint32_t op = x & 0xFFu;
@@ -654,6 +654,21 @@ namespace tg
 		__device__ __forceinline__ float4 Load(int q) const { return Window[q & 63]; }
 	};
 
+	// A distance brush's distance at two points, from its record's quads, and the size its float
+	// error goes with.
+	template<typename Load>
+	__device__ __forceinline__ float2 DistanceBrush(Load load, uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size)
+	{
+		const float2 x[1] = { px }, y[1] = { py }, z[1] = { pz };
+		float2 qx[1], qy[1], qz[1], d[1];
+		float4 h;
+		BrushStep<1, false>(load, 0, head, x, y, z, u, qx, qy, qz, h, d);
+		const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
+		size = make_float2(fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(d[0].x),
+			fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(d[0].y));
+		return d[0];
+	}
+
 	// What BuildTape reads: the records of a program in order, each with its event.
 	//
 	// A cell's distance program; events name the surface records too (the same brushes and
@@ -675,17 +690,9 @@ namespace tg
 			Pc += DistanceRecordQuads(head);
 			Surface += (head & 0xFFu) <= OpPlane ? 4 : 1;
 		}
-		// The brush's distance at the two points, and the size its float error goes with.
 		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
 		{
-			const float2 x[1] = { px }, y[1] = { py }, z[1] = { pz };
-			float2 qx[1], qy[1], qz[1], d[1];
-			float4 h;
-			BrushStep<1, false>([&](int q) { return In.Load(q); }, Pc, head, x, y, z, u, qx, qy, qz, h, d);
-			const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
-			size = make_float2(fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(d[0].x),
-				fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(d[0].y));
-			return d[0];
+			return DistanceBrush([&](int q) { return In.Load(Pc + q); }, head, px, py, pz, u, size);
 		}
 	};
 
@@ -795,6 +802,74 @@ namespace tg
 			const float2 d = SurfaceBrushStep<false>(head & 0xFFu, h, Quad(1), T, px, py, pz, u);
 			size = SurfaceBrushSize(h, T, px, py, pz, d);
 			return d;
+		}
+	};
+
+	// The same for distance records: four events at a time, eight lanes each (a brush takes up to
+	// five quads), with the next four in flight.
+	struct DistanceEventSource
+	{
+		const float4* Code;     // the distance program
+		const uint2* Events;
+		int Count;
+		float4* Window;         // 8 events x 8 quads
+		uint2* Heads;           // 8 events
+		int At = 0, Chunk = 0;
+		float4 Ahead;           // of this lane's event of the chunk after the two in the window,
+		uint2 AheadEvent, NextEvent;    // its event, and that of the chunk after it
+
+		__device__ __forceinline__ uint2 FetchEvent(int chunk) const
+		{
+			const int e = chunk * 4 + (int)((threadIdx.x & 31) >> 3);
+			return e < Count ? __ldg(Events + e) : make_uint2(0u, 0u);
+		}
+		__device__ __forceinline__ float4 FetchQuad(uint2 ev) const
+		{
+			const int q = (int)(threadIdx.x & 7);
+			const uint32_t op = ev.x & 0xFFu;
+			return op != 0u && op < OpTapeNegate && q < DistanceRecordQuads(ev.x) ? __ldg(Code + (ev.x >> 16) + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+		}
+		__device__ __forceinline__ void Put(int half, uint2 ev, float4 quad)
+		{
+			const int lane = (int)(threadIdx.x & 31);
+			Window[half * 32 + lane] = quad;
+			if ((lane & 7) == 0) Heads[half * 4 + (lane >> 3)] = ev;
+		}
+		__device__ __forceinline__ void Open(const float4* code, const uint2* events, int count, float4* window, uint2* heads)
+		{
+			Code = code;
+			Events = events;
+			Count = count;
+			Window = window;
+			Heads = heads;
+			const uint2 e0 = FetchEvent(0), e1 = FetchEvent(1);
+			AheadEvent = FetchEvent(2);
+			NextEvent = FetchEvent(3);
+			Put(0, e0, FetchQuad(e0));
+			Put(1, e1, FetchQuad(e1));
+			Ahead = FetchQuad(AheadEvent);
+			__syncwarp();
+		}
+		__device__ __forceinline__ uint32_t Head()
+		{
+			while (Chunk < (At >> 2))
+			{
+				__syncwarp();
+				Put(Chunk & 1, AheadEvent, Ahead);
+				++Chunk;
+				AheadEvent = NextEvent;
+				Ahead = FetchQuad(AheadEvent);
+				NextEvent = FetchEvent(Chunk + 3);
+				__syncwarp();
+			}
+			return At < Count ? Heads[At & 7].x & 0xFFFFu : OpStop;
+		}
+		__device__ __forceinline__ uint2 Event(uint32_t) const { const uint2 ev = Heads[At & 7]; return make_uint2(ev.x & ~RecThenSet, ev.y); }
+		__device__ __forceinline__ float Operand() const { return Window[(At & 7) * 8].y; }
+		__device__ __forceinline__ void Advance(uint32_t) { ++At; }
+		__device__ __forceinline__ float2 Brush(uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size) const
+		{
+			return DistanceBrush([&](int q) { return Window[(At & 7) * 8 + q]; }, head, px, py, pz, u, size);
 		}
 	};
 

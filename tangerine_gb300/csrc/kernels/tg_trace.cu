@@ -211,11 +211,17 @@ namespace tg
 		// The root cube in bricks for the renderer's tapes: 8^3 points a brick at the centres of
 		// the cube's (8 N)^3 cells.  The octree halves the cube, so a brick lies in one cell where
 		// the cells are no smaller.
-		struct RenderLattice
+		// Level 1: bricks of 4^3 of those, for the tapes that theirs are built from: 32 768 passes of
+		// programs of several hundred records took longer than the rays (2364 of 2550 us for 512
+		// primitives at 2 x 300 x 200, 1811 of 5920 for 1024 at 2 x 1920 x 1080); by way of 512
+		// larger bricks' tapes the images take 738 and 5011.
+		template<int Level>
+		struct RenderBricksOf
 		{
 			static constexpr int kStride = parts::kBox;
 			static constexpr int kBox = parts::kBox, kMost = 24;
-			static constexpr bool kOutside = true, kBetween = true;
+			static constexpr bool kOutside = true, kBetween = true, kAbove = Level == 0;
+			static constexpr int kShortest = Level == 0 ? 0 : parts::kAboveQuads;
 			float Origin[3];
 			float Step;
 			int N;
@@ -232,7 +238,13 @@ namespace tg
 				const uint32_t z = (uint32_t)fminf(fmaxf((p.z - Origin[2]) * over, 0.0f), most);
 				return x + (uint32_t)N * (y + (uint32_t)N * z);
 			}
+			__device__ __forceinline__ uint32_t Above(uint32_t b) const
+			{
+				const uint32_t n = (uint32_t)N, coarse = n / 4;
+				return b % n / 4 + coarse * (b / n % n / 4 + coarse * (b / (n * n) / 4));
+			}
 		};
+		using RenderLattice = RenderBricksOf<0>;
 
 		// MarchBounded by the bricks' tapes: the same distances, and so the same steps.
 		__device__ __forceinline__ March MarchTapes(const DeviceProgram& prog, const RenderLattice& lat, const BrickTapes& tapes, Vec3 start,
@@ -274,7 +286,7 @@ namespace tg
 					if (run.Events != kNoTape)
 					{
 						const uint2* ev = tapes.Events + run.Value;
-						f = RunTapePoint([&](int q) { return __ldg(code + q); }, run.Distance, [&](uint32_t e) { return __ldg(ev + e); }, run.Events,
+						f = RunTapePoint([&](int q) { return __ldg(code + q); }, run.Distance, run.First.x, [&](uint32_t e) { return __ldg(ev + e); }, run.Events,
 							pos.x, pos.y, pos.z, spill, 2 * 32);
 					}
 					else f = RunWholePoint(code, run.Distance, pos.x, pos.y, pos.z, spill, 2 * 32);
@@ -416,7 +428,7 @@ namespace tg
 		return n <= 64 && pixels >= (int64_t)n * n * n / 4 ? n : 0;
 	}
 
-	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes,
+	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes, const BrickTapes& above,
 		const CameraBasis* cameras, int count, int width, int height, int max_steps, float epsilon, float* depth, float* normals,
 		uint8_t* colors, int sms, cudaStream_t stream)
 	{
@@ -425,7 +437,17 @@ namespace tg
 		lat.N = bricks;
 		lat.Step = 2.0f * half / (float)(bricks * parts::kBox);
 		for (int a = 0; a < 3; ++a) lat.Origin[a] = pivot[a] - half;
-		cudaError_t e = parts::LaunchParts(prog, lat, nullptr, nullptr, nullptr, tapes, sms, stream);
+		cudaError_t e = cudaSuccess;
+		if (above.Bricks)
+		{
+			RenderBricksOf<1> coarse;
+			coarse.N = bricks / 4;
+			coarse.Step = 4.0f * lat.Step;
+			for (int a = 0; a < 3; ++a) coarse.Origin[a] = lat.Origin[a];
+			e = parts::LaunchParts(prog, coarse, nullptr, nullptr, nullptr, above, sms, stream);
+			if (e != cudaSuccess) return e;
+		}
+		e = parts::LaunchParts(prog, lat, nullptr, nullptr, nullptr, tapes, sms, stream, above);
 		if (e != cudaSuccess) return e;
 		// The colour's walk takes two words a level, the gradient one pair.
 		const size_t smem = parts::SpillPairs(prog, 2) * 32 * sizeof(float2);

@@ -125,13 +125,33 @@ def test_point_cloud_tapes_match_oracle(lib, port, prims, ops, paint, step, refi
         assert m.colors is None
 
 
-@pytest.mark.parametrize("prims,ops", [(3, ALL_OPS), (150, ALL_OPS), (600, W.OPS_60_20_10_10)])
-def test_render_by_tapes_equals_render_without(lib, prims, ops):
-    """Enough pixels together go by the root cube's tapes; the same poses one by one do not.
-    Odd image sides, a camera inside the root cube, one that misses it."""
+def _large_cells(prims, ops, paint):
+    """A tree with long programs in most of its space: few cells, so few of them were split."""
     seed = 31
-    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops))):
-        seed += 1
+    for seed in range(31, 400):
+        spec = W.random_tree(seed, prims, ops=ops, paint=paint)
+        if not sdf.has_export_octree(sdf.from_spec(spec)):
+            continue
+        with sdf.compile(sdf.from_spec(spec)) as prog:
+            info = prog.info()
+        if info.distance_quads >= 100 * info.octree_cells:
+            return spec
+    raise AssertionError("no such tree")
+
+
+@pytest.mark.parametrize("prims,ops,large,paint", [(3, ALL_OPS, False, True), (150, ALL_OPS, False, True), (600, W.OPS_60_20_10_10, False, True),
+                                                   (400, W.OPS_60_20_10_10, True, True), (400, ALL_OPS, True, True),
+                                                   (300, W.OPS_60_20_10_10, True, False)])
+def test_render_by_tapes_equals_render_without(lib, prims, ops, large, paint):
+    """Enough pixels together go by the root cube's tapes (built by way of larger bricks' where
+    the cells are large); the same poses one by one do not.  Odd image sides, a camera inside
+    the root cube, one that misses it."""
+    if large:
+        spec = _large_cells(prims, ops, paint)
+    else:
+        seed = 31
+        while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops))):
+            seed += 1
     poses = np.concatenate([W.camera_poses(7, 7), [[0.3, 0.2, 0.1], [60.0, 50.0, 70.0]]]).astype(np.float32)
     with sdf.compile(sdf.from_spec(spec)) as prog:
         depth, normals, colors = prog.render(sdf.cameras(poses), 83, 61)
