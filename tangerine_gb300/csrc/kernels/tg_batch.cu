@@ -585,8 +585,8 @@ namespace tg
 					const uint32_t* base = s.CellWordBase + m.CellWord0;
 					const uint32_t w = words[c >> 5];
 					const uint32_t vid = base[c >> 5] + __popc(w & ((1u << (c & 31)) - 1u));
-					const int64_t i = c % cg.sx, j = (c / cg.sx) % cg.sy, k = c / (cg.sx * cg.sy);
-					EmitCellVertex(s.Lattice + m.Lattice, m.Grid, cg, words, c, i, j, k, vid, s.Vertices, s.Cubes, s.FaceCounts);
+					const CellIndex at = CellAt((uint32_t)c, cg);
+					EmitCellVertex(s.Lattice + m.Lattice, m.Grid, cg, words, c, at.i, at.j, at.k, vid, s.Vertices, s.Cubes, s.FaceCounts);
 				}
 			}
 			if (!GridSync(s)) return;
@@ -609,35 +609,8 @@ namespace tg
 				{
 					const int mi = ModelOf(s.VertexBase, s.Count, (uint32_t)v0);
 					const BatchModel& m = s.Models[mi];
-					const CellGeom cg = Geom(m.Grid);
-					const float* lat = s.Lattice + m.Lattice;
-					const uint32_t* words = s.CellBits + m.CellWord0;
-					const uint32_t* base = s.CellWordBase + m.CellWord0;
-					const uint32_t vb = s.VertexBase[mi];
-					const int64_t c = s.Cubes[v0];
-					const int64_t i = c % cg.sx, j = (c / cg.sx) % cg.sy, k = c / (cg.sx * cg.sy);
-					if (i == 0 || j == 0 || k == 0) continue;
-					const int64_t dy = cg.sx, dz = cg.sx * cg.sy;
-					const int64_t nb[6] = { c - 1, c - 1 - dy, c - dy, c - dy - dz, c - dz, c - 1 - dz };
-					const int quads[3][3] = { {0, 1, 2}, {0, 5, 4}, {2, 3, 4} };
-					const float c0 = Corner(lat, cg, i, j, k);
-					const float sv[3][2] = { { c0, Corner(lat, cg, i, j, k + 1) }, { Corner(lat, cg, i, j + 1, k), c0 },
-						{ c0, Corner(lat, cg, i + 1, j, k) } };
-					uint32_t out = s.FaceBase[v0];
-					const uint32_t self = (uint32_t)v0 - vb;
-					for (int q = 0; q < 3; ++q)
-					{
-						const int64_t a = nb[quads[q][0]], b = nb[quads[q][1]], d = nb[quads[q][2]];
-						if (!(IsActive(words, a) && IsActive(words, b) && IsActive(words, d))) continue;
-						const uint32_t nv[3] = { VertexOf(words, base, a) - vb, VertexOf(words, base, b) - vb, VertexOf(words, base, d) - vb };
-						uint32_t v1, v2, v3;
-						if (sv[q][1] > sv[q][0]) { v1 = nv[0]; v2 = nv[1]; v3 = nv[2]; }
-						else { v1 = nv[2]; v2 = nv[1]; v3 = nv[0]; }
-						uint32_t* f = s.Faces + (int64_t)out * 3;
-						f[0] = self; f[1] = v1; f[2] = v2;
-						f[3] = self; f[4] = v2; f[5] = v3;
-						out += 2;
-					}
+					EmitCellFaces(s.Lattice + m.Lattice, Geom(m.Grid), s.CellBits + m.CellWord0, s.CellWordBase + m.CellWord0, s.Cubes[v0],
+						(uint32_t)v0 - s.VertexBase[mi], s.VertexBase[mi], s.FaceBase[v0], s.Faces);
 				}
 			}
 

@@ -72,10 +72,16 @@ namespace tg
 		__global__ void ListBricksByCostKernel(const uint32_t* __restrict__ bits, int64_t bricks, DeviceProgram prog, GridSpec g,
 			BrickGrid bg, uint32_t* __restrict__ tops, uint32_t* counts, uint32_t* total, uint32_t* __restrict__ list)
 		{
+			// Per block one atomic a class: a warp each, they were all of its time on fine grids.
+			__shared__ uint32_t found[kCostClasses], first[kCostClasses];
 			const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
 			const int lane = (int)(threadIdx.x & 31);
 			int cls = kCostClasses;           // not kept
-			if (b < bricks && ((__ldg(bits + (b >> 5)) >> (b & 31)) & 1u))
+			const bool kept = b < bricks && ((__ldg(bits + (b >> 5)) >> (b & 31)) & 1u);
+			if (!__syncthreads_or(kept)) return;
+			if (threadIdx.x < kCostClasses) found[threadIdx.x] = 0;
+			__syncthreads();
+			if (kept)
 			{
 				uint32_t top;
 				if constexpr (Descend)
@@ -92,21 +98,24 @@ namespace tg
 				cls = CostClass(prog, top);
 			}
 			const unsigned peers = __match_any_sync(0xFFFFFFFFu, cls);
-			if (cls == kCostClasses) return;
 			const int leader = __ffs((int)peers) - 1;
-			const uint32_t k = (uint32_t)__popc(peers);
-			if (!Place)
-			{
-				if (lane == leader) { atomicAdd(counts + cls, k); atomicAdd(total, k); }
-				return;
-			}
 			uint32_t at = 0;
-			if (lane == leader) at = atomicAdd(counts + kCostClasses + cls, k);
-			at = __shfl_sync(peers, at, leader);
-			uint32_t start = 0;
+			if (kept && lane == leader) at = atomicAdd(found + cls, (uint32_t)__popc(peers));
+			at = __shfl_sync(0xFFFFFFFFu, at, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+			__syncthreads();
+			if (threadIdx.x < kCostClasses && found[threadIdx.x])
+			{
+				const uint32_t k = found[threadIdx.x];
+				if (Place) first[threadIdx.x] = atomicAdd(counts + kCostClasses + threadIdx.x, k);
+				else { atomicAdd(counts + threadIdx.x, k); atomicAdd(total, k); }
+			}
+			if (!Place) return;
+			__syncthreads();
+			if (!kept) return;
+			uint32_t start = first[cls];
 #pragma unroll
 			for (int c = 0; c < kCostClasses - 1; ++c) if (c < cls) start += counts[c];
-			list[start + at + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = (uint32_t)b;
+			list[start + at] = (uint32_t)b;
 		}
 
 		// Bricks whose bit is set, in brick-index order (x fastest): consecutive list entries
@@ -447,11 +456,11 @@ namespace tg
 			const CellGeom cg = Geom(g);
 			const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
 			if (t >= cell_count) return;
-			const int64_t c = __ldg(cells + t);
+			const uint32_t c = __ldg(cells + t);
 			const uint32_t w = __ldg(words + (c >> 5));
 			const uint32_t vid = __ldg(base + (c >> 5)) + __popc(w & ((1u << (c & 31)) - 1u));
-			const int64_t i = c % cg.sx, j = (c / cg.sx) % cg.sy, k = c / (cg.sx * cg.sy);
-			EmitCellVertex(lat, g, cg, words, c, i, j, k, vid, vertices, cubes, face_counts);
+			const CellIndex at = CellAt(c, cg);
+			EmitCellVertex(lat, g, cg, words, c, at.i, at.j, at.k, vid, vertices, cubes, face_counts);
 		}
 
 	}

@@ -22,11 +22,9 @@ namespace tg
 			bool active = false;
 			if (c < cells)
 			{
-				const int64_t i = c % cg.sx;
-				const int64_t j = (c / cg.sx) % cg.sy;
-				const int64_t k = c / (cg.sx * cg.sy);
+				const CellIndex at = CellAt((uint32_t)c, cg);
 				float v[8];
-				LoadCorners(lat, cg, i, j, k, v);
+				LoadCorners(lat, cg, at.i, at.j, at.k, v);
 				// "Positive" is >= isovalue (0); a cell with two signs has a bipolar edge.
 				unsigned pos = 0;
 #pragma unroll
@@ -47,10 +45,8 @@ namespace tg
 			const uint32_t w = __ldg(words + (c >> 5));
 			if (!((w >> (c & 31)) & 1u)) return;
 			const uint32_t vid = __ldg(base + (c >> 5)) + __popc(w & ((1u << (c & 31)) - 1u));
-			const int64_t i = c % cg.sx;
-			const int64_t j = (c / cg.sx) % cg.sy;
-			const int64_t k = c / (cg.sx * cg.sy);
-			EmitCellVertex(lat, g, cg, words, c, i, j, k, vid, vertices, cubes, face_counts);
+			const CellIndex at = CellAt((uint32_t)c, cg);
+			EmitCellVertex(lat, g, cg, words, c, at.i, at.j, at.k, vid, vertices, cubes, face_counts);
 		}
 
 		__global__ void FacesKernel(const float* __restrict__ lat, GridSpec g, const uint32_t* __restrict__ words,
@@ -60,31 +56,7 @@ namespace tg
 			const CellGeom cg = Geom(g);
 			const uint32_t v0 = blockIdx.x * blockDim.x + threadIdx.x;
 			if (v0 >= vertex_count) return;
-			const int64_t c = __ldg(cubes + v0);
-			const int64_t i = c % cg.sx;
-			const int64_t j = (c / cg.sx) % cg.sy;
-			const int64_t k = c / (cg.sx * cg.sy);
-			if (i == 0 || j == 0 || k == 0) return;
-			const int64_t dy = cg.sx, dz = cg.sx * cg.sy;
-			const int64_t nb[6] = { c - 1, c - 1 - dy, c - dy, c - dy - dz, c - dz, c - 1 - dz };
-			const int quads[3][3] = { {0, 1, 2}, {0, 5, 4}, {2, 3, 4} };
-			// Directed edges (0,4), (3,0), (0,1) decide the winding (surface_nets.cpp:1041-1105).
-			const float c0 = Corner(lat, cg, i, j, k);
-			const float s[3][2] = { { c0, Corner(lat, cg, i, j, k + 1) }, { Corner(lat, cg, i, j + 1, k), c0 }, { c0, Corner(lat, cg, i + 1, j, k) } };
-			uint32_t out = __ldg(face_base + v0);
-			for (int q = 0; q < 3; ++q)
-			{
-				const int64_t a = nb[quads[q][0]], b = nb[quads[q][1]], d = nb[quads[q][2]];
-				if (!(IsActive(words, a) && IsActive(words, b) && IsActive(words, d))) continue;
-				const uint32_t nv[3] = { VertexOf(words, base, a), VertexOf(words, base, b), VertexOf(words, base, d) };
-				uint32_t v1, v2, v3;
-				if (s[q][1] > s[q][0]) { v1 = nv[0]; v2 = nv[1]; v3 = nv[2]; }
-				else { v1 = nv[2]; v2 = nv[1]; v3 = nv[0]; }
-				uint32_t* f = faces + (int64_t)out * 3;
-				f[0] = v0; f[1] = v1; f[2] = v2;
-				f[3] = v0; f[4] = v2; f[5] = v3;
-				out += 2;
-			}
+			EmitCellFaces(lat, cg, words, base, __ldg(cubes + v0), v0, 0u, __ldg(face_base + v0), faces);
 		}
 
 		// Face normals (the STL writer): five threads per point (the four tetrahedral offsets
@@ -235,16 +207,35 @@ namespace tg
 			out[t] = r[0];
 		}
 
-		// ---- exclusive scan: 1024 threads x 4 items per block -------------------------
+		// ---- exclusive scan: 1024 threads x 16 items per block ------------------------
+		// Of counts, or of words' popcounts; then only the words that have bits get their base
+		// (nobody looks up another's), which spares most of the writes.  Bound by memory.  The
+		// 33 million cell words of a 1024^3 export: 145 us by four single words
+		// a thread and every base written, 74 so; up to two blocks' items by one block (8 for 12 us).
 		constexpr int kScanThreads = 1024;
-		constexpr int kScanItems = 4;
+		constexpr int kScanItems = 16;
 		constexpr int kScanTile = kScanThreads * kScanItems;
 
-		__device__ __forceinline__ uint32_t ScanItem(const uint32_t* in, int64_t i, int64_t n, bool pop)
+		// This thread's items from `base` on, 0 beyond n.
+		__device__ __forceinline__ void ScanItems(const uint32_t* __restrict__ in, int64_t base, int64_t n, bool pop, uint32_t (&v)[kScanItems])
 		{
-			if (i >= n) return 0u;
-			const uint32_t x = __ldg(in + i);
-			return pop ? (uint32_t)__popc(x) : x;
+			if (base + kScanItems <= n && (reinterpret_cast<uintptr_t>(in) & 15u) == 0)
+			{
+#pragma unroll
+				for (int q = 0; q < kScanItems / 4; ++q)
+				{
+					const uint4 x = __ldg(reinterpret_cast<const uint4*>(in + base) + q);
+					v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+				}
+			}
+			else
+			{
+#pragma unroll
+				for (int q = 0; q < kScanItems; ++q) v[q] = base + q < n ? __ldg(in + base + q) : 0u;
+			}
+			if (!pop) return;
+#pragma unroll
+			for (int q = 0; q < kScanItems; ++q) v[q] = (uint32_t)__popc(v[q]);
 		}
 
 		// Block-wide exclusive scan of one value per thread; returns the block total.
@@ -284,9 +275,10 @@ namespace tg
 		__global__ void __launch_bounds__(kScanThreads) ScanReduceKernel(const uint32_t* __restrict__ in, int64_t n, bool pop, uint32_t* __restrict__ sums)
 		{
 			const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-			uint32_t s = 0;
+			uint32_t v[kScanItems], s = 0;
+			ScanItems(in, base, n, pop, v);
 #pragma unroll
-			for (int q = 0; q < kScanItems; ++q) s += ScanItem(in, base + q, n, pop);
+			for (int q = 0; q < kScanItems; ++q) s += v[q];
 			uint32_t ex;
 			const uint32_t total = BlockExclusiveScan(s, ex);
 			if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = total;
@@ -312,23 +304,65 @@ namespace tg
 			if (threadIdx.x == 0) *total = carry;
 		}
 
+		// Writes this thread's items' exclusive sums from `run` on.
+		__device__ __forceinline__ void PutScan(uint32_t* __restrict__ out, int64_t base, int64_t n, bool pop, const uint32_t (&v)[kScanItems],
+			uint32_t s, uint32_t run)
+		{
+			if (pop && s == 0) return;
+			if (!pop && base + kScanItems <= n && (reinterpret_cast<uintptr_t>(out) & 15u) == 0)
+			{
+#pragma unroll
+				for (int q = 0; q < kScanItems; q += 4)
+				{
+					const uint4 x = make_uint4(run, run + v[q], run + v[q] + v[q + 1], run + v[q] + v[q + 1] + v[q + 2]);
+					reinterpret_cast<uint4*>(out + base)[q / 4] = x;
+					run = x.w + v[q + 3];
+				}
+				return;
+			}
+#pragma unroll
+			for (int q = 0; q < kScanItems; ++q)
+			{
+				if (base + q < n && (!pop || v[q])) out[base + q] = run;
+				run += v[q];
+			}
+		}
+
 		__global__ void __launch_bounds__(kScanThreads) ScanDownKernel(const uint32_t* __restrict__ in, int64_t n, bool pop,
 			const uint32_t* __restrict__ offsets, uint32_t* __restrict__ out)
 		{
 			const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-			uint32_t v[kScanItems];
-			uint32_t s = 0;
+			uint32_t v[kScanItems], s = 0;
+			ScanItems(in, base, n, pop, v);
 #pragma unroll
-			for (int q = 0; q < kScanItems; ++q) { v[q] = ScanItem(in, base + q, n, pop); s += v[q]; }
+			for (int q = 0; q < kScanItems; ++q) s += v[q];
 			uint32_t ex;
 			BlockExclusiveScan(s, ex);
-			uint32_t run = __ldg(offsets + blockIdx.x) + ex;
-#pragma unroll
-			for (int q = 0; q < kScanItems; ++q)
+			PutScan(out, base, n, pop, v, s, __ldg(offsets + blockIdx.x) + ex);
+		}
+
+		// All of a short scan by one block, a tile after the other: one launch in place of three.
+		__global__ void __launch_bounds__(kScanThreads) ScanShortKernel(const uint32_t* __restrict__ in, int64_t n, bool pop,
+			uint32_t* __restrict__ out, uint32_t* __restrict__ total)
+		{
+			__shared__ uint32_t carry;
+			if (threadIdx.x == 0) carry = 0;
+			const int64_t own = (int64_t)threadIdx.x * kScanItems;
+			for (int64_t tile = 0; tile < n; tile += kScanTile)
 			{
-				if (base + q < n) out[base + q] = run;
-				run += v[q];
+				uint32_t v[kScanItems], s = 0;
+				ScanItems(in, tile + own, n, pop, v);
+#pragma unroll
+				for (int q = 0; q < kScanItems; ++q) s += v[q];
+				__syncthreads();
+				const uint32_t c = carry;
+				uint32_t ex;
+				const uint32_t t = BlockExclusiveScan(s, ex);
+				PutScan(out, tile + own, n, pop, v, s, c + ex);
+				if (threadIdx.x == kScanThreads - 1) carry = c + t;
 			}
+			__syncthreads();
+			if (threadIdx.x == 0) *total = carry;
 		}
 
 		inline unsigned Blocks(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -346,6 +380,11 @@ namespace tg
 		if (nb == 0)
 		{
 			return cudaMemsetAsync(total, 0, sizeof(uint32_t), stream);
+		}
+		if (nb <= 2)
+		{
+			ScanShortKernel<<<1, kScanThreads, 0, stream>>>(in, n, popcount, out, total);
+			return cudaGetLastError();
 		}
 		ScanReduceKernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(in, n, popcount, scratch);
 		ScanTopKernel<<<1, kScanThreads, 0, stream>>>(scratch, nb, total);

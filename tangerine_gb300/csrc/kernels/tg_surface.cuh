@@ -53,6 +53,75 @@ namespace tg
 	}
 
 
+	// Cell c's coordinates, in 32 bits: cell numbers fit, and a 64-bit division is some hundred
+	// instructions.
+	struct CellIndex { int64_t i, j, k; };
+
+	__device__ __forceinline__ CellIndex CellAt(uint32_t c, const CellGeom& cg)
+	{
+		const uint32_t sx = (uint32_t)cg.sx, sy = (uint32_t)cg.sy, row = c / sx, k = row / sy;
+		return { (int64_t)(c - row * sx), (int64_t)(row - k * sy), (int64_t)k };
+	}
+
+	// SecondLoopThunk's triangles (surface_nets.cpp:1016-1115) of the vertex of active cell c,
+	// from triangle `out` on; vertex numbers less `first`.
+	__device__ __forceinline__ void EmitCellFaces(const float* __restrict__ lat, const CellGeom& cg, const uint32_t* __restrict__ words,
+		const uint32_t* __restrict__ base, uint32_t cell, uint32_t self, uint32_t first, uint32_t out, uint32_t* __restrict__ faces)
+	{
+		const CellIndex at = CellAt(cell, cg);
+		const int64_t i = at.i, j = at.j, k = at.k, c = cell;
+		if (i == 0 || j == 0 || k == 0) return;
+		const int64_t dy = cg.sx, dz = cg.sx * cg.sy;
+		const int64_t nb[6] = { c - 1, c - 1 - dy, c - dy, c - dy - dz, c - dz, c - 1 - dz };
+		// All the neighbours' words at once, then all the numbers.
+		uint32_t w[6];
+		bool on[6];
+		uint32_t id[6];
+#pragma unroll
+		for (int q = 0; q < 6; ++q) w[q] = __ldg(words + (nb[q] >> 5));
+#pragma unroll
+		for (int q = 0; q < 6; ++q)
+		{
+			on[q] = (w[q] >> (nb[q] & 31)) & 1u;
+			id[q] = on[q] ? __ldg(base + (nb[q] >> 5)) + __popc(w[q] & ((1u << (nb[q] & 31)) - 1u)) - first : 0u;
+		}
+		// Directed edges (0,4), (3,0), (0,1) decide the winding (surface_nets.cpp:1041-1105).
+		const float c0 = Corner(lat, cg, i, j, k);
+		const float s[3][2] = { { c0, Corner(lat, cg, i, j, k + 1) }, { Corner(lat, cg, i, j + 1, k), c0 }, { c0, Corner(lat, cg, i + 1, j, k) } };
+		constexpr int quads[3][3] = { {0, 1, 2}, {0, 5, 4}, {2, 3, 4} };
+#pragma unroll
+		for (int q = 0; q < 3; ++q)
+		{
+			if (!(on[quads[q][0]] && on[quads[q][1]] && on[quads[q][2]])) continue;
+			const bool rising = s[q][1] > s[q][0];
+			const uint32_t a = id[quads[q][0]], v2 = id[quads[q][1]], d = id[quads[q][2]];
+			const uint32_t v1 = rising ? a : d, v3 = rising ? d : a;
+			uint32_t* f = faces + (int64_t)out * 3;
+			f[0] = self; f[1] = v1; f[2] = v2;
+			f[3] = self; f[4] = v2; f[5] = v3;
+			out += 2;
+		}
+	}
+
+	// The sum of a cell's edge points whatever its values (infinities, NaN).
+	static __device__ __noinline__ void CellSumGeneral(const float (&v)[8], float fi, float fj, float fk, float& sx, float& sy, float& sz)
+	{
+		sx = sy = sz = 0.0f;
+#pragma unroll 1
+		for (int e = 0; e < 12; ++e)
+		{
+			const int a = kEdges[e][0], b = kEdges[e][1];
+			const float s1 = v[a], s2 = v[b];
+			if ((s1 >= 0.0f) == (s2 >= 0.0f)) continue;
+			const float p1x = fi + (float)kCornerOfs[a][0], p1y = fj + (float)kCornerOfs[a][1], p1z = fk + (float)kCornerOfs[a][2];
+			const float p2x = fi + (float)kCornerOfs[b][0], p2y = fj + (float)kCornerOfs[b][1], p2z = fk + (float)kCornerOfs[b][2];
+			const float t = (0.0f - s1) / (s2 - s1);
+			sx = sx + (p1x + t * (p2x - p1x));
+			sy = sy + (p1y + t * (p2y - p1y));
+			sz = sz + (p1z + t * (p2z - p1z));
+		}
+	}
+
 	// FirstLoopInnerThunk's vertex (surface_nets.cpp:915-965) for active cell c = (i, j, k)
 	// at its rank `vid`, and the number of triangles SecondLoopThunk will emit for it
 	// (surface_nets.cpp:1016-1115).
@@ -65,20 +134,33 @@ namespace tg
 		const float fi = (float)i, fj = (float)j, fk = (float)k;
 		float sx = 0.0f, sy = 0.0f, sz = 0.0f;
 		int count = 0;
+		// An edge's point is its first corner and, along its axis, t or -t more: the other axes'
+		// t * 0 changes nothing while t is a number from 0 to 1.  All edges are computed and the
+		// bipolar ones counted, without branches.  With the edges looked up and taken one by one
+		// the vertex pass took 1370 instructions a warp and was bound by issue (1.2 million vertices
+		// 53 us), now 600 and half waits for memory (36).
+		constexpr int kFrom[12] = { 0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3 }, kTo[12] = { 1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7 };
+		constexpr int kX[8] = { 0, 1, 1, 0, 0, 1, 1, 0 }, kY[8] = { 0, 0, 1, 1, 0, 0, 1, 1 }, kZ[8] = { 0, 0, 0, 0, 1, 1, 1, 1 };
+		const float x[2] = { fi, fi + 1.0f }, y[2] = { fj, fj + 1.0f }, z[2] = { fk, fk + 1.0f };
+		bool usual = true;
 #pragma unroll
 		for (int e = 0; e < 12; ++e)
 		{
-			const int a = kEdges[e][0], b = kEdges[e][1];
+			const int a = kFrom[e], b = kTo[e];
 			const float s1 = v[a], s2 = v[b];
-			if ((s1 >= 0.0f) == (s2 >= 0.0f)) continue;
-			const float p1x = fi + (float)kCornerOfs[a][0], p1y = fj + (float)kCornerOfs[a][1], p1z = fk + (float)kCornerOfs[a][2];
-			const float p2x = fi + (float)kCornerOfs[b][0], p2y = fj + (float)kCornerOfs[b][1], p2z = fk + (float)kCornerOfs[b][2];
-			const float t = (0.0f - s1) / (s2 - s1);
-			sx = sx + (p1x + t * (p2x - p1x));
-			sy = sy + (p1y + t * (p2y - p1y));
-			sz = sz + (p1z + t * (p2z - p1z));
-			++count;
+			const bool bipolar = (s1 >= 0.0f) != (s2 >= 0.0f);
+			const float t = (0.0f - s1) / (bipolar ? s2 - s1 : 1.0f);
+			usual = usual && (!bipolar || (t >= 0.0f && t <= 1.0f));
+			const int dx = kX[b] - kX[a], dy = kY[b] - kY[a], dz = kZ[b] - kZ[a];
+			const float px = dx > 0 ? x[0] + t : dx < 0 ? x[1] - t : x[kX[a]];
+			const float py = dy > 0 ? y[0] + t : dy < 0 ? y[1] - t : y[kY[a]];
+			const float pz = dz > 0 ? z[0] + t : dz < 0 ? z[1] - t : z[kZ[a]];
+			sx = bipolar ? sx + px : sx;
+			sy = bipolar ? sy + py : sy;
+			sz = bipolar ? sz + pz : sz;
+			count += bipolar ? 1 : 0;
 		}
+		if (!usual) CellSumGeneral(v, fi, fj, fk, sx, sy, sz);
 		const float n = (float)count;
 		const float cx = sx / n, cy = sy / n, cz = sz / n;
 		const float fsx = (float)cg.sx, fsy = (float)cg.sy, fsz = (float)cg.sz;
