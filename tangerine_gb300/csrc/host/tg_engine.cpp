@@ -266,14 +266,16 @@ namespace tg
 	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
 	// A tape saves about what its cell's program has beyond a dozen quads (two brushes), on
 	// every pass over the brick, and costs one pass of the whole program and two launches: it
-	// pays from a number of bricks that falls as the programs get longer.  Measured on a
-	// GB300, export to the device, tapes against whole programs, in us: 64 primitives (23
-	// quads a cell) 384^3 356 / 333, 512^3 414 / 417, 700^3 596 / 660; 16 primitives (16
-	// quads) 512^3 256 / 241, 700^3 346 / 356; 256 primitives (54 quads) 256^3 695 / 735,
-	// 512^3 861 / 1062, and 128^3 721 / 653.
+	// pays from a number of bricks that falls as the programs get longer, and later while whole
+	// programs go by eight warps a brick (kWideBricks).  Measured on a GB300, export to the
+	// device, whole programs / tapes, in us: 64 primitives (19 quads a cell) 448^3 330 / 348,
+	// 512^3 389 / 383, 700^3 599 / 531; 16 primitives (14 quads) 600^3 252 / 259, 700^3 321 /
+	// 304; 256 primitives (46 quads) 320^3 582 / 600, 384^3 693 / 644, 512^3 966 / 767; 256 others
+	// (33 quads) 384^3 451 / 514, 448^3 571 / 551.
 	static bool TapesPay(const Program& p, int64_t bricks)
 	{
-		return p.View.Lipschitz && (p.View.Form & kFormPrunable) && (double)bricks * (CellQuads(p) - 12.0) >= 3.5e6;
+		return p.View.Lipschitz && (p.View.Form & kFormPrunable) &&
+			(double)bricks * (CellQuads(p) - 12.0) >= (bricks <= kWideBricks ? 5e6 : 3.5e6);
 	}
 
 	// Whether a whole lattice goes by tapes, in bricks of 16^3 points (a quarter full at least).

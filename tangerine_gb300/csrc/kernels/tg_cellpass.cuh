@@ -45,22 +45,23 @@ namespace tg
 	// x fastest): every cell with corners of both signs sets its bit in `words` and is
 	// appended to `cells` (one atomic per brick).  Called by the whole CTA (it
 	// synchronises); `warpBase` is shared scratch, one word per warp.
-	template<int BT>
+	template<int BT, int Threads = kTiledThreads>
 	__device__ __forceinline__ void BrickCellFlags(const float* box, const BrickCells& bc, const CellGeom& cg, uint32_t* __restrict__ words,
 		uint32_t* __restrict__ cells, uint32_t* __restrict__ cell_count, uint32_t* warpBase)
 	{
+		constexpr int kRounds = (7 * 7 * 7 + Threads - 1) / Threads;
 		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 		const int ex = BT ? BT : bc.nx, ey = BT ? BT : bc.ny;
 		const int total = BT ? BT * BT * BT : bc.nx * bc.ny * bc.nz;
 		const int64_t sxy = cg.sx * cg.sy;
 		const int64_t c0 = bc.i0 + bc.j0 * cg.sx + bc.k0 * sxy;
-		unsigned ballots[kTiledRounds];
-		uint32_t cellOf[kTiledRounds];
+		unsigned ballots[kRounds];
+		uint32_t cellOf[kRounds];
 		uint32_t mine = 0;
 #pragma unroll
-		for (int r = 0; r < kTiledRounds; ++r)
+		for (int r = 0; r < kRounds; ++r)
 		{
-			const int t = r * kTiledThreads + (int)threadIdx.x;
+			const int t = r * Threads + (int)threadIdx.x;
 			bool active = false;
 			cellOf[r] = 0;
 			const int x = t % ex, y = (t / ex) % ey, z = t / (ex * ey);
@@ -85,18 +86,18 @@ namespace tg
 		if (threadIdx.x == 0)
 		{
 			uint32_t sum = 0;
-			uint32_t counts[kTiledThreads / 32];
+			uint32_t counts[Threads / 32];
 #pragma unroll
-			for (int w = 0; w < kTiledThreads / 32; ++w) { counts[w] = warpBase[w]; sum += counts[w]; }
+			for (int w = 0; w < Threads / 32; ++w) { counts[w] = warpBase[w]; sum += counts[w]; }
 			uint32_t at = sum ? atomicAdd(cell_count, sum) : 0u;
 #pragma unroll
-			for (int w = 0; w < kTiledThreads / 32; ++w) { warpBase[w] = at; at += counts[w]; }
+			for (int w = 0; w < Threads / 32; ++w) { warpBase[w] = at; at += counts[w]; }
 		}
 		__syncthreads();
 		uint32_t at = warpBase[warp];
 		const unsigned below = (1u << lane) - 1u;
 #pragma unroll
-		for (int r = 0; r < kTiledRounds; ++r)
+		for (int r = 0; r < kRounds; ++r)
 		{
 			if ((ballots[r] >> lane) & 1u) cells[at + __popc(ballots[r] & below)] = cellOf[r];
 			at += (uint32_t)__popc(ballots[r]);

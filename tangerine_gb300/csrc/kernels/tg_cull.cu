@@ -149,11 +149,11 @@ namespace tg
 		// __ldg, or with generic loads when Generic: a staged copy).  Box: the values also go
 		// to `box`, the brick's C^3 corner box in shared memory (x fastest), for the cell pass
 		// folded into EvalBricksCellsKernel.
-		template<int C, int K, bool Generic, bool Box>
+		template<int C, int K, bool Generic, bool Box, int Threads = kBrickThreads>
 		__device__ __forceinline__ void EvalSlice(const DeviceProgram& prog, const GridSpec& g, int i0, int i1, int j0, int j1, int k0,
 			int k1, int top, bool shared, int slice, int lane, const float4* code, float* __restrict__ lattice, float* spill, float* box)
 		{
-			constexpr int ZSpan = 2 * K;
+			constexpr int ZSpan = Threads / 64 * K;
 			const int tx = lane & 7, ty = (lane >> 3) + 4 * (slice & 1), tz = slice >> 1;
 			for (int oz = 0; oz < C; oz += ZSpan)
 			for (int oy = 0; oy < C; oy += 8)
@@ -190,17 +190,17 @@ namespace tg
 						if (Generic)
 						{
 							RunDistancePaired<K>([&](int q) { return code[q]; }, __ldg(&prog.Nodes[c].DistanceCode), px, py, pz, r,
-								spill + 2 * threadIdx.x, kBrickThreads);
+								spill + 2 * threadIdx.x, Threads);
 						}
 						else
 						{
 							RunDistancePaired<K>([&](int q) { return __ldg(code + q); }, __ldg(&prog.Nodes[c].DistanceCode), px,
-								py, pz, r, spill + 2 * threadIdx.x, kBrickThreads);
+								py, pz, r, spill + 2 * threadIdx.x, Threads);
 						}
 					}
 					else
 					{
-						RunDistance<K>(prog.Code, __ldg(&prog.Nodes[c].DistanceCode), px, py, pz, r, spill + threadIdx.x, kBrickThreads);
+						RunDistance<K>(prog.Code, __ldg(&prog.Nodes[c].DistanceCode), px, py, pz, r, spill + threadIdx.x, Threads);
 					}
 #pragma unroll
 					for (int k = 0; k < K; ++k)
@@ -412,17 +412,16 @@ namespace tg
 		// its four slices (EvalSlice) into the lattice and into the brick's 8^3 corner box in
 		// shared memory, and the CTA then flags and lists the brick's active cells from that
 		// box (BrickCellFlags) -- the separate cell pass read the boxes back from memory.
-		template<int K>
-		__global__ void __launch_bounds__(kBrickThreads, EvalBricksCtasPerSm<8>()) EvalBricksCellsKernel(DeviceProgram prog, GridSpec g,
+		template<int K, int Threads>
+		__global__ void __launch_bounds__(Threads, EvalBricksCtasPerSm<8>() * kBrickThreads / Threads) EvalBricksCellsKernel(DeviceProgram prog, GridSpec g,
 			BrickGrid bg, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count, const uint32_t* __restrict__ tops,
 			float* __restrict__ lattice, uint32_t* __restrict__ words, uint32_t* __restrict__ cells, uint32_t* __restrict__ cell_count,
 			uint32_t* __restrict__ next)
 		{
 			extern __shared__ __align__(16) float spill[];
 			__shared__ float box[kTiledBox * kTiledBox * kTiledBox];
-			__shared__ uint32_t warpBase[kBrickWarps];
+			__shared__ uint32_t warpBase[Threads / 32];
 			__shared__ uint32_t itemSlot;
-			static_assert(kBrickWarps == kTiledThreads / 32, "the cell pass takes the CTA's warps");
 			const CellGeom cg = Geom(g);
 			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
 			const uint32_t n = *count;
@@ -439,10 +438,10 @@ namespace tg
 				const int i0 = bx * bg.B, j0 = by * bg.B, k0 = bz * bg.B;
 				const int i1 = min(i0 + bg.B, g.NX - 1), j1 = min(j0 + bg.B, g.NY - 1), k1 = min(k0 + bg.B, g.NZ - 1);
 				const uint32_t packed = tops ? __ldg(tops + b) : BrickTop(prog, g, i0, i1, j0, j1, k0, k1);
-				EvalSlice<8, K, false, true>(prog, g, i0, i1, j0, j1, k0, k1, (int)(packed & 0x7FFFFFFFu), (packed >> 31) != 0u, warp, lane,
+				EvalSlice<8, K, false, true, Threads>(prog, g, i0, i1, j0, j1, k0, k1, (int)(packed & 0x7FFFFFFFu), (packed >> 31) != 0u, warp, lane,
 					prog.Code, lattice, spill, box);
 				__syncthreads();
-				BrickCellFlags<kTiledBox - 1>(box, CellsOf(b, bg, cg), cg, words, cells, cell_count, warpBase);
+				BrickCellFlags<kTiledBox - 1, Threads>(box, CellsOf(b, bg, cg), cg, words, cells, cell_count, warpBase);
 			}
 		}
 
@@ -586,19 +585,19 @@ namespace tg
 
 	namespace
 	{
-		template<int K>
+		template<int K, int Threads>
 		cudaError_t LaunchEvalBricksCellsK(const DeviceProgram& prog, const GridSpec& g, const uint32_t* list, const uint32_t* count,
 			const uint32_t* tops, float* lattice, uint32_t* words, uint32_t* cells, uint32_t* cell_count, int sms, cudaStream_t stream,
 			int* status)
 		{
 			const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
-			const size_t smem = (size_t)depth * K * kBrickThreads * sizeof(float);
+			const size_t smem = (size_t)depth * K * Threads * sizeof(float);
 			if (smem > 40 * 1024)
 			{
-				cudaError_t e = cudaFuncSetAttribute(EvalBricksCellsKernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+				cudaError_t e = cudaFuncSetAttribute(EvalBricksCellsKernel<K, Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 				if (e != cudaSuccess) return e;
 			}
-			EvalBricksCellsKernel<K><<<sms * EvalBricksCtasPerSm<8>(), kBrickThreads, smem, stream>>>(prog, g, MakeBrickGrid(g, kTiledBox - 1),
+			EvalBricksCellsKernel<K, Threads><<<sms * EvalBricksCtasPerSm<8>() * kBrickThreads / Threads, Threads, smem, stream>>>(prog, g, MakeBrickGrid(g, kTiledBox - 1),
 				list, count, tops, lattice, words, cells, cell_count, reinterpret_cast<uint32_t*>(status) + 1);
 			return cudaGetLastError();
 		}
@@ -614,9 +613,17 @@ namespace tg
 		if (e != cudaSuccess) return e;
 		switch (lanes)
 		{
-		case 1: return LaunchEvalBricksCellsK<1>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
-		case 2: return LaunchEvalBricksCellsK<2>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
-		default: return LaunchEvalBricksCellsK<4>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
+		case 1: return LaunchEvalBricksCellsK<1, 128>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
+		case 2:
+			// On small grids a launch is as long as its longest brick: eight warps take a brick's
+			// points in one pass of the program, four in two.  Whole exports to the device, four / eight
+			// warps, us: 256 primitives 192^3 540 / 466, 384^3 751 / 693; 64 primitives 192^3 215 / 202,
+			// 384^3 297 / 294, 448^3 330 / 340; 16 primitives 192^3 153 / 139, 384^3 184 / 172, 512^3
+			// 217 / 228, where the bricks fill the GPU several times over.
+			if (BrickCount(g, kTiledBox - 1) <= kWideBricks)
+				return LaunchEvalBricksCellsK<2, 256>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
+			return LaunchEvalBricksCellsK<2, 128>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
+		default: return LaunchEvalBricksCellsK<4, 128>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
 		}
 	}
 

@@ -109,6 +109,8 @@ namespace tg
 	// tops: the classifier's brick_tops for every listed brick, or nullptr (the kernel descends).
 	cudaError_t LaunchEvalBricks(const DeviceProgram& prog, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,
 		const uint32_t* tops, float* lattice, int sms, cudaStream_t stream, int lanes, bool staged, int* status);
+	// Grids of up to this many bricks are evaluated eight warps to a brick.
+	constexpr int64_t kWideBricks = 200000;
 	// LaunchEvalBricks and LaunchCellFlagsListed in one launch, for 7^3-cell bricks with the
 	// programs read from global memory: the same lattice, cell bits and active-cell list
 	// (list order differs).  status as LaunchEvalBricks's.
