@@ -308,38 +308,8 @@ namespace tg
 			}
 		}
 
-		// Cell pass over the lattice of listed bricks only: cells of skipped bricks are
-		// inactive without looking at their corners.
-		__global__ void CellFlagsBricksKernel(const float* __restrict__ lat, GridSpec g, BrickGrid bg,
-			const uint32_t* __restrict__ brick_bits, uint32_t* __restrict__ words, int64_t cells)
-		{
-			const int64_t sx = g.NX - 1, sy = g.NY - 1;
-			const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-			bool active = false;
-			if (c < cells)
-			{
-				const int64_t i = c % sx;
-				const int64_t j = (c / sx) % sy;
-				const int64_t k = c / (sx * sy);
-				const int64_t brick = (i / bg.B) + (int64_t)bg.NBX * ((j / bg.B) + (int64_t)bg.NBY * (k / bg.B));
-				if ((__ldg(brick_bits + (brick >> 5)) >> (brick & 31)) & 1u)
-				{
-					const int64_t nx = g.NX, ny = g.NY;
-					const int64_t base = (k * ny + j) * nx + i;
-					const int64_t dy = nx, dz = nx * ny;
-					const float v[8] = { __ldg(lat + base), __ldg(lat + base + 1), __ldg(lat + base + dy + 1), __ldg(lat + base + dy),
-						__ldg(lat + base + dz), __ldg(lat + base + dz + 1), __ldg(lat + base + dz + dy + 1), __ldg(lat + base + dz + dy) };
-					unsigned pos = 0;
-#pragma unroll
-					for (int q = 0; q < 8; ++q) pos |= (v[q] >= 0.0f ? 1u : 0u) << q;
-					active = pos != 0u && pos != 0xFFu;
-				}
-			}
-			const unsigned ballot = __ballot_sync(0xFFFFFFFFu, active);
-			if ((threadIdx.x & 31) == 0 && c < cells) words[c >> 5] = ballot;
-		}
-
-		// Also appends each active cell's index to `cells` (in no particular order: vertex
+		// Cell pass over the cells of listed bricks only: sets their bits and appends each active
+		// cell's index to `cells` (in no particular order: vertex
 		// numbers come from the bitmask rank, which is independent of this order).
 		__global__ void __launch_bounds__(128) CellFlagsListedKernel(const float* __restrict__ lat, GridSpec g, BrickGrid bg,
 			const uint32_t* __restrict__ list, const uint32_t* __restrict__ count, uint32_t* __restrict__ words,
@@ -409,8 +379,8 @@ namespace tg
 
 		// The brick evaluation with the cell pass folded in (7^3-cell bricks, programs read
 		// from global memory): a CTA draws a brick from a counter, each warp evaluates one of
-		// its four slices (EvalSlice) into the lattice and into the brick's 8^3 corner box in
-		// shared memory, and the CTA then flags and lists the brick's active cells from that
+		// its slices (EvalSlice; as many as warps) into the lattice and into the brick's 8^3 corner
+		// box in shared memory, and the CTA then flags and lists the brick's active cells from that
 		// box (BrickCellFlags) -- the separate cell pass read the boxes back from memory.
 		template<int K, int Threads>
 		__global__ void __launch_bounds__(Threads, EvalBricksCtasPerSm<8>() * kBrickThreads / Threads) EvalBricksCellsKernel(DeviceProgram prog, GridSpec g,
@@ -625,16 +595,6 @@ namespace tg
 			return LaunchEvalBricksCellsK<2, 128>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
 		default: return LaunchEvalBricksCellsK<4, 128>(prog, g, list, count, tops, lattice, words, cells, cell_count, sms, stream, status);
 		}
-	}
-
-	cudaError_t LaunchCellFlagsBricks(const float* lattice, const GridSpec& g, int B, const uint32_t* brick_bits, uint32_t* words,
-		cudaStream_t stream)
-	{
-		const BrickGrid bg = MakeBrickGrid(g, B);
-		const int64_t cells = (int64_t)(g.NX - 1) * (g.NY - 1) * (g.NZ - 1);
-		if (cells <= 0) return cudaSuccess;
-		CellFlagsBricksKernel<<<(unsigned)((cells + 255) / 256), 256, 0, stream>>>(lattice, g, bg, brick_bits, words, cells);
-		return cudaGetLastError();
 	}
 
 	cudaError_t LaunchCellFlagsListed(const float* lattice, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,

@@ -292,7 +292,7 @@ namespace tg
 	// to *material_out.  Operands below the top of the stack spill to shared memory:
 	// distance (depth, lane) at spill[(depth * (K + 1) + lane) * stride] and the material
 	// lane's material index at spill[(depth * (K + 1) + K) * stride].
-	template<int K, bool FuseSet = true>
+	template<int K>
 	__device__ __forceinline__ void RunSurfaceBatch(const float4* __restrict__ code, int pc,
 		const float (&px)[K], const float (&py)[K], const float (&pz)[K], float (&out)[K],
 		int mat_lane, int* material_out, float* spill, int stride)
@@ -344,7 +344,7 @@ namespace tg
 			{
 				// RecThenSet: the set operator after this brush takes the current accumulator
 				// (and material) as its left operand, so nothing is pushed.
-				const bool thenSet = FuseSet && (head & RecThenSet) != 0;
+				const bool thenSet = (head & RecThenSet) != 0;
 				float left[K];
 #pragma unroll
 				for (int k = 0; k < K; ++k) left[k] = acc[k];

@@ -160,8 +160,6 @@ namespace tg
 	cudaError_t LaunchBrickAttributes(const DeviceProgram& prog, const GridSpec& g, int B, const BrickTapes& tapes, const uint32_t* cells,
 		const uint32_t* words, const uint32_t* word_base, const float* vertices, uint32_t vertex_count, float* normals, uint8_t* colors,
 		cudaStream_t stream);
-	cudaError_t LaunchCellFlagsBricks(const float* lattice, const GridSpec& g, int B, const uint32_t* brick_bits, uint32_t* words,
-		cudaStream_t stream);
 	// Cell pass over the cells of listed bricks only: clears and fills the bitmask and
 	// lists the active cells (`cells` holds up to the lattice's cell count).
 	cudaError_t LaunchCellFlagsListed(const float* lattice, const GridSpec& g, int B, const uint32_t* list, const uint32_t* count,
