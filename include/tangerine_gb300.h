@@ -588,6 +588,11 @@ typedef struct tg_surrogate_info
 	int64_t mlp_floats;                       /* 10497: W1[64][32] b1 W2[64][64] b2 W3[64][64] b3 W4[64] b4 */
 } tg_surrogate_info;
 
+/* A block of page-locked host memory, for results that a call copies to the host at the link's
+ * rate (any thread; given back blocks are kept for the next ones, up to 2 GB). */
+TANGERINE_API tg_status tg_host_take(size_t bytes, void** block);
+TANGERINE_API void tg_host_give(void* block);
+
 TANGERINE_API void tg_surrogate_default_options(tg_surrogate_options* out);
 /* Allocates the network on the current device with seeded initial parameters. */
 TANGERINE_API tg_status tg_surrogate_create(const tg_surrogate_options* options, tg_surrogate** out);

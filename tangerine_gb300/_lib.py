@@ -137,6 +137,8 @@ SIGNATURES = {
     "tg_export_point_cloud": (_i, [_vp, _vp, _vp, _vp, _i, _u32, C.POINTER(HostMesh), _vp]),
     "tg_export_voxels": (_i, [_vp, _f, _i, C.POINTER(Voxels), _vp]),
     "tg_voxels_free": (None, [C.POINTER(Voxels)]),
+    "tg_host_take": (C.c_int, [C.c_size_t, C.POINTER(C.c_void_p)]),
+    "tg_host_give": (None, [C.c_void_p]),
     "tg_write_vox": (_i, [C.POINTER(Voxels), C.c_char_p]),
     "ExportMagicaVoxel": (None, [_vp, _f, _i, C.c_char_p]),
     "MeshExport": (_i, [_vp, C.c_char_p, _vp, _vp, _vp, _i, _i, C.c_bool, _f]),

@@ -1753,6 +1753,16 @@ extern "C"
 		return e == cudaSuccess ? TG_OK : CudaFail(e, "evaluating the surrogate");
 	}
 
+	TANGERINE_API tg_status tg_host_take(size_t bytes, void** out)
+	{
+		if (!out) { SetError("null argument"); return TG_ERR_INVALID; }
+		*out = HostPool::Get().Take(bytes);
+		if (!*out) { SetError("no pinned host memory"); return TG_ERR_MEMORY; }
+		return TG_OK;
+	}
+
+	TANGERINE_API void tg_host_give(void* block) { HostPool::Get().Give(block); }
+
 	TANGERINE_API tg_status tg_surrogate_gradients(tg_surrogate* s, const float* samples, int64_t n, float* table_grad, float* mlp_grad,
 		float* loss)
 	{
@@ -1760,11 +1770,10 @@ extern "C"
 		Engine& eng = Engine::Get();
 		std::lock_guard<std::mutex> lock(eng.Mutex);
 		const cudaStream_t st = eng.DefaultStream();
-		DeviceBuffer d;
+		DeviceBuffer& d = s->Given;
 		cudaError_t e = d.Reserve((size_t)n * 16);
 		if (e == cudaSuccess) e = cudaMemcpyAsync(d.Ptr, samples, (size_t)n * 16, cudaMemcpyHostToDevice, st);
 		if (e == cudaSuccess) e = s->Gradients(d.As<float4>(), n, table_grad, mlp_grad, loss, st);
-		d.Release();
 		if (e == cudaErrorLaunchTimeout) { SetError("a tensor-core wait timed out in the surrogate kernels"); return TG_ERR_CUDA; }
 		return e == cudaSuccess ? TG_OK : CudaFail(e, "surrogate gradients");
 	}

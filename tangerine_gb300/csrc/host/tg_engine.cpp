@@ -58,8 +58,12 @@ namespace tg
 		{
 			if (Used[i].first == p)
 			{
-				Free.push_back(Used[i]);
+				auto blk = Used[i];
 				Used.erase(Used.begin() + (long)i);
+				size_t kept = blk.second;
+				for (const auto& f : Free) kept += f.second;
+				if (kept > kMostFree) cudaFreeHost(blk.first);
+				else Free.push_back(blk);
 				return true;
 			}
 		}

@@ -248,6 +248,7 @@ namespace tg
 		void* Take(size_t bytes);            // nullptr when pinned memory is unavailable
 		bool Give(void* p);                  // false: p is not from this pool
 	private:
+		static constexpr size_t kMostFree = (size_t)2 << 30;    // bytes kept for reuse
 		std::mutex Mutex;
 		std::vector<std::pair<void*, size_t>> Free;
 		std::vector<std::pair<void*, size_t>> Used;

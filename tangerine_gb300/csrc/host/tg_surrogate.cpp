@@ -48,7 +48,7 @@ namespace tg
 	{
 		int prev = 0;
 		const bool switched = cudaGetDevice(&prev) == cudaSuccess && prev != DeviceId && cudaSetDevice(DeviceId) == cudaSuccess;
-		for (DeviceBuffer* b : { &Table, &TableGrad, &TableM, &TableV, &Mlp, &MlpGrad, &MlpM, &MlpV, &Image, &Status, &Loss }) b->Release();
+		for (DeviceBuffer* b : { &Table, &TableGrad, &TableM, &TableV, &Mlp, &MlpGrad, &MlpM, &MlpV, &Image, &Status, &Loss, &Given }) b->Release();
 		if (switched) cudaSetDevice(prev);
 	}
 

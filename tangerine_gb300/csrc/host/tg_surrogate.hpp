@@ -84,6 +84,7 @@ namespace tg
 		// |clamp(d)| <= r decide: m = Safety x max(max over them of |net| - r, P99Error).
 		float MarginFor(float radius) const;
 		int DeviceId = 0;
+		DeviceBuffer Given;                     // the caller's samples of a gradient call
 
 	private:
 		cudaError_t Step(const float4* samples, int64_t n, float rate, cudaStream_t s);

@@ -258,3 +258,19 @@ def test_point_queries_match_oracle(lib, port, golden, name):
         for n in (1, 15, 16, 17, 63, 65, 20005):
             np.testing.assert_array_equal(prog.eval_tree(points[:n]), values[:n])
             np.testing.assert_array_equal(prog.gradient_tree(points[:n]), gradients[:n])
+
+
+@pytest.mark.parametrize("log2_table", [14, 15])
+def test_gradient_arrays_are_the_callers_own(lib, log2_table):
+    """Gradients come in page-locked blocks that the library reuses: not while an array views them."""
+    with sdf.Surrogate(log2_table=log2_table) as net:
+        rng = np.random.default_rng(2)
+        a, b = (np.concatenate([rng.uniform(-1, 1, (n, 3)), rng.uniform(-0.5, 0.5, (n, 1))], 1).astype(np.float32) for n in (700, 300))
+        table, mlp, loss = net.gradients(a)
+        kept = table.copy(), mlp.copy()
+        other = net.gradients(b)
+        assert not np.shares_memory(other[0], table) and not np.shares_memory(other[1], mlp)
+        np.testing.assert_array_equal(table, kept[0])
+        np.testing.assert_array_equal(mlp, kept[1])
+        table[:] = 0.0          # writable, and nobody else's
+        assert np.any(other[0]) and not np.array_equal(other[1], kept[1])
