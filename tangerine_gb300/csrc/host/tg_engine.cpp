@@ -302,13 +302,9 @@ namespace tg
 	cudaError_t Engine::EvalGrid(const Program& p, const GridSpec& g, float* out, cudaStream_t s)
 	{
 		BrickTapes tapes{};
-		const bool byTapes = GridTapesPay(p, g);
-		if (byTapes)
-		{
-			const int64_t slab = DenseSlabBricks(g);
-			TG_TRY(ReadSmCount());
-			TG_TRY(ReserveTapes(slab, (size_t)slab * 16 + 4096, tapes));
-		}
+		const int64_t slab = DenseSlabBricks(g);
+		TG_TRY(ReadSmCount());
+		const bool byTapes = GridTapesPay(p, g) && TapesFit(Tapes, slab, (size_t)slab * 16 + 4096, tapes);
 		Begin("eval_grid", s);
 		const cudaError_t e = byTapes ? LaunchEvalGridTapes(p.View, g, tapes, out, SmCount, s) : LaunchEvalGrid(p.View, g, out, s);
 		End(s);
@@ -397,6 +393,15 @@ namespace tg
 		out.Counters = buffers.Counters.As<uint32_t>();
 		out.Long = out.Counters + kBrickTapeCounters;
 		return cudaSuccess;
+	}
+
+	bool Engine::TapesFit(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out)
+	{
+		if (ReserveTapes(buffers, bricks, parts, out) == cudaSuccess) return true;
+		cudaGetLastError();
+		for (DeviceBuffer* b : { &buffers.Bricks, &buffers.Parts, &buffers.Events, &buffers.Counters }) b->Release();
+		out = BrickTapes{};
+		return false;
 	}
 
 	cudaError_t Engine::Export(const Program& p, const GridSpec& g, const ExportOptions& opt, DeviceMesh& out, cudaStream_t s)
@@ -495,7 +500,8 @@ namespace tg
 			TG_TRY(ActiveCells.Reserve((size_t)(nb * (int64_t)B * B * B < cells ? nb * (int64_t)B * B * B : cells) * 4));
 			int* evalStatus = reinterpret_cast<int*>(Counts.As<uint32_t>() + 4);      // status and work counter
 			TG_TRY(cudaMemsetAsync(evalStatus, 0, 2 * sizeof(int), s));
-			if (B == 7 && !opt.Staged && !(opt.Tapes || TapesPay(p, nb)))
+			const bool byTapes = B == 7 && !opt.Staged && (opt.Tapes || TapesPay(p, nb)) && TapesFit(Tapes, nb, BrickPartCapacity(nb), tapes);
+			if (B == 7 && !opt.Staged && !byTapes)
 			{
 				// The cell pass runs inside the brick evaluation, on each brick's values in
 				// shared memory.
@@ -504,11 +510,10 @@ namespace tg
 					Words.As<uint32_t>(), ActiveCells.As<uint32_t>(), Counts.As<uint32_t>() + 3, SmCount, s, opt.Lanes, evalStatus));
 				End(s);
 			}
-			else if (B == 7 && !opt.Staged)
+			else if (byTapes)
 			{
 				// Each brick's shortened programs, then the evaluation by them with the cell pass
 				// folded in, on each brick's values in shared memory.
-				TG_TRY(ReserveTapes(nb, BrickPartCapacity(nb), tapes));
 				Begin("brick_tapes", s);
 				TG_TRY(LaunchBrickTapes(p.View, g, B, BrickList.As<uint32_t>(), brickCount, tops, tapes, SmCount, s));
 				End(s);
@@ -799,12 +804,13 @@ namespace tg
 		else
 		{
 			const OctNode& root = p.Host.Nodes[0];
-			const int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px);
+			int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px);
+			const int64_t all = (int64_t)bricks * bricks * bricks;
 			BrickTapes tapes{}, above{};
+			if (bricks && !TapesFit(Tapes, all, BrickPartCapacity(all), tapes)) bricks = 0;
 			if (bricks)
 			{
 				TG_TRY(ReadSmCount());
-				TG_TRY(ReserveTapes((int64_t)bricks * bricks * bricks, BrickPartCapacity((int64_t)bricks * bricks * bricks), tapes));
 				// By way of larger bricks' tapes where much of the space runs long programs: two more
 				// launches, the first as long as one pass of the longest program.  Without / with, us an
 				// image, by quads a point runs: 36 425 / 458, 58 2463 / 2502, 78 1181 / 1188, 124 800 /
@@ -812,7 +818,7 @@ namespace tg
 				if (p.Host.VolumeQuads >= 100.0)
 				{
 					const int64_t coarse = (int64_t)(bricks / 4) * (bricks / 4) * (bricks / 4);
-					TG_TRY(ReserveTapes(CoarseTapes, coarse, (size_t)coarse * 24, above));
+					TapesFit(CoarseTapes, coarse, (size_t)coarse * 24, above);
 				}
 			}
 			Begin("render", s);

@@ -209,8 +209,9 @@ namespace tg
 		cudaStream_t CopyStream = nullptr;          // early device-to-host copies of an export
 		// The buffers of a grid's brick tapes (LaunchBrickTapes), kept between exports.
 		struct TapeBuffers { DeviceBuffer Bricks, Parts, Events, Counters; };
-		cudaError_t ReserveTapes(int64_t bricks, size_t parts, BrickTapes& out) { return ReserveTapes(Tapes, bricks, parts, out); }
 		cudaError_t ReserveTapes(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out);
+		// The same where there is room for them; false (and none held) where whole programs must do.
+		bool TapesFit(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out);
 		cudaError_t ReadSmCount();
 		cudaEvent_t MeshReady = nullptr;
 		cudaEvent_t CodeReady = nullptr;            // RestageCode's copy of an export is done

@@ -100,13 +100,12 @@ namespace tg
 		TG_TRY(WordBase.Reserve((size_t)(words ? words : 1) * 4));
 		TG_TRY(Counts.Reserve(4 * sizeof(uint32_t)));
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4 + 4));
-		const bool byTapes = CloudByTapes(p.View, s, CellQuads(p));
 		BrickTapes tapes{};
+		const int64_t bricks = CloudBricks(s);
+		const bool byTapes = CloudByTapes(p.View, s, CellQuads(p)) && TapesFit(Tapes, bricks, BrickPartCapacity(bricks), tapes);
 		if (byTapes)
 		{
-			const int64_t bricks = CloudBricks(s);
 			TG_TRY(ReadSmCount());
-			TG_TRY(ReserveTapes(bricks, BrickPartCapacity(bricks), tapes));
 			TG_TRY(VoxScratch.Reserve((size_t)bricks * 8));
 			uint32_t* list = VoxScratch.As<uint32_t>();
 			TG_TRY(ActiveCells.Reserve((size_t)s.Total * 4));
