@@ -655,7 +655,8 @@ namespace tg
 	};
 
 	// A distance brush's distance at two points, from its record's quads, and the size its float
-	// error goes with.
+	// error goes with: that of its local coordinates and parameters, times the brush's scale,
+	// which multiplies their rounding too.
 	template<typename Load>
 	__device__ __forceinline__ float2 DistanceBrush(Load load, uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size)
 	{
@@ -664,8 +665,9 @@ namespace tg
 		float4 h;
 		BrushStep<1, false>(load, 0, head, x, y, z, u, qx, qy, qz, h, d);
 		const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
-		size = make_float2(fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(d[0].x),
-			fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(d[0].y));
+		const float scale = (head & RecScale) ? fmaxf(1.0f, fabsf(load(DistanceRecordQuads(head) - 1).x)) : 1.0f;
+		size = make_float2(scale * (fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes) + fabsf(d[0].x),
+			scale * (fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes) + fabsf(d[0].y));
 		return d[0];
 	}
 

@@ -274,3 +274,32 @@ def test_gradient_arrays_are_the_callers_own(lib, log2_table):
         np.testing.assert_array_equal(mlp, kept[1])
         table[:] = 0.0          # writable, and nobody else's
         assert np.any(other[0]) and not np.array_equal(other[1], kept[1])
+
+
+def _unit(*q):
+    q = np.asarray(q, np.float64)
+    return [float(v) for v in (q / np.linalg.norm(q)).astype(np.float32)]
+
+
+def _tilted():
+    """A slab whose top crosses z = 0.1 at a slight slant."""
+    return sdf.box(0.9, 0.9, 0.5).rotate(*_unit(0.0, 0.02, 0.0, 0.9998)).move(0.0, 0.0, -0.4)
+
+
+@pytest.mark.parametrize("scale", [1e4, 3e4, 1e5])
+def test_brick_tapes_of_large_scales(lib, scale):
+    """A brush's own rounding grows with its scale: the top of a unit sphere or box scaled to 1e4
+    and more lies in steps of some thousandths, across a slab's that it crosses slowly."""
+    grid = _lib.Grid(-0.43, -0.41, -0.1, 0.0021, 410, 391, 150)
+    for big in (lambda: sdf.sphere(1.0), lambda: sdf.box(1.0, 0.9, 1.0), lambda: sdf.cylinder(1.0, 1.0)):
+        cut = big().rotate(*_unit(0.3, 0.1, 0.2, 0.927)).scale(scale)
+        # The brush's extent along z by the tree's own distance: the cut's top goes to 0.1.
+        lo, hi = 0.0, 2.0 * scale
+        for _ in range(60):
+            mid = 0.5 * (lo + hi)
+            lo, hi = (mid, hi) if cut.eval(0.0, 0.0, mid) < 0.0 else (lo, mid)
+        tree = sdf.inter(sdf.box(0.4, 0.38, 0.5), sdf.union(cut.move(0.0, 0.0, 0.1 - lo), _tilted()))
+        with sdf.compile(tree) as prog:
+            whole = prog.export_mesh(grid, staged=True)
+            assert whole.vertices.shape[0] > 1000
+            _same(whole, prog.export_mesh(grid, tapes=True))
