@@ -944,7 +944,8 @@ namespace tg
 	// the difference of two operands can move inside a ball, with the fixed part of the
 	// rounding (TapeReach); the part that grows with the operands' own coordinates (brushes
 	// far from the box) is added here: each brush's float error is at most a few roundings of
-	// its local coordinates and sizes.  Returns false when a list outgrows its room.
+	// its local coordinates and sizes, that of a flate or a blend a few of what goes in and of
+	// its own width.  Returns false when a list outgrows its room.
 	template<bool Materials, typename Source>
 	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, const PairUnits& u, float2* spill,
 		int stride, const TapeLists& ts, TapeCounts& out)
@@ -1011,7 +1012,12 @@ namespace tg
 				const uint2 ev = src.Event(head);
 				ts.Value[nv++] = ev;
 				if (Materials) ts.Material[nm++] = ev;
-				if (op == OpFlate) acc = Sub2(acc, Pair(src.Operand()), u);
+				if (op == OpFlate)
+				{
+					const float k = src.Operand();
+					size = make_float2(fmaxf(size.x, fabsf(acc.x) + fabsf(k)), fmaxf(size.y, fabsf(acc.y) + fabsf(k)));
+					acc = Sub2(acc, Pair(k), u);
+				}
 				else acc = op == OpTapeNegate ? make_float2(-acc.x, -acc.y) : make_float2(acc.x + 0.0f, acc.y + 0.0f);
 				src.Advance(head);
 				continue;
@@ -1020,6 +1026,7 @@ namespace tg
 			const bool blend = op >= OpBlendUnion;
 			const bool diff = op == OpDiff || op == OpBlendDiff;
 			const bool unions = op == OpUnion || op == OpBlendUnion;
+			if (blend) size = make_float2(fmaxf(size.x, fabsf(k)), fmaxf(size.y, fabsf(k)));
 			// s > 0 where the left operand wins: by more than the reach everywhere, it always does.
 			const float2 s = unions ? make_float2(acc.x - left.x, acc.y - left.y)
 				: diff ? make_float2(left.x + acc.x, left.y + acc.y) : make_float2(left.x - acc.x, left.y - acc.y);

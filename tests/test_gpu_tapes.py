@@ -303,3 +303,19 @@ def test_brick_tapes_of_large_scales(lib, scale):
             whole = prog.export_mesh(grid, staged=True)
             assert whole.vertices.shape[0] > 1000
             _same(whole, prog.export_mesh(grid, tapes=True))
+
+
+def test_shortened_programs_of_large_steps_between(lib):
+    """Operators that go far from the surface and back (a flate by 2e6 and one by -2e6; a blend
+    8e6 wide, a quarter of that below its operands, lifted again) leave distances in steps of
+    1/8: a step may lie between the points that are looked at and the others."""
+    step, n = 1.0 / 256.0, 330
+    block = lambda w: sdf.box(w, 0.8, 0.3).rotate(*_unit(0.02, 0.05, 0.3, 1.0))
+    slab = lambda: sdf.box(0.7, 0.7, 0.2).rotate(*_unit(0.3, 0.1, 0.2, 1.0))
+    for far in (sdf.flate(sdf.flate(block(0.8), 2e6), -2e6), sdf.flate(sdf.blend_union(8e6, block(0.8), block(0.7)), -2e6)):
+        with sdf.compile(sdf.diff(sdf.union(far, slab()), sdf.sphere(0.2).move(0.1, 0.1, 0.1))) as prog:
+            whole = prog.eval_grid(_lib.Grid(-n // 2 * step, -n // 2 * step, -n // 2 * step, step, n, n, n))
+            for z in range(0, n, 55):
+                for y in range(0, n, 55):
+                    piece = prog.eval_grid(_lib.Grid(-n // 2 * step, (y - n // 2) * step, (z - n // 2) * step, step, n, 55, 55))
+                    np.testing.assert_array_equal(piece, whole[z:z + 55, y:y + 55])
