@@ -153,6 +153,7 @@ namespace tg
 			p.View.CodeQuads = p.Host.Header.CodeQuads;
 			p.View.FullBrushes = p.Host.Header.FullBrushes;
 			p.View.FullOps = p.Host.Header.FullOps;
+			p.View.Slack = p.Host.Header.Slack;
 		}
 	}
 

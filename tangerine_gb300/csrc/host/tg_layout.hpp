@@ -79,10 +79,15 @@ namespace tg
 		int32_t Form;               // kForm* below
 		int32_t FullBrushes;        // brushes and operators of the whole tree, stencils' masks left out
 		int32_t FullOps;
+		float Slack;                // kRoundingSlack, and more for rotations off the unit quaternion
 	};
 
+	// The float error of two operands at two points, by the size of what goes into them, with
+	// some thirty roundings' reserve.
+	constexpr float kRoundingSlack = 2e-5f;
+
 	// What the shortened programs (kernels/tg_tape.cuh) may assume of the whole tree.
-	constexpr int32_t kFormPrunable = 1;     // every rotation within 1e-3 of a unit quaternion, finite scales
+	constexpr int32_t kFormPrunable = 1;     // every rotation within 1e-3 of a unit quaternion (Slack covers that), finite scales
 	constexpr int32_t kFormPlain = 2;        // no stencils: a surface program's records follow the distance program's
 	constexpr int32_t kFormPainted = 4;      // plain, and every brush has a material
 }

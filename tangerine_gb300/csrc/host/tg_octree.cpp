@@ -859,6 +859,21 @@ namespace tg
 		return 0;
 	}
 
+	// How far the squared norm of any brush's rotation is from 1.
+	static double RotationError(const Node& n)
+	{
+		switch (n.Kind)
+		{
+		case NodeKind::Brush:
+		{
+			const Quat& q = n.Xf.Rotation;
+			return std::fabs((double)q.w * q.w + (double)q.x * q.x + (double)q.y * q.y + (double)q.z * q.z - 1.0);
+		}
+		case NodeKind::Set: return std::max(RotationError(*n.Lhs), RotationError(*n.Rhs));
+		default: return RotationError(*n.Lhs);
+		}
+	}
+
 	// Brushes and operators the tree's distance takes (a stencil's mask changes none).
 	static void CountNodes(const Node& n, int32_t& brushes, int32_t& ops)
 	{
@@ -1169,6 +1184,10 @@ namespace tg
 		out.Header.Lipschitz = HasNonLipschitzBrush(*root) ? 0 : 1;
 		out.Header.Form = FormOf(*root);
 		CountNodes(*root, out.Header.FullBrushes, out.Header.FullOps);
+		// With a rotation of squared norm 1 + e the inverse matrix of a distance record and the
+		// inverse quaternion of the surface record take a point v from the brush's origin up to
+		// 2 e |v| apart; a tape that serves both programs allows for that in both operands.
+		out.Header.Slack = kRoundingSlack + (float)(4.0 * RotationError(*root));
 		if (maxStack > kMaxStack)
 		{
 			error = "tree needs a deeper evaluation stack than the kernels hold";

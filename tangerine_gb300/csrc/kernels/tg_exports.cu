@@ -536,7 +536,7 @@ namespace tg
 			SurfaceSource src;
 			src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, window);
 			TapeCounts counts;
-			const bool ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), LoadPairUnits(), spill, 32,
+			const bool ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, LoadPairUnits(), spill, 32,
 				TapeLists{ value, nullptr, start, kVoxCoarseCap }, counts);
 			if (ok)
 				for (int i = lane; i < counts.Value; i += 32) st.Events[(int64_t)b * kVoxCoarseCap + i] = value[i];
@@ -590,13 +590,13 @@ namespace tg
 				{
 					SurfaceSource src;
 					src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, sc.Window);
-					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32, lists, counts);
+					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
 				}
 				else if (given != kNoTape)
 				{
 					SurfaceEventSource src;
 					src.Open(prog.Code + prog.FullSurfaceCode, st.Events + first, (int)given, sc.Window, sc.Heads);
-					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), units, spill, 32, lists, counts);
+					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
 				}
 				// The box goes by its own tape, where there is room for it.
 				uint2 tape = make_uint2(first, given);

@@ -371,15 +371,15 @@ namespace tg
 						const BrickPart& p = above.Parts[around];
 						DistanceEventSource src;
 						src.Open(code + base, above.Events + p.Material, (int)(p.Counts >> 16), ts.Window, ts.Heads);
-						ok = BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach, units, spill, 32,
-							lists, counts);
+						ok = BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach, prog.Slack, units,
+							spill, 32, lists, counts);
 					}
 					else
 					{
 						DistanceSource src;
 						src.In.Open(code + base, quads, ts.Window);
 						ok = quads <= 0xFFF0 && BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach,
-							units, spill, 32, lists, counts);
+							prog.Slack, units, spill, 32, lists, counts);
 					}
 				}
 				if (!ok) continue;

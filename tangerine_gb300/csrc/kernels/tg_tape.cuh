@@ -945,10 +945,11 @@ namespace tg
 	// rounding (TapeReach); the part that grows with the operands' own coordinates (brushes
 	// far from the box) is added here: each brush's float error is at most a few roundings of
 	// its local coordinates and sizes, that of a flate or a blend a few of what goes in and of
-	// its own width.  Returns false when a list outgrows its room.
+	// its own width (`slack` times the largest of them).  Returns false when a list outgrows its
+	// room.
 	template<bool Materials, typename Source>
-	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, const PairUnits& u, float2* spill,
-		int stride, const TapeLists& ts, TapeCounts& out)
+	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, float slack, const PairUnits& u,
+		float2* spill, int stride, const TapeLists& ts, TapeCounts& out)
 	{
 		const int lane = (int)(threadIdx.x & 31);
 		float2 acc = make_float2(0.0f, 0.0f), left = acc;
@@ -1030,7 +1031,7 @@ namespace tg
 			// s > 0 where the left operand wins: by more than the reach everywhere, it always does.
 			const float2 s = unions ? make_float2(acc.x - left.x, acc.y - left.y)
 				: diff ? make_float2(left.x + acc.x, left.y + acc.y) : make_float2(left.x - acc.x, left.y - acc.y);
-			const float2 t = make_float2(reach + 2e-5f * size.x + (blend ? k : 0.0f), reach + 2e-5f * size.y + (blend ? k : 0.0f));
+			const float2 t = make_float2(reach + slack * size.x + (blend ? k : 0.0f), reach + slack * size.y + (blend ? k : 0.0f));
 			const bool decides = !blend || k > 0.0f;
 			__syncwarp();       // every lane's list writes so far come before any slot is reused
 			const bool leftWins = __all_sync(0xFFFFFFFFu, decides && s.x > t.x && s.y > t.y);
@@ -1087,7 +1088,7 @@ namespace tg
 		out.Material = nm;
 		out.Same = same;
 		out.Distance = acc;
-		out.Error = make_float2(2e-5f * size.x, 2e-5f * size.y);
+		out.Error = make_float2(slack * size.x, slack * size.y);
 		return true;
 	}
 

@@ -319,3 +319,29 @@ def test_shortened_programs_of_large_steps_between(lib):
                 for y in range(0, n, 55):
                     piece = prog.eval_grid(_lib.Grid(-n // 2 * step, (y - n // 2) * step, (z - n // 2) * step, step, n, 55, 55))
                     np.testing.assert_array_equal(piece, whole[z:z + 55, y:y + 55])
+
+
+def _top_at(make, z):
+    """The brush moved along z until its top over the origin is at z, by the tree's own distance."""
+    shape, (lo, hi) = make(), (0.0, 1e3)
+    for _ in range(60):
+        mid = 0.5 * (lo + hi)
+        lo, hi = (mid, hi) if shape.eval(0.0, 0.0, mid) < 0.0 else (lo, mid)
+    return shape.move(0.0, 0.0, z - lo)
+
+
+@pytest.mark.parametrize("norm", [0.9992, 1.0009])
+@pytest.mark.parametrize("size", [4.0, 40.0])
+def test_brick_tapes_of_rotations_off_the_unit(lib, norm, size):
+    """Rotations typed with three digits: the distance program's inverse matrix and the surface
+    program's inverse quaternion then place a brush some thousandths of its extent apart, and
+    the normals are those of the surface program."""
+    grid = _lib.Grid(-0.43, -0.41, -0.1, 0.0021, 410, 391, 150)
+    for axis in ((0.3, 0.1, 0.2, 0.927), (0.1, -0.2, 0.4, 0.8), (0.05, 0.04, 0.6, 0.8)):
+        q = [norm * v for v in _unit(*axis)]
+        for lift in (-0.02, 0.0, 0.02):
+            big = _top_at(lambda: sdf.box(size, 0.9 * size, size).rotate(*q), 0.1 + lift)
+            with sdf.compile(sdf.inter(sdf.box(0.4, 0.38, 0.5), sdf.union(big, _tilted()))) as prog:
+                whole = prog.export_mesh(grid, staged=True)
+                assert whole.vertices.shape[0] > 1000
+                _same(whole, prog.export_mesh(grid, tapes=True))
