@@ -535,6 +535,10 @@ TANGERINE_API tg_status tg_batch_debug_barrier(tg_batch* batch, uint64_t limit_n
  * returns an error ("did not complete in time" / "timed out").  limit_ns = 0 restores the
  * normal waits. */
 TANGERINE_API tg_status tg_debug_wait_test(int which, uint64_t limit_ns);
+/* Test hook: the device memory that the library's buffers may hold together (0: no limit); a
+ * reservation beyond it fails as cudaMalloc does when the device is full.  release nonzero: the
+ * engine gives its buffers back first.  Returns the bytes held (compiled programs left out). */
+TANGERINE_API uint64_t tg_debug_device_limit(uint64_t bytes, int release);
 /* Output capacity for the next run (default: an estimate from the lattices); a run that
  * finds more vertices or faces grows the buffers and runs again (tg_batch_info.reruns). */
 TANGERINE_API tg_status tg_batch_reserve(tg_batch* batch, uint64_t vertices, uint64_t faces);

@@ -1521,6 +1521,15 @@ extern "C"
 		return TG_OK;
 	}
 
+	TANGERINE_API uint64_t tg_debug_device_limit(uint64_t bytes, int release)
+	{
+		Engine& eng = Engine::Get();
+		std::lock_guard<std::mutex> lock(eng.Mutex);
+		if (release) eng.ReleaseBuffers();
+		DeviceBuffer::Limit = bytes ? (size_t)bytes : (size_t)-1;
+		return DeviceBuffer::Held;
+	}
+
 	TANGERINE_API tg_status tg_debug_wait_test(int which, uint64_t limit_ns)
 	{
 		if ((which != 0 && which != 1) || limit_ns > 1000000000ull)

@@ -70,22 +70,81 @@ namespace tg
 		return false;
 	}
 
+	std::atomic<size_t> DeviceBuffer::Held{ 0 }, DeviceBuffer::Limit{ (size_t)-1 };
+
+	namespace
+	{
+		cudaError_t AllocateDevice(void** out, size_t bytes)
+		{
+			for (bool again = true; ; again = false)
+			{
+				const cudaError_t e = DeviceBuffer::Held + bytes > DeviceBuffer::Limit ? cudaErrorMemoryAllocation : cudaMalloc(out, bytes);
+				if (e == cudaSuccess) return e;
+				*out = nullptr;
+				if (e != cudaErrorMemoryAllocation || !again || !Engine::Get().ReleaseSpare()) return e;
+				cudaGetLastError();
+			}
+		}
+	}
+
 	cudaError_t DeviceBuffer::Reserve(size_t bytes)
 	{
 		if (bytes <= Bytes && Ptr) return cudaSuccess;
 		Release();
 		size_t want = bytes < 256 ? 256 : bytes;
-		cudaError_t e = cudaMalloc(&Ptr, want);
-		if (e != cudaSuccess) { Ptr = nullptr; Bytes = 0; return e; }
+		const cudaError_t e = AllocateDevice(&Ptr, want);
+		if (e != cudaSuccess) return e;
 		Bytes = want;
+		Held += want;
 		return cudaSuccess;
 	}
 
 	void DeviceBuffer::Release()
 	{
 		if (Ptr) cudaFree(Ptr);
+		Held -= Bytes;
 		Ptr = nullptr;
 		Bytes = 0;
+	}
+
+	void Engine::SpareUse::Hold()
+	{
+		if (Held) return;
+		std::lock_guard<std::mutex> lock(E.SpareMutex);
+		++E.SpareUses;
+		Held = true;
+	}
+
+	void Engine::SpareUse::Drop()
+	{
+		if (!Held) return;
+		std::lock_guard<std::mutex> lock(E.SpareMutex);
+		--E.SpareUses;
+		Held = false;
+	}
+
+	bool Engine::ReleaseSpare()
+	{
+		std::lock_guard<std::mutex> lock(SpareMutex);
+		bool any = false;
+		if (SpareUses) return false;
+		for (TapeBuffers* t : { &Tapes, &CoarseTapes })
+		{
+			for (DeviceBuffer* b : { &t->Bricks, &t->Parts, &t->Events, &t->Counters }) { any = any || b->Ptr; b->Release(); }
+		}
+		any = any || VoxScratch.Ptr;
+		VoxScratch.Release();
+		return any;
+	}
+
+	void Engine::ReleaseBuffers()
+	{
+		ReleaseSpare();
+		for (DeviceBuffer* b : { &LatticeBuf, &Words, &WordBase, &Scratch, &Counts, &Vertices, &Cubes, &FaceCounts, &FaceBase, &Faces, &Normals,
+			&Colors, &Points, &PointOut, &BrickBits, &BrickList, &BrickTops, &ClassCounts, &ProgramScratch, &ActiveCells, &RayIn, &RayOut,
+			&Cameras, &Image, &RenderCounters, &SodaBoxes, &SodaCache, &SodaColors, &RootScratch }) b->Release();
+		PreValid = false;
+		ActiveBricks = 0;
 	}
 
 	Program::~Program()
@@ -202,8 +261,8 @@ namespace tg
 		const ProgramLayout l = LayoutOf(p);
 		cudaError_t e = cudaGetDevice(&p.DeviceId);
 		if (e != cudaSuccess) return e;
-		e = cudaMalloc(&p.Device, l.Total);
-		if (e != cudaSuccess) { p.Device = nullptr; return e; }
+		e = AllocateDevice(&p.Device, l.Total);
+		if (e != cudaSuccess) return e;
 		std::vector<uint8_t> staging(l.Total, 0);
 		Pack(p, l, staging.data());
 		e = cudaMemcpy(p.Device, staging.data(), l.Total, cudaMemcpyHostToDevice);
@@ -305,11 +364,12 @@ namespace tg
 		BrickTapes tapes{};
 		const int64_t slab = DenseSlabBricks(g);
 		TG_TRY(ReadSmCount());
-		const bool byTapes = GridTapesPay(p, g) && TapesFit(Tapes, slab, (size_t)slab * 16 + 4096, tapes);
+		SpareUse spare(*this);
+		const bool byTapes = GridTapesPay(p, g) && TapesFit(Tapes, slab, (size_t)slab * 16 + 4096, tapes, spare);
 		Begin("eval_grid", s);
-		const cudaError_t e = byTapes ? LaunchEvalGridTapes(p.View, g, tapes, out, SmCount, s) : LaunchEvalGrid(p.View, g, out, s);
+		TG_TRY(byTapes ? LaunchEvalGridTapes(p.View, g, tapes, out, SmCount, s) : LaunchEvalGrid(p.View, g, out, s));
 		End(s);
-		return e;
+		return byTapes ? cudaStreamSynchronize(s) : cudaSuccess;
 	}
 
 	cudaError_t Engine::EvalPoints(const Program& p, const float* host_points, int64_t n, float* host_out, cudaStream_t s)
@@ -396,8 +456,9 @@ namespace tg
 		return cudaSuccess;
 	}
 
-	bool Engine::TapesFit(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out)
+	bool Engine::TapesFit(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out, SpareUse& use)
 	{
+		use.Hold();
 		if (ReserveTapes(buffers, bricks, parts, out) == cudaSuccess) return true;
 		cudaGetLastError();
 		for (DeviceBuffer* b : { &buffers.Bricks, &buffers.Parts, &buffers.Events, &buffers.Counters }) b->Release();
@@ -442,6 +503,20 @@ namespace tg
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4));
 
 		BrickTapes tapes{};
+		SpareUse spare(*this);
+		// What is reserved once the bricks have been evaluated: the tapes give way to it (the
+		// attributes then go by whole programs).
+		auto reserve = [&](DeviceBuffer& b, size_t bytes) -> cudaError_t
+		{
+			cudaError_t e = b.Reserve(bytes);
+			if (e != cudaErrorMemoryAllocation || !spare.Held) return e;
+			cudaGetLastError();
+			e = cudaStreamSynchronize(s);
+			if (e != cudaSuccess) return e;
+			tapes = BrickTapes{};
+			spare.Drop();
+			return b.Reserve(bytes);
+		};
 		if (opt.Dense)
 		{
 			Bricks = ActiveBricks = 0;
@@ -501,7 +576,7 @@ namespace tg
 			TG_TRY(ActiveCells.Reserve((size_t)(nb * (int64_t)B * B * B < cells ? nb * (int64_t)B * B * B : cells) * 4));
 			int* evalStatus = reinterpret_cast<int*>(Counts.As<uint32_t>() + 4);      // status and work counter
 			TG_TRY(cudaMemsetAsync(evalStatus, 0, 2 * sizeof(int), s));
-			const bool byTapes = B == 7 && !opt.Staged && (opt.Tapes || TapesPay(p, nb)) && TapesFit(Tapes, nb, BrickPartCapacity(nb), tapes);
+			const bool byTapes = B == 7 && !opt.Staged && (opt.Tapes || TapesPay(p, nb)) && TapesFit(Tapes, nb, BrickPartCapacity(nb), tapes, spare);
 			if (B == 7 && !opt.Staged && !byTapes)
 			{
 				// The cell pass runs inside the brick evaluation, on each brick's values in
@@ -562,11 +637,11 @@ namespace tg
 		}
 		if (stopped(0.6f)) return cudaSuccess;
 
-		TG_TRY(Vertices.Reserve((size_t)vcount * 12));
-		TG_TRY(Cubes.Reserve((size_t)vcount * 4));
-		TG_TRY(FaceCounts.Reserve((size_t)vcount * 4));
-		TG_TRY(FaceBase.Reserve((size_t)vcount * 4));
-		TG_TRY(Scratch.Reserve(ScanScratchWords(vcount) * 4));
+		TG_TRY(reserve(Vertices, (size_t)vcount * 12));
+		TG_TRY(reserve(Cubes, (size_t)vcount * 4));
+		TG_TRY(reserve(FaceCounts, (size_t)vcount * 4));
+		TG_TRY(reserve(FaceBase, (size_t)vcount * 4));
+		TG_TRY(reserve(Scratch, ScanScratchWords(vcount) * 4));
 		Begin("cell_vertices", s);
 		if (opt.Dense)
 		{
@@ -588,7 +663,7 @@ namespace tg
 		const uint32_t fcount = HostCounts[1];
 		if (stopped(0.8f)) return cudaSuccess;
 
-		TG_TRY(Faces.Reserve((size_t)fcount * 12));
+		TG_TRY(reserve(Faces, (size_t)fcount * 12));
 		Begin("faces", s);
 		TG_TRY(LaunchFaces(LatticeBuf.As<float>(), g, Words.As<uint32_t>(), WordBase.As<uint32_t>(), Cubes.As<uint32_t>(),
 			FaceBase.As<uint32_t>(), vcount, Faces.As<uint32_t>(), s));
@@ -643,11 +718,11 @@ namespace tg
 		}
 		if (opt.Attributes)
 		{
-			TG_TRY(Normals.Reserve((size_t)vcount * 12));
+			TG_TRY(reserve(Normals, (size_t)vcount * 12));
 			uint8_t* colors = nullptr;
 			if (p.Host.Header.HasPaint)
 			{
-				TG_TRY(Colors.Reserve((size_t)vcount * 3));
+				TG_TRY(reserve(Colors, (size_t)vcount * 3));
 				colors = Colors.As<uint8_t>();
 			}
 			// The culled export visits the vertices in its active-cell list's order (cells
@@ -776,6 +851,7 @@ namespace tg
 	{
 		const int64_t px = (int64_t)width * height * count;
 		if (px <= 0) return cudaSuccess;
+		SpareUse spare(*this);
 		TG_TRY(Cameras.Reserve(sizeof(CameraBasis) * (size_t)count));
 		TG_TRY(cudaMemcpyAsync(Cameras.Ptr, cams, sizeof(CameraBasis) * (size_t)count, cudaMemcpyHostToDevice, s));
 		float* dDepth = depth;
@@ -808,7 +884,7 @@ namespace tg
 			int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px);
 			const int64_t all = (int64_t)bricks * bricks * bricks;
 			BrickTapes tapes{}, above{};
-			if (bricks && !TapesFit(Tapes, all, BrickPartCapacity(all), tapes)) bricks = 0;
+			if (bricks && !TapesFit(Tapes, all, BrickPartCapacity(all), tapes, spare)) bricks = 0;
 			if (bricks)
 			{
 				TG_TRY(ReadSmCount());
@@ -819,7 +895,7 @@ namespace tg
 				if (p.Host.VolumeQuads >= 100.0)
 				{
 					const int64_t coarse = (int64_t)(bricks / 4) * (bricks / 4) * (bricks / 4);
-					TapesFit(CoarseTapes, coarse, (size_t)coarse * 24, above);
+					TapesFit(CoarseTapes, coarse, (size_t)coarse * 24, above, spare);
 				}
 			}
 			Begin("render", s);

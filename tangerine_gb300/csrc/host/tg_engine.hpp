@@ -19,13 +19,16 @@ namespace tg
 {
 	class FieldNet;
 
-	// A grow-only device allocation.
+	// A grow-only device allocation.  Where there is no room the engine's spare buffers
+	// (Engine::ReleaseSpare) make some.
 	struct DeviceBuffer
 	{
 		void* Ptr = nullptr;
 		size_t Bytes = 0;
 		cudaError_t Reserve(size_t bytes);
 		void Release();
+		// Test hook (tg_debug_device_limit): bytes that all buffers hold, and may hold.
+		static std::atomic<size_t> Held, Limit;
 		template<typename T> T* As() const { return static_cast<T*>(Ptr); }
 	};
 
@@ -187,6 +190,11 @@ namespace tg
 		// Network iterations and exact steps of the last network-stepped render.
 		uint64_t LastNetworkSteps = 0, LastExactSteps = 0;
 		DeviceBuffer& Lattice() { return LatticeBuf; }
+		// Frees what only makes calls faster (tapes, the voxel blocks' scratch), unless a call is
+		// using it.  True when there was any.
+		bool ReleaseSpare();
+		// Frees every buffer of the engine (test hook: a call then finds what a first one does).
+		void ReleaseBuffers();
 
 		// Profiling of kernel launches (CUDA events on the launching stream).
 		void SetProfiling(bool on);
@@ -207,11 +215,24 @@ namespace tg
 
 		cudaStream_t Stream = nullptr;
 		cudaStream_t CopyStream = nullptr;          // early device-to-host copies of an export
+		// A call's hold on the spare buffers: taken before it reserves them, given up when it ends or
+		// goes on without them (its launches that use them are over then).
+		struct SpareUse
+		{
+			explicit SpareUse(Engine& e) : E(e) {}
+			~SpareUse() { Drop(); }
+			void Hold();
+			void Drop();
+			Engine& E;
+			bool Held = false;
+		};
+		std::mutex SpareMutex;
+		int SpareUses = 0;
 		// The buffers of a grid's brick tapes (LaunchBrickTapes), kept between exports.
 		struct TapeBuffers { DeviceBuffer Bricks, Parts, Events, Counters; };
 		cudaError_t ReserveTapes(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out);
 		// The same where there is room for them; false (and none held) where whole programs must do.
-		bool TapesFit(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out);
+		bool TapesFit(TapeBuffers& buffers, int64_t bricks, size_t parts, BrickTapes& out, SpareUse& use);
 		cudaError_t ReadSmCount();
 		cudaEvent_t MeshReady = nullptr;
 		cudaEvent_t CodeReady = nullptr;            // RestageCode's copy of an export is done
@@ -220,7 +241,7 @@ namespace tg
 		TapeBuffers Tapes, CoarseTapes;
 		DeviceBuffer RayIn, RayOut, Cameras, Image, RenderCounters;
 		DeviceBuffer SodaBoxes, SodaCache, SodaColors;
-		DeviceBuffer VoxScratch, VoxelsOut;
+		DeviceBuffer VoxScratch;
 		void* Staging = nullptr;
 		size_t StagingBytes = 0;
 		// PreClassify's one-cell program: pinned staging, its device copy, the event after

@@ -102,13 +102,24 @@ namespace tg
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4 + 4));
 		BrickTapes tapes{};
 		const int64_t bricks = CloudBricks(s);
-		const bool byTapes = CloudByTapes(p.View, s, CellQuads(p)) && TapesFit(Tapes, bricks, BrickPartCapacity(bricks), tapes);
+		SpareUse spare(*this);
+		bool byTapes = CloudByTapes(p.View, s, CellQuads(p)) && TapesFit(Tapes, bricks, BrickPartCapacity(bricks), tapes, spare);
+		if (byTapes)
+		{
+			cudaError_t e = VoxScratch.Reserve((size_t)bricks * 8);
+			if (e == cudaSuccess) e = ActiveCells.Reserve((size_t)s.Total * 4);
+			if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return e;
+			if (e != cudaSuccess)
+			{
+				cudaGetLastError();
+				byTapes = false;
+				spare.Drop();
+			}
+		}
 		if (byTapes)
 		{
 			TG_TRY(ReadSmCount());
-			TG_TRY(VoxScratch.Reserve((size_t)bricks * 8));
 			uint32_t* list = VoxScratch.As<uint32_t>();
-			TG_TRY(ActiveCells.Reserve((size_t)s.Total * 4));
 			Begin("cloud_flags", st);
 			TG_TRY(LaunchCloudVoxels(p.View, s, list, list + bricks, tapes, Words.As<uint32_t>(),
 				ActiveCells.As<uint32_t>(), Counts.As<uint32_t>() + 1, SmCount, st));
@@ -148,23 +159,37 @@ namespace tg
 			}
 			if (control->Stage && control->Stage->load() > 2) refine = 0;
 		}
-		TG_TRY(Vertices.Reserve((size_t)n * 12 + 12));
+		const bool listed = !byTapes;       // the voxels' numbers are in Cubes already
+		// The tapes give way to the results: the points then go by whole programs.
+		auto reserve = [&](DeviceBuffer& b, size_t bytes) -> cudaError_t
+		{
+			const cudaError_t e = b.Reserve(bytes);
+			if (e != cudaErrorMemoryAllocation || !spare.Held) return e;
+			cudaGetLastError();
+			byTapes = false;
+			spare.Drop();
+			return b.Reserve(bytes);
+		};
+		TG_TRY(reserve(Vertices, (size_t)n * 12 + 12));
 		float* normals = nullptr;
 		uint8_t* colors = nullptr;
 		if (attributes)
 		{
-			TG_TRY(Normals.Reserve((size_t)n * 12 + 12));
+			TG_TRY(reserve(Normals, (size_t)n * 12 + 12));
 			normals = Normals.As<float>();
 			if (p.Host.Header.HasPaint)
 			{
-				TG_TRY(Colors.Reserve((size_t)n * 3 + 3));
+				TG_TRY(reserve(Colors, (size_t)n * 3 + 3));
 				colors = Colors.As<uint8_t>();
 			}
 		}
+		if (!listed) TG_TRY(reserve(Cubes, (size_t)n * 4 + 4));
+		if (!listed && !byTapes)
+			TG_TRY(LaunchListBricks(Words.As<uint32_t>(), s.Total, WordBase.As<uint32_t>(), Scratch.As<uint32_t>(), Cubes.As<uint32_t>(),
+				Counts.As<uint32_t>(), st));
 		Begin("cloud_refine", st);
 		if (byTapes)
 		{
-			TG_TRY(Cubes.Reserve((size_t)n * 4 + 4));
 			TG_TRY(LaunchCloudPoints(p.View, s, tapes, ActiveCells.As<uint32_t>(), n, Words.As<uint32_t>(), WordBase.As<uint32_t>(), refine,
 				Cubes.As<uint32_t>(), Vertices.As<float>(), normals, colors, st));
 		}
@@ -200,10 +225,30 @@ namespace tg
 		TG_TRY(WordBase.Reserve((size_t)(words ? words : 1) * 4));
 		TG_TRY(Counts.Reserve(4 * sizeof(uint32_t)));
 		TG_TRY(Scratch.Reserve(ScanScratchWords(words) * 4 + 4));
-		TG_TRY(VoxScratch.Reserve(VoxScratchBytes(p.View, s)));
 		TG_TRY(ReadSmCount());
+		SpareUse spare(*this);
+		const size_t blockBytes = VoxBlockBytes(p.View, s);
+		bool byBlocks = blockBytes != 0;
+		if (byBlocks)
+		{
+			spare.Hold();
+			const cudaError_t e = VoxScratch.Reserve(blockBytes);
+			if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return e;
+			if (e != cudaSuccess)
+			{
+				cudaGetLastError();
+				byBlocks = false;
+				spare.Drop();
+			}
+		}
+		if (!byBlocks)
+		{
+			PreValid = false;   // these bits replace a pending PreClassify's
+			TG_TRY(BrickBits.Reserve(VoxelBrickWords(s.SX, s.SY, s.SZ) * 4));
+		}
 		Begin("vox_flags", st);
-		TG_TRY(LaunchVoxFlags(p.View, s, VoxScratch.Ptr, Words.As<uint32_t>(), SmCount, st));
+		if (byBlocks) TG_TRY(LaunchVoxBlocks(p.View, s, VoxScratch.Ptr, Words.As<uint32_t>(), SmCount, st));
+		else TG_TRY(LaunchVoxFlags(p.View, s, BrickBits.As<uint32_t>(), Words.As<uint32_t>(), st));
 		End(st);
 		Begin("list_cells", st);
 		TG_TRY(LaunchExclusiveScan(Words.As<uint32_t>(), words, true, WordBase.As<uint32_t>(), Counts.As<uint32_t>(), Scratch.As<uint32_t>(), st));
@@ -211,6 +256,7 @@ namespace tg
 		TG_TRY(cudaMemcpyAsync(HostCounts, Counts.Ptr, 4, cudaMemcpyDeviceToHost, st));
 		TG_TRY(cudaStreamSynchronize(st));
 		const uint32_t n = HostCounts[0];
+		spare.Drop();
 		// The voxels are written out on the GPU, straight in the caller's layout, and come back
 		// in one copy to a page-locked block.
 		const size_t bytes = (size_t)(n ? n : 1) * sizeof(int4);
@@ -218,11 +264,11 @@ namespace tg
 		if (!block) block = std::malloc(bytes);
 		host_full = !block;
 		if (!block) return cudaErrorMemoryAllocation;
-		cudaError_t e = VoxelsOut.Reserve(bytes);
+		cudaError_t e = Cubes.Reserve(bytes);
 		if (e == cudaSuccess && n)
 		{
-			e = LaunchVoxList(s, Words.As<uint32_t>(), WordBase.As<uint32_t>(), color, VoxelsOut.As<int4>(), st);
-			if (e == cudaSuccess) e = cudaMemcpyAsync(block, VoxelsOut.Ptr, (size_t)n * sizeof(int4), cudaMemcpyDeviceToHost, st);
+			e = LaunchVoxList(s, Words.As<uint32_t>(), WordBase.As<uint32_t>(), color, Cubes.As<int4>(), st);
+			if (e == cudaSuccess) e = cudaMemcpyAsync(block, Cubes.Ptr, (size_t)n * sizeof(int4), cudaMemcpyDeviceToHost, st);
 		}
 		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
 		Collect();

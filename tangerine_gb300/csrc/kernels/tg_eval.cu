@@ -191,7 +191,7 @@ namespace tg
 		}
 	}
 
-	// Slabs bound the tapes' memory, whatever the lattice.
+	// Slabs bound the tapes' memory: kSlabBricks bricks, or one layer of them where that is more.
 	int64_t DenseSlabBricks(const GridSpec& g)
 	{
 		const int64_t plane = DensePlane(g), layers = (g.NZ + DenseLattice::kBox - 1) / DenseLattice::kBox;

@@ -917,38 +917,37 @@ namespace tg
 		return at;
 	}
 
-	size_t VoxScratchBytes(const DeviceProgram& prog, const VoxSpec& s)
+	size_t VoxBlockBytes(const DeviceProgram& prog, const VoxSpec& s)
 	{
-		if (s.Total <= 0) return 16;
-		if (!VoxByBlocks(prog, s)) return VoxelBrickWords(s.SX, s.SY, s.SZ) * sizeof(uint32_t);
+		if (s.Total <= 0 || !VoxByBlocks(prog, s)) return 0;
 		VoxState st;
 		return VoxLayout(s, nullptr, st);
 	}
 
-	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream)
+	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, uint32_t* brick_bits, uint32_t* words, cudaStream_t stream)
 	{
 		if (s.Total <= 0) return cudaSuccess;
-		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
-		if (!VoxByBlocks(prog, s))
+		const VoxelBricks vb = BricksOf(s.SX, s.SY, s.SZ);
+		const int nb = vb.NX * vb.NY * vb.NZ;
+		cudaError_t e = cudaMemsetAsync(brick_bits, 0, VoxelBrickWords(s.SX, s.SY, s.SZ) * 4, stream);
+		if (e != cudaSuccess) return e;
+		const size_t smem = DistanceSpillBytes(prog, 128);
+		if (smem > 48 * 1024)
 		{
-			uint32_t* brick_bits = static_cast<uint32_t*>(scratch);
-			const VoxelBricks vb = BricksOf(s.SX, s.SY, s.SZ);
-			const int nb = vb.NX * vb.NY * vb.NZ;
-			cudaError_t e = cudaMemsetAsync(brick_bits, 0, VoxelBrickWords(s.SX, s.SY, s.SZ) * 4, stream);
+			e = cudaFuncSetAttribute(VoxFlagsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			if (e == cudaSuccess) e = cudaFuncSetAttribute(VoxBricksKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 			if (e != cudaSuccess) return e;
-			const size_t smem = DistanceSpillBytes(prog, 128);
-			if (smem > 48 * 1024)
-			{
-				e = cudaFuncSetAttribute(VoxFlagsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-				if (e == cudaSuccess) e = cudaFuncSetAttribute(VoxBricksKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-				if (e != cudaSuccess) return e;
-			}
-			VoxBricksKernel<<<Blocks(nb, 128), 128, smem, stream>>>(prog, s, vb, brick_bits);
-			e = cudaGetLastError();
-			if (e != cudaSuccess) return e;
-			VoxFlagsKernel<<<Blocks(s.Total, 128), 128, smem, stream>>>(prog, s, vb, brick_bits, words);
-			return cudaGetLastError();
 		}
+		VoxBricksKernel<<<Blocks(nb, 128), 128, smem, stream>>>(prog, s, vb, brick_bits);
+		e = cudaGetLastError();
+		if (e != cudaSuccess) return e;
+		VoxFlagsKernel<<<Blocks(s.Total, 128), 128, smem, stream>>>(prog, s, vb, brick_bits, words);
+		return cudaGetLastError();
+	}
+
+	cudaError_t LaunchVoxBlocks(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream)
+	{
+		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
 		const VoxGrid vg = VoxGridOf(s);
 		VoxState st;
 		VoxLayout(s, scratch, st);

@@ -345,3 +345,64 @@ def test_brick_tapes_of_rotations_off_the_unit(lib, norm, size):
                 whole = prog.export_mesh(grid, staged=True)
                 assert whole.vertices.shape[0] > 1000
                 _same(whole, prog.export_mesh(grid, tapes=True))
+
+
+def _call(kind, prog):
+    """A call that goes by tapes or blocks where there is room, and what it returns."""
+    if kind == "mesh":
+        m = prog.export_mesh(W.export_grid(resolution=150), tapes=True)
+        return m.vertices, m.faces, m.cubes, m.normals, m.colors
+    if kind == "cloud":
+        m = prog.export_point_cloud((-1.6,) * 3, (1.6,) * 3, 0.013, 2)
+        return m.vertices, m.cubes, m.normals, m.colors
+    if kind == "voxels":
+        voxels, size, _ = prog.export_voxels(40.0, 3)
+        return voxels, np.asarray(size)
+    if kind == "render":
+        return prog.render(sdf.cameras(W.camera_poses(7, 2)), 210, 190)
+    return (prog.eval_grid(_lib.Grid(-1.6, -1.6, -1.6, 3.2 / 219, 220, 220, 220)),)
+
+
+CALLS = ("mesh", "cloud", "voxels", "render", "lattice")
+
+
+@pytest.mark.parametrize("kind", CALLS)
+def test_calls_go_without_tapes_where_memory_ends(lib, kind):
+    """Device memory that ends at any point of a call: from the least that the call needs on, all
+    of it or a part by whole programs, it returns the same."""
+    with sdf.compile(sdf.from_spec(W.random_tree(1, 256))) as prog:
+        try:
+            lib.tg_debug_device_limit(0, 1)
+            want = _call(kind, prog)
+            full = int(lib.tg_debug_device_limit(0, 0))
+            fits = []
+            for limit in np.linspace(full // 64, full, 90, dtype=np.int64):
+                lib.tg_debug_device_limit(int(limit), 1)
+                try:
+                    got = _call(kind, prog)
+                except _lib.TangerineError:
+                    fits.append(False)
+                    continue
+                fits.append(True)
+                for a, b in zip(got, want):
+                    np.testing.assert_array_equal(a, b)
+        finally:
+            lib.tg_debug_device_limit(0, 1)
+    least = fits.index(True)
+    assert 0 < least < 80       # the limit bites, and the call goes without something
+    assert all(fits[least:]), [i for i in range(least, len(fits)) if not fits[i]]
+
+
+def test_kept_tapes_give_way_to_other_calls(lib):
+    """What a call keeps to be faster the next time takes no other call's room."""
+    with sdf.compile(sdf.from_spec(W.random_tree(1, 256))) as prog:
+        try:
+            lib.tg_debug_device_limit(0, 1)
+            _call("mesh", prog)
+            lib.tg_debug_device_limit(int(lib.tg_debug_device_limit(0, 0)), 0)
+            depth, _, _ = prog.render(sdf.cameras(W.camera_poses(7, 1)), 640, 360, exact=True)
+            with sdf.compile(sdf.from_spec(W.random_tree(2, 16))) as other:
+                assert other.export_mesh(W.export_grid(resolution=32)).vertices.shape[0] > 0
+        finally:
+            lib.tg_debug_device_limit(0, 1)
+    assert np.isfinite(depth).any()
