@@ -593,7 +593,8 @@ typedef struct tg_surrogate_info
 } tg_surrogate_info;
 
 /* A block of page-locked host memory, for results that a call copies to the host at the link's
- * rate (any thread; given back blocks are kept for the next ones, up to 2 GB). */
+ * rate (any thread; given back blocks are kept for the next ones, up to 2 GB).  TG_ERR_MEMORY where
+ * there is none to be had or 2 GB of such blocks and voxels are in use: take ordinary memory. */
 TANGERINE_API tg_status tg_host_take(size_t bytes, void** block);
 TANGERINE_API void tg_host_give(void* block);
 

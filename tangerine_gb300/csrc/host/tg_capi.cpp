@@ -1765,8 +1765,8 @@ extern "C"
 	TANGERINE_API tg_status tg_host_take(size_t bytes, void** out)
 	{
 		if (!out) { SetError("null argument"); return TG_ERR_INVALID; }
-		*out = HostPool::Get().Take(bytes);
-		if (!*out) { SetError("no pinned host memory"); return TG_ERR_MEMORY; }
+		*out = HostPool::Get().TakeBounded(bytes);
+		if (!*out) { SetError("no pinned host memory, or 2 GB of it in use"); return TG_ERR_MEMORY; }
 		return TG_OK;
 	}
 

@@ -28,46 +28,50 @@ namespace tg
 		return *pool;
 	}
 
-	void* HostPool::Take(size_t bytes)
+	void* HostPool::TakeBlock(size_t bytes, size_t most, bool bounded)
 	{
 		std::lock_guard<std::mutex> lock(Mutex);
+		if (bounded && (bytes > kMostHeld || BoundedBytes > kMostHeld - bytes)) return nullptr;
 		size_t best = (size_t)-1;
 		for (size_t i = 0; i < Free.size(); ++i)
 		{
-			if (Free[i].second >= bytes && (best == (size_t)-1 || Free[i].second < Free[best].second)) best = i;
+			if (Free[i].Bytes >= bytes && Free[i].Bytes <= most && (best == (size_t)-1 || Free[i].Bytes < Free[best].Bytes)) best = i;
 		}
+		Block blk{ nullptr, bytes < 4096 ? 4096 : bytes + bytes / 8, bounded };
 		if (best != (size_t)-1)
 		{
-			auto blk = Free[best];
+			blk.Ptr = Free[best].Ptr;
+			blk.Bytes = Free[best].Bytes;
 			Free.erase(Free.begin() + (long)best);
-			Used.push_back(blk);
-			return blk.first;
 		}
-		void* p = nullptr;
-		const size_t want = bytes < 4096 ? 4096 : bytes + bytes / 8;
-		if (cudaMallocHost(&p, want) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-		Used.push_back({ p, want });
-		return p;
+		else if (cudaMallocHost(&blk.Ptr, blk.Bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+		if (bounded) BoundedBytes += blk.Bytes;
+		Used.push_back(blk);
+		return blk.Ptr;
 	}
+
+	void* HostPool::Take(size_t bytes) { return TakeBlock(bytes, (size_t)-1, false); }
+
+	void* HostPool::TakeBounded(size_t bytes) { return TakeBlock(bytes, bytes < 4096 ? 8192 : 2 * bytes, true); }
 
 	bool HostPool::Give(void* p)
 	{
 		if (!p) return true;
-		std::lock_guard<std::mutex> lock(Mutex);
-		for (size_t i = 0; i < Used.size(); ++i)
 		{
-			if (Used[i].first == p)
-			{
-				auto blk = Used[i];
-				Used.erase(Used.begin() + (long)i);
-				size_t kept = blk.second;
-				for (const auto& f : Free) kept += f.second;
-				if (kept > kMostFree) cudaFreeHost(blk.first);
-				else Free.push_back(blk);
-				return true;
-			}
+			std::lock_guard<std::mutex> lock(Mutex);
+			size_t i = 0;
+			while (i < Used.size() && Used[i].Ptr != p) ++i;
+			if (i == Used.size()) return false;
+			const Block blk = Used[i];
+			Used.erase(Used.begin() + (long)i);
+			if (blk.Bounded) BoundedBytes -= blk.Bytes;
+			size_t kept = blk.Bytes;
+			for (const Block& f : Free) kept += f.Bytes;
+			if (kept <= kMostFree) { Free.push_back(blk); return true; }
 		}
-		return false;
+		// Beyond the bound: freeing waits for the device, which other threads' takes need not.
+		cudaFreeHost(p);
+		return true;
 	}
 
 	std::atomic<size_t> DeviceBuffer::Held{ 0 }, DeviceBuffer::Limit{ (size_t)-1 };

@@ -268,12 +268,20 @@ namespace tg
 	public:
 		static HostPool& Get();
 		void* Take(size_t bytes);            // nullptr when pinned memory is unavailable
+		// The same for results that callers may keep for long and that can as well be in ordinary
+		// memory: nullptr too once kMostHeld bytes are out, and no block of more than twice the size
+		// (a small result would keep it from the next large one).
+		void* TakeBounded(size_t bytes);
 		bool Give(void* p);                  // false: p is not from this pool
 	private:
 		static constexpr size_t kMostFree = (size_t)2 << 30;    // bytes kept for reuse
+		static constexpr size_t kMostHeld = (size_t)2 << 30;    // bytes of TakeBounded's blocks in use
+		struct Block { void* Ptr; size_t Bytes; bool Bounded; };
+		void* TakeBlock(size_t bytes, size_t most, bool bounded);
 		std::mutex Mutex;
-		std::vector<std::pair<void*, size_t>> Free;
-		std::vector<std::pair<void*, size_t>> Used;
+		std::vector<Block> Free;
+		std::vector<Block> Used;
+		size_t BoundedBytes = 0;
 	};
 
 	struct ExportTiming

@@ -260,7 +260,7 @@ namespace tg
 		// The voxels are written out on the GPU, straight in the caller's layout, and come back
 		// in one copy to a page-locked block.
 		const size_t bytes = (size_t)(n ? n : 1) * sizeof(int4);
-		void* block = HostPool::Get().Take(bytes);
+		void* block = HostPool::Get().TakeBounded(bytes);
 		if (!block) block = std::malloc(bytes);
 		host_full = !block;
 		if (!block) return cudaErrorMemoryAllocation;

@@ -344,7 +344,8 @@ class Program:
         return _take_mesh(hm)
 
     def export_voxels(self, grid_size, color_index=0, stream=None):
-        """VoxExport's voxels on the GPU: ((n, 4) int32 x y z colour, size, radius)."""
+        """VoxExport's voxels on the GPU: ((n, 4) int32 x y z colour, size, radius).  The array is in
+        page-locked memory (up to 2 GB of such results): copy it to keep it for long."""
         v = _lib.Voxels()
         check(load().tg_export_voxels(self.ptr, float(grid_size), int(color_index), C.byref(v), stream), "tg_export_voxels")
         n = int(v.count)
@@ -643,7 +644,8 @@ class Surrogate:
         return out
 
     def gradients(self, samples):
-        """(table_grad, mlp_grad, summed squared error) of the mean squared error."""
+        """(table_grad, mlp_grad, summed squared error) of the mean squared error.  The arrays are in
+        page-locked memory (up to 2 GB of such results): copy them to keep them for long."""
         s = np.ascontiguousarray(np.asarray(samples, np.float32).reshape(-1, 4))
         tg_, mg = _host_floats(self.table_floats), _host_floats(self.mlp_floats)
         loss = C.c_float()

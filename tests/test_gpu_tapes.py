@@ -406,3 +406,27 @@ def test_kept_tapes_give_way_to_other_calls(lib):
         finally:
             lib.tg_debug_device_limit(0, 1)
     assert np.isfinite(depth).any()
+
+
+def test_page_locked_results_are_bounded(lib):
+    """Blocks for results that callers may keep: at most 2 GB in use, none far larger than asked
+    for, and room again once they are given back."""
+    C = _lib.C
+
+    def take(size):
+        ptr = C.c_void_p()
+        return ptr.value if lib.tg_host_take(size, C.byref(ptr)) == 0 else None
+
+    taken = []
+    try:
+        while len(taken) < 12 and (block := take(200 << 20)):
+            taken.append(block)
+        assert 8 <= len(taken) <= 10            # an eighth more is pinned than asked for
+        lib.tg_host_give(taken[0])
+        small = take(1 << 20)
+        assert small and small != taken[0]
+        assert take(200 << 20) == taken[0]
+        lib.tg_host_give(small)
+    finally:
+        for block in taken:
+            lib.tg_host_give(block)
