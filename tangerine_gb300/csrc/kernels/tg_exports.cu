@@ -437,6 +437,7 @@ namespace tg
 		constexpr int kVoxCoarseCap = 2048, kVoxBlockCap = 192;
 		constexpr int kVoxWarps = 4, kVoxCtasPerSm = 6, kVoxEvalCtasPerSm = 8;
 		constexpr int kVoxDirectBlocks = 1000;
+		constexpr int kVoxWholeBoxes = 4096;
 
 		// A warp's scratch while it builds a 16^3 block's tape.
 		struct VoxScratch
@@ -536,7 +537,7 @@ namespace tg
 			SurfaceSource src;
 			src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, window);
 			TapeCounts counts;
-			const bool ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, LoadPairUnits(), spill, 32,
+			const bool ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, LoadPairUnits(), spill, 32,
 				TapeLists{ value, nullptr, start, kVoxCoarseCap }, counts);
 			if (ok)
 				for (int i = lane; i < counts.Value; i += 32) st.Events[(int64_t)b * kVoxCoarseCap + i] = value[i];
@@ -546,7 +547,7 @@ namespace tg
 			{
 				const float d = j ? counts.Distance.y : counts.Distance.x, r = j ? l.R.y : l.R.x;
 				const float margin = (j ? l.Margin.y : l.Margin.x) + (j ? counts.Error.y : counts.Error.x);
-				const bool keep = l.In[j] && !(ok && fabsf(d) > r + s.Radius + margin);
+				const bool keep = l.In[j] && !(fabsf(d) > r + s.Radius + margin);
 				const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
 				uint32_t at = 0;
 				if (lane == 0 && kept) at = atomicAdd(st.Counters, (uint32_t)__popc(kept));
@@ -555,9 +556,13 @@ namespace tg
 			}
 		}
 
+		// A list that finds no room still leaves the distances, which drop the boxes out of reach: 2000
+		// primitives at 92^3 voxels 4933 us a call with every box of such a block kept, 3377 so; at 230^3
+		// 11033 and 5306.
+		//
 		// One warp per listed 16^3 block, drawn from a counter: its tape from its 64^3 block's,
 		// and the 4^3 boxes in it that may hold a kept voxel.  Direct: every 16^3 block, from the
-		// whole tree's program.
+		// whole tree's program (as where the 64^3 block's tape had no room).
 		template<bool Direct>
 		__global__ void __launch_bounds__(kVoxWarps * 32, kVoxCtasPerSm) VoxBlockKernel(DeviceProgram prog, VoxSpec s, VoxGrid vg, VoxState st,
 			int spill_pairs)
@@ -583,20 +588,20 @@ namespace tg
 				const uint32_t first = Direct ? 0u : (entry >> 6) * (uint32_t)kVoxCoarseCap;
 				const VoxLane l = VoxLaneOf(s, from, kVoxFine, rootClip);
 				const TapeLists lists{ sc.Value, nullptr, sc.Start, kVoxBlockCap };
-				bool ok = false;
+				bool ok;
 				TapeCounts counts;
 				__syncwarp();       // the previous block's events have been copied out
-				if (Direct)
+				if (Direct || given == kNoTape)
 				{
 					SurfaceSource src;
 					src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, sc.Window);
-					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
+					ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
 				}
-				else if (given != kNoTape)
+				else
 				{
 					SurfaceEventSource src;
 					src.Open(prog.Code + prog.FullSurfaceCode, st.Events + first, (int)given, sc.Window, sc.Heads);
-					ok = BuildTape<false>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
+					ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
 				}
 				// The box goes by its own tape, where there is room for it.
 				uint2 tape = make_uint2(first, given);
@@ -617,12 +622,34 @@ namespace tg
 				{
 					const float d = j ? counts.Distance.y : counts.Distance.x, r = j ? l.R.y : l.R.x;
 					const float margin = (j ? l.Margin.y : l.Margin.x) + (j ? counts.Error.y : counts.Error.x);
-					const bool keep = l.In[j] && !(ok && fabsf(d) > r + s.Radius + margin);
+					const bool keep = l.In[j] && !(fabsf(d) > r + s.Radius + margin);
 					const unsigned kept = __ballot_sync(0xFFFFFFFFu, keep);
 					uint32_t at = 0;
 					if (lane == 0 && kept) at = atomicAdd(st.Counters + 3, (uint32_t)__popc(kept));
 					at = __shfl_sync(0xFFFFFFFFu, at, 0);
 					if (keep) st.Boxes[at + (uint32_t)__popc(kept & ((1u << lane) - 1u))] = item * 64u + (uint32_t)(lane + 32 * j);
+				}
+			}
+		}
+
+		// The kept ones of a 4^3 box's voxels, by a warp: lane l has (x, y, z) and the voxel two above
+		// it, with their distances.
+		__device__ __forceinline__ void PutVoxBits(const VoxSpec& s, int x, int y, int z, float2 d, uint32_t* __restrict__ words)
+		{
+			const int lane = (int)(threadIdx.x & 31);
+#pragma unroll
+			for (int j = 0; j < 2; ++j)
+			{
+				const bool keep = x < s.SX && y < s.SY && z + 2 * j < s.SZ && fabsf(j ? d.y : d.x) <= s.Radius;
+				const unsigned bits = __ballot_sync(0xFFFFFFFFu, keep);
+				// A row of four voxels of the box is four neighbouring lanes.
+				const uint32_t row = (bits >> (lane & 28)) & 15u;
+				if ((lane & 3) == 0 && row)
+				{
+					const int64_t t = x + (int64_t)s.SX * (y + (int64_t)s.SY * (z + 2 * j));
+					const int shift = (int)(t & 31);
+					atomicOr(words + (t >> 5), row << shift);
+					if (shift > 28 && (row >> (32 - shift))) atomicOr(words + (t >> 5) + 1, row >> (32 - shift));
 				}
 			}
 		}
@@ -649,8 +676,7 @@ namespace tg
 				int from[3];
 				VoxBlockStart(vg, block, from);
 				const int part = (int)(entry & 63u);
-				const int vx = lane & 3;
-				const int x = from[0] + (part & 3) * kVoxFine + vx, y = from[1] + ((part >> 2) & 3) * kVoxFine + ((lane >> 2) & 3);
+				const int x = from[0] + (part & 3) * kVoxFine + (lane & 3), y = from[1] + ((part >> 2) & 3) * kVoxFine + ((lane >> 2) & 3);
 				const int z = from[2] + (part >> 4) * kVoxFine + (lane >> 4);
 				const float cx = VoxCentre(s.Min[0], s.Max[0], x, s.SX), cy = VoxCentre(s.Min[1], s.Max[1], y, s.SY);
 				const float2 px[1] = { make_float2(cx, cx) }, py[1] = { make_float2(cy, cy) };
@@ -661,22 +687,28 @@ namespace tg
 				else
 					RunSurfaceTapePairs<1>(load, 0, [&](uint32_t e) { return __ldg(events + e); }, tape.y, px, py, pz, units, d, spill2 + threadIdx.x,
 						kVoxWarps * 32);
-#pragma unroll
-				for (int j = 0; j < 2; ++j)
-				{
-					const bool keep = x < s.SX && y < s.SY && z + 2 * j < s.SZ && fabsf(j ? d[0].y : d[0].x) <= s.Radius;
-					const unsigned bits = __ballot_sync(0xFFFFFFFFu, keep);
-					// A row of four voxels of the box is four neighbouring lanes.
-					const uint32_t row = (bits >> (lane & 28)) & 15u;
-					if (vx == 0 && row)
-					{
-						const int64_t t = x + (int64_t)s.SX * (y + (int64_t)s.SY * (z + 2 * j));
-						const int shift = (int)(t & 31);
-						atomicOr(words + (t >> 5), row << shift);
-						if (shift > 28 && (row >> (32 - shift))) atomicOr(words + (t >> 5) + 1, row >> (32 - shift));
-					}
-				}
+				PutVoxBits(s, x, y, z, d[0], words);
 			}
+		}
+
+		// Small lattices: every 4^3 box by the whole tree's program, one warp each.  A pass over the
+		// blocks first is as long as that by itself, and leaves few of so few boxes out.
+		__global__ void __launch_bounds__(kVoxWarps * 32) VoxWholeKernel(DeviceProgram prog, VoxSpec s, int nx, int ny, int nz, int spill_pairs,
+			uint32_t* __restrict__ words)
+		{
+			extern __shared__ __align__(16) float4 shared4[];
+			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+			const int box = (int)blockIdx.x * kVoxWarps + warp;
+			if (box >= nx * ny * nz) return;
+			const int x = box % nx * kVoxFine + (lane & 3), y = box / nx % ny * kVoxFine + ((lane >> 2) & 3);
+			const int z = box / (nx * ny) * kVoxFine + (lane >> 4);
+			const float cx = VoxCentre(s.Min[0], s.Max[0], x, s.SX), cy = VoxCentre(s.Min[1], s.Max[1], y, s.SY);
+			SurfaceSource src;
+			src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, shared4 + warp * 64);
+			const float2 d = RunSourcePair(src, make_float2(cx, cx), make_float2(cy, cy),
+				make_float2(VoxCentre(s.Min[2], s.Max[2], z, s.SZ), VoxCentre(s.Min[2], s.Max[2], z + 2, s.SZ)), LoadPairUnits(),
+				reinterpret_cast<float2*>(shared4 + kVoxWarps * 64) + warp * spill_pairs * 32 + lane, 32);
+			PutVoxBits(s, x, y, z, d, words);
 		}
 
 		// Trees whose programs cannot be shortened (a brush that is not 1-Lipschitz, rotations that
@@ -917,9 +949,20 @@ namespace tg
 		return at;
 	}
 
+	static int VoxBoxes(int voxels) { return (voxels + kVoxFine - 1) / kVoxFine; }
+
+	// Lattices whose 4^3 boxes the GPU runs at once go without blocks.  Measured on a GB300, with
+	// blocks / without, us a call: 60 primitives 6^3 voxels 144 / 84, 48^3 122 / 94, 80^3 115 / 170;
+	// 400 primitives 15^3 653 / 285, 60^3 683 / 416; 2000 primitives 13^3 2979 / 1192, 55^3 3186 / 1613.
+	static bool VoxWhole(const VoxSpec& s)
+	{
+		return (int64_t)VoxBoxes(s.SX) * VoxBoxes(s.SY) * VoxBoxes(s.SZ) <= kVoxWholeBoxes;
+	}
+
 	size_t VoxBlockBytes(const DeviceProgram& prog, const VoxSpec& s)
 	{
 		if (s.Total <= 0 || !VoxByBlocks(prog, s)) return 0;
+		if (VoxWhole(s)) return 16;
 		VoxState st;
 		return VoxLayout(s, nullptr, st);
 	}
@@ -948,11 +991,19 @@ namespace tg
 	cudaError_t LaunchVoxBlocks(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream)
 	{
 		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
+		cudaError_t e = cudaMemsetAsync(words, 0, (size_t)((s.Total + 31) / 32) * 4, stream);
+		if (e != cudaSuccess) return e;
+		if (VoxWhole(s))
+		{
+			const int nx = VoxBoxes(s.SX), ny = VoxBoxes(s.SY), nz = VoxBoxes(s.SZ);
+			const size_t smem = kVoxWarps * (64 * sizeof(float4) + (size_t)depth * 32 * sizeof(float2));
+			VoxWholeKernel<<<(unsigned)((nx * ny * nz + kVoxWarps - 1) / kVoxWarps), kVoxWarps * 32, smem, stream>>>(prog, s, nx, ny, nz, depth, words);
+			return cudaGetLastError();
+		}
 		const VoxGrid vg = VoxGridOf(s);
 		VoxState st;
 		VoxLayout(s, scratch, st);
-		cudaError_t e = cudaMemsetAsync(words, 0, (size_t)((s.Total + 31) / 32) * 4, stream);
-		if (e == cudaSuccess) e = cudaMemsetAsync(st.Counters, 0, kVoxCounters * sizeof(uint32_t), stream);
+		e = cudaMemsetAsync(st.Counters, 0, kVoxCounters * sizeof(uint32_t), stream);
 		if (e != cudaSuccess) return e;
 		const size_t coarse = 64 * sizeof(float4) + (kVoxCoarseCap + kMaxStack + 2) * sizeof(uint2) + (size_t)depth * 32 * sizeof(float2);
 		const size_t fine = kVoxWarps * (sizeof(VoxScratch) + (size_t)depth * 32 * sizeof(float2));

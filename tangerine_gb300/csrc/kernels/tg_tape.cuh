@@ -946,8 +946,8 @@ namespace tg
 	// far from the box) is added here: each brush's float error is at most a few roundings of
 	// its local coordinates and sizes, that of a flate or a blend a few of what goes in and of
 	// its own width (`slack` times the largest of them).  Returns false when a list outgrows its
-	// room.
-	template<bool Materials, typename Source>
+	// room; with Finish the rest of the program still runs then, for the distances.
+	template<bool Materials, bool Finish = false, typename Source>
 	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, float slack, const PairUnits& u,
 		float2* spill, int stride, const TapeLists& ts, TapeCounts& out)
 	{
@@ -956,7 +956,7 @@ namespace tg
 		float2 size = make_float2(0.0f, 0.0f);
 		int depth = 0;
 		int nv = 0, nm = 0;
-		bool same = true;
+		bool same = true, full = false;
 		// [from, to) of a list moves down to `down`.
 		auto move = [&](uint2* list, int down, int from, int to)
 		{
@@ -971,7 +971,13 @@ namespace tg
 		};
 		for (int guard = 0; guard < (1 << 24); ++guard)
 		{
-			if (nv + 4 > ts.Cap || (Materials && nm + 4 > ts.Cap)) return false;
+			if (nv + 4 > ts.Cap || (Materials && nm + 4 > ts.Cap))
+			{
+				if (!Finish) return false;
+				full = true;
+			}
+			// A list that is full: nothing is left out any more, and what is written goes over its start.
+			if (Finish && full) nv = nm = 0;
 			uint32_t head = src.Head();
 			uint32_t op = head & 0xFFu;
 			int rv = nv, rm = nm;       // first events of the right operand
@@ -1032,7 +1038,7 @@ namespace tg
 			const float2 s = unions ? make_float2(acc.x - left.x, acc.y - left.y)
 				: diff ? make_float2(left.x + acc.x, left.y + acc.y) : make_float2(left.x - acc.x, left.y - acc.y);
 			const float2 t = make_float2(reach + slack * size.x + (blend ? k : 0.0f), reach + slack * size.y + (blend ? k : 0.0f));
-			const bool decides = !blend || k > 0.0f;
+			const bool decides = (!blend || k > 0.0f) && !full;
 			__syncwarp();       // every lane's list writes so far come before any slot is reused
 			const bool leftWins = __all_sync(0xFFFFFFFFu, decides && s.x > t.x && s.y > t.y);
 			const bool rightWins = __all_sync(0xFFFFFFFFu, decides && s.x < -t.x && s.y < -t.y);
@@ -1089,7 +1095,7 @@ namespace tg
 		out.Same = same;
 		out.Distance = acc;
 		out.Error = make_float2(slack * size.x, slack * size.y);
-		return true;
+		return !full;
 	}
 
 	// How far the difference of two operands can move inside a ball of radius r about a point

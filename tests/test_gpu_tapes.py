@@ -430,3 +430,48 @@ def test_page_locked_results_are_bounded(lib):
     finally:
         for block in taken:
             lib.tg_host_give(block)
+
+
+@pytest.mark.parametrize("prims,cells", [(1200, 130), (1500, 150), (1900, 200)])
+def test_voxel_blocks_with_full_lists_equal_bricks(lib, prims, cells):
+    """Trees with more records in a block than its list holds (all of the tree in one or a few,
+    and a far sphere), against the same without room for the blocks' scratch."""
+    seed = 11
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims))):
+        seed += 1
+    tree = sdf.union(sdf.from_spec(spec).scale(0.2), sdf.sphere(0.1).move(1.2, 1.0, 1.1))
+    with sdf.compile(tree) as prog:
+        info = prog.info()
+        grid = cells / float(np.max(np.asarray(info.bounds_max[:]) - np.asarray(info.bounds_min[:])))
+        voxels, size, _ = prog.export_voxels(grid, 3)
+        blocks, words = int(np.prod([-(-n // 64) for n in size])), int(np.prod(size)) // 4
+        try:        # room for the words and their ranks, and for less than the blocks' 41.7 KB each
+            lib.tg_debug_device_limit(int(lib.tg_debug_device_limit(0, 1)) + words + blocks * 41000, 0)
+            want, want_size, _ = prog.export_voxels(grid, 3)
+        finally:
+            lib.tg_debug_device_limit(0, 1)
+    assert size == want_size and voxels.shape[0] > 500
+    np.testing.assert_array_equal(voxels, want)
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_voxels_around_the_first_blocks_match_oracle(lib, port, whole):
+    """The largest lattices of at most 4096 boxes of 4^3 go box by box, larger ones by blocks."""
+    seed = 11
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, 90, ops=ALL_OPS))):
+        seed += 1
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        def boxes(grid):
+            return int(np.prod([-(-n // 4) for n in prog.export_voxels(grid, 3)[1]]))
+        grid = 4.0
+        while boxes(grid + 0.25) <= 4096:
+            grid += 0.25
+        grid += 0.0 if whole else 0.25
+        voxels, size, _ = prog.export_voxels(grid, 3)
+    h = port.build(spec)
+    try:
+        want, want_size, _ = port.vox(h, grid, 3)
+    finally:
+        port.free(h)
+    assert size == want_size
+    np.testing.assert_array_equal(voxels, want)
