@@ -1521,6 +1521,16 @@ extern "C"
 		return TG_OK;
 	}
 
+	TANGERINE_API int tg_debug_goes_by_tapes(void* tree, int call, const tg_grid* g, int64_t pixels)
+	{
+		GridSpec gs{};
+		Program p;
+		std::string err;
+		if (!tree || call < 0 || call > 3 || (call < 3 && !ToGridSpec(g, gs))) return -1;
+		if (!CompileTree(Borrow(tree), p.Host, err)) { SetError(err); return -1; }
+		return GoesByTapes(p, (CallKind)call, gs, pixels) ? 1 : 0;
+	}
+
 	TANGERINE_API uint64_t tg_debug_device_limit(uint64_t bytes, int release)
 	{
 		Engine& eng = Engine::Get();

@@ -363,6 +363,25 @@ namespace tg
 			points >= 1024.0 * bricks(g.NX) * bricks(g.NY) * bricks(g.NZ);
 	}
 
+	bool GoesByTapes(Program& p, CallKind kind, const GridSpec& g, int64_t pixels)
+	{
+		Bind(p, LayoutOf(p), nullptr);
+		switch (kind)
+		{
+		case CallKind::Export: return TapesPay(p, BrickCount(g, 7));
+		case CallKind::Lattice: return GridTapesPay(p, g);
+		case CallKind::Cloud:
+		{
+			CloudSpec s{};
+			s.IX = g.NX; s.IY = g.NY; s.IZ = g.NZ;
+			s.Total = (int64_t)g.NX * g.NY * g.NZ;
+			return CloudByTapes(p.View, s, CellQuads(p));
+		}
+		case CallKind::Render: return RenderBricks(p.View, p.Host.Nodes[0].ClipRadius, pixels, p.Host.VolumeQuads) != 0;
+		}
+		return false;
+	}
+
 	cudaError_t Engine::EvalGrid(const Program& p, const GridSpec& g, float* out, cudaStream_t s)
 	{
 		BrickTapes tapes{};
@@ -885,7 +904,7 @@ namespace tg
 		else
 		{
 			const OctNode& root = p.Host.Nodes[0];
-			int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px);
+			int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px, p.Host.VolumeQuads);
 			const int64_t all = (int64_t)bricks * bricks * bricks;
 			BrickTapes tapes{}, above{};
 			if (bricks && !TapesFit(Tapes, all, BrickPartCapacity(all), tapes, spare)) bricks = 0;

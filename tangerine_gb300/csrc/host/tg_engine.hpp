@@ -74,6 +74,12 @@ namespace tg
 		return (double)p.Host.DistanceQuadsTotal / (p.Host.Header.NodeCount > 0 ? p.Host.Header.NodeCount : 1);
 	}
 
+	// Whether a call on the tree that p was compiled from (its host image; p is not on a device)
+	// goes by shortened programs, where memory allows: a culled export of g by 7^3-cell bricks,
+	// tg_eval_grid of it, a point cloud of as many voxels, a render of so many pixels.
+	enum class CallKind { Export, Lattice, Cloud, Render };
+	bool GoesByTapes(Program& p, CallKind kind, const GridSpec& g, int64_t pixels);
+
 	struct ExportOptions
 	{
 		bool Attributes = true;     // gradient normals and colours

@@ -209,8 +209,9 @@ namespace tg
 
 	// LaunchRender's octree-bounded form by tapes of the root cube's bricks (the same steps and
 	// images): how many bricks per axis pay for that many pixels (0: none), and the launch, with
-	// the tapes' buffers for bricks^3 bricks.  pivot, root_clip: the root cell's.
-	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels);
+	// the tapes' buffers for bricks^3 bricks.  pivot, root_clip: the root cell's; quads: what a point
+	// runs on average.
+	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels, double quads);
 	// above: the buffers for tapes of the 4^3 times larger bricks first ((bricks / 4)^3), from which
 	// the others are then built (Bricks == nullptr: without).
 	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes,

@@ -412,20 +412,23 @@ namespace tg
 	}
 
 	// Bricks per axis for the renderer's tapes, 0 for none.  A tape costs a pass of its cell's
-	// program by one warp; without, a render of any size lasts as long as the ray that grazes
-	// the surface longest, some hundred whole programs one after the other.  Measured on a
-	// GB300, tapes against none, us an image: 16 primitives 64 x 48 238 / 184, 200 x 150 287 /
-	// 330; 64 primitives 422 / 352 and 429 / 675; 512 primitives 780 / 1349 and 1291 / 2170;
-	// 1024 primitives two of 1920 x 1080 2.39 / 6.2 ms.
-	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels)
+	// program by one warp, and building them all 120 us at least; without, a render of any size
+	// lasts as long as the ray that grazes the surface longest, some hundred whole programs one
+	// after the other.  So what counts are the pixels and what a program has beyond two brushes
+	// (ten quads), which a tape mostly leaves.  Measured on a GB300, none against tapes, us an image
+	// (quads a point runs in brackets): 1 primitive (5) 1920 x 1080 168 / 238, 2 (10) 256 / 270, 4 (12)
+	// 200 x 150 137 / 185, 800 x 500 385 / 260, 8 (18) 64 x 48 152 / 193, 128 x 96 231 / 216, 16 (25)
+	// 355 / 280, 32 (61) 64 x 48 356 / 258, 64 (50) 382 / 237, 256 (107) 1757 / 667; the rule's worst,
+	// 16 (44) 128 x 96 159 / 224.
+	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels, double quads)
 	{
-		if (!prog.Lipschitz || !(prog.Form & kFormPrunable)) return 0;
+		if (!prog.Lipschitz || !(prog.Form & kFormPrunable) || (double)pixels * (quads - 10.0) < 1.2e5) return 0;
 		const float span = 2.0f * fabsf(root_clip) * 0.57735f;
 		// The cells' edge: the cube halved until no more than the octree's target.
 		int cells = 1;
 		while (cells < 128 && span / (float)cells > 0.25f) cells *= 2;
 		const int n = cells < 32 ? 32 : cells;
-		return n <= 64 && pixels >= (int64_t)n * n * n / 4 ? n : 0;
+		return n <= 64 ? n : 0;
 	}
 
 	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes, const BrickTapes& above,

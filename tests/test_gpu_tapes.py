@@ -475,3 +475,34 @@ def test_voxels_around_the_first_blocks_match_oracle(lib, port, whole):
         port.free(h)
     assert size == want_size
     np.testing.assert_array_equal(voxels, want)
+
+
+def _by_whole_programs(lib, room, call):
+    """A call with `room` bytes of device memory beside what is held: not enough for tapes."""
+    try:
+        lib.tg_debug_device_limit(int(lib.tg_debug_device_limit(0, 1)) + room, 0)
+        return call()
+    finally:
+        lib.tg_debug_device_limit(0, 1)
+
+
+@pytest.mark.parametrize("prims,ops,large,paint", [(24, ALL_OPS, False, True), (150, ALL_OPS, False, True), (600, W.OPS_60_20_10_10, False, True),
+                                                   (400, W.OPS_60_20_10_10, True, True), (300, W.OPS_60_20_10_10, True, False)])
+def test_render_by_tapes_equals_whole_programs(lib, prims, ops, large, paint):
+    """The same images with room for the tapes (by way of larger bricks' where the cells are
+    large) and without.  Odd image sides, a camera inside the root cube, one that misses it."""
+    seed = 31
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops, paint=paint))):
+        seed += 1
+    if large:
+        spec = _large_cells(prims, ops, paint)
+    width, height = 83, 61
+    poses = np.concatenate([W.camera_poses(7, 7), [[0.3, 0.2, 0.1], [60.0, 50.0, 70.0]]]).astype(np.float32)
+    pixels = len(poses) * width * height
+    assert lib.tg_debug_goes_by_tapes(sdf.from_spec(spec).handle, 3, None, pixels) == 1
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        images = prog.render(sdf.cameras(poses), width, height)
+        want = _by_whole_programs(lib, 19 * pixels + (1 << 20), lambda: prog.render(sdf.cameras(poses), width, height))
+    assert np.isfinite(images[0]).any()
+    for a, b in zip(images, want):
+        np.testing.assert_array_equal(a, b)

@@ -1,0 +1,43 @@
+"""Which calls go by shortened programs: the rules weigh what a call could save against what building
+them costs, and both sides were measured where a test here draws the line.  No GPU needed."""
+
+import ctypes as C
+
+import pytest
+
+from tangerine_gb300 import _lib, sdf
+from tangerine_gb300 import workloads as W
+
+U, D, I, BU, BD, BI = W.UNION, W.DIFF, W.INTER, W.BLEND_UNION, W.BLEND_DIFF, W.BLEND_INTER
+BLENDS = ((U, 0.3), (D, 0.2), (I, 0.05), (BU, 0.25), (BD, 0.1), (BI, 0.1))
+EXPORT, LATTICE, CLOUD, RENDER = range(4)
+
+
+def _tree(prims, seed, blends=False):
+    kw = {"ops": BLENDS} if blends else {}
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, **kw))):
+        seed += 7919
+    return sdf.from_spec(spec)
+
+
+def _by_tapes(lib, tree, call, grid=None, pixels=0):
+    answer = lib.tg_debug_goes_by_tapes(tree.handle, call, C.byref(grid) if grid is not None else None, pixels)
+    assert answer >= 0
+    return bool(answer)
+
+
+# Measured without / with tapes, us an image.
+@pytest.mark.parametrize("prims,seed,blends,width,height,tapes", [
+    (1, 3, False, 1920, 1080, False),       # 168 / 238
+    (1, 2, False, 400, 300, False),         # 211 / 279
+    (2, 3, False, 1920, 1080, False),       # 256 / 270
+    (4, 4, True, 128, 96, False),           # 122 / 177
+    (4, 3, False, 800, 500, True),          # 385 / 260
+    (16, 3, False, 64, 48, False),          # 191 / 227
+    (8, 2, False, 200, 150, True),          # 627 / 441
+    (32, 6, True, 128, 96, True),           # 459 / 283
+    (64, 3, False, 64, 48, True),           # 382 / 237
+    (256, 2, False, 64, 48, True),          # 1757 / 667
+])
+def test_render(lib, prims, seed, blends, width, height, tapes):
+    assert _by_tapes(lib, _tree(prims, seed, blends), RENDER, pixels=width * height) == tapes
