@@ -348,18 +348,19 @@ namespace tg
 
 	// Whether a whole lattice goes by tapes, in bricks of 16^3 points (a quarter full at least).
 	// By whole programs it takes about 0.7 to 0.9 us per million quads that its points run
-	// together; by tapes 6 us per million points, and 100 to 350 us whatever the size, the more
-	// the larger the tree (the chains of splitting bricks and of the longest program's one pass).
-	// Whole programs / tapes in us by millions of quads: 8 primitives 89 / 111 at 89, 136 / 133 at
-	// 174, 433 / 253 at 713; 30 primitives 157 / 204 at 109, 261 / 229 at 213, 789 / 340 at 876; 64
-	// primitives 229 / 229 at 232, 405 / 260 at 455, 1415 / 257 at 1877; 128 primitives 296 / 202 at
-	// 294, 231 / 256 at 177; 256 primitives 372 / 422 at 270, 384 / 366 at 401, 5515 / 618 at 8900.
+	// together; by tapes 6 us per million points (as long as six quads take otherwise), and 40 to
+	// 600 us whatever the size, the more the larger the tree (the chains of splitting bricks and of
+	// the longest program's one pass).  Whole programs / tapes in us (quads a point runs in
+	// brackets): 1 primitive (5) 300^3 163 / 177, 2 (10) 300^3 182 / 188, 4 (12.5) 300^3 251 / 208, 8
+	// (16) 190^3 101 / 97, 240^3 169 / 139, 16 (42) 150^3 110 / 115, 190^3 189 / 134, 64 (32) 190^3 238
+	// / 199, 128 (43) 190^3 329 / 244, 256 (107) 150^3 429 / 298, 512 (57) 190^3 495 / 408, (1500)
+	// 110^3 2152 / 1743.
 	static bool GridTapesPay(const Program& p, const GridSpec& g)
 	{
 		if (!p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
 		const double points = (double)g.NX * g.NY * g.NZ;
 		const auto bricks = [](int n) { return (double)((n + 15) / 16); };
-		return points * p.Host.VolumeQuads >= 1e6 * (200.0 + p.Host.Header.FullBrushes) &&
+		return points * (p.Host.VolumeQuads - 6.0) >= 1e6 * (120.0 + 0.6 * p.Host.Header.FullBrushes) &&
 			points >= 1024.0 * bricks(g.NX) * bricks(g.NY) * bricks(g.NZ);
 	}
 

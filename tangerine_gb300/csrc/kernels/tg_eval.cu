@@ -120,7 +120,12 @@ namespace tg
 
 	namespace
 	{
-		constexpr int kSlice = 4;                // levels of a brick that a warp takes at a time
+		// Levels of a brick that a warp takes at a time: two, one where there are few bricks.  At four
+		// a warp whose part has no tape (a long program, a coarse lattice) ran the whole program 16
+		// times over, longer than all others took together: 512 primitives at 110^3 2764 us by whole
+		// programs, 5310 at four levels, 3077 at two, 2175 at one; 32 primitives at 190^3 710, 201, 173,
+		// 162, at 300^3 2639, 334, 321, 332.
+		constexpr int64_t kFewBricks = 2000;
 		constexpr int64_t kSlabBricks = 16384;
 		constexpr int kDenseCtasPerSm = 8;
 
@@ -150,12 +155,13 @@ namespace tg
 		};
 
 		// A warp per slice of a brick, drawn from a counter.
+		template<int Slice>
 		__global__ void __launch_bounds__(parts::kThreads, kDenseCtasPerSm) EvalGridTapesKernel(DeviceProgram prog, DenseLattice lat, BrickTapes tapes,
 			float* __restrict__ out)
 		{
 			extern __shared__ __align__(16) float2 spill2[];
 			__shared__ float axes[parts::kWarps][3][DenseLattice::kBox];
-			constexpr int kSlices = DenseLattice::kBox / kSlice;
+			constexpr int kSlices = DenseLattice::kBox / Slice;
 			const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
 			float (*axis)[DenseLattice::kBox] = axes[warp];
 			const PairUnits units = LoadPairUnits();
@@ -168,7 +174,7 @@ namespace tg
 				item = __shfl_sync(0xFFFFFFFFu, item, 0);
 				if (item >= n * kSlices) break;
 				const uint32_t b = item / kSlices;
-				const int lowest = (int)(item % kSlices) * kSlice;
+				const int lowest = (int)(item % kSlices) * Slice;
 				int first[3], extent[3];
 				parts::BrickSpan(lat, b, first, extent);
 				if (lowest > extent[2]) continue;
@@ -180,7 +186,7 @@ namespace tg
 					[&](int at, float v, bool live)
 					{
 						if (live) corner[(at >> 8) * plane + ((at >> 4) & 15) * lat.Grid.NX + (at & 15)] = v;
-					}, lowest, lowest + kSlice - 1);
+					}, lowest, lowest + Slice - 1);
 			}
 		}
 
@@ -202,9 +208,11 @@ namespace tg
 	cudaError_t LaunchEvalGridTapes(const DeviceProgram& prog, const GridSpec& g, const BrickTapes& tapes, float* out, int sms, cudaStream_t stream)
 	{
 		const size_t smem = parts::SpillPairs(prog, 1) * parts::kThreads * sizeof(float2);
+		const int64_t bricks = DensePlane(g) * ((g.NZ + DenseLattice::kBox - 1) / DenseLattice::kBox);
+		auto* kernel = bricks <= kFewBricks ? EvalGridTapesKernel<1> : EvalGridTapesKernel<2>;
 		if (smem > 46 * 1024)
 		{
-			const cudaError_t e = cudaFuncSetAttribute(EvalGridTapesKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 			if (e != cudaSuccess) return e;
 		}
 		const int levels = (int)(DenseSlabBricks(g) / DensePlane(g)) * DenseLattice::kBox;
@@ -213,7 +221,7 @@ namespace tg
 			const DenseLattice lat{ g, k0, g.NZ - k0 < levels ? g.NZ - k0 : levels };
 			cudaError_t e = parts::LaunchParts(prog, lat, nullptr, nullptr, nullptr, tapes, sms, stream);
 			if (e != cudaSuccess) return e;
-			EvalGridTapesKernel<<<sms * kDenseCtasPerSm, parts::kThreads, smem, stream>>>(prog, lat, tapes, out);
+			kernel<<<sms * kDenseCtasPerSm, parts::kThreads, smem, stream>>>(prog, lat, tapes, out);
 			e = cudaGetLastError();
 			if (e != cudaSuccess) return e;
 		}

@@ -2,6 +2,8 @@
 lose everywhere in its box, so every value it gives is the whole program's, bit for bit (the
 tolerance is 0)."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -506,3 +508,21 @@ def test_render_by_tapes_equals_whole_programs(lib, prims, ops, large, paint):
     assert np.isfinite(images[0]).any()
     for a, b in zip(images, want):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("prims,ops,shape", [(5, ALL_OPS, (353, 320, 300)), (64, ALL_OPS, (257, 193, 209)), (64, ALL_OPS, (15, 633, 641)),
+                                             (200, W.OPS_60_20_10_10, (33, 17, 9000)), (200, ALL_OPS, (1601, 16, 241)), (90, ALL_OPS, (129, 3001, 14)),
+                                             (100, ALL_OPS, (1025, 1025, 66)), (500, ALL_OPS, (190, 191, 193))])
+def test_lattices_by_tapes_equal_whole_programs(lib, prims, ops, shape):
+    """Lattices with remainders of bricks on every axis, one brick thin on some, in one and in
+    several slabs, by levels one and two at a time: with room for the tapes and without."""
+    seed = 21
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops))):
+        seed += 1
+    steps = [3.2 / n for n in shape]
+    grid = _lib.Grid(-1.6, -1.6, -1.6, steps[0], *shape, steps[1], steps[2])
+    assert lib.tg_debug_goes_by_tapes(sdf.from_spec(spec).handle, 1, C.byref(grid), 0) == 1
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        lattice = prog.eval_grid(grid)
+        want = _by_whole_programs(lib, 4 * int(np.prod(shape)) + (1 << 18), lambda: prog.eval_grid(grid))
+    np.testing.assert_array_equal(lattice, want)

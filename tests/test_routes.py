@@ -41,3 +41,22 @@ def _by_tapes(lib, tree, call, grid=None, pixels=0):
 ])
 def test_render(lib, prims, seed, blends, width, height, tapes):
     assert _by_tapes(lib, _tree(prims, seed, blends), RENDER, pixels=width * height) == tapes
+
+
+# Measured by whole programs / by tapes, us a call.
+@pytest.mark.parametrize("prims,seed,blends,n,tapes", [
+    (1, 4, True, 300, False),               # 163 / 177
+    (2, 4, True, 300, False),               # 182 / 188
+    (4, 3, False, 300, True),               # 251 / 208
+    (16, 3, False, 150, False),             # 110 / 115
+    (16, 3, False, 190, True),              # 189 / 134
+    (32, 4, True, 150, True),               # 378 / 137
+    (128, 2, False, 190, True),             # 329 / 244
+    (256, 2, False, 64, False),             # 269 / 448
+    (512, 3, False, 110, False),            # 314 / 471
+    (512, 4, True, 64, False),              # 1455 / 2244
+    (512, 4, True, 110, True),              # 2764 / 2175
+])
+def test_lattice(lib, prims, seed, blends, n, tapes):
+    grid = _lib.Grid(-1.6, -1.6, -1.6, 3.2 / (n - 1), n, n, n)
+    assert _by_tapes(lib, _tree(prims, seed, blends), LATTICE, grid) == tapes
