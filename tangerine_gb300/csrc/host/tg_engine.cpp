@@ -333,17 +333,27 @@ namespace tg
 
 	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
 	// A tape saves about what its cell's program has beyond a dozen quads (two brushes), on
-	// every pass over the brick, and costs one pass of the whole program and two launches: it
-	// pays from a number of bricks that falls as the programs get longer, and later while whole
-	// programs go by eight warps a brick (kWideBricks).  Measured on a GB300, export to the
-	// device, whole programs / tapes, in us: 64 primitives (19 quads a cell) 448^3 330 / 348,
-	// 512^3 389 / 383, 700^3 599 / 531; 16 primitives (14 quads) 600^3 252 / 259, 700^3 321 /
-	// 304; 256 primitives (46 quads) 320^3 582 / 600, 384^3 693 / 644, 512^3 966 / 767; 256 others
-	// (33 quads) 384^3 451 / 514, 448^3 571 / 551.
-	static bool TapesPay(const Program& p, int64_t bricks)
+	// every pass over a kept brick, and costs one pass of the whole program and two launches.
+	// Which bricks will be kept is not known here; their number goes with the model's surface,
+	// as the bricks on a side of its bounds (within the lattice) do.  Tapes pay from a number that
+	// falls as the programs get longer, and four times later while whole programs go by eight
+	// warps a brick (kWideBricks).  Measured on a GB300, export to the device, whole programs /
+	// tapes, in us (quads of a cell's program in brackets): 16 primitives (22) 512^3 164 / 197,
+	// 900^3 249 / 271, 32 (17) 600^3 274 / 289, 900^3 476 / 458, 64 (19) 512^3 387 / 385, 600^3
+	// 476 / 459, 64 others (63) 400^3 169 / 222, 900^3 282 / 278, 128 (24) 400^3 447 / 459, 450^3
+	// 520 / 497, 256 (38) 400^3 546 / 587, 512^3 755 / 658, 512 (181) 320^3 902 / 1011, 450^3 1235 / 1018.
+	static bool TapesPay(const Program& p, const GridSpec& g)
 	{
-		return p.View.Lipschitz && (p.View.Form & kFormPrunable) &&
-			(double)bricks * (CellQuads(p) - 12.0) >= (bricks <= kWideBricks ? 5e6 : 3.5e6);
+		if (!p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
+		const AABB& b = p.Host.Bounds;
+		const auto side = [](float lo, float hi, float start, float step, int points)
+		{
+			const double end = (double)start + (double)step * (points - 1);
+			return std::max(0.0, (std::min<double>(hi, end) - std::max<double>(lo, start)) / (7.0 * step));
+		};
+		const double x = side(b.Min.x, b.Max.x, g.X0, g.DX, g.NX), y = side(b.Min.y, b.Max.y, g.Y0, g.DY, g.NY);
+		const double z = side(b.Min.z, b.Max.z, g.Z0, g.DZ, g.NZ);
+		return (x * y + y * z + z * x) / 3.0 * (CellQuads(p) - 12.0) >= (BrickCount(g, 7) <= kWideBricks ? 2e5 : 5e4);
 	}
 
 	// Whether a whole lattice goes by tapes, in bricks of 16^3 points (a quarter full at least).
@@ -369,7 +379,7 @@ namespace tg
 		Bind(p, LayoutOf(p), nullptr);
 		switch (kind)
 		{
-		case CallKind::Export: return TapesPay(p, BrickCount(g, 7));
+		case CallKind::Export: return TapesPay(p, g);
 		case CallKind::Lattice: return GridTapesPay(p, g);
 		case CallKind::Cloud:
 		{
@@ -600,7 +610,7 @@ namespace tg
 			TG_TRY(ActiveCells.Reserve((size_t)(nb * (int64_t)B * B * B < cells ? nb * (int64_t)B * B * B : cells) * 4));
 			int* evalStatus = reinterpret_cast<int*>(Counts.As<uint32_t>() + 4);      // status and work counter
 			TG_TRY(cudaMemsetAsync(evalStatus, 0, 2 * sizeof(int), s));
-			const bool byTapes = B == 7 && !opt.Staged && (opt.Tapes || TapesPay(p, nb)) && TapesFit(Tapes, nb, BrickPartCapacity(nb), tapes, spare);
+			const bool byTapes = B == 7 && !opt.Staged && (opt.Tapes || TapesPay(p, g)) && TapesFit(Tapes, nb, BrickPartCapacity(nb), tapes, spare);
 			if (B == 7 && !opt.Staged && !byTapes)
 			{
 				// The cell pass runs inside the brick evaluation, on each brick's values in

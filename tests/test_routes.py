@@ -60,3 +60,23 @@ def test_render(lib, prims, seed, blends, width, height, tapes):
 def test_lattice(lib, prims, seed, blends, n, tapes):
     grid = _lib.Grid(-1.6, -1.6, -1.6, 3.2 / (n - 1), n, n, n)
     assert _by_tapes(lib, _tree(prims, seed, blends), LATTICE, grid) == tapes
+
+
+# Measured by whole programs / by tapes, us an export to the device.
+@pytest.mark.parametrize("prims,seed,blends,res,tapes", [
+    (1, 2, False, 900, False),              # 264 / 270
+    (16, 3, False, 512, False),             # 164 / 197
+    (16, 3, False, 900, False),             # 249 / 271
+    (16, 4, True, 720, False),              # 215 / 233
+    (32, 3, False, 720, False),             # 255 / 285
+    (64, 4, True, 400, False),              # 169 / 222
+    (64, 2, False, 900, True),              # 922 / 820
+    (128, 2, False, 720, True),             # 948 / 779
+    (256, 2, False, 400, False),            # 546 / 587
+    (256, 2, False, 512, True),             # 755 / 658
+    (512, 4, True, 320, False),             # 902 / 1011
+    (512, 6, True, 450, True),              # 1029 / 817
+])
+def test_export(lib, prims, seed, blends, res, tapes):
+    grid = sdf._grid(W.export_grid(resolution=res))
+    assert _by_tapes(lib, _tree(prims, seed, blends), EXPORT, grid) == tapes
