@@ -3,6 +3,7 @@
 #include "tg_surrogate.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -332,16 +333,17 @@ namespace tg
 #define TG_TRY(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
 
 	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
-	// A tape saves about what its cell's program has beyond a dozen quads (two brushes), on
-	// every pass over a kept brick, and costs one pass of the whole program and two launches.
-	// Which bricks will be kept is not known here; their number goes with the model's surface,
-	// as the bricks on a side of its bounds (within the lattice) do.  Tapes pay from a number that
-	// falls as the programs get longer, and four times later while whole programs go by eight
-	// warps a brick (kWideBricks).  Measured on a GB300, export to the device, whole programs /
-	// tapes, in us (quads of a cell's program in brackets): 16 primitives (22) 512^3 164 / 197,
-	// 900^3 249 / 271, 32 (17) 600^3 274 / 289, 900^3 476 / 458, 64 (19) 512^3 387 / 385, 600^3
-	// 476 / 459, 64 others (63) 400^3 169 / 222, 900^3 282 / 278, 128 (24) 400^3 447 / 459, 450^3
-	// 520 / 497, 256 (38) 400^3 546 / 587, 512^3 755 / 658, 512 (181) 320^3 902 / 1011, 450^3 1235 / 1018.
+	// A tape saves most of its cell's program on every pass over a kept brick, and costs one pass
+	// of that program and two launches.  Which bricks will be kept is not known here; their number
+	// goes with the model's surface: as the bricks on a side of its bounds (within the lattice),
+	// and a little with the octree's cells, the more of them the more convoluted it is.  The line
+	// is fitted to 668 exports of 62 trees: 4 of them are slower by its choice, 6 % at most.  While
+	// whole programs go by eight warps a brick (kWideBricks) tapes pay eight times later.
+	// Measured on a GB300, export to the device, whole programs / tapes, in us (quads of a cell's
+	// program in brackets): 16 primitives (22) 512^3 164 / 197, 900^3 249 / 271, 32 (17) 600^3 274 /
+	// 289, 900^3 476 / 458, 64 (19) 512^3 387 / 385, 600^3 476 / 459, 64 others (63) 400^3 169 / 222,
+	// 900^3 282 / 278, 128 (24) 400^3 447 / 459, 450^3 520 / 497, 256 (38) 400^3 546 / 587, 512^3
+	// 755 / 658, 512 (181) 320^3 902 / 1011, 450^3 1235 / 1018.
 	static bool TapesPay(const Program& p, const GridSpec& g)
 	{
 		if (!p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
@@ -353,7 +355,8 @@ namespace tg
 		};
 		const double x = side(b.Min.x, b.Max.x, g.X0, g.DX, g.NX), y = side(b.Min.y, b.Max.y, g.Y0, g.DY, g.NY);
 		const double z = side(b.Min.z, b.Max.z, g.Z0, g.DZ, g.NZ);
-		return (x * y + y * z + z * x) / 3.0 * (CellQuads(p) - 12.0) >= (BrickCount(g, 7) <= kWideBricks ? 2e5 : 5e4);
+		const double gain = (x * y + y * z + z * x) / 3.0 * std::pow((double)p.Host.Header.NodeCount, 0.2) * std::pow(CellQuads(p), 1.3);
+		return gain >= (BrickCount(g, 7) <= kWideBricks ? 4e6 : 5e5);
 	}
 
 	// Whether a whole lattice goes by tapes, in bricks of 16^3 points (a quarter full at least).
