@@ -332,6 +332,19 @@ namespace tg
 
 #define TG_TRY(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
 
+	double BoundsSide(const Program& p, const float start[3], const float step[3], const int points[3], int edge)
+	{
+		const AABB& b = p.Host.Bounds;
+		const float lo[3] = { b.Min.x, b.Min.y, b.Min.z }, hi[3] = { b.Max.x, b.Max.y, b.Max.z };
+		double n[3];
+		for (int a = 0; a < 3; ++a)
+		{
+			const double end = (double)start[a] + (double)step[a] * (points[a] - 1);
+			n[a] = std::max(0.0, (std::min<double>(hi[a], end) - std::max<double>(lo[a], start[a])) / ((double)edge * step[a]));
+		}
+		return (n[0] * n[1] + n[1] * n[2] + n[2] * n[0]) / 3.0;
+	}
+
 	// Whether 7^3-cell bricks go by tapes (kernels/tg_tape.cuh) or by their cells' programs.
 	// A tape saves most of its cell's program on every pass over a kept brick, and costs one pass
 	// of that program and two launches.  Which bricks will be kept is not known here; their number
@@ -347,15 +360,9 @@ namespace tg
 	static bool TapesPay(const Program& p, const GridSpec& g)
 	{
 		if (!p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
-		const AABB& b = p.Host.Bounds;
-		const auto side = [](float lo, float hi, float start, float step, int points)
-		{
-			const double end = (double)start + (double)step * (points - 1);
-			return std::max(0.0, (std::min<double>(hi, end) - std::max<double>(lo, start)) / (7.0 * step));
-		};
-		const double x = side(b.Min.x, b.Max.x, g.X0, g.DX, g.NX), y = side(b.Min.y, b.Max.y, g.Y0, g.DY, g.NY);
-		const double z = side(b.Min.z, b.Max.z, g.Z0, g.DZ, g.NZ);
-		const double gain = (x * y + y * z + z * x) / 3.0 * std::pow((double)p.Host.Header.NodeCount, 0.2) * std::pow(CellQuads(p), 1.3);
+		const float start[3] = { g.X0, g.Y0, g.Z0 }, step[3] = { g.DX, g.DY, g.DZ };
+		const int points[3] = { g.NX, g.NY, g.NZ };
+		const double gain = BoundsSide(p, start, step, points, 7) * std::pow((double)p.Host.Header.NodeCount, 0.2) * std::pow(CellQuads(p), 1.3);
 		return gain >= (BrickCount(g, 7) <= kWideBricks ? 4e6 : 5e5);
 	}
 
@@ -389,7 +396,9 @@ namespace tg
 			CloudSpec s{};
 			s.IX = g.NX; s.IY = g.NY; s.IZ = g.NZ;
 			s.Total = (int64_t)g.NX * g.NY * g.NZ;
-			return CloudByTapes(p.View, s, CellQuads(p));
+			const float start[3] = { g.X0, g.Y0, g.Z0 }, step[3] = { g.DX, g.DY, g.DZ };
+			for (int a = 0; a < 3; ++a) { s.Start[a] = start[a]; s.Step[a] = step[a]; }
+			return CloudTapesPay(p, s);
 		}
 		case CallKind::Render: return RenderBricks(p.View, p.Host.Nodes[0].ClipRadius, pixels, p.Host.VolumeQuads) != 0;
 		}

@@ -74,6 +74,10 @@ namespace tg
 		return (double)p.Host.DistanceQuadsTotal / (p.Host.Header.NodeCount > 0 ? p.Host.Header.NodeCount : 1);
 	}
 
+	// The bricks of edge^3 steps on a side of p's bounds, as far as they lie in a lattice.
+	double BoundsSide(const Program& p, const float start[3], const float step[3], const int points[3], int edge);
+	// Whether a point cloud goes by tapes.
+	bool CloudTapesPay(const Program& p, const CloudSpec& s);
 	// Whether a call on the tree that p was compiled from (its host image; p is not on a device)
 	// goes by shortened programs, where memory allows: a culled export of g by 7^3-cell bricks,
 	// tg_eval_grid of it, a point cloud of as many voxels, a render of so many pixels.

@@ -90,6 +90,21 @@ namespace tg
 		return true;
 	}
 
+	// Few bricks keep the direct tests: the splitting and building cost more there, the more the
+	// larger the bricks are against the octree's cells.  Fitted to 438 clouds of 62 trees, of which
+	// 6 are slower by the choice, up to 30 % (by bricks x (quads - 12) alone 12 were, up to fourfold).
+	// Measured on a GB300, direct / tapes, us a call (quads of a cell's program in brackets), in
+	// [-1.6, 1.6]^3: 1 primitive (5) 0.02 voxels 146 / 147, 0.015 174 / 152, 16 (15) 0.03 253 / 266,
+	// 0.02 321 / 293, 64 (19) 399 / 470 and 519 / 428, 256 (38) 0.04 1074 / 1329, 0.03 1198 / 1035,
+	// 256 others (443) 0.06 342 / 438, 0.04 565 / 459, 512 (181) 0.06 2299 / 7287, 0.03 3598 / 4308.
+	bool CloudTapesPay(const Program& p, const CloudSpec& s)
+	{
+		if (s.Total <= 0 || !p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
+		const int points[3] = { s.IX, s.IY, s.IZ };
+		const double side = BoundsSide(p, s.Start, s.Step, points, 8);
+		return std::pow((double)CloudBricks(s), 0.75) * std::pow(side, 0.25) * std::sqrt(CellQuads(p)) >= 7550.0;
+	}
+
 	cudaError_t Engine::PointCloud(const Program& p, const CloudSpec& s, int refine, bool attributes, DeviceMesh& out, cudaStream_t st,
 		const ExportOptions* control)
 	{
@@ -103,7 +118,7 @@ namespace tg
 		BrickTapes tapes{};
 		const int64_t bricks = CloudBricks(s);
 		SpareUse spare(*this);
-		bool byTapes = CloudByTapes(p.View, s, CellQuads(p)) && TapesFit(Tapes, bricks, BrickPartCapacity(bricks), tapes, spare);
+		bool byTapes = CloudTapesPay(p, s) && TapesFit(Tapes, bricks, BrickPartCapacity(bricks), tapes, spare);
 		if (byTapes)
 		{
 			cudaError_t e = VoxScratch.Reserve((size_t)bricks * 8);

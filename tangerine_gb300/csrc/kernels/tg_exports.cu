@@ -844,16 +844,6 @@ namespace tg
 		return (int64_t)lat.Bricks(0) * lat.Bricks(1) * lat.Bricks(2);
 	}
 
-	// Short programs and few bricks keep the direct tests (two launches and a pass of the whole
-	// programs cost more there).  Measured on a GB300, tapes against direct, us a call: 16
-	// primitives (16 quads a cell) 0.04 voxels 203 / 193, 0.02 222 / 275; 64 (23 quads) 556 /
-	// 429 and 470 / 634; 256 (54 quads) 0.08 voxels 1971 / 1188, 0.04 1549 / 1527, 0.02 1108 /
-	// 2295.  quads: those of an octree cell's distance program, on average.
-	bool CloudByTapes(const DeviceProgram& prog, const CloudSpec& s, double quads)
-	{
-		return s.Total > 0 && prog.Lipschitz && (prog.Form & kFormPrunable) && (double)CloudBricks(s) * (quads - 12.0) >= 45000.0;
-	}
-
 	cudaError_t LaunchCloudVoxels(const DeviceProgram& prog, const CloudSpec& s, uint32_t* list, uint32_t* tops, const BrickTapes& tapes,
 		uint32_t* words, uint32_t* voxels, uint32_t* counts, int sms, cudaStream_t stream)
 	{

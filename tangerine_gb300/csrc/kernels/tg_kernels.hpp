@@ -298,10 +298,9 @@ namespace tg
 	size_t VoxelBrickWords(int sx, int sy, int sz);
 	// One bit per voxel (cell number order): |octree distance at the centre| < Diagonal.
 	cudaError_t LaunchCloudFlags(const DeviceProgram& prog, const CloudSpec& s, uint32_t* brick_bits, uint32_t* words, cudaStream_t stream);
-	// The same by shortened programs (tg_parts.cuh), where the tree's can be (CloudByTapes):
+	// The same by shortened programs (tg_parts.cuh), where the tree's can be (CloudTapesPay):
 	// one bit per kept voxel and the voxels listed by brick; counts: bricks, voxels.  Scratch:
 	// list and tops hold a word per brick (CloudBricks), voxels one per voxel.
-	bool CloudByTapes(const DeviceProgram& prog, const CloudSpec& s, double quads);
 	int64_t CloudBricks(const CloudSpec& s);
 	cudaError_t LaunchCloudVoxels(const DeviceProgram& prog, const CloudSpec& s, uint32_t* list, uint32_t* tops, const BrickTapes& tapes,
 		uint32_t* words, uint32_t* voxels, uint32_t* counts, int sms, cudaStream_t stream);

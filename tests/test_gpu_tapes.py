@@ -526,3 +526,29 @@ def test_lattices_by_tapes_equal_whole_programs(lib, prims, ops, shape):
         lattice = prog.eval_grid(grid)
         want = _by_whole_programs(lib, 4 * int(np.prod(shape)) + (1 << 18), lambda: prog.eval_grid(grid))
     np.testing.assert_array_equal(lattice, want)
+
+
+@pytest.mark.parametrize("prims,ops,paint,step,refine", [(200, ALL_OPS, True, (0.014, 0.017, 0.012), 4), (200, W.OPS_60_20_10_10, False, 0.013, 0),
+                                                         (100, ALL_OPS, True, 0.012, 1), (20, ALL_OPS, True, 0.011, 6)])
+def test_clouds_by_tapes_equal_whole_programs(lib, prims, ops, paint, step, refine):
+    """The same points, normals and colours with room for the tapes and without; bricks cut on
+    every axis, refined points that leave their voxel's brick and its parts on the way."""
+    seed = 21
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ops, paint=paint))):
+        seed += 1
+    step = [float(v) for v in np.broadcast_to(np.asarray(step, np.float32), (3,))]
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        info = prog.info()
+        lo, hi = np.asarray(info.bounds_min[:]), np.asarray(info.bounds_max[:])
+        shape = [int(np.ceil((h - l) / s)) for l, h, s in zip(lo, hi, step)]
+        grid = _lib.Grid(*[float(v) for v in lo], step[0], *shape, step[1], step[2])
+        assert lib.tg_debug_goes_by_tapes(sdf.from_spec(spec).handle, 2, C.byref(grid), 0) == 1
+        cloud = prog.export_point_cloud(lo, hi, step, refine)
+        count = cloud.vertices.shape[0]
+        want = _by_whole_programs(lib, int(4.5 * np.prod(shape)) + 31 * count + (1 << 20), lambda: prog.export_point_cloud(lo, hi, step, refine))
+    assert count > 1000
+    for a, b in ((cloud.vertices, want.vertices), (cloud.cubes, want.cubes), (cloud.normals, want.normals)):
+        np.testing.assert_array_equal(a, b)
+    assert (cloud.colors is None) == (want.colors is None) == (not paint)
+    if paint:
+        np.testing.assert_array_equal(cloud.colors, want.colors)

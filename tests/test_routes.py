@@ -2,6 +2,7 @@
 them costs, and both sides were measured where a test here draws the line.  No GPU needed."""
 
 import ctypes as C
+import math
 
 import pytest
 
@@ -80,3 +81,23 @@ def test_lattice(lib, prims, seed, blends, n, tapes):
 def test_export(lib, prims, seed, blends, res, tapes):
     grid = sdf._grid(W.export_grid(resolution=res))
     assert _by_tapes(lib, _tree(prims, seed, blends), EXPORT, grid) == tapes
+
+
+# Measured without / with tapes, us a call.
+@pytest.mark.parametrize("prims,seed,blends,step,tapes", [
+    (1, 3, False, 0.03, False),             # 124 / 141
+    (8, 2, False, 0.03, False),             # 213 / 225
+    (8, 2, False, 0.015, True),             # 322 / 243
+    (64, 4, True, 0.04, False),             # 422 / 569
+    (64, 3, False, 0.02, True),             # 338 / 241
+    (128, 3, False, 0.03, False),           # 495 / 604
+    (256, 2, False, 0.02, True),            # 1705 / 1056
+    (512, 4, True, 0.06, False),            # 2299 / 7287
+    (512, 4, True, 0.04, False),            # 2585 / 4712
+    (512, 4, True, 0.02, True),             # 5552 / 2038
+    (512, 6, True, 0.06, False),            # 845 / 3471
+])
+def test_cloud(lib, prims, seed, blends, step, tapes):
+    n = math.ceil(3.2 / step)
+    grid = _lib.Grid(-1.6, -1.6, -1.6, step, n, n, n)
+    assert _by_tapes(lib, _tree(prims, seed, blends), CLOUD, grid) == tapes
