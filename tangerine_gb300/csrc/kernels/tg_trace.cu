@@ -115,8 +115,11 @@ namespace tg
 		// walk, read through a window in shared memory.  Bound by issue.  Calls from and to the
 		// host, a thread a point (one evaluation after the other) against this: gradients of 64
 		// primitives 100 000 188 / 155, 30 000 142 / 84, of 256 primitives 200 000 1177 / 825, 30 000
-		// 455 / 231, of 8 primitives 1000 35 / 31; values of 256 primitives 200 000 376 / 293.
-		constexpr int kQueryThreads = 128;
+		// 455 / 231, of 8 primitives 1000 35 / 31; values of 256 primitives 200 000 376 / 293.  A warp
+		// a CTA: with four, some SMs got a quarter more of the work than others at middling counts
+		// (values of 400 primitives at 120 000 321 us by a thread a point, 356 by CTAs of four, 320 so;
+		// gradients 1041, 830, 743).
+		constexpr int kQueryThreads = 32;
 
 		template<bool Gradient>
 		__global__ void __launch_bounds__(kQueryThreads) PointQueryKernel(DeviceProgram prog, const float* __restrict__ points, int64_t n,
