@@ -930,7 +930,8 @@ namespace tg
 			int bricks = exact ? 0 : RenderBricks(p.View, root.ClipRadius, px, p.Host.VolumeQuads);
 			const int64_t all = (int64_t)bricks * bricks * bricks;
 			BrickTapes tapes{}, above{};
-			if (bricks && !TapesFit(Tapes, all, BrickPartCapacity(all), tapes, spare)) bricks = 0;
+			// All bricks get parts, not only those with surface.
+			if (bricks && !TapesFit(Tapes, all, (size_t)all * 3 / 2 + 32768, tapes, spare)) bricks = 0;
 			if (bricks)
 			{
 				TG_TRY(ReadSmCount());

@@ -422,16 +422,18 @@ namespace tg
 	// (quads a point runs in brackets): 1 primitive (5) 1920 x 1080 168 / 238, 2 (10) 256 / 270, 4 (12)
 	// 200 x 150 137 / 185, 800 x 500 385 / 260, 8 (18) 64 x 48 152 / 193, 128 x 96 231 / 216, 16 (25)
 	// 355 / 280, 32 (61) 64 x 48 356 / 258, 64 (50) 382 / 237, 256 (107) 1757 / 667; the rule's worst,
-	// 16 (44) 128 x 96 159 / 224.
+	// 16 (44) 128 x 96 159 / 224.  Scenes so wide that their cells ask for 64 bricks an axis build
+	// eight times the tapes, of space that is mostly empty: 60 strewn primitives 640 x 360 566 / 815,
+	// 1920 x 1080 1453 / 1024.
 	int RenderBricks(const DeviceProgram& prog, float root_clip, int64_t pixels, double quads)
 	{
-		if (!prog.Lipschitz || !(prog.Form & kFormPrunable) || (double)pixels * (quads - 10.0) < 1.2e5) return 0;
+		if (!prog.Lipschitz || !(prog.Form & kFormPrunable)) return 0;
 		const float span = 2.0f * fabsf(root_clip) * 0.57735f;
 		// The cells' edge: the cube halved until no more than the octree's target.
 		int cells = 1;
 		while (cells < 128 && span / (float)cells > 0.25f) cells *= 2;
 		const int n = cells < 32 ? 32 : cells;
-		return n <= 64 ? n : 0;
+		return n <= 64 && (double)pixels * (quads - 10.0) >= (n > 32 ? 8e6 : 1.2e5) ? n : 0;
 	}
 
 	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes, const BrickTapes& above,

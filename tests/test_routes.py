@@ -4,6 +4,7 @@ them costs, and both sides were measured where a test here draws the line.  No G
 import ctypes as C
 import math
 
+import numpy as np
 import pytest
 
 from tangerine_gb300 import _lib, sdf
@@ -101,3 +102,17 @@ def test_cloud(lib, prims, seed, blends, step, tapes):
     n = math.ceil(3.2 / step)
     grid = _lib.Grid(-1.6, -1.6, -1.6, step, n, n, n)
     assert _by_tapes(lib, _tree(prims, seed, blends), CLOUD, grid) == tapes
+
+
+# Wide scenes build eight times as many tapes: without / with, us an image.
+@pytest.mark.parametrize("width,height,tapes", [(640, 360, False), (1920, 1080, True)])      # 566 / 815, 1453 / 1024
+def test_render_of_wide_scenes(lib, width, height, tapes):
+    rng = np.random.default_rng(4)
+    tree = None
+    for i in range(60):
+        a = rng.uniform(0.5, 1.0)
+        q = rng.normal(size=4)
+        brush = (sdf.sphere(a), sdf.box(a, 0.7 * a, 0.9 * a), sdf.torus(a, 0.3 * a))[i % 3].rotate(*[float(v) for v in q / np.linalg.norm(q)])
+        brush.move(*[float(v) for v in rng.uniform(-6, 6, 3)])
+        tree = brush if tree is None else sdf.union(tree, brush)
+    assert _by_tapes(lib, tree, RENDER, pixels=width * height) == tapes
