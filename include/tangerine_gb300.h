@@ -539,6 +539,8 @@ TANGERINE_API tg_status tg_debug_wait_test(int which, uint64_t limit_ns);
  * allowing; -1 without an octree.  call 0: a culled export of grid by 7^3-cell bricks, 1: tg_eval_grid
  * of it, 2: a point cloud of nx x ny x nz voxels, 3: a render of so many pixels.  Needs no GPU. */
 TANGERINE_API int tg_debug_goes_by_tapes(void* tree, int call, const tg_grid* grid, int64_t pixels);
+/* Test hook: how many parts and events the tapes of the next calls may have (0: no limit). */
+TANGERINE_API void tg_debug_tape_room(uint32_t parts, uint32_t events);
 /* Test hook: the device memory that the library's buffers may hold together (0: no limit); a
  * reservation beyond it fails as cudaMalloc does when the device is full.  release nonzero: the
  * engine gives its buffers back first.  Returns the bytes held (compiled programs left out). */

@@ -183,6 +183,7 @@ SIGNATURES = {
     "tg_batch_cancel": (_i, [_vp, _i]),
     "tg_batch_debug_barrier": (_i, [_vp, C.c_uint64, _i, C.c_uint64]),
     "tg_debug_wait_test": (_i, [_i, C.c_uint64]),
+    "tg_debug_tape_room": (None, [C.c_uint32, C.c_uint32]),
     "tg_debug_goes_by_tapes": (_i, [_vp, _i, C.POINTER(Grid), _i64]),
     "tg_debug_device_limit": (C.c_uint64, [C.c_uint64, _i]),
     "tg_surrogate_save": (_i64, [_vp, _vp, _i64]),

@@ -1531,6 +1531,14 @@ extern "C"
 		return GoesByTapes(p, (CallKind)call, gs, pixels) ? 1 : 0;
 	}
 
+	TANGERINE_API void tg_debug_tape_room(uint32_t parts, uint32_t events)
+	{
+		Engine& eng = Engine::Get();
+		std::lock_guard<std::mutex> lock(eng.Mutex);
+		eng.MostParts = parts ? parts : 0x7FFFFFFFu;
+		eng.MostEvents = events ? events : 0x7FFFFFFFu;
+	}
+
 	TANGERINE_API uint64_t tg_debug_device_limit(uint64_t bytes, int release)
 	{
 		Engine& eng = Engine::Get();

@@ -499,6 +499,8 @@ namespace tg
 		out.Events = buffers.Events.As<uint2>();
 		out.Counters = buffers.Counters.As<uint32_t>();
 		out.Long = out.Counters + kBrickTapeCounters;
+		out.PartCapacity = std::min(out.PartCapacity, MostParts);
+		out.EventCapacity = std::min(out.EventCapacity, MostEvents);
 		return cudaSuccess;
 	}
 

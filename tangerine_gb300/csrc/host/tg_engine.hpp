@@ -203,6 +203,8 @@ namespace tg
 		// Frees what only makes calls faster (tapes, the voxel blocks' scratch), unless a call is
 		// using it.  True when there was any.
 		bool ReleaseSpare();
+		// Test hook (tg_debug_tape_room): parts and events that tapes may take.
+		uint32_t MostParts = 0x7FFFFFFFu, MostEvents = 0x7FFFFFFFu;
 		// Frees every buffer of the engine (test hook: a call then finds what a first one does).
 		void ReleaseBuffers();
 

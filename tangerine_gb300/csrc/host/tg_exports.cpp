@@ -262,7 +262,7 @@ namespace tg
 			TG_TRY(BrickBits.Reserve(VoxelBrickWords(s.SX, s.SY, s.SZ) * 4));
 		}
 		Begin("vox_flags", st);
-		if (byBlocks) TG_TRY(LaunchVoxBlocks(p.View, s, VoxScratch.Ptr, Words.As<uint32_t>(), SmCount, st));
+		if (byBlocks) TG_TRY(LaunchVoxBlocks(p.View, s, VoxScratch.Ptr, MostEvents, Words.As<uint32_t>(), SmCount, st));
 		else TG_TRY(LaunchVoxFlags(p.View, s, BrickBits.As<uint32_t>(), Words.As<uint32_t>(), st));
 		End(st);
 		Begin("list_cells", st);

@@ -978,7 +978,8 @@ namespace tg
 		return cudaGetLastError();
 	}
 
-	cudaError_t LaunchVoxBlocks(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream)
+	cudaError_t LaunchVoxBlocks(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t most_events, uint32_t* words, int sms,
+		cudaStream_t stream)
 	{
 		const int depth = prog.MaxStack > 1 ? prog.MaxStack - 1 : 1;
 		cudaError_t e = cudaMemsetAsync(words, 0, (size_t)((s.Total + 31) / 32) * 4, stream);
@@ -993,6 +994,7 @@ namespace tg
 		const VoxGrid vg = VoxGridOf(s);
 		VoxState st;
 		VoxLayout(s, scratch, st);
+		if (st.EventCap > most_events) st.EventCap = most_events;
 		e = cudaMemsetAsync(st.Counters, 0, kVoxCounters * sizeof(uint32_t), stream);
 		if (e != cudaSuccess) return e;
 		const size_t coarse = 64 * sizeof(float4) + (kVoxCoarseCap + kMaxStack + 2) * sizeof(uint2) + (size_t)depth * 32 * sizeof(float2);

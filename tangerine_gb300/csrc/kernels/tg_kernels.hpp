@@ -314,9 +314,11 @@ namespace tg
 		uint32_t capacity, int iterations, float* points, cudaStream_t stream);
 	// One bit per voxel: |full-tree distance at the centre| <= Radius.
 	cudaError_t LaunchVoxFlags(const DeviceProgram& prog, const VoxSpec& s, uint32_t* brick_bits, uint32_t* words, cudaStream_t stream);
-	// The same by blocks of shortened programs; scratch: VoxBlockBytes (0: not for this tree or lattice).
+	// The same by blocks of shortened programs; scratch: VoxBlockBytes (0: not for this tree or
+	// lattice); most_events: what the blocks' own lists may hold together.
 	size_t VoxBlockBytes(const DeviceProgram& prog, const VoxSpec& s);
-	cudaError_t LaunchVoxBlocks(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t* words, int sms, cudaStream_t stream);
+	cudaError_t LaunchVoxBlocks(const DeviceProgram& prog, const VoxSpec& s, void* scratch, uint32_t most_events, uint32_t* words, int sms,
+		cudaStream_t stream);
 	// The flagged voxels in order, each x, y, z, color; word_base: LaunchExclusiveScan of the words.
 	cudaError_t LaunchVoxList(const VoxSpec& s, const uint32_t* words, const uint32_t* word_base, int color, int4* out, cudaStream_t stream);
 }

@@ -552,3 +552,35 @@ def test_clouds_by_tapes_equal_whole_programs(lib, prims, ops, paint, step, refi
     assert (cloud.colors is None) == (want.colors is None) == (not paint)
     if paint:
         np.testing.assert_array_equal(cloud.colors, want.colors)
+
+
+@pytest.mark.parametrize("kind", CALLS)
+@pytest.mark.parametrize("parts,events", [(1, 1), (100, 0), (3001, 0), (0, 100), (0, 5003)])
+def test_calls_with_little_room_for_tapes(lib, kind, parts, events):
+    """Bricks whose parts and parts whose events found no room go by whole programs."""
+    with sdf.compile(sdf.from_spec(W.random_tree(1, 256))) as prog:
+        want = _call(kind, prog)
+        lib.tg_debug_tape_room(parts, events)
+        try:
+            got = _call(kind, prog)
+        finally:
+            lib.tg_debug_tape_room(0, 0)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_more_long_parts_than_are_listed(lib):
+    """A tree whose few cells all have long programs, and more bricks than the list of long parts
+    holds (16384): the others are built in their turn."""
+    blends = ((W.UNION, 0.3), (W.DIFF, 0.2), (W.INTER, 0.05), (W.BLEND_UNION, 0.25), (W.BLEND_DIFF, 0.1), (W.BLEND_INTER, 0.1))
+    seed = 6
+    while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, 256, ops=blends))):
+        seed += 7919
+    n = 430
+    grid = _lib.Grid(-1.6, -1.6, -1.6, 3.2 / n, n, n, n)
+    with sdf.compile(sdf.from_spec(spec)) as prog:
+        info = prog.info()
+        assert info.octree_cells <= 4 and info.distance_quads > 300 * info.octree_cells
+        lattice = prog.eval_grid(grid)
+        want = _by_whole_programs(lib, 4 * n ** 3 + (1 << 18), lambda: prog.eval_grid(grid))
+    np.testing.assert_array_equal(lattice, want)
