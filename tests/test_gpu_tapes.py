@@ -584,3 +584,23 @@ def test_more_long_parts_than_are_listed(lib):
         lattice = prog.eval_grid(grid)
         want = _by_whole_programs(lib, 4 * n ** 3 + (1 << 18), lambda: prog.eval_grid(grid))
     np.testing.assert_array_equal(lattice, want)
+
+
+def test_queries_at_special_points(lib, port):
+    """Zeros, denormal, huge and infinite coordinates, NaN: the oracle's values by a block, a warp
+    and half a lane a point."""
+    v = np.asarray([0, -0.0, 1e-40, -1e-30, 1e10, -1e30, 3e38, np.inf, -np.inf, np.nan, 0.3, -0.7], np.float32)
+    points = np.stack(np.meshgrid(v, v, v, indexing="ij"), -1).reshape(-1, 3)
+    for prims in (1, 3, 60):
+        seed = 4
+        while not sdf.has_export_octree(sdf.from_spec(spec := W.random_tree(seed, prims, ops=ALL_OPS))):
+            seed += 1
+        handle = port.build(spec)
+        try:
+            values, gradients = port.eval(handle, points), port.gradient(handle, points)
+        finally:
+            port.free(handle)
+        with sdf.compile(sdf.from_spec(spec)) as prog:
+            for n in (100, 1728, 40000):
+                np.testing.assert_array_equal(prog.eval_tree(np.resize(points, (n, 3))), np.resize(values, n))
+                np.testing.assert_array_equal(prog.gradient_tree(np.resize(points, (n, 3))), np.resize(gradients, (n, 3)))
