@@ -472,8 +472,10 @@ TANGERINE_API tg_status tg_last_export_timing(double* compile_s, double* upload_
 
 /* Per-kernel device time of the export pipeline, accumulated while enabled (CUDA events
  * on the launching stream).  Names: "eval_grid", "cell_flags", "scan", "cell_vertices",
- * "faces", "attributes", "face_normals", "eval_points", "classify_bricks", "eval_bricks",
- * "ray_march", "render". */
+ * "faces", "attributes", "face_normals", "eval_points", "classify_bricks", "classify_root",
+ * "classify_field", "refine_bricks", "list_bricks", "brick_tapes", "eval_bricks", "ray_march",
+ * "tree_eval", "tree_gradient", "render", "render_field", "cloud_flags", "list_cells",
+ * "cloud_refine", "vox_flags". */
 TANGERINE_API void tg_profile_enable(int enable);
 TANGERINE_API int tg_profile_read(const char* kernel, double* total_ms, int64_t* launches);
 TANGERINE_API void tg_profile_reset(void);
