@@ -218,6 +218,7 @@ namespace tg
 			p.View.FullBrushes = p.Host.Header.FullBrushes;
 			p.View.FullOps = p.Host.Header.FullOps;
 			p.View.Slack = p.Host.Header.Slack;
+			p.View.Widths = p.Host.Header.Widths;
 		}
 	}
 

@@ -79,7 +79,8 @@ namespace tg
 		int32_t Form;               // kForm* below
 		int32_t FullBrushes;        // brushes and operators of the whole tree, stencils' masks left out
 		int32_t FullOps;
-		float Slack;                // kRoundingSlack, and more for rotations off the unit quaternion
+		float Slack;                // kRoundingSlack, and more for scales above 1 and rotations off the unit quaternion
+		float Widths;               // of all flates and blends together
 	};
 
 	// The float error of two operands at two points, by the size of what goes into them, with

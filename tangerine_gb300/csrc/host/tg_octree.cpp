@@ -859,19 +859,25 @@ namespace tg
 		return 0;
 	}
 
-	// How far the squared norm of any brush's rotation is from 1.
-	static double RotationError(const Node& n)
+	// What the float error of the tree's distances goes with, beside the brushes' own sizes: how far
+	// the squared norm of a rotation is from 1, the largest scale, all flates' and blends' widths.
+	struct RoundingFacts
 	{
-		switch (n.Kind)
-		{
-		case NodeKind::Brush:
+		double Rotation = 0.0, Scale = 1.0, Widths = 0.0;
+	};
+
+	static void AddRounding(const Node& n, RoundingFacts& r)
+	{
+		if (n.Kind == NodeKind::Brush)
 		{
 			const Quat& q = n.Xf.Rotation;
-			return std::fabs((double)q.w * q.w + (double)q.x * q.x + (double)q.y * q.y + (double)q.z * q.z - 1.0);
+			r.Rotation = std::max(r.Rotation, std::fabs((double)q.w * q.w + (double)q.x * q.x + (double)q.y * q.y + (double)q.z * q.z - 1.0));
+			r.Scale = std::max(r.Scale, std::fabs((double)n.Xf.Scalation));
+			return;
 		}
-		case NodeKind::Set: return std::max(RotationError(*n.Lhs), RotationError(*n.Rhs));
-		default: return RotationError(*n.Lhs);
-		}
+		if (n.Kind == NodeKind::Flate || (n.Kind == NodeKind::Set && IsBlendOp(n.Op))) r.Widths += std::fabs((double)n.Threshold);
+		AddRounding(*n.Lhs, r);
+		if (n.Kind == NodeKind::Set) AddRounding(*n.Rhs, r);
 	}
 
 	// Brushes and operators the tree's distance takes (a stencil's mask changes none).
@@ -1184,10 +1190,14 @@ namespace tg
 		out.Header.Lipschitz = HasNonLipschitzBrush(*root) ? 0 : 1;
 		out.Header.Form = FormOf(*root);
 		CountNodes(*root, out.Header.FullBrushes, out.Header.FullOps);
-		// With a rotation of squared norm 1 + e the inverse matrix of a distance record and the
-		// inverse quaternion of the surface record take a point v from the brush's origin up to
-		// 2 e |v| apart; a tape that serves both programs allows for that in both operands.
-		out.Header.Slack = kRoundingSlack + (float)(4.0 * RotationError(*root));
+		// A brush's scale multiplies the rounding of its local coordinates.  With a rotation of squared
+		// norm 1 + e the inverse matrix of a distance record and the inverse quaternion of the surface
+		// record take a point v from the brush's origin up to 2 e |v| apart; a tape that serves both
+		// programs allows for that in both operands.
+		RoundingFacts rounding;
+		AddRounding(*root, rounding);
+		out.Header.Slack = (float)((kRoundingSlack + 4.0 * rounding.Rotation) * rounding.Scale);
+		out.Header.Widths = (float)rounding.Widths;
 		if (maxStack > kMaxStack)
 		{
 			error = "tree needs a deeper evaluation stack than the kernels hold";

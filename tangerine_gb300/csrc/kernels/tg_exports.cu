@@ -537,7 +537,7 @@ namespace tg
 			SurfaceSource src;
 			src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, window);
 			TapeCounts counts;
-			const bool ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, LoadPairUnits(), spill, 32,
+			const bool ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, prog.Widths, LoadPairUnits(), spill, 32,
 				TapeLists{ value, nullptr, start, kVoxCoarseCap }, counts);
 			if (ok)
 				for (int i = lane; i < counts.Value; i += 32) st.Events[(int64_t)b * kVoxCoarseCap + i] = value[i];
@@ -595,13 +595,13 @@ namespace tg
 				{
 					SurfaceSource src;
 					src.In.Open(prog.Code + prog.FullSurfaceCode, prog.CodeQuads - prog.FullSurfaceCode, sc.Window);
-					ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
+					ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, prog.Widths, units, spill, 32, lists, counts);
 				}
 				else
 				{
 					SurfaceEventSource src;
 					src.Open(prog.Code + prog.FullSurfaceCode, st.Events + first, (int)given, sc.Window, sc.Heads);
-					ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, units, spill, 32, lists, counts);
+					ok = BuildTape<false, true>(src, l.X, l.Y, l.Z, VoxReach(l, rootClip), kRoundingSlack, prog.Widths, units, spill, 32, lists, counts);
 				}
 				// The box goes by its own tape, where there is room for it.
 				uint2 tape = make_uint2(first, given);

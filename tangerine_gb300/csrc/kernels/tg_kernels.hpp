@@ -21,7 +21,8 @@ namespace tg
 		int Form;               // kForm* (tg_layout.hpp): what may be left out of its programs
 		int CodeQuads;          // quads of Code; the whole tree's surface program is the last in it
 		int FullBrushes, FullOps;   // brushes and operators of that program (stencils' masks left out)
-		float Slack;            // rounding of two operands by the size of what goes into them (tg_layout.hpp)
+		float Slack;            // rounding of two operands by the size of what goes into them (tg_layout.hpp),
+		float Widths;           // to which those of the flates and blends belong
 	};
 
 	// Pinhole camera: pixel (x, y) looks along forward + right*u + up*v with

@@ -371,7 +371,7 @@ namespace tg
 						const BrickPart& p = above.Parts[around];
 						DistanceEventSource src;
 						src.Open(code + base, above.Events + p.Material, (int)(p.Counts >> 16), ts.Window, ts.Heads);
-						ok = BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach, prog.Slack, units,
+						ok = BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach, prog.Slack, prog.Widths, units,
 							spill, 32, lists, counts);
 					}
 					else
@@ -379,7 +379,7 @@ namespace tg
 						DistanceSource src;
 						src.In.Open(code + base, quads, ts.Window);
 						ok = quads <= 0xFFF0 && BuildTape<true>(src, make_float2(cx, cx), make_float2(cy, cy), make_float2(cz, cz + 2.0f * wz), reach,
-							prog.Slack, units, spill, 32, lists, counts);
+							prog.Slack, prog.Widths, units, spill, 32, lists, counts);
 					}
 				}
 				if (!ok) continue;

@@ -655,8 +655,7 @@ namespace tg
 	};
 
 	// A distance brush's distance at two points, from its record's quads, and the size its float
-	// error goes with: that of its local coordinates and parameters, times the brush's scale,
-	// which multiplies their rounding too.
+	// error goes with (its scale apart: DeviceProgram::Slack).
 	template<typename Load>
 	__device__ __forceinline__ float2 DistanceBrush(Load load, uint32_t head, float2 px, float2 py, float2 pz, const PairUnits& u, float2& size)
 	{
@@ -665,9 +664,8 @@ namespace tg
 		float4 h;
 		BrushStep<1, false>(load, 0, head, x, y, z, u, qx, qy, qz, h, d);
 		const float sizes = fabsf(h.y) + fabsf(h.z) + fabsf(h.w);
-		const float scale = (head & RecScale) ? fmaxf(1.0f, fabsf(load(DistanceRecordQuads(head) - 1).x)) : 1.0f;
-		size = make_float2(scale * (fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes) + fabsf(d[0].x),
-			scale * (fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes) + fabsf(d[0].y));
+		size = make_float2(fabsf(qx[0].x) + fabsf(qy[0].x) + fabsf(qz[0].x) + sizes + fabsf(d[0].x),
+			fabsf(qx[0].y) + fabsf(qy[0].y) + fabsf(qz[0].y) + sizes + fabsf(d[0].y));
 		return d[0];
 	}
 
@@ -945,15 +943,17 @@ namespace tg
 	// rounding (TapeReach); the part that grows with the operands' own coordinates (brushes
 	// far from the box) is added here: each brush's float error is at most a few roundings of
 	// its local coordinates and sizes, that of a flate or a blend a few of what goes in and of
-	// its own width (`slack` times the largest of them).  Returns false when a list outgrows its
-	// room; with Finish the rest of the program still runs then, for the distances.
+	// its own width: `slack` times the largest of the brushes' sizes and of all widths together.
+	// (Scales, rotations and widths are the whole tree's, from the host: looked at record by record
+	// here they took 2 to 4 % of the building.)  Returns false when a list outgrows its room; with
+	// Finish the rest of the program still runs then, for the distances.
 	template<bool Materials, bool Finish = false, typename Source>
-	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, float slack, const PairUnits& u,
+	__device__ __forceinline__ bool BuildTape(Source& src, float2 px, float2 py, float2 pz, float reach, float slack, float widths, const PairUnits& u,
 		float2* spill, int stride, const TapeLists& ts, TapeCounts& out)
 	{
 		const int lane = (int)(threadIdx.x & 31);
 		float2 acc = make_float2(0.0f, 0.0f), left = acc;
-		float2 size = make_float2(0.0f, 0.0f);
+		float2 size = make_float2(widths, widths);
 		int depth = 0;
 		int nv = 0, nm = 0;
 		bool same = true, full = false;
@@ -1019,12 +1019,7 @@ namespace tg
 				const uint2 ev = src.Event(head);
 				ts.Value[nv++] = ev;
 				if (Materials) ts.Material[nm++] = ev;
-				if (op == OpFlate)
-				{
-					const float k = src.Operand();
-					size = make_float2(fmaxf(size.x, fabsf(acc.x) + fabsf(k)), fmaxf(size.y, fabsf(acc.y) + fabsf(k)));
-					acc = Sub2(acc, Pair(k), u);
-				}
+				if (op == OpFlate) acc = Sub2(acc, Pair(src.Operand()), u);
 				else acc = op == OpTapeNegate ? make_float2(-acc.x, -acc.y) : make_float2(acc.x + 0.0f, acc.y + 0.0f);
 				src.Advance(head);
 				continue;
@@ -1033,7 +1028,6 @@ namespace tg
 			const bool blend = op >= OpBlendUnion;
 			const bool diff = op == OpDiff || op == OpBlendDiff;
 			const bool unions = op == OpUnion || op == OpBlendUnion;
-			if (blend) size = make_float2(fmaxf(size.x, fabsf(k)), fmaxf(size.y, fabsf(k)));
 			// s > 0 where the left operand wins: by more than the reach everywhere, it always does.
 			const float2 s = unions ? make_float2(acc.x - left.x, acc.y - left.y)
 				: diff ? make_float2(left.x + acc.x, left.y + acc.y) : make_float2(left.x - acc.x, left.y - acc.y);
