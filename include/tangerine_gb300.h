@@ -653,7 +653,8 @@ enum
 	   into shared memory (one bulk copy) and reads its records there (same results). */
 	TG_MESH_STAGED = 1u << 21,
 	/* Brick evaluation of the default 7^3-cell bricks through shortened programs whatever the
-	   grid's size (by default only where that is the faster way; same results). */
+	   grid's size (by default only where that is the faster way; same results; lattice points per
+	   thread then have no effect). */
 	TG_MESH_TAPES = 1u << 22,
 };
 TANGERINE_API tg_status tg_export_mesh_surrogate(tg_program* program, tg_surrogate* s, const tg_grid* grid, uint32_t flags,
