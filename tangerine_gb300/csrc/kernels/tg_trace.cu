@@ -418,7 +418,7 @@ namespace tg
 	// program by one warp, and building them all 120 us at least; without, a render of any size
 	// lasts as long as the ray that grazes the surface longest, some hundred whole programs one
 	// after the other.  So what counts are the pixels and what a program has beyond two brushes
-	// (ten quads), which a tape mostly leaves.  Measured on a GB300, none against tapes, us an image
+	// (ten quads), which a tape mostly leaves; fitted to 240 images of 40 trees.  Measured on a GB300, none against tapes, us an image
 	// (quads a point runs in brackets): 1 primitive (5) 1920 x 1080 168 / 238, 2 (10) 256 / 270, 4 (12)
 	// 200 x 150 137 / 185, 800 x 500 385 / 260, 8 (18) 64 x 48 152 / 193, 128 x 96 231 / 216, 16 (25)
 	// 355 / 280, 32 (61) 64 x 48 356 / 258, 64 (50) 382 / 237, 256 (107) 1757 / 667; the rule's worst,
@@ -433,7 +433,8 @@ namespace tg
 		int cells = 1;
 		while (cells < 128 && span / (float)cells > 0.25f) cells *= 2;
 		const int n = cells < 32 ? 32 : cells;
-		return n <= 64 && (double)pixels * (quads - 10.0) >= (n > 32 ? 8e6 : 1.2e5) ? n : 0;
+		const double gain = quads > 10.0 ? (double)pixels * std::sqrt(quads - 10.0) : 0.0;
+		return n <= 64 && gain >= (n > 32 ? 2e6 : 1.8e4) ? n : 0;
 	}
 
 	cudaError_t LaunchRenderTapes(const DeviceProgram& prog, const float* pivot, float root_clip, int bricks, const BrickTapes& tapes, const BrickTapes& above,

@@ -34,6 +34,8 @@ def _by_tapes(lib, tree, call, grid=None, pixels=0):
     (1, 2, False, 400, 300, False),         # 211 / 279
     (2, 3, False, 1920, 1080, False),       # 256 / 270
     (4, 4, True, 128, 96, False),           # 122 / 177
+    (8, 6, True, 64, 48, False),            # 152 / 193
+    (8, 4, True, 128, 96, True),            # 237 / 221
     (4, 3, False, 800, 500, True),          # 385 / 260
     (16, 3, False, 64, 48, False),          # 191 / 227
     (8, 2, False, 200, 150, True),          # 627 / 441
@@ -62,6 +64,15 @@ def test_render(lib, prims, seed, blends, width, height, tapes):
 def test_lattice(lib, prims, seed, blends, n, tapes):
     grid = _lib.Grid(-1.6, -1.6, -1.6, 3.2 / (n - 1), n, n, n)
     assert _by_tapes(lib, _tree(prims, seed, blends), LATTICE, grid) == tapes
+
+
+def test_lattice_of_long_programs_and_few_points(lib):
+    """125 primitives of some 300 quads: 250 us by whole programs, 482 by tapes."""
+    spec = W.random_tree(11 * 1000003 + 125, 125)
+    assert sdf.has_export_octree(sdf.from_spec(spec))
+    n = (34, 318, 59)
+    step = [3.2 / (k - 1) for k in n]
+    assert not _by_tapes(lib, sdf.from_spec(spec), LATTICE, _lib.Grid(-1.6, -1.6, -1.6, step[0], *n, step[1], step[2]))
 
 
 # Measured by whole programs / by tapes, us an export to the device.
