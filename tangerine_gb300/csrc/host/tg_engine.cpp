@@ -219,6 +219,7 @@ namespace tg
 			p.View.FullOps = p.Host.Header.FullOps;
 			p.View.Slack = p.Host.Header.Slack;
 			p.View.Widths = p.Host.Header.Widths;
+			p.View.Deflate = p.Host.Header.Deflate;
 		}
 	}
 
@@ -473,6 +474,7 @@ namespace tg
 		v.Code = reinterpret_cast<const float4*>(RootScratch.As<uint8_t>() + codeOff);
 		v.MaxStack = root.Node.StackSize;
 		v.Lipschitz = root.Node.ClipRadius >= 0.0f ? 1 : 0;
+		v.Deflate = root.Deflate;
 		Begin("classify_root", s);
 		TG_TRY(LaunchClassifyBricks(v, g, B, BrickBits.As<uint32_t>(), s));
 		End(s);

@@ -81,6 +81,7 @@ namespace tg
 		int32_t FullOps;
 		float Slack;                // kRoundingSlack, and more for scales above 1 and rotations off the unit quaternion
 		float Widths;               // of all flates and blends together
+		float Deflate;              // how far the surface may lie outside the root cube
 	};
 
 	// The float error of two operands at two points, by the size of what goes into them, with

@@ -88,6 +88,7 @@ namespace tg
 	{
 		OctNode Node{};
 		std::vector<float> Code;
+		float Deflate = 0.0f;               // ProgramHeader's
 	};
 	using RootHook = std::function<void(const RootProgram&)>;
 

@@ -41,8 +41,9 @@ namespace tg
 	{
 		const float rootClip = __ldg(&prog.Nodes[0].ClipRadius);
 		// Outside the root cube every brush, and so every clipped program, is positive
-		// (the cube holds the tree's bounds): a ball missing the cube has no surface.
-		const float half = fabsf(rootClip) * 0.57736f;           // span / 2 = radius / sqrt(3), rounded up
+		// (the cube holds the tree's bounds, of negative flates too little by Deflate): a ball
+		// missing the cube has no surface.
+		const float half = fabsf(rootClip) * 0.57736f + prog.Deflate;    // span / 2 = radius / sqrt(3), rounded up
 		const float ox = fmaxf(fabsf(b.cx - __ldg(&prog.Nodes[0].Pivot[0])) - half, 0.0f);
 		const float oy = fmaxf(fabsf(b.cy - __ldg(&prog.Nodes[0].Pivot[1])) - half, 0.0f);
 		const float oz = fmaxf(fabsf(b.cz - __ldg(&prog.Nodes[0].Pivot[2])) - half, 0.0f);

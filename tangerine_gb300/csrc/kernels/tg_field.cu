@@ -738,7 +738,7 @@ namespace tg
 			Pipe p;
 			bool failed = !Setup(&S.TmemSlot, S.Bars, S.Image, image, kInferColumns, p);
 			const float rootClip = fabsf(__ldg(&prog.Nodes[0].ClipRadius));
-			const float half = rootClip * 0.57736f;
+			const float half = rootClip * 0.57736f + prog.Deflate;
 			const float rx = __ldg(&prog.Nodes[0].Pivot[0]), ry = __ldg(&prog.Nodes[0].Pivot[1]), rz = __ldg(&prog.Nodes[0].Pivot[2]);
 			for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
 			{

@@ -23,6 +23,7 @@ namespace tg
 		int FullBrushes, FullOps;   // brushes and operators of that program (stencils' masks left out)
 		float Slack;            // rounding of two operands by the size of what goes into them (tg_layout.hpp),
 		float Widths;           // to which those of the flates and blends belong
+		float Deflate;          // how far the surface may lie outside the root cube
 	};
 
 	// Pinhole camera: pixel (x, y) looks along forward + right*u + up*v with

@@ -604,3 +604,29 @@ def test_queries_at_special_points(lib, port):
             for n in (100, 1728, 40000):
                 np.testing.assert_array_equal(prog.eval_tree(np.resize(points, (n, 3))), np.resize(values, n))
                 np.testing.assert_array_equal(prog.gradient_tree(np.resize(points, (n, 3))), np.resize(gradients, (n, 3)))
+
+
+def test_culled_exports_of_deflated_trees_equal_dense(lib):
+    """The reference's bounds of a flate by a negative radius are too small by it: the surface leaves
+    the octree's cube, by way of the compiled program, the root's alone (export_tree) and a batch."""
+    def trees():
+        yield sdf.flate(sdf.union(sdf.sphere(0.5), sdf.box(0.4, 0.3, 0.6).move(0.2, 0.1, 0.0)), -0.08)
+        yield sdf.union(sdf.flate(sdf.torus(0.5, 0.2).rotate(0.6, 0.0, 0.0, 0.8), -0.03).scale(1.3), sdf.sphere(0.2).move(0.1, 0.0, 0.0))
+        yield sdf.flate(sdf.flate(sdf.blend_union(0.1, sdf.cylinder(0.4, 0.5), sdf.sphere(0.3).move(0.3, 0.2, 0.1)), 0.02), -0.06).paint(0.2, 0.4, 0.6)
+    lo, hi, step = (-1.0, -1.0, -1.0), (1.0, 1.0, 1.0), 0.011
+    programs = [sdf.compile(t) for t in trees()]
+    grid = sdf.export_grid(lo, hi, step)
+    for tree, prog in zip(trees(), programs):
+        dense = prog.export_mesh(grid, dense=True)
+        info = prog.info()
+        assert (dense.vertices.max(0) > np.asarray(info.bounds_max[:])).any()
+        for brick in (3, 7, 16):
+            _same(dense, prog.export_mesh(grid, brick=brick))
+        _same(dense, prog.export_mesh(grid, tapes=True))
+        _same(dense, sdf.export_tree(tree, lo, hi, step))
+    with sdf.Batch(programs, [grid] * len(programs)) as batch:
+        batch.run()
+        for i, prog in enumerate(programs):
+            _same(prog.export_mesh(grid, dense=True), batch.mesh(i))
+    for prog in programs:
+        prog.close()
