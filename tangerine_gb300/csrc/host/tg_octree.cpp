@@ -861,12 +861,9 @@ namespace tg
 
 	// What the float error of the tree's distances goes with, beside the brushes' own sizes: how far
 	// the squared norm of a rotation is from 1, the largest scale, all flates' and blends' widths.
-	// And how far the surface may lie outside the tree's bounds: those of a flate by r are the
-	// operand's grown by 2 r (sdf_evaluator.cpp:1082-1096), too small by |r| where r is negative.
 	struct RoundingFacts
 	{
 		double Rotation = 0.0, Scale = 1.0, Widths = 0.0;
-		double Deflate = 0.0;       // negative flates' together
 	};
 
 	static void AddRounding(const Node& n, RoundingFacts& r)
@@ -878,10 +875,23 @@ namespace tg
 			r.Scale = std::max(r.Scale, std::fabs((double)n.Xf.Scalation));
 			return;
 		}
-		if (n.Kind == NodeKind::Flate && n.Threshold < 0.0f) r.Deflate -= (double)n.Threshold;
 		if (n.Kind == NodeKind::Flate || (n.Kind == NodeKind::Set && IsBlendOp(n.Op))) r.Widths += std::fabs((double)n.Threshold);
 		AddRounding(*n.Lhs, r);
 		if (n.Kind == NodeKind::Set) AddRounding(*n.Rhs, r);
+	}
+
+	// How far the surface may lie outside the tree's bounds: those of a flate by r are the operand's
+	// grown by 2 r (sdf_evaluator.cpp:1082-1096), too small by |r| where r is negative.
+	static float Deflation(const Node& n)
+	{
+		switch (n.Kind)
+		{
+		case NodeKind::Brush: return 0.0f;
+		case NodeKind::Set: return std::max(Deflation(*n.Lhs), Deflation(*n.Rhs));
+		case NodeKind::Flate: return Deflation(*n.Lhs) + std::max(0.0f, -n.Threshold);
+		case NodeKind::Stencil: return Deflation(*n.Lhs);
+		}
+		return 0.0f;
 	}
 
 	// Brushes and operators the tree's distance takes (a stencil's mask changes none).
@@ -1000,8 +1010,7 @@ namespace tg
 			int q, pk;
 			shared.SurfaceSize(*root, q, pk);
 		}
-		RoundingFacts rounding;
-		AddRounding(*root, rounding);
+		const float deflation = Deflation(*root);
 		// The root cell's program, emitted as the programs below emit node 0's.
 		Octree::RootSeen rootSeen;
 		if (on_root && *on_root && kind == OctreeKind::Export)
@@ -1009,7 +1018,7 @@ namespace tg
 			rootSeen = [&](const Vec3& pivot, float radius, const NodeRef& evaluator)
 			{
 				RootProgram rp;
-				rp.Deflate = (float)rounding.Deflate;
+				rp.Deflate = deflation;
 				Emitter em(rp.Code, ds->Materials, &shared);
 				const int depth = em.Distance(*evaluator);
 				em.Quad(OpStop, 0.0f, 0.0f, 0.0f);
@@ -1201,9 +1210,11 @@ namespace tg
 		// norm 1 + e the inverse matrix of a distance record and the inverse quaternion of the surface
 		// record take a point v from the brush's origin up to 2 e |v| apart; a tape that serves both
 		// programs allows for that in both operands.
+		RoundingFacts rounding;
+		AddRounding(*root, rounding);
 		out.Header.Slack = (float)((kRoundingSlack + 4.0 * rounding.Rotation) * rounding.Scale);
 		out.Header.Widths = (float)rounding.Widths;
-		out.Header.Deflate = (float)rounding.Deflate;
+		out.Header.Deflate = deflation;
 		if (maxStack > kMaxStack)
 		{
 			error = "tree needs a deeper evaluation stack than the kernels hold";

@@ -36,7 +36,9 @@ namespace tg
 	// The part of the exact test that needs no program: the root cube and dropped-octant
 	// tests, then the deepest cell on the centre's descent path whose clip sphere holds
 	// the ball (with no cell at or below it that is not 1-Lipschitz).  Returns that cell,
-	// kBoxEmpty or kBoxUndecided.
+	// kBoxEmpty or kBoxUndecided.  Below a flate by a negative radius -t the reference clips with
+	// t less (sdf_evaluator.cpp:1098-1110): an intersection's operand above -2 t in the sphere
+	// less t may be gone, so the program has the tree's sign in the sphere less 2 t.
 	__device__ __forceinline__ int BoxHolder(const DeviceProgram& prog, const BoxBall& b)
 	{
 		const float rootClip = __ldg(&prog.Nodes[0].ClipRadius);
@@ -62,7 +64,7 @@ namespace tg
 			else
 			{
 				const float dx = b.cx - px, dy = b.cy - py, dz = b.cz - pz;
-				if (sqrtf(dx * dx + dy * dy + dz * dz) + b.r + b.margin <= clip) holder = at;
+				if (sqrtf(dx * dx + dy * dy + dz * dz) + b.r + b.margin + 2.0f * prog.Deflate <= clip) holder = at;
 			}
 			if (flags & kNodeTerminus) break;
 			const int octant = (b.cx > px ? 1 : 0) | (b.cy > py ? 2 : 0) | (b.cz > pz ? 4 : 0);
@@ -197,7 +199,7 @@ namespace tg
 				{
 					const float4 n = __ldg(reinterpret_cast<const float4*>(prog.Nodes + at));
 					const float dx = b.cx - n.x, dy = b.cy - n.y, dz = b.cz - n.z;
-					if (!(sqrtf(dx * dx + dy * dy + dz * dz) + b.r + b.margin <= __ldg(&prog.Nodes[at].ClipRadius))) break;
+					if (!(sqrtf(dx * dx + dy * dy + dz * dz) + b.r + b.margin + 2.0f * prog.Deflate <= __ldg(&prog.Nodes[at].ClipRadius))) break;
 					common = at;
 					if (__float_as_int(n.w) & kNodeTerminus) break;
 					at = __ldg(&prog.Nodes[at].Child[(b.cx > n.x ? 1 : 0) | (b.cy > n.y ? 2 : 0) | (b.cz > n.z ? 4 : 0)]);

@@ -630,3 +630,39 @@ def test_culled_exports_of_deflated_trees_equal_dense(lib):
             _same(prog.export_mesh(grid, dense=True), batch.mesh(i))
     for prog in programs:
         prog.close()
+
+
+def _deflated(seed, prims=8):
+    """Few brushes with flates by negative radii at any depth."""
+    rng = np.random.default_rng(seed)
+    def build(n):
+        if n == 1:
+            a, b, c = (float(v) for v in rng.uniform(0.2, 0.6, 3))
+            t = (sdf.sphere(a), sdf.box(a, b, c), sdf.cylinder(a, b))[int(rng.integers(3))].move(*[float(v) for v in rng.uniform(-0.8, 0.8, 3)])
+        else:
+            m = int(rng.integers(1, n))
+            l, r = build(m), build(n - m)
+            x = rng.uniform()
+            t = sdf.union(l, r) if x < 0.5 else sdf.diff(l, r) if x < 0.7 else sdf.inter(l, r) if x < 0.8 else sdf.blend_union(0.1, l, r)
+        return sdf.flate(t, float(rng.uniform(-0.1, -0.02))) if rng.uniform() < 0.3 else t
+    return build(prims)
+
+
+@pytest.mark.parametrize("seed", [20, 74, 121, 159, 220, 351])
+def test_culled_exports_below_negative_flates_equal_dense(lib, seed):
+    """Below a negative flate the octree's clips hold in less than their sphere: cells that hold a
+    brick's ball by less than that decide nothing about it.  All cells where the tree's own sign
+    changes are kept, whatever the bricks (the clip's errors put others into the dense mesh)."""
+    with sdf.compile(_deflated(seed)) as prog:
+        grid = sdf.export_grid((-1.5, -1.5, -1.5), (1.5, 1.5, 1.5), 0.02)
+        dense = prog.export_mesh(grid, dense=True)
+        _same(dense, prog.export_mesh(grid))
+        _same(dense, prog.export_mesh(grid, tapes=True))
+        c = dense.cubes.astype(np.int64)
+        at = np.stack([c % (grid.nx - 1), c // (grid.nx - 1) % (grid.ny - 1), c // ((grid.nx - 1) * (grid.ny - 1))], 1)
+        corners = at[:, None] + np.asarray(list(np.ndindex(2, 2, 2)))
+        points = (np.float32([grid.x0, grid.y0, grid.z0]) + corners.astype(np.float32) * np.float32(grid.step)).reshape(-1, 3)
+        inside = (prog.eval_tree(points) < 0).reshape(-1, 8)
+        surface = dense.cubes[inside.any(1) & ~inside.all(1)]
+        for brick in (2, 4, 15, 32):
+            assert np.isin(surface, prog.export_mesh(grid, brick=brick).cubes).all()
