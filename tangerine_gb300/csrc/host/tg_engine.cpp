@@ -369,7 +369,7 @@ namespace tg
 	}
 
 	// Whether a whole lattice goes by tapes, in bricks of 16^3 points (a quarter full at least).
-	// Up to half a million points whole programs are one wave of warps, as long as one walk of the
+	// Up to some half a million points whole programs are one wave of warps, as long as one walk of the
 	// longest; bricks are then coarse and their tapes long (125 primitives, 300 quads, 34 x 318 x 59
 	// points 250 / 482).
 	// By whole programs it takes about 0.7 to 0.9 us per million quads that its points run
@@ -385,7 +385,7 @@ namespace tg
 		if (!p.View.Lipschitz || !(p.View.Form & kFormPrunable)) return false;
 		const double points = (double)g.NX * g.NY * g.NZ;
 		const auto bricks = [](int n) { return (double)((n + 15) / 16); };
-		return points >= 1e6 && points * (p.Host.VolumeQuads - 6.0) >= 1e6 * (120.0 + 0.6 * p.Host.Header.FullBrushes) &&
+		return points >= 7e5 && points * (p.Host.VolumeQuads - 6.0) >= 1e6 * (120.0 + 0.6 * p.Host.Header.FullBrushes) &&
 			points >= 1024.0 * bricks(g.NX) * bricks(g.NY) * bricks(g.NZ);
 	}
 
